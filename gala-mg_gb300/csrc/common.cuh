@@ -147,6 +147,15 @@ __device__ __forceinline__ void atomic_add_w(long long *p, long long v)
     atomicAdd((unsigned long long *)p, (unsigned long long)v);  // two's complement: also subtracts
 }
 
+// int64 as FP32 within 2^-23 (the 64-bit conversion instructions run at the
+// FP64 rate; the halves' 32-bit conversions do not).
+__device__ __forceinline__ float f32_of(long long x)
+{
+    const unsigned long long u = x < 0 ? 0ull - (unsigned long long)x : (unsigned long long)x;
+    const float f = __fmaf_rn((float)(unsigned)(u >> 32), 4294967296.f, (float)(unsigned)u);
+    return x < 0 ? -f : f;
+}
+
 // ---------------------------------------------------------------------------
 // FP64 gain of a candidate community, same operation order as the reference
 // (kernel_functions.cu:136, :171, :202, :362):
@@ -183,7 +192,10 @@ __device__ __forceinline__ bool prune_bound(WT in_w, WT self_w, WT ki, WT min_to
 // The same bound decided in exact integers: P = ip*m2 + (minTot - (Tot_c - K))*K
 // has the sign of the FP64 expression whenever P != 0 and K*m2 < 2^49 (the
 // FP64 error is below K*2^-50, non-zero P/m2 is at least 1/m2 away from 0);
-// otherwise the FP64 expression decides, as in the reference.
+// otherwise the FP64 expression decides, as in the reference.  For 64-bit
+// fixed-point weights the sign comes from FP32 when it is beyond doubt: every
+// operand is an exact integer rounded to FP32 (2^-23), four roundings follow,
+// and the FP64 expression errs by a few 2^-53 of the same two terms.
 template <typename WT>
 __device__ __forceinline__ bool prune_bound_fast(WT in_w, WT self_w, WT ki, WT min_tot, WT tot_c, double constant,
                                                  long long m2)
@@ -194,6 +206,11 @@ __device__ __forceinline__ bool prune_bound_fast(WT in_w, WT self_w, WT ki, WT m
             const long long p = (long long)ip * m2 + (long long)(min_tot - (tot_c - ki)) * (long long)ki;
             if (p != 0) return p > 0;
         }
+    } else {
+        const float ip = f32_of(2 * (in_w - self_w) - (ki - self_w));
+        const float d = f32_of(min_tot - (tot_c - ki)) * (float)constant * f32_of(ki);
+        const float e = (fabsf(ip) + fabsf(d)) * 0x1p-20f;
+        if (fabsf(ip + d) > e) return ip + d > 0.f;
     }
     return prune_bound(in_w, self_w, ki, min_tot, tot_c, constant);
 }
