@@ -156,6 +156,26 @@ __device__ __forceinline__ float f32_of(long long x)
     return x < 0 ? -f : f;
 }
 
+// The same add to a shared-memory table.  Shared memory has native 32-bit adds
+// only (a 64-bit add is a compare-and-swap loop, which queues on the slot of a
+// vertex's own community): two 32-bit adds instead, the carry taken from the
+// low word's old value, so the sum does not depend on the order.  Read the
+// slot only after a barrier.  Float-weight LFR graph of 500k vertices, kernel
+// times of a run: 33-8192-entry decide tables 9.9 -> 5.7 ms, long-row chunk
+// combine of the contraction 1.8 -> 0.17 ms.
+__device__ __forceinline__ void atomic_add_sm(int *p, int v) { atomicAdd(p, v); }
+__device__ __forceinline__ void atomic_add_sm(long long *p, long long v)
+{
+    unsigned *q = (unsigned *)p;
+    const unsigned lo = (unsigned)(unsigned long long)v;
+    unsigned hi = (unsigned)((unsigned long long)v >> 32);
+    if (lo) {
+        const unsigned old = atomicAdd(q, lo);
+        hi += old + lo < old;
+    }
+    if (hi) atomicAdd(q + 1, hi);
+}
+
 // ---------------------------------------------------------------------------
 // FP64 gain of a candidate community, same operation order as the reference
 // (kernel_functions.cu:136, :171, :202, :362):

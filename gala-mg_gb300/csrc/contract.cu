@@ -468,8 +468,8 @@ __device__ __forceinline__ int agg_insert(const AggArgs<WT> &a, long long st, in
 
 // Add (key, w) to a table (dense when keys is null); returns 1 when this call
 // created the key, 0 when it existed, -1 when the probe ran out.  `slot`
-// receives the slot (hash tables).
-template <typename WT>
+// receives the slot (hash tables).  SM: the table is in shared memory.
+template <bool SM, typename WT>
 __device__ __forceinline__ int table_add(int *keys, WT *vals, int T, int lg, int key, WT w, int &slot)
 {
     if (!keys) {
@@ -488,7 +488,10 @@ __device__ __forceinline__ int table_add(int *keys, WT *vals, int T, int lg, int
             }
         }
         if (k == key) {
-            atomic_add_w(&vals[h], w);
+            if constexpr (SM)
+                atomic_add_sm(&vals[h], w);
+            else
+                atomic_add_w(&vals[h], w);
             slot = (int)h;
             return created;
         }
@@ -520,7 +523,7 @@ __device__ __forceinline__ void agg_insert_list(const AggArgs<WT> &a, long long 
         // match first, where repeated keys would queue on one address
         int created = 0, slot = -1;
         if (valid) {
-            created = table_add(keys, vals, T, lg, key, wt, slot);
+            created = table_add<true>(keys, vals, T, lg, key, wt, slot);
             if (created < 0) {
                 atomicOr(&a.st->err, kErrHashOverflow);
                 created = 0;
@@ -570,7 +573,7 @@ __global__ void __launch_bounds__(256) k_agg_warp_list(AggArgs<WT> a, const int3
             const int j = b0 + lane;
             int created = 0, slot = -1;
             if (j < E) {
-                created = table_add(keys, vals, T, LG, a.skey[st + j], a.w_at(st + j), slot);
+                created = table_add<true>(keys, vals, T, LG, a.skey[st + j], a.w_at(st + j), slot);
                 if (created < 0) {
                     atomicOr(&a.st->err, kErrHashOverflow);
                     created = 0;
@@ -843,7 +846,7 @@ __global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b,
                 int k = *(volatile int *)&skeys[h];  // a repeated key skips the claim
                 if (k == -1) k = atomicCAS(&skeys[h], -1, key);
                 if (k == -1 || k == key) {
-                    atomic_add_w(&svals[h], wt);
+                    atomic_add_sm(&svals[h], wt);
                     if (k == -1) socc[atomicAdd(&s_n, 1)] = (unsigned short)h;
                     break;
                 }
@@ -865,7 +868,7 @@ __global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b,
             if (q < n) {
                 const int h = socc[q];
                 int slot;
-                const int r = table_add(keys, vals, (int)T, lg, skeys[h], svals[h], slot);
+                const int r = table_add<false>(keys, vals, (int)T, lg, skeys[h], svals[h], slot);
                 if (r < 0) atomicOr(&a.st->err, kErrHashOverflow);
                 if (r == 1) {
                     mask |= 1u << it;
@@ -1172,7 +1175,7 @@ __global__ void __launch_bounds__(kRadCombineThreads, 2) k_rad_combine(AggArgs<W
                 int k = *(volatile int *)&skeys[h];  // a repeated key skips the claim
                 if (k == -1) k = atomicCAS(&skeys[h], -1, key);
                 if (k == -1 || k == key) {
-                    atomic_add_w(&svals[h], wt);
+                    atomic_add_sm(&svals[h], wt);
                     if (k == -1) {
                         socc[atomicAdd(&s_n, 1)] = (unsigned short)h;
                         const int bk = key >> kRadLg;
@@ -1505,14 +1508,14 @@ __global__ void __launch_bounds__(512) k_rad_agg(AggArgs<WT> a, BigArgs b, int32
                     if (dense) {
                         const unsigned s = (unsigned)(key[u] - kbase);
                         if (s < (unsigned)kRadW) {
-                            atomic_add_w(&vals[s], v[u]);
+                            atomic_add_sm(&vals[s], v[u]);
                             if (v[u] <= 0) atomicOr(&bits[s >> 5], 1u << (s & 31));
                         } else {
                             atomicOr(&st->err, kErrBadIndex);
                         }
                     } else {
                         int slot;
-                        const int r = table_add(keys, vals, T, lg, key[u], v[u], slot);
+                        const int r = table_add<true>(keys, vals, T, lg, key[u], v[u], slot);
                         if (r < 0) atomicOr(&st->err, kErrHashOverflow);
                         else if (r == 1) {
                             const int o = atomicAdd(&s_n, 1);

@@ -958,7 +958,7 @@ __device__ __forceinline__ int hash_add_slot(int *keys, VT *vals, int T, int log
         const int k = atomicCAS(&keys[h], -1, key);
         if (k == -1 || k == key) {
             created = k == -1;
-            atomic_add_w(&vals[h], w);
+            atomic_add_sm(&vals[h], w);
             return (int)h;
         }
         h = (h + 1) & (unsigned)(T - 1);
@@ -2033,7 +2033,7 @@ __global__ void __launch_bounds__(256) k_hub_insert(DecideArgs<WT> a, HubPlan p,
                 for (int q = 0; q < kHubCacheProbe; ++q) {
                     const int k = atomicCAS(&ckeys[h], -1, c);
                     if (k == -1 || k == c) {
-                        atomic_add_w(&cvals[h], wt);
+                        atomic_add_sm(&cvals[h], wt);
                         cached = true;
                         break;
                     }

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(32 * ref_warps<WT>())
                     const int k = atomicCAS(&keys[h], -1, r);
                     if (k == -1 || k == r) {
                         created = k == -1;
-                        atomic_add_w(&vals[h], wt);
+                        atomic_add_sm(&vals[h], wt);
                         slot = (int)h;
                         break;
                     }
