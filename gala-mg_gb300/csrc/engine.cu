@@ -70,6 +70,8 @@ struct gala_context {
     int32_t *h_chunk = nullptr;      // page-locked copy of vstart and lo
     DevStats *d_stats2 = nullptr;    // level-init sums of a level whose rows were still in flight
     DevStats *h_stats2 = nullptr;
+    void *small_ctl = nullptr;       // small levels: sweep counters and result
+    SmallOut *small_out = nullptr, *h_small_out = nullptr;
     // per-graph state of gala_louvain_batch, kept between calls (reallocated
     // only for a larger batch)
     BatchRun *batch = nullptr;
@@ -304,6 +306,15 @@ long long decide_bytes_for(long long nv, long long ne, bool weighted)
     return nv * (2 * 8 + 4 * 4) + ne * (8 + (weighted ? 4 : 0));
 }
 
+// Levels whose sweeps run in one cooperative launch (small_level.cu).  Below
+// this many entries a sweep costs less than its launches and its host read:
+// phase 1 of planted graphs (one GB300, ms per call, separate launches / one
+// launch) 2.28 / 1.03 at 0.4M entries, 2.57 / 1.90 at 2.4M, 7.75 / 7.72 at
+// 9.6M, and 17.3 / 22.3 at 16M, where the one-bin kernels' higher occupancy
+// (48-64 warps per SM against 32) counts for more.
+constexpr int64_t kSmallLevelEntries = 1 << 22;
+bool small_level(const LevelGraph &g) { return g.E <= kSmallLevelEntries; }
+
 // One phase-1 run on level graph g (louvain_main_process).  The accepted
 // partition is left in ctx->p1.comm.
 //
@@ -345,6 +356,15 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     int32_t *const d_lo = d_vstart + PendingRows::kMax + 1;
     int32_t *const d_cnt = d_lo + (PendingRows::kMax + 1) * kNumBins;
     const int32_t *const h_lo = ctx->h_chunk + PendingRows::kMax + 1;
+
+    // a small level runs all its sweeps in one launch, with its own bin limits
+    const bool small = small_level(g) && !pend && !bt && pmode == GALA_PROPOSAL_OFF && !use_graphs &&
+                       ctx->update_mode != 2;
+    struct LimGuard {
+        BinLimits &l, keep;
+        ~LimGuard() { l = keep; }
+    } lim_guard{b.lim, b.lim};
+    if (small) b.lim = small_limits(b.lim, g.wide);
 
     p1_reset_level_stats(b, st);
     p1_level_init(g, b, st);
@@ -538,7 +558,35 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     // enqueued only after a sweep that moved under a third of them)
     unsigned long long prev_mv_edges = ~0ull;
     cudaEventRecord(ctx->ev[0], st);
-    for (;;) {
+    for (bool done = false; small && !done;) {
+        SmallRun r{ctx->small_ctl, ctx->small_out, bin_start, m2, min_tot_init, min_mod, prev_q, fp64_only, iteration};
+        if ((s = check(small_level_run(g, b, hp, r, st), "small level"))) return s;
+        SmallOut &o = *ctx->h_small_out;
+        cudaMemcpyAsync(&o, ctx->small_out, sizeof(SmallOut), cudaMemcpyDeviceToHost, st);
+        if ((s = sync_check(st, "small level"))) return s;
+        if (o.err) {
+            set_error("phase 1: device error bits %d", o.err);
+            return GALA_ERR_OVERFLOW;
+        }
+        for (int k = 0; k < o.sweeps; ++k) {
+            if (trace) trace->push_back(o.trace[k]);
+            if (verbose) printf("Iteration:%d Q:%f\n", iteration + k, o.trace[k]);
+        }
+        const long long dec_nv = o.decisions + (iteration == 1 ? act_nv : 0);
+        const long long dec_ne = (long long)o.entries + (iteration == 1 ? act_ne : 0);
+        out->decisions += dec_nv;
+        out->movers += o.movers;
+        out->active_entries += dec_ne;
+        out->decide_ms += (double)o.decide_ns * 1e-6;
+        out->update_ms += (double)o.update_ns * 1e-6;
+        out->decide_bytes += decide_bytes_for(dec_nv, dec_ne, weighted);
+        out->update_bytes += o.sweeps * (nv_all * (2 * 8 + 4 * 4) + g.E * (8 + (weighted ? 4 : 0)));
+        out->sweeps += o.sweeps;
+        prev_q = o.q;
+        done = o.done != 0;
+        iteration += o.sweeps - (done ? 1 : 0);
+    }
+    while (!small) {
         const int nxt = cur ^ 1;
         const int32_t *lists = iteration == 1 ? b.order : b.act[cur];
         const int *counts = &b.stats->act_count[cur][0];
@@ -1193,6 +1241,7 @@ void gala_context_destroy(gala_context *ctx)
     if (ctx->offs_ev) cudaEventDestroy(ctx->offs_ev);
     if (ctx->h_chunk) cudaFreeHost(ctx->h_chunk);
     if (ctx->h_stats2) cudaFreeHost(ctx->h_stats2);
+    if (ctx->h_small_out) cudaFreeHost(ctx->h_small_out);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     cudaSetDevice(prev);
     delete ctx;
@@ -1245,6 +1294,10 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
     ok = ok && cudaMallocHost(&ctx->h_chunk, kChunkInts * sizeof(int32_t)) == cudaSuccess;
     ok = ok && cudaMallocHost(&ctx->h_stats2, sizeof(DevStats)) == cudaSuccess;
     ok = ok && dalloc(ctx, &ctx->d_chunk, kChunkInts) && dalloc(ctx, &ctx->d_stats2, 1);
+    char *ctl = nullptr;
+    ok = ok && dalloc(ctx, &ctl, small_ctl_bytes()) && dalloc(ctx, &ctx->small_out, 1);
+    ok = ok && cudaMallocHost(&ctx->h_small_out, sizeof(SmallOut)) == cudaSuccess;
+    ctx->small_ctl = ctl;
     for (int i = 0; i < 2 && ok; ++i)
         ok = dalloc(ctx, &ctx->offs[i], n + 1) && dalloc(ctx, &ctx->nbr[i], E) && dalloc8(ctx, &ctx->w[i], E);
     Phase1Buffers &b = ctx->p1;
@@ -1263,9 +1316,10 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
          dalloc(ctx, &c.medge, n + 1) && dalloc(ctx, &c.stream_key, E) && dalloc8(ctx, &c.stream_w, E) &&
          dalloc(ctx, &c.tmp_off, n + 1) && dalloc(ctx, &c.tmp_nbr, E) && dalloc8(ctx, &c.tmp_w, E) &&
          dalloc(ctx, &c.kc, n + 1) && dalloc(ctx, &c.cls_list, 6 * n);
-    // tables of the rows longer than 4096 entries: at most 4 slots per entry
-    // (keys + values), chunk list of at most E / 4096 + n entries
-    c.big_pool_ints = 8LL * (long long)E + 64;
+    // tables of the rows longer than 4096 entries (hubs of a small level: 2048):
+    // at most 3 slots per entry of a key and up to 8 bytes of value, chunk
+    // list of at most E / 4096 + n entries
+    c.big_pool_ints = 9LL * (long long)E + 64;
     c.big_work_cap = (long long)E / 4096 + (long long)n + 1;
     c.big_twork_cap = (long long)E / 1024 + (long long)n + 1;  // table slots <= 4E, 4096 per chunk
     ok = ok && dalloc(ctx, &c.big_pool, (size_t)c.big_pool_ints) && dalloc(ctx, &c.big_T, n) &&

@@ -205,6 +205,30 @@ void p1_hub_decide(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, doub
 void p1_hub_update(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, int next, int bin_start, double constant,
                    long long m2, cudaStream_t st);
 
+// ---- all sweeps of a small level in one launch (small_level.cu) ----
+constexpr int kSmallSweeps = 256;  // sweeps of one launch at most
+struct SmallOut {  // what a launch reports (copied to the host in one piece)
+    double q;      // Q of the partition kept
+    int32_t sweeps, done, err, pad;
+    long long movers, decisions;  // decisions, entries: without the level's first sweep
+    unsigned long long entries, decide_ns, update_ns;
+    double trace[kSmallSweeps];
+};
+struct SmallRun {
+    void *ctl;       // small_ctl_bytes() of device memory, kept between launches of a level
+    SmallOut *out;   // device
+    const int *bin_start;
+    long long m2, min_tot_init;
+    double min_mod, prev_q;
+    int fp64_only;
+    int s0;          // first sweep (1 = the level's first: every vertex is active)
+};
+size_t small_ctl_bytes();
+// Degree-bin limits of a level run this way (rows above go to the hub path).
+BinLimits small_limits(const BinLimits &lim, bool wide);
+cudaError_t small_level_run(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, const SmallRun &r,
+                            cudaStream_t st);
+
 // ---- batched graphs (batch.cu) ----
 constexpr int kSumIn = 1, kSumTot2 = 2, kMinTot = 4, kSumK = 8, kCountComm = 16;
 struct GraphSums {  // per-graph outputs (device arrays of G entries)
