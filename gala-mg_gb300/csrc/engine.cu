@@ -456,10 +456,10 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
         p1_hub_work_launch(hp, st);
     }
     cudaMemsetAsync(b.act_flag, 1, (size_t)g.n, st);
-    // incremental weight updates: plain runs of one graph on a symmetric
-    // graph (the symmetry hash of the run's first level, summed by its
-    // level-init row kernels, is 0)
-    const bool incr_level = !bt && pmode == GALA_PROPOSAL_OFF && ctx->update_mode != 1;
+    // incremental weight updates: plain runs (single graphs and batches) on a
+    // symmetric graph (the symmetry hash of the run's first level, summed by
+    // its level-init row kernels, is 0)
+    const bool incr_level = pmode == GALA_PROPOSAL_OFF && ctx->update_mode != 1;
     if (incr_level) {
         cudaMemsetAsync(b.moved, 0, (size_t)g.n, st);
         if (ctx->sym_state < 0 && !pend) ctx->sym_state = (!g.ks_ready && h->sym_hash == 0) ? 1 : 0;

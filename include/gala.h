@@ -297,8 +297,8 @@ gala_status gala_context_set_hub_table_cap(gala_context *ctx, int64_t slots);
  * mirror (u, v, w), checked once per run; mode 1: always the full update;
  * mode 2: incrementally whenever allowed (symmetric graph, from a level's
  * second sweep on).  Integer sums: every mode gives the same In, active sets
- * and results bit for bit.  Plain runs of one graph only; proposal runs and
- * batches always take the full update. */
+ * and results bit for bit.  Plain runs, of one graph or of a batch's union;
+ * proposal runs always take the full update. */
 gala_status gala_context_set_update_mode(gala_context *ctx, int32_t mode);
 
 /* Aggregation of the contraction rows longer than 8192 entries inside a
