@@ -6,6 +6,8 @@
 // The vertices of graph g occupy the contiguous id range [goff[g], goff[g+1])
 // at every level: contraction renumbers communities by ascending old id and a
 // community never spans two graphs, so the ranges stay contiguous.
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -45,20 +47,46 @@ __device__ __forceinline__ int block_min_i32(int v, int *red)
     return t;
 }
 
-// One block per graph: the sums `what` asks for over the graph's range.
-// Graphs with stop[g] set are left alone (their values are final).
-__global__ void __launch_bounds__(256) k_graph_sums(int what, int G, const int64_t *__restrict__ goff,
+// S blocks per graph, each over a slice of its range: the sums `what` asks
+// for.  One block per graph writes them (S = 1); several add to values that
+// k_graph_sums_zero reset.  Graphs with stop[g] set are left alone (their
+// values are final).
+__global__ void k_graph_sums_zero(int what, int G, const uint8_t *__restrict__ stop, GraphSums out)
+{
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < G; g += gridDim.x * blockDim.x) {
+        if (stop && stop[g]) continue;
+        if (what & kSumIn) out.sum_in[g] = 0;
+        if (what & kSumTot2) out.sum_tot2[g] = 0;
+        if (what & kSumK) out.sum_k[g] = 0;
+        if (what & kCountComm) out.ncomm[g] = 0;
+        if (what & kMinTot) out.min_tot[g] = 0x7fffffff;
+    }
+}
+
+__device__ __forceinline__ void put_sum(unsigned long long *p, unsigned long long v, bool add)
+{
+    if (add)
+        atomicAdd(p, v);
+    else
+        *p = v;
+}
+
+__global__ void __launch_bounds__(256) k_graph_sums(int what, int G, int S, const int64_t *__restrict__ goff,
                                                     const uint8_t *__restrict__ stop, const int32_t *__restrict__ In,
                                                     const int32_t *__restrict__ Tot, const int32_t *__restrict__ K,
                                                     const int32_t *__restrict__ size, GraphSums out)
 {
     __shared__ unsigned long long red[32];
     __shared__ int redi[32];
-    for (int g = blockIdx.x; g < G; g += gridDim.x) {
+    const bool add = S > 1;
+    for (long long i = blockIdx.x; i < (long long)G * S; i += gridDim.x) {
+        const int g = (int)(i / S), slice = (int)(i % S);
         if (stop && stop[g]) continue;
-        const long long v0 = goff[g], v1 = goff[g + 1];
+        const long long r0 = goff[g], len = goff[g + 1] - r0;
+        const long long v0 = r0 + len * slice / S, v1 = r0 + len * (slice + 1) / S;
         unsigned long long si = 0, st2 = 0, sk = 0, nc = 0;
         int mn = 0x7fffffff;
+#pragma unroll 4
         for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
             if (what & kSumIn) si += (unsigned long long)In[v];
             if (what & (kSumTot2 | kMinTot)) {
@@ -73,23 +101,33 @@ __global__ void __launch_bounds__(256) k_graph_sums(int what, int G, const int64
         }
         if (what & kSumIn) {
             si = block_sum_u64(si, red);
-            if (threadIdx.x == 0) out.sum_in[g] = si;
+            if (threadIdx.x == 0) put_sum(&out.sum_in[g], si, add);
         }
         if (what & kSumTot2) {
             st2 = block_sum_u64(st2, red);
-            if (threadIdx.x == 0) out.sum_tot2[g] = st2;
+            if (threadIdx.x == 0) put_sum(&out.sum_tot2[g], st2, add);
         }
         if (what & kSumK) {
             sk = block_sum_u64(sk, red);
-            if (threadIdx.x == 0) out.sum_k[g] = sk;
+            if (threadIdx.x == 0) put_sum(&out.sum_k[g], sk, add);
         }
         if (what & kCountComm) {
             nc = block_sum_u64(nc, red);
-            if (threadIdx.x == 0) out.ncomm[g] = (int32_t)nc;
+            if (threadIdx.x == 0) {
+                if (add)
+                    atomicAdd(&out.ncomm[g], (int32_t)nc);
+                else
+                    out.ncomm[g] = (int32_t)nc;
+            }
         }
         if (what & kMinTot) {
             mn = block_min_i32(mn, redi);
-            if (threadIdx.x == 0) out.min_tot[g] = mn;
+            if (threadIdx.x == 0) {
+                if (add)
+                    atomicMin(&out.min_tot[g], mn);
+                else
+                    out.min_tot[g] = mn;
+            }
         }
         __syncthreads();
     }
@@ -122,53 +160,91 @@ __global__ void k_gid_fill(int G, const int64_t *__restrict__ goff, int32_t *gid
         for (long long v = goff[g] + threadIdx.x; v < goff[g + 1]; v += blockDim.x) gid[v] = g;
 }
 
+int sm_count_batch()
+{
+    static int s = 0;
+    if (s == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&s, cudaDevAttrMultiProcessorCount, dev);
+        if (s <= 0) s = 148;
+    }
+    return s;
+}
+
 int grid_for(int G) { return G < 65535 ? G : 65535; }
 
+// Graph of union position x: the last g with start[g] <= x.
+__device__ __forceinline__ int graph_of(const int64_t *__restrict__ start, int G, long long x)
+{
+    int lo = 0, hi = G - 1;
+    while (lo < hi) {
+        const int m = (lo + hi + 1) >> 1;
+        if (start[m] <= x)
+            lo = m;
+        else
+            hi = m - 1;
+    }
+    return lo;
+}
+
 // Union CSR of page-locked host graphs, read by the GPU through their
-// device-mapped addresses: one block per graph shifts the graph's offsets by
-// its first entry and its neighbour ids by its first vertex.  Four loads in
-// flight per thread (host memory behind the chip-to-chip link has a long
-// latency).
+// device-mapped addresses.  A block takes chunks of kGatherChunk union
+// entries (or vertices) whatever graphs they lie in, so that one large graph
+// does not keep one block busy, with eight loads in flight per thread (host
+// memory behind the chip-to-chip link has a long latency).  Ids are shifted
+// by their graph's first vertex, offsets by its first entry.
+constexpr int kGatherChunk = 8192;
+template <typename T, typename Src, typename Put>
+__device__ __forceinline__ void gather_chunk(const int64_t *__restrict__ start, int G, long long c0, long long c1,
+                                             Src src, Put put)
+{
+    constexpr int U = 8;
+    for (int g = graph_of(start, G, c0); c0 < c1; ++g) {
+        const long long b = start[g], e = start[g + 1] < c1 ? start[g + 1] : c1;
+        const T *p = src(g);
+        for (long long j0 = c0; j0 < e; j0 += (long long)U * blockDim.x) {
+            T t[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const long long j = j0 + u * blockDim.x + threadIdx.x;
+                t[u] = (j < e && p) ? p[j - b] : (T)1;  // graphs without weights: 1
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const long long j = j0 + u * blockDim.x + threadIdx.x;
+                if (j < e) put(g, j, t[u]);
+            }
+        }
+        if (e > c0) c0 = e;
+    }
+}
+
 __global__ void __launch_bounds__(256) k_batch_gather(int G, BatchSrc s, int64_t *offs, int32_t *nbr, int32_t *w)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) offs[0] = 0;
-    for (int g = blockIdx.x; g < G; g += gridDim.x) {
-        const long long v0 = s.vstart[g], n = s.vstart[g + 1] - v0;
-        const long long e0 = s.estart[g], E = s.estart[g + 1] - e0;
-        const int64_t *so = s.offs[g];
-        const int32_t *sn = s.nbr[g];
-        const int32_t *sw = s.w[g];
-        const int32_t shift = (int32_t)v0;
-        for (long long v = threadIdx.x; v < n; v += blockDim.x) offs[v0 + v + 1] = e0 + so[v];
-        constexpr int U = 4;
-        for (long long j0 = 0; j0 < E; j0 += (long long)U * blockDim.x) {
-            int32_t t[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const long long j = j0 + u * blockDim.x + threadIdx.x;
-                t[u] = j < E ? sn[j] : 0;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const long long j = j0 + u * blockDim.x + threadIdx.x;
-                if (j < E) nbr[e0 + j] = t[u] + shift;
-            }
+    const long long n = s.vstart[G], E = s.estart[G];
+    const long long ec = (E + kGatherChunk - 1) / kGatherChunk, vc = (n + kGatherChunk - 1) / kGatherChunk;
+    const long long all = vc + ec + (w ? ec : 0);
+    for (long long c = blockIdx.x; c < all; c += gridDim.x) {
+        if (c < vc) {
+            const long long c0 = c * kGatherChunk, c1 = c0 + kGatherChunk < n ? c0 + kGatherChunk : n;
+            gather_chunk<int64_t>(
+                s.vstart, G, c0, c1, [&](int g) { return s.offs[g]; },
+                [&](int g, long long v, int64_t x) { offs[v + 1] = s.estart[g] + x; });
+            continue;
         }
-        if (w) {
-            for (long long j0 = 0; j0 < E; j0 += (long long)U * blockDim.x) {
-                int32_t t[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const long long j = j0 + u * blockDim.x + threadIdx.x;
-                    t[u] = (j < E && sw) ? sw[j] : 1;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const long long j = j0 + u * blockDim.x + threadIdx.x;
-                    if (j < E) w[e0 + j] = t[u];
-                }
-            }
-        }
+        const bool wt = c >= vc + ec;
+        const long long c0 = (c - vc - (wt ? ec : 0)) * kGatherChunk;
+        const long long c1 = c0 + kGatherChunk < E ? c0 + kGatherChunk : E;
+        if (wt)
+            gather_chunk<int32_t>(
+                s.estart, G, c0, c1, [&](int g) { return s.w[g]; },
+                [&](int, long long j, int32_t x) { w[j] = x; });
+        else
+            gather_chunk<int32_t>(
+                s.estart, G, c0, c1, [&](int g) { return s.nbr[g]; },
+                [&](int g, long long j, int32_t x) { nbr[j] = x + (int32_t)s.vstart[g]; });
     }
 }
 
@@ -205,7 +281,7 @@ __global__ void k_batch_local_labels(int G, const int64_t *__restrict__ vstart, 
 void batch_gather(int G, const BatchSrc &src, int64_t *offs, int32_t *nbr, int32_t *w, cudaStream_t st)
 {
     if (G <= 0) return;
-    k_batch_gather<<<grid_for(G), 256, 0, st>>>(G, src, offs, nbr, w);
+    k_batch_gather<<<sm_count_batch() * 8, 256, 0, st>>>(G, src, offs, nbr, w);
     note_launch(1);
 }
 
@@ -227,7 +303,15 @@ void batch_graph_sums(int what, int G, const int64_t *goff, const uint8_t *stop,
                       const GraphSums &out, cudaStream_t st)
 {
     if (G <= 0) return;
-    k_graph_sums<<<grid_for(G), 256, 0, st>>>(what, G, goff, stop, b.In, b.Tot, b.K, b.size, out);
+    // few graphs: several blocks each, about eight per SM in all (128 graphs
+    // of 2,000-60,000 vertices: 36 us a launch with one block per graph, 6 us
+    // with nine, the reset included)
+    const int S = std::max(1, std::min(64, sm_count_batch() * 8 / G));
+    if (S > 1) {
+        k_graph_sums_zero<<<(G + 255) / 256, 256, 0, st>>>(what, G, stop, out);
+        note_launch(1);
+    }
+    k_graph_sums<<<grid_for(G * S), 256, 0, st>>>(what, G, S, goff, stop, b.In, b.Tot, b.K, b.size, out);
     note_launch(1);
 }
 
