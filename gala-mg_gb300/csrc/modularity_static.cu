@@ -9,7 +9,7 @@
 // scratch the computation needs - the total weight of every community and
 // four sums - lives in the file-scope arrays below, sized for at most
 // kStaticMaxVertices vertices.  Every GPU that loads this library holds that
-// memory (8 MB + 36 B) until the process exits.
+// memory (8 MB + 40 B) until the process exits.
 //
 // The computation is the one phase 1 uses for Q: sum of In over vertices and
 // total weight m2 as exact 64-bit integers, sum of Tot^2 over communities as
@@ -30,59 +30,124 @@ constexpr int kStaticMaxDevices = 64;
 
 // Scratch shared by every call on a device: community totals and the sums.
 static __device__ __align__(256) unsigned long long g_static_tot[kStaticMaxVertices];
-// sum In, sum K, sum Tot^2 (low word), sum Tot^2 (high word)
-static __device__ __align__(256) unsigned long long g_static_sums[4];
-// bit 0: a label lies outside [0, n); bit 1: a weight is not positive
-static __device__ __align__(256) int g_static_bad;
+// sum In, sum K, sum Tot^2 (low word), sum Tot^2 (high word), and the error
+// bits (bit 0: a label lies outside [0, n); bit 1: a weight is not positive):
+// one copy brings all five back
+static __device__ __align__(256) unsigned long long g_static_sums[5];
 
-// Device addresses of the three arrays, looked up once per device (in host
+// Device addresses of the two arrays, looked up once per device (in host
 // code the symbols are host-side stand-ins, not device addresses).
 static unsigned long long *g_tot_ptr[kStaticMaxDevices];
 static unsigned long long *g_sums_ptr[kStaticMaxDevices];
-static int *g_bad_ptr[kStaticMaxDevices];
 static std::mutex g_static_mu;
 
-__global__ void k_static_zero(unsigned long long *tot, int n, unsigned long long *sums, int *bad)
+__global__ void k_static_zero(unsigned long long *tot, int n, unsigned long long *sums)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) tot[i] = 0ull;
-    if (blockIdx.x == 0 && threadIdx.x < 4) sums[threadIdx.x] = 0ull;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *bad = 0;
+    if (blockIdx.x == 0 && threadIdx.x < 5) sums[threadIdx.x] = 0ull;
 }
 
-// One warp per vertex: K (row weight), In (weight to the own community);
-// community totals by atomics, sums by warp then block reduction.
-__global__ void __launch_bounds__(256) k_static_rows(int n, const int64_t *__restrict__ offs,
-                                                     const int32_t *__restrict__ nbr, const int32_t *__restrict__ w,
-                                                     const int32_t *__restrict__ comm, unsigned long long *tot,
-                                                     unsigned long long *sums, int *bad)
+// Weight (W) and own-community weight of the row entries first, first + step,
+// ... < deg.
+template <bool W>
+__device__ __forceinline__ void static_row(const int32_t *__restrict__ nbr, const int32_t *__restrict__ w,
+                                           const int32_t *__restrict__ comm, int n, int c, long long first,
+                                           long long deg, int step, unsigned long long &k, unsigned long long &in,
+                                           int &bad)
+{
+    constexpr int U = 4;  // predicated batches: a short row's loads are in flight together too
+    for (; first < deg; first += (long long)U * step) {
+        int u[U], wi[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const long long j = first + q * step;
+            u[q] = j < deg ? nbr[j] : -1;
+            if (W) {
+                wi[q] = j < deg ? w[j] : 0;
+                if (j < deg && wi[q] <= 0) bad |= 2;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) u[q] = (unsigned)u[q] < (unsigned)n ? comm[u[q]] : ~c;
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            if (W) {
+                const unsigned long long wt = wi[q] > 0 ? (unsigned long long)wi[q] : 0ull;
+                k += wt;
+                if (u[q] == c) in += wt;
+            } else {
+                in += u[q] == c;
+            }
+        }
+    }
+}
+
+// K (row weight) and In (weight to the own community) of every vertex;
+// community totals by atomics, sums by warp then block reduction.  A group of
+// kStaticG lanes takes a row, four loads in flight per lane and four rows per
+// warp; rows longer than kStaticLong entries go to the whole warp afterwards.
+// One wave of blocks.  300k vertices, 7.2M entries: 59 us with a warp per row,
+// 42 us so, where the label gathers (one 32-byte L2 sector each, about
+// 6 TB/s of sectors) bound it: neither more warps nor more loads in flight
+// change it.
+constexpr int kStaticG = 8;
+constexpr int kStaticLong = 512;
+template <bool W>
+__global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int64_t *__restrict__ offs,
+                                                        const int32_t *__restrict__ nbr,
+                                                        const int32_t *__restrict__ w,
+                                                        const int32_t *__restrict__ comm, unsigned long long *tot,
+                                                        unsigned long long *sums)
 {
     __shared__ unsigned long long s_in[8], s_k[8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int sub = lane & (kStaticG - 1), gw = lane / kStaticG;
+    constexpr int GPW = 32 / kStaticG;
     const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     unsigned long long my_in = 0, my_k = 0;
-    for (int v = wg; v < n; v += nw) {
+    int bad = 0;
+    for (long long v0 = (long long)wg * GPW; v0 < n; v0 += (long long)nw * GPW) {
+        const bool has = v0 + gw < n;
+        const int v = has ? (int)(v0 + gw) : n - 1;
         const int c = comm[v];
+        const long long s = offs[v], deg = has ? offs[v + 1] - s : 0;
+        const bool is_long = deg > kStaticLong;
         unsigned long long k = 0, in = 0;
-        for (long long j = offs[v] + lane; j < offs[v + 1]; j += 32) {
-            const int32_t wi = w ? w[j] : 1;
-            if (wi <= 0) atomicOr(bad, 2);
-            const unsigned long long wt = wi > 0 ? (unsigned long long)wi : 0ull;
-            k += wt;
-            const int u = nbr[j];
-            if (u >= 0 && u < n && comm[u] == c) in += wt;
+        if (!is_long) static_row<W>(nbr + s, W ? w + s : nullptr, comm, n, c, sub, deg, kStaticG, k, in, bad);
+        unsigned todo = __ballot_sync(GALA_FULL_MASK, is_long && sub == 0);
+        while (todo) {  // warp-uniform
+            const int src = __ffs((int)todo) - 1;
+            todo &= todo - 1;
+            const long long ls = __shfl_sync(GALA_FULL_MASK, s, src), ld = __shfl_sync(GALA_FULL_MASK, deg, src);
+            const int lc = __shfl_sync(GALA_FULL_MASK, c, src);
+            unsigned long long lk = 0, lin = 0;
+            static_row<W>(nbr + ls, W ? w + ls : nullptr, comm, n, lc, lane, ld, 32, lk, lin, bad);
+            if (W) lk = warp_sum(lk);
+            lin = warp_sum(lin);
+            if (lane == src) {
+                k = lk;
+                in = lin;
+            }
         }
-        k = warp_sum(k);
-        in = warp_sum(in);
-        if (lane == 0) {
-            if (c >= 0 && c < n)
+#pragma unroll
+        for (int o = kStaticG / 2; o >= 1; o >>= 1) {
+            if (W) k += __shfl_xor_sync(GALA_FULL_MASK, k, o);
+            in += __shfl_xor_sync(GALA_FULL_MASK, in, o);
+        }
+        if (has && sub == 0) {
+            if (!W) k = (unsigned long long)deg;
+            if ((unsigned)c < (unsigned)n)
                 atomicAdd(&tot[c], k);
             else
-                atomicOr(bad, 1);
+                bad |= 1;
             my_in += in;
             my_k += k;
         }
     }
+    if (bad) atomicOr(&sums[4], (unsigned long long)bad);
+    my_in = warp_sum(my_in);
+    my_k = warp_sum(my_k);
     if (lane == 0) {
         s_in[wid] = my_in;
         s_k[wid] = my_k;
@@ -159,40 +224,39 @@ extern "C" gala_status gala_modularity_device_static(int32_t n, const int64_t *d
         return GALA_ERR_INVALID;
     }
     unsigned long long *tot = nullptr, *sums = nullptr;
-    int *bad = nullptr;
     {
         // first call on this device (with it current): look up the device
         // addresses of the static arrays
         std::lock_guard<std::mutex> lock(g_static_mu);
         if (!g_tot_ptr[dev]) {
-            void *p = nullptr, *q = nullptr, *r = nullptr;
+            void *p = nullptr, *q = nullptr;
             if ((ce = cudaGetSymbolAddress(&p, g_static_tot)) != cudaSuccess ||
-                (ce = cudaGetSymbolAddress(&q, g_static_sums)) != cudaSuccess ||
-                (ce = cudaGetSymbolAddress(&r, g_static_bad)) != cudaSuccess)
+                (ce = cudaGetSymbolAddress(&q, g_static_sums)) != cudaSuccess)
                 return cuda_fail(ce, "gala_modularity_device_static: symbol address");
-            g_tot_ptr[dev] = (unsigned long long *)p;
             g_sums_ptr[dev] = (unsigned long long *)q;
-            g_bad_ptr[dev] = (int *)r;
+            g_tot_ptr[dev] = (unsigned long long *)p;
         }
         tot = g_tot_ptr[dev];
         sums = g_sums_ptr[dev];
-        bad = g_bad_ptr[dev];
     }
     // the scratch keeps the previous call's contents: clear it first
     const int grid = (n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024;
-    k_static_zero<<<grid, 256>>>(tot, n, sums, bad);
-    const int rgrid = (int)(((long long)n * 32 + 255) / 256 < 2048 ? ((long long)n * 32 + 255) / 256 : 2048);
-    k_static_rows<<<rgrid, 256>>>(n, d_offsets, d_neighbors, d_weights, d_community, tot, sums, bad);
+    k_static_zero<<<grid, 256>>>(tot, n, sums);
+    const long long rblocks = ((long long)n * kStaticG + 255) / 256, wave = (long long)hub_grid_size() * (d_weights ? 5 : 6);
+    const int rgrid = (int)(rblocks < wave ? rblocks : wave);
+    if (d_weights)
+        k_static_rows<true><<<rgrid, 256>>>(n, d_offsets, d_neighbors, d_weights, d_community, tot, sums);
+    else
+        k_static_rows<false><<<rgrid, 256>>>(n, d_offsets, d_neighbors, nullptr, d_community, tot, sums);
     k_static_tot2<<<grid, 256>>>(n, tot, sums);
     note_launch(3);
     // a launch that failed for its configuration would leave the previous
     // call's sums in the scratch: report it instead of reading them
     if ((ce = cudaGetLastError()) != cudaSuccess) return cuda_fail(ce, "gala_modularity_device_static: launch");
-    unsigned long long h[4] = {0, 0, 0, 0};
-    int hbad = 0;
-    if ((ce = cudaMemcpy(h, sums, sizeof(h), cudaMemcpyDeviceToHost)) != cudaSuccess ||
-        (ce = cudaMemcpy(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
+    unsigned long long h[5] = {0, 0, 0, 0, 0};
+    if ((ce = cudaMemcpy(h, sums, sizeof(h), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return cuda_fail(ce, "gala_modularity_device_static");
+    const int hbad = (int)h[4];
     if (hbad & 1) {
         set_error("gala_modularity_device_static: a community label lies outside [0, %d)", n);
         return GALA_ERR_INVALID;
