@@ -101,94 +101,150 @@ __global__ void __launch_bounds__(256) k_mlp_logits(const __nv_bfloat16 *__restr
 
 // Gradient of the weighted binary cross-entropy over samples [0, n) with FP32
 // master weights: loss = sum_s wt_s * BCE(sigmoid(out_s), y_s), wt = pos_weight
-// for y = 1, else 1.  Per-sample gradients are summed over the warp by
-// shuffles into the warp's own row of shared memory, the rows of a block in
-// fixed order into the block's partial (global), and the partials of all
-// blocks in fixed order by k_grad_sum: the gradient does not depend on
-// scheduling, so training repeats bit-exactly.
+// for y = 1, else 1.  A warp takes 32 samples at a time: the forward pass and
+// the backward deltas one sample per lane, then the weight gradients (outer
+// products summed over the samples) one output column per lane, the samples'
+// activations and deltas read from shared memory.  Every lane keeps its part
+// of the gradient in registers over all its samples; the warps of a block are
+// summed in fixed order into the block's partial and the partials in fixed
+// order by k_grad_sum, so the gradient does not depend on scheduling and
+// training repeats bit-exactly.
+// Bound by its FMA and shared-memory issue: about 4,500 instructions a warp
+// and 32 samples (one 5-shuffle warp sum per parameter took over 11,000, on
+// 512 warps).  65,536 samples: 148 + 7 -> 23 + 6 us (gradient kernel + sums).
 constexpr int kGradBlock = 128;
 constexpr int kGradWarps = kGradBlock / 32;
-constexpr int kGradMaxBlocks = 128;
+constexpr int kGradMaxBlocks = 304;  // two per SM
+struct __align__(16) GradTile {  // one warp's 32 samples
+    float x[32][kIn];
+    float h[32][kH + 1];  // h1 (odd row length: columns and rows conflict-free)
+    float d[32][kH + 4];  // dout * h2, then dz2, then dz1 (rows 16-byte aligned)
+};
+__device__ __forceinline__ float tile_column_sum(const GradTile &t, int c)
+{
+    float s = 0.f;
+#pragma unroll
+    for (int r = 0; r < 32; ++r) s += t.d[r][c];
+    return s;
+}
+
 __global__ void __launch_bounds__(kGradBlock) k_mlp_grad(const float *__restrict__ Pm, const float *__restrict__ X,
                                                          const float *__restrict__ Y, long long n, float pos_weight,
                                                          float *grad_part, float *loss_part)
 {
-    __shared__ float P[kPropParams];
-    __shared__ float Gw[kGradWarps][kPropParams];
+    __shared__ __align__(16) float P[kPropParams + 3];
+    extern __shared__ __align__(16) unsigned char grad_sm[];
+    GradTile *tiles = (GradTile *)grad_sm;
     __shared__ float Lw[kGradWarps];
-    for (int i = threadIdx.x; i < kPropParams; i += blockDim.x) {
-        P[i] = Pm[i];
-        for (int w = 0; w < kGradWarps; ++w) Gw[w][i] = 0.f;
-    }
-    if (threadIdx.x < kGradWarps) Lw[threadIdx.x] = 0.f;
+    for (int i = threadIdx.x; i < kPropParams; i += blockDim.x) P[i] = Pm[i];
     __syncthreads();
-    float *G = Gw[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    // all lanes of a warp run the same number of rounds (warp reductions inside)
-    const long long base0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31);
-    for (long long base = base0; base < n; base += stride) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    GradTile &T = tiles[wid];
+    // this lane's part: columns w1[lane][*], w2[*][lane], b1, b2, w3 at lane;
+    // b3 and the loss one sample per lane
+    float g1[kIn], g2[kH], gb1 = 0.f, gb2 = 0.f, g3 = 0.f, gb3 = 0.f, loss = 0.f;
+#pragma unroll
+    for (int i = 0; i < kIn; ++i) g1[i] = 0.f;
+#pragma unroll
+    for (int i = 0; i < kH; ++i) g2[i] = 0.f;
+    const long long stride = (long long)gridDim.x * kGradBlock;
+    for (long long base = (long long)blockIdx.x * kGradBlock + wid * 32; base < n; base += stride) {
         const long long s = base + lane;
         const bool valid = s < n;
-        float x[kIn], z1[kH], z2[kH];
-        float y = 0.f;
-#pragma unroll
-        for (int i = 0; i < kIn; ++i) x[i] = valid ? X[s * kIn + i] : 0.f;
-        if (valid) y = Y[s];
-        const float out = mlp_forward(P, x, z1, z2);
-        const float p = sigmoidf_(out);
-        const float wt = valid ? (y > 0.5f ? pos_weight : 1.f) : 0.f;
-        // loss (stable form): wt * (softplus(out) - y*out)
-        const float sp = out > 0.f ? out + log1pf(__expf(-out)) : log1pf(__expf(out));
-        float l = wt * (sp - y * out);
-        const float dout = wt * (p - y);
-        // output layer
-        float dh2[kH];
-#pragma unroll
-        for (int i = 0; i < kH; ++i) {
-            const float h2 = fmaxf(z2[i], 0.f);
-            float g = warp_sum(dout * h2);
-            if (lane == 0) G[kOffW3 + i] += g;
-            dh2[i] = z2[i] > 0.f ? dout * P[kOffW3 + i] : 0.f;
-        }
+        float z1[kH], dh1[kH];
+        float dout;
         {
-            float g = warp_sum(dout);
-            if (lane == 0) G[kOffB3] += g;
-            float lw = warp_sum(l);
-            if (lane == 0) Lw[threadIdx.x >> 5] += lw;
-        }
-        // hidden layer 2: dW2[o][i] = dz2[o] * h1[i]
-        float dh1[kH];
+            float x[kIn], z2[kH];
+            float y = 0.f;
 #pragma unroll
-        for (int i = 0; i < kH; ++i) dh1[i] = 0.f;
-        for (int o = 0; o < kH; ++o) {
-            const float dz = dh2[o];
-            float g = warp_sum(dz);
-            if (lane == 0) G[kOffB2 + o] += g;
+            for (int i = 0; i < kIn; ++i) x[i] = valid ? X[s * kIn + i] : 0.f;
+            if (valid) y = Y[s];
+            const float out = mlp_forward(P, x, z1, z2);
+            const float p = sigmoidf_(out);
+            const float wt = valid ? (y > 0.5f ? pos_weight : 1.f) : 0.f;
+            // loss (stable form): wt * (softplus(out) - y*out)
+            const float sp = out > 0.f ? out + log1pf(__expf(-out)) : log1pf(__expf(out));
+            loss += wt * (sp - y * out);
+            dout = wt * (p - y);
+            gb3 += dout;
+#pragma unroll
+            for (int i = 0; i < kIn; ++i) T.x[lane][i] = x[i];
 #pragma unroll
             for (int i = 0; i < kH; ++i) {
-                const float h1 = fmaxf(z1[i], 0.f);
-                float gg = warp_sum(dz * h1);
-                if (lane == 0) G[kOffW2 + o * kH + i] += gg;
-                dh1[i] = fmaf(dz, P[kOffW2 + o * kH + i], dh1[i]);
+                T.h[lane][i] = fmaxf(z1[i], 0.f);
+                T.d[lane][i] = dout * fmaxf(z2[i], 0.f);
             }
-        }
-        // hidden layer 1
-        for (int o = 0; o < kH; ++o) {
-            const float dz = z1[o] > 0.f ? dh1[o] : 0.f;
-            float g = warp_sum(dz);
-            if (lane == 0) G[kOffB1 + o] += g;
+            __syncwarp();
+            g3 += tile_column_sum(T, lane);
+            __syncwarp();
+            // hidden layer 2: dz2 = dout * w3 where z2 > 0
 #pragma unroll
-            for (int i = 0; i < kIn; ++i) {
-                float gg = warp_sum(dz * x[i]);
-                if (lane == 0) G[kOffW1 + o * kIn + i] += gg;
+            for (int i = 0; i < kH; ++i) dh1[i] = 0.f;
+#pragma unroll
+            for (int o = 0; o < kH; ++o) {
+                const float dz = z2[o] > 0.f ? dout * P[kOffW3 + o] : 0.f;
+                T.d[lane][o] = dz;
+#pragma unroll
+                for (int i = 0; i < kH; ++i) dh1[i] = fmaf(dz, P[kOffW2 + o * kH + i], dh1[i]);
             }
         }
+        __syncwarp();
+        gb2 += tile_column_sum(T, lane);
+        // dW2[o][lane] = sum over the samples of dz2[o] h1[lane]
+#pragma unroll 4
+        for (int r = 0; r < 32; ++r) {
+            const float h = T.h[r][lane];
+            const float4 *d4 = (const float4 *)T.d[r];
+#pragma unroll
+            for (int q = 0; q < kH / 4; ++q) {
+                const float4 d = d4[q];
+                g2[4 * q] = fmaf(d.x, h, g2[4 * q]);
+                g2[4 * q + 1] = fmaf(d.y, h, g2[4 * q + 1]);
+                g2[4 * q + 2] = fmaf(d.z, h, g2[4 * q + 2]);
+                g2[4 * q + 3] = fmaf(d.w, h, g2[4 * q + 3]);
+            }
+        }
+        __syncwarp();
+        // hidden layer 1: dz1 = dh1 where z1 > 0
+#pragma unroll
+        for (int o = 0; o < kH; ++o) T.d[lane][o] = z1[o] > 0.f ? dh1[o] : 0.f;
+        __syncwarp();
+        gb1 += tile_column_sum(T, lane);
+#pragma unroll 4
+        for (int r = 0; r < 32; ++r) {
+            const float d = T.d[r][lane];
+            const float4 *x4 = (const float4 *)T.x[r];
+#pragma unroll
+            for (int q = 0; q < kIn / 4; ++q) {
+                const float4 x = x4[q];
+                g1[4 * q] = fmaf(d, x.x, g1[4 * q]);
+                g1[4 * q + 1] = fmaf(d, x.y, g1[4 * q + 1]);
+                g1[4 * q + 2] = fmaf(d, x.z, g1[4 * q + 2]);
+                g1[4 * q + 3] = fmaf(d, x.w, g1[4 * q + 3]);
+            }
+        }
+        __syncwarp();
+    }
+    gb3 = warp_sum(gb3);
+    loss = warp_sum(loss);
+    // the tiles are free: one gradient row per warp, summed in warp order
+    __syncthreads();
+    float *G = (float *)grad_sm + wid * kPropParams;
+#pragma unroll
+    for (int i = 0; i < kIn; ++i) G[kOffW1 + lane * kIn + i] = g1[i];
+#pragma unroll
+    for (int o = 0; o < kH; ++o) G[kOffW2 + o * kH + lane] = g2[o];
+    G[kOffB1 + lane] = gb1;
+    G[kOffB2 + lane] = gb2;
+    G[kOffW3 + lane] = g3;
+    if (lane == 0) {
+        G[kOffB3] = gb3;
+        Lw[wid] = loss;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kPropParams; i += blockDim.x) {
         float t = 0.f;
-        for (int w = 0; w < kGradWarps; ++w) t += Gw[w][i];
+        for (int w = 0; w < kGradWarps; ++w) t += ((const float *)grad_sm)[w * kPropParams + i];
         grad_part[(long long)blockIdx.x * kPropParams + i] = t;
     }
     if (threadIdx.x == 0) {
@@ -197,22 +253,38 @@ __global__ void __launch_bounds__(kGradBlock) k_mlp_grad(const float *__restrict
         loss_part[blockIdx.x] = t;
     }
 }
+constexpr size_t kGradSmem = kGradWarps * sizeof(GradTile);
+static_assert(kGradWarps * kPropParams * sizeof(float) <= kGradSmem, "gradient rows reuse the tiles");
+static_assert(kGradSmem <= 48 * 1024, "no opt-in for more shared memory");
 
-// grad = sum of the block partials in block order (and the loss likewise,
-// added to *loss).
-__global__ void k_grad_sum(const float *__restrict__ grad_part, const float *__restrict__ loss_part, int nblocks,
-                           float *grad, float *loss)
+// grad = sum of the block partials (and the loss likewise, added to *loss):
+// kSumParts threads per parameter sum contiguous runs of blocks in block
+// order, thread 0 adds the runs in order.
+constexpr int kSumParts = 8;
+__global__ void __launch_bounds__(32 * kSumParts) k_grad_sum(const float *__restrict__ grad_part,
+                                                            const float *__restrict__ loss_part, int nblocks,
+                                                            float *grad, float *loss)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ float part[kSumParts][32];
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    const int per = (nblocks + kSumParts - 1) / kSumParts;
+    const int b0 = min(nblocks, (int)threadIdx.y * per), b1 = min(nblocks, b0 + per);
+    float t = 0.f;
     if (i < kPropParams) {
-        float t = 0.f;
-        for (int b = 0; b < nblocks; ++b) t += grad_part[(long long)b * kPropParams + i];
-        grad[i] = t;
+#pragma unroll 8
+        for (int b = b0; b < b1; ++b) t += grad_part[(long long)b * kPropParams + i];
+    } else if (i == kPropParams) {
+#pragma unroll 8
+        for (int b = b0; b < b1; ++b) t += loss_part[b];
     }
-    if (i == kPropParams) {
-        float t = 0.f;
-        for (int b = 0; b < nblocks; ++b) t += loss_part[b];
-        *loss += t;
+    part[threadIdx.y][threadIdx.x] = t;
+    __syncthreads();
+    if (threadIdx.y == 0) {
+        for (int q = 1; q < kSumParts; ++q) t += part[q][threadIdx.x];
+        if (i < kPropParams)
+            grad[i] = t;
+        else if (i == kPropParams)
+            *loss += t;
     }
 }
 
@@ -698,8 +770,8 @@ gala_status gala_proposal_gradient(gala_proposal *p, const float *features, cons
     cudaMemcpyAsync(p->Yb, labels, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(p->loss, 0, sizeof(float), st);
     const int gb = grad_blocks(n);
-    k_mlp_grad<<<gb, kGradBlock, 0, st>>>(p->Pm, p->Xb, p->Yb, n, pos_weight, p->grad_part, p->loss_part);
-    k_grad_sum<<<(kPropParams + 256) / 256, 256, 0, st>>>(p->grad_part, p->loss_part, gb, p->grad, p->loss);
+    k_mlp_grad<<<gb, kGradBlock, kGradSmem, st>>>(p->Pm, p->Xb, p->Yb, n, pos_weight, p->grad_part, p->loss_part);
+    k_grad_sum<<<(kPropParams + 32) / 32, dim3(32, kSumParts), 0, st>>>(p->grad_part, p->loss_part, gb, p->grad, p->loss);
     note_launch(2);
     cudaMemcpyAsync(grad_out, p->grad, kPropParams * sizeof(float), cudaMemcpyDeviceToHost, st);
     float l = 0.f;
@@ -785,8 +857,8 @@ gala_status gala_proposal_train(gala_proposal *p, int32_t epochs, int32_t batch_
             const int nb = (int)std::min<int64_t>(batch_size, n - b0);
             k_gather_batch<<<(nb + 255) / 256, 256, 0, st>>>(p->X, p->Y, p->idx + b0, nb, p->Xb, p->Yb);
             const int gb = grad_blocks(nb);
-            k_mlp_grad<<<gb, kGradBlock, 0, st>>>(p->Pm, p->Xb, p->Yb, nb, pos_weight, p->grad_part, p->loss_part);
-            k_grad_sum<<<(kPropParams + 256) / 256, 256, 0, st>>>(p->grad_part, p->loss_part, gb, p->grad, p->loss);
+            k_mlp_grad<<<gb, kGradBlock, kGradSmem, st>>>(p->Pm, p->Xb, p->Yb, nb, pos_weight, p->grad_part, p->loss_part);
+            k_grad_sum<<<(kPropParams + 32) / 32, dim3(32, kSumParts), 0, st>>>(p->grad_part, p->loss_part, gb, p->grad, p->loss);
             p->adam_t++;
             k_adam<<<(kPropParams + 255) / 256, 256, 0, st>>>(p->Pm, p->m, p->v, p->grad, 1.f / nb, lr, 0.9f, 0.999f,
                                                              1e-8f, p->adam_t, p->wb);
