@@ -88,7 +88,6 @@ struct DevStats {
     long long new_entries;  // entries of the contracted level
     long long big_slots;    // long rows: table slots
     long long big_nwork;    // long rows: stream chunks
-    long long big_ntwork;   // long rows: table chunks
     long long big_lwork;    // long rows: slot-list chunks
     // long rows by key range: pool offsets (ints) and counts
     long long rad_offm;     // per-chunk bucket offsets (uint16)
@@ -100,6 +99,7 @@ struct DevStats {
     int rad_nitems;         // items planned
     int rad_nacc;           // accumulators taken
     int rad_next;           // item queue head
+    int sort_cnt[5];        // sorted rows of more than 128 / 512 / 1024 / 4096 / 16384 pairs
     // incremental weight update
     unsigned long long mv_edges;  // row entries of this sweep's movers
     long long push_total;         // the same, summed by the movers' prefix

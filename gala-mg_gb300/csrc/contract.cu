@@ -9,21 +9,18 @@
 //      the neighbour's community and the weight, contiguous per community
 //   4. per community, sum the weights per neighbour community, by row length:
 //        <= 32 entries      one warp, __match_any_sync + __reduce_add_sync
+//        <= 128 entries     one warp, its own shared-memory hash table
 //        <= 512 entries     one 128-thread CTA, shared-memory hash table
-//        <= 4096 entries    one CTA (1024 threads; 256 when rows are sorted),
-//                           shared-memory hash table
-//        <= 8192 entries    one 1024-thread CTA (rows in table order only)
-//        larger             a global table per community filled by many CTAs
-//                           (4096-entry chunks of the stream); a dense table
-//                           indexed by community id when a hash table would not
-//                           be smaller
-//      and emit the distinct neighbours in ascending id order (rank by
-//      shuffle compare, bitonic sort in shared memory, or - rows with more
-//      than 16384 distinct neighbours - a bitmap over all communities ranked
-//      by a prefix sum of popcounts, all spread over many CTAs)
-//   5. CSR offsets by scan and a compaction copy.
-// Rows come out sorted by neighbour id, so the contracted graph of a given
-// partition is unique and can be compared bit for bit.
+//        <= 4096 / 8192     one 1024-thread CTA, shared-memory hash table
+//        larger             by key range: chunks summed in shared memory,
+//                           buckets of 8192 communities summed by one CTA
+//                           each (or global hash tables, when that does not
+//                           fit the scratch or is asked for)
+//   5. CSR offsets by scan and a compaction copy; gala_contract_device sorts
+//      every row on the way (registers, shared memory, or a bitmap over the
+//      communities).
+// With sorted rows the contracted graph of a given partition is unique and can
+// be compared bit for bit.
 //
 // The stream fill and the compaction walk contiguous entry ranges: every
 // warp takes 1024 consecutive CSR entries and finds the row of each entry
@@ -263,14 +260,14 @@ __global__ void __launch_bounds__(256) k_stream_fill(long long E, const int32_t 
     }
 }
 
-__device__ __forceinline__ int row_class(long long E, int sort_rows)
+__device__ __forceinline__ int row_class(long long E)
 {
     if (E == 0) return -1;
     if (E <= kSmallMax) return 0;
-    if (E <= kWarpAggMax && !sort_rows) return kWarpCls;
+    if (E <= kWarpAggMax) return kWarpCls;
     if (E <= kMid1Max) return 1;
     if (E <= kMid2Max) return 2;
-    if (E <= kMid3Max && !sort_rows) return 3;
+    if (E <= kMid3Max) return 3;
     return kLongCls;
 }
 
@@ -279,7 +276,7 @@ __device__ __forceinline__ int row_class(long long E, int sort_rows)
 // its communities from lists + k * lstride.  Communities without entries get
 // an empty row right away.
 __global__ void __launch_bounds__(256) k_classify(const long long *__restrict__ ec, int32_t *lists, long long lstride,
-                                                  int32_t *kc, DevStats *st, int sort_rows)
+                                                  int32_t *kc, DevStats *st)
 {
     __shared__ int wc[8][kNumCls];  // per-warp counts of a tile
     __shared__ int next[kNumCls];   // the block's next list position per class
@@ -292,7 +289,7 @@ __global__ void __launch_bounds__(256) k_classify(const long long *__restrict__ 
 #pragma unroll
     for (int k = 0; k < kNumCls; ++k) cnt[k] = 0;
     for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-        const int cls = row_class(ec[c], sort_rows);
+        const int cls = row_class(ec[c]);
 #pragma unroll
         for (int k = 0; k < kNumCls; ++k) cnt[k] += cls == k;
     }
@@ -309,7 +306,7 @@ __global__ void __launch_bounds__(256) k_classify(const long long *__restrict__ 
     __syncthreads();
     for (int t0 = c0; t0 < c1; t0 += blockDim.x) {  // block-uniform
         const int c = t0 + threadIdx.x;
-        const int cls = c < c1 ? row_class(ec[c], sort_rows) : -2;
+        const int cls = c < c1 ? row_class(ec[c]) : -2;
         if (cls == -1) kc[c] = 0;
         int rank = 0;
 #pragma unroll
@@ -349,8 +346,8 @@ struct AggArgs {
     __device__ __forceinline__ WT w_at(long long i) const { return sw ? sw[i] : (WT)1; }
 };
 
-// Rows of at most 32 entries: one warp, rank of each distinct key by a
-// shuffle compare against all others.
+// Rows of at most 32 entries: one warp, equal keys by a warp match; the
+// distinct keys keep the order of their first entries.
 template <typename WT>
 __global__ void __launch_bounds__(256) k_agg_small(AggArgs<WT> a, const int32_t *__restrict__ list)
 {
@@ -373,97 +370,19 @@ __global__ void __launch_bounds__(256) k_agg_small(AggArgs<WT> a, const int32_t 
         const WT sum = group_sum(m, wt);
         const bool head = valid && (__ffs(m) - 1 == lane);
         const unsigned hm = __ballot_sync(GALA_FULL_MASK, head);
-        int rank = 0;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            int kj = __shfl_sync(GALA_FULL_MASK, key, j);
-            rank += ((hm >> j) & 1u) && kj < key;
-        }
         if (head) {
-            a.tmp_nbr[a.tmp_off[c] + rank] = key;
-            a.tmp_w[a.tmp_off[c] + rank] = sum;
+            const long long o = a.tmp_off[c] + __popc(hm & lanemask_lt());
+            a.tmp_nbr[o] = key;
+            a.tmp_w[o] = sum;
         }
         if (lane == 0) a.kc[c] = __popc(hm);
     }
 }
 
-// Sort (key, val) pairs in shared memory by key, P a power of two.
-template <typename VT>
-__device__ __forceinline__ void bitonic_sort_smem(int *k, VT *v, int P)
-{
-    for (int size = 2; size <= P; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = threadIdx.x; t < (P >> 1); t += blockDim.x) {
-                int i = 2 * t - (t & (stride - 1));
-                int j = i + stride;
-                bool asc = (i & size) == 0;
-                int ki = k[i], kj = k[j];
-                if ((ki > kj) == asc) {
-                    k[i] = kj;
-                    k[j] = ki;
-                    VT tv = v[i];
-                    v[i] = v[j];
-                    v[j] = tv;
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
-// Insert stream entries [st, st + len) into a table (dense when keys is
-// null).  Returns this thread's count of newly created keys.  All threads of
-// the block call it.
 __device__ __forceinline__ bool add_was_zero(int *p, int v) { return atomicAdd(p, v) == 0; }
 __device__ __forceinline__ bool add_was_zero(long long *p, long long v)
 {
     return atomicAdd((unsigned long long *)p, (unsigned long long)v) == 0ull;
-}
-
-template <typename WT>
-__device__ __forceinline__ int agg_insert(const AggArgs<WT> &a, long long st, int len, int *keys, WT *vals, int T,
-                                          int lg)
-{
-    const int lane = threadIdx.x & 31;
-    int created = 0;
-    for (int b0 = 0; b0 < len; b0 += blockDim.x) {
-        const int j = b0 + threadIdx.x;
-        const bool valid = j < len;
-        int key = -1;
-        WT wt = 0;
-        if (valid) {
-            key = a.skey[st + j];
-            wt = a.w_at(st + j);
-        }
-        const unsigned m = __match_any_sync(GALA_FULL_MASK, key);
-        const WT sum = group_sum(m, wt);
-        if (valid && __ffs(m) - 1 == lane) {
-            if (!keys) {
-                created += add_was_zero(&vals[key], sum);
-            } else {
-                unsigned h = hash_slot(key, lg);
-                bool ok = false;
-                for (int p = 0; p < T; ++p) {
-                    int k = *(volatile int *)&keys[h];
-                    if (k == -1) {
-                        k = atomicCAS(&keys[h], -1, key);
-                        if (k == -1) {
-                            k = key;
-                            created++;
-                        }
-                    }
-                    if (k == key) {
-                        atomic_add_w(&vals[h], sum);
-                        ok = true;
-                        break;
-                    }
-                    h = (h + 1) & (unsigned)(T - 1);
-                }
-                if (!ok) atomicOr(&a.st->err, kErrHashOverflow);
-            }
-        }
-    }
-    return created;
 }
 
 // Add (key, w) to a table (dense when keys is null); returns 1 when this call
@@ -640,86 +559,20 @@ __global__ void __launch_bounds__(BLOCK) k_agg_mid_list(AggArgs<WT> a, const int
     }
 }
 
-// Rows of 33..kMid2Max entries: one CTA per community, shared-memory hash
-// table of TMAX slots, distinct keys sorted by a bitonic sort of LMAX slots.
-template <typename WT, int BLOCK, int TMAX, int LMAX>
-__global__ void __launch_bounds__(BLOCK) k_agg_mid(AggArgs<WT> a, const int32_t *__restrict__ list, int cls)
-{
-    extern __shared__ long long sm_ll[];
-    int *keys = (int *)sm_ll;
-    WT *vals = (WT *)(keys + TMAX);
-    int *lk = (int *)(vals + TMAX);
-    WT *lv = (WT *)(lk + LMAX);
-    __shared__ int s_k;
-    const int cnt = a.st->small_cnt[cls];
-    for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
-        const int c = list[i];
-        const long long st = a.medge[a.moff[c]];
-        const int E = (int)a.ec[c];
-        const int C = (int)a.st->ccount;
-        const int cap = E < C ? E : C;
-        int T = next_pow2_int(2LL * cap);
-        if (T < 64) T = 64;
-        if (T > TMAX) T = TMAX;
-        const int lg = __ffs(T) - 1;
-        for (int j = threadIdx.x; j < T; j += BLOCK) {
-            keys[j] = -1;
-            vals[j] = 0;
-        }
-        if (threadIdx.x == 0) s_k = 0;
-        __syncthreads();
-        agg_insert(a, st, E, keys, vals, T, lg);
-        __syncthreads();
-        for (int j = threadIdx.x; j < T; j += BLOCK) {
-            int kk = keys[j];
-            if (kk >= 0) {
-                int p = atomicAdd(&s_k, 1);
-                lk[p] = kk;
-                lv[p] = vals[j];
-            }
-        }
-        __syncthreads();
-        const int k = s_k;
-        const int P = next_pow2_int(k);
-        for (int j = k + threadIdx.x; j < P; j += BLOCK) {
-            lk[j] = 0x7fffffff;
-            lv[j] = 0;
-        }
-        __syncthreads();
-        bitonic_sort_smem(lk, lv, P);
-        const long long o = a.tmp_off[c];
-        for (int j = threadIdx.x; j < k; j += BLOCK) {
-            a.tmp_nbr[o + j] = lk[j];
-            a.tmp_w[o + j] = lv[j];
-        }
-        if (threadIdx.x == 0) a.kc[c] = k;
-        __syncthreads();
-    }
-}
-
 // ---- rows of more than kMid2Max entries --------------------------------
 
 struct BigArgs {
     const int32_t *__restrict__ list;  // class-3 communities
     long long *T;
     long long *chunks;
-    long long *tchunks;
     const long long *__restrict__ toff;
     const long long *__restrict__ coff;
-    const long long *__restrict__ tcoff;
     int32_t *mode;
     int32_t *work;
-    int32_t *twork;
-    int32_t *kdist;
     int32_t *cursor;
-    long long *gwords;
-    const long long *__restrict__ gofs;
     int32_t *pool;
     long long pool_half;  // keys at pool[0, half), values (WT, 8-byte aligned) from pool[half]
     long long work_cap;   // capacity of work
-    long long twork_cap;  // capacity of twork
-    unsigned *bits;       // bitmaps of the rows ranked by bitmap
-    unsigned *pref;       // exclusive prefix of their popcounts
 };
 
 // Long-row kernels run only while the tables fit their scratch.
@@ -741,13 +594,11 @@ __global__ void k_big_plan(AggArgs<WT> a, BigArgs b)
         b.T[i] = T;
         b.mode[i] = dense;
         b.chunks[i] = (E + kChunk - 1) / kChunk;
-        b.tchunks[i] = (T + kChunk - 1) / kChunk;
-        b.kdist[i] = 0;
         b.cursor[i] = 0;
     }
 }
 
-// toff[cnt] / coff[cnt] / tcoff[cnt] close the last segments; tables or
+// toff[cnt] / coff[cnt] close the last segments; tables or
 // chunk lists beyond their scratch set kErrCapacity, which stops the other
 // long-row kernels (the host reports it after the contraction).
 __global__ void k_big_tail(BigArgs b, DevStats *st)
@@ -755,9 +606,7 @@ __global__ void k_big_tail(BigArgs b, DevStats *st)
     const int cnt = st->small_cnt[kLongCls];
     ((long long *)b.toff)[cnt] = st->big_slots;
     ((long long *)b.coff)[cnt] = st->big_nwork;
-    ((long long *)b.tcoff)[cnt] = st->big_ntwork;
-    if (st->big_slots > b.pool_half || st->big_nwork > b.work_cap || st->big_ntwork > b.twork_cap)
-        st->err |= kErrCapacity;
+    if (st->big_slots > b.pool_half || st->big_nwork > b.work_cap) st->err |= kErrCapacity;
 }
 
 // Empty tables: keys -1, values 0, over the slots the plan counted.
@@ -774,8 +623,7 @@ __global__ void k_big_clear(BigArgs b, const DevStats *st)
     }
 }
 
-// stream chunk -> community and table chunk -> community, one warp per
-// community (list index)
+// stream chunk -> community, one warp per community (list index)
 template <typename WT>
 __global__ void k_big_work(AggArgs<WT> a, BigArgs b)
 {
@@ -784,11 +632,8 @@ __global__ void k_big_work(AggArgs<WT> a, BigArgs b)
     const int nw = (gridDim.x * blockDim.x) >> 5;
     const int cnt = big_off(a.st) ? 0 : a.st->small_cnt[kLongCls];
     for (int i = wg; i < cnt; i += nw) {
-        long long o = b.coff[i], k = b.coff[i + 1] - o;
+        const long long o = b.coff[i], k = b.coff[i + 1] - o;
         for (long long j = lane; j < k; j += 32) b.work[o + j] = i;
-        o = b.tcoff[i];
-        k = b.tcoff[i + 1] - o;
-        for (long long j = lane; j < k; j += 32) b.twork[o + j] = i;
     }
 }
 
@@ -809,7 +654,7 @@ constexpr size_t big_sm_smem()
     return (size_t)kSmT * (sizeof(WT) + sizeof(int) + sizeof(unsigned short));
 }
 template <typename WT>
-__global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b, int lists)
+__global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b)
 {
     const long long nwork = big_off(a.st) ? 0 : a.st->big_nwork;
     if (nwork <= blockIdx.x) return;
@@ -855,8 +700,8 @@ __global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b,
         }
         __syncthreads();
         const int n = s_n;
-        // the chunk's distinct keys go to the global table; with lists, the
-        // slots this chunk created are appended to the row's slot list (in the
+        // the chunk's distinct keys go to the global table; the slots this
+        // chunk created are appended to the row's slot list (in the
         // row's own tmp range), one counter add per chunk
         constexpr int kIt = kChunk / 512;
         int made[kIt];
@@ -895,12 +740,11 @@ __global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b,
                 red[q] = tot;
                 tot += t;
             }
-            if (tot) atomicAdd(&b.kdist[i], tot);
-            s_base = (lists && tot) ? atomicAdd(&b.cursor[i], tot) : 0;
+            s_base = tot ? atomicAdd(&b.cursor[i], tot) : 0;
             s_n = 0;
         }
         __syncthreads();
-        if (lists && mask) {
+        if (mask) {
             int p = s_base + red[wid] + incl - mine;
             const long long o = a.tmp_off[c];
 #pragma unroll
@@ -908,21 +752,6 @@ __global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b,
                 if (mask & (1u << it)) a.tmp_nbr[o + p++] = made[it];
         }
         __syncthreads();
-    }
-}
-
-// Rows with more distinct neighbours than a shared-memory sort holds are
-// ranked by a bitmap over all communities: words per row (0 for the others);
-// every class-3 row gets its final length here.
-template <typename WT>
-__global__ void k_big_mark(AggArgs<WT> a, BigArgs b, int sort_rows)
-{
-    const int cnt = a.st->small_cnt[kLongCls];
-    const long long words = (a.st->ccount + 31) >> 5;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-        const int k = b.kdist[i];
-        b.gwords[i] = (sort_rows && k > kSortMax) ? words : 0;
-        a.kc[b.list[i]] = k;
     }
 }
 
@@ -1572,106 +1401,276 @@ __global__ void __launch_bounds__(512) k_rad_agg(AggArgs<WT> a, BigArgs b, int32
     }
 }
 
-// Table chunks: distinct entries of sorted rows go to the row unsorted
-// (atomic cursor); rows ranked by bitmap set their bits.
-template <typename WT>
-__global__ void __launch_bounds__(256) k_big_collect(AggArgs<WT> a, BigArgs b, long long ntwork)
+// ---- sorted rows ---------------------------------------------------------
+//
+// gala_contract_device (and sorted_levels) return every row in ascending
+// neighbour id.  The rows come out of the aggregation in any order; this stage
+// takes the place of the compaction and writes every row sorted to its final
+// place.  A warp sorts up to 512 (key, sum) pairs in its registers, lane l
+// holding the positions [l R, l R + R), so that compares at distances under R
+// stay inside a lane; the pieces of longer rows, up to kSortMax pairs, are
+// sorted the same way (512 keys with their places) and merged in shared memory
+// by rank (a key's place in the merged run is its own plus the count of
+// smaller keys in the other run: binary searches, one barrier a round); longer
+// rows are ranked by a bitmap over the communities.  Bound by the issue of the
+// register compares and, in the CTA kernels, by latency; the classes run side
+// by side on the auxiliary streams.  Contraction of a 17M-entry R-MAT graph:
+// 2.26 ms with the sort inside the aggregation (a CTA per row, a barrier per
+// compare distance), 1.04 ms so.
+
+// Compare distances stride, stride / 2, ... 1 (stride < 32 R) of a bitonic
+// sort of 32 R pairs at step `size`; (lane, r) holds position lane R + r.
+template <typename WT, int R>
+__device__ __forceinline__ void bitonic_regs(int (&k)[R], WT (&v)[R], int size, int stride)
 {
-    for (long long wi = blockIdx.x; wi < ntwork; wi += gridDim.x) {
-        const int i = b.twork[wi];
-        const long long j0 = (wi - b.tcoff[i]) * kChunk;
-        const long long T = b.T[i];
-        const int c = b.list[i];
-        const WT *vals = big_vals<WT>(b, i);
-        const int *keys = b.pool + b.toff[i];
-        const bool dense = b.mode[i];
-        const bool bitmap = b.gwords[i] > 0;
-        const long long o = a.tmp_off[c];
-        unsigned *bits = bitmap ? b.bits + b.gofs[i] : nullptr;
-        for (long long s0 = j0; s0 < j0 + kChunk && s0 < T; s0 += blockDim.x) {
-            const long long s = s0 + threadIdx.x;
-            int key = -1;
-            WT val = 0;
-            if (s < T && s < j0 + kChunk) {
-                val = vals[s];
-                key = dense ? (val > 0 ? (int)s : -1) : keys[s];
+    const int lane = threadIdx.x & 31;
+    for (; stride >= R; stride >>= 1) {
+        const int ls = stride / R;
+        const bool lower = (lane & ls) == 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int ok = __shfl_xor_sync(GALA_FULL_MASK, k[r], ls);
+            const WT ov = __shfl_xor_sync(GALA_FULL_MASK, v[r], ls);
+            const bool asc = ((lane * R + r) & size) == 0;
+            if ((ok < k[r]) == (lower == asc)) {  // equal keys are padding
+                k[r] = ok;
+                v[r] = ov;
             }
-            const bool occ = key >= 0;
-            if (bitmap) {
-                if (occ) atomicOr(&bits[key >> 5], 1u << (key & 31));
-            } else {
-                const unsigned bal = __ballot_sync(GALA_FULL_MASK, occ);
-                if (bal) {
-                    const int lane = threadIdx.x & 31, leader = __ffs(bal) - 1;
-                    int base = 0;
-                    if (lane == leader) base = atomicAdd(&b.cursor[i], __popc(bal));
-                    base = __shfl_sync(GALA_FULL_MASK, base, leader);
-                    if (occ) {
-                        const long long p = o + base + __popc(bal & lanemask_lt());
-                        a.tmp_nbr[p] = key;
-                        a.tmp_w[p] = val;
-                    }
+        }
+    }
+#pragma unroll
+    for (int s = R / 2; s >= 1; s >>= 1) {
+        if (s > stride) continue;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (r & s) continue;
+            const bool asc = ((lane * R + r) & size) == 0;
+            if ((k[r] > k[r + s]) == asc) {
+                const int tk = k[r];
+                const WT tv = v[r];
+                k[r] = k[r + s];
+                v[r] = v[r + s];
+                k[r + s] = tk;
+                v[r + s] = tv;
+            }
+        }
+    }
+}
+
+// Keys [q0, q0 + 32 R) of a row of n (past the end: INT_MAX), loaded in any
+// order with their values val(q), sorted ascending.
+template <int R, typename WT, typename Val>
+__device__ __forceinline__ void sort_regs(const int32_t *nbr, int q0, int n, int (&k)[R], WT (&v)[R], Val val)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int q = q0 + r * 32 + lane;
+        k[r] = q < n ? nbr[q] : 0x7fffffff;
+        v[r] = q < n ? val(q) : (WT)0;
+    }
+    for (int size = 2; size <= 32 * R; size <<= 1) bitonic_regs<WT, R>(k, v, size, size >> 1);
+}
+
+template <typename WT>
+struct SortArgs {
+    const long long *__restrict__ tmp_off;
+    const int32_t *tmp_nbr;
+    const WT *tmp_w;
+    const int32_t *__restrict__ kc;
+    const int64_t *__restrict__ new_offs;
+    int32_t *out_nbr;
+    WT *out_w;
+    WT *self_out;      // null: not wanted
+    int32_t *list;     // rows by kSortCls class, lstride apart
+    long long lstride;
+    DevStats *st;
+    __device__ __forceinline__ void put(int c, long long o, int key, WT w) const
+    {
+        out_nbr[o] = key;
+        out_w[o] = w;
+        if (self_out && key == c) self_out[c] = w;
+    }
+};
+constexpr int kSortSmall = 128;  // pairs a warp sorts at high occupancy
+constexpr int kSortWarp = 512;   // pairs a warp sorts
+constexpr int kSortCta1 = 1024;  // pairs a 64-thread CTA sorts
+constexpr int kSortCta2 = 4096;  // pairs a 256-thread CTA sorts; above: 1024 threads
+constexpr int kSortLists = 5;    // classes of rows of more than kSortSmall pairs
+
+template <typename WT, int R>
+__device__ __forceinline__ void sort_row_warp(const SortArgs<WT> &a, int c, int n)
+{
+    const int lane = threadIdx.x & 31;
+    const long long t = a.tmp_off[c], o = a.new_offs[c];
+    int k[R];
+    WT v[R];
+    const WT *w = a.tmp_w + t;
+    sort_regs<R>(a.tmp_nbr + t, 0, n, k, v, [=](int q) { return w[q]; });
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int q = lane * R + r;
+        if (q < n) a.put(c, o + q, k[r], v[r]);
+    }
+}
+
+// Rows of more than kSortSmall pairs, listed by class.
+template <typename WT>
+__global__ void __launch_bounds__(256) k_sort_list(SortArgs<WT> a)
+{
+    const int C = (int)a.st->ccount;
+    const int stride = gridDim.x * blockDim.x;
+    for (int c0 = blockIdx.x * blockDim.x; c0 < C; c0 += stride) {  // block-uniform
+        const int c = c0 + threadIdx.x;
+        const int n = c < C ? a.kc[c] : 0;
+        const int cls = n <= kSortSmall  ? -1
+                        : n <= kSortWarp ? 0
+                        : n <= kSortCta1 ? 1
+                        : n <= kSortCta2 ? 2
+                        : n <= kSortMax  ? 3
+                                         : 4;
+#pragma unroll
+        for (int k = 0; k < kSortLists; ++k) warp_append(cls == k, c, a.list + k * a.lstride, &a.st->sort_cnt[k]);
+    }
+}
+
+// One warp per row of up to kSortSmall pairs.
+template <typename WT>
+__global__ void __launch_bounds__(256) k_sort_small(SortArgs<WT> a)
+{
+    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    const int C = (int)a.st->ccount;
+    for (int c = wg; c < C; c += nw) {
+        const int n = a.kc[c];
+        if (n <= 0 || n > kSortSmall) continue;
+        if (n <= 32)
+            sort_row_warp<WT, 1>(a, c, n);
+        else if (n <= 64)
+            sort_row_warp<WT, 2>(a, c, n);
+        else
+            sort_row_warp<WT, 4>(a, c, n);
+    }
+}
+
+// One warp per row of kSortSmall + 1 ... kSortWarp pairs.
+template <typename WT>
+__global__ void __launch_bounds__(128) k_sort_warp(SortArgs<WT> a)
+{
+    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    const int cnt = a.st->sort_cnt[0];
+    for (int i = wg; i < cnt; i += nw) {
+        const int c = a.list[i], n = a.kc[c];
+        if (n <= 256)
+            sort_row_warp<WT, 8>(a, c, n);
+        else
+            sort_row_warp<WT, 16>(a, c, n);
+    }
+}
+
+// One CTA per row of up to MAX pairs: keys and their places in two buffers.
+constexpr size_t sort_cta_smem(int max) { return (size_t)max * 2 * (sizeof(int) + sizeof(unsigned short)); }
+template <typename WT, int BLOCK, int MAX>
+__global__ void __launch_bounds__(BLOCK) k_sort_cta(SortArgs<WT> a, int cls)
+{
+    extern __shared__ int sort_sm[];
+    constexpr int R = 16, N = 32 * R;
+    static_assert(MAX <= 65536, "16-bit places");
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int cnt = a.st->sort_cnt[cls];
+    for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
+        int *src = sort_sm, *dst = sort_sm + MAX;
+        unsigned short *sq = (unsigned short *)(sort_sm + 2 * MAX), *dq = sq + MAX;
+        const int c = a.list[cls * a.lstride + i];
+        const int n = a.kc[c];
+        const long long t = a.tmp_off[c], o = a.new_offs[c];
+        for (int q0 = wid * N; q0 < n; q0 += BLOCK / 32 * N) {
+            int k[R], q[R];
+            sort_regs<R>(a.tmp_nbr + t, q0, n, k, q, [](int x) { return x; });
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int e = q0 + lane * R + r;
+                if (e < n) {
+                    src[e] = k[r];
+                    sq[e] = (unsigned short)q[r];
                 }
             }
         }
+        for (int run = N; run < n; run <<= 1) {
+            __syncthreads();
+            constexpr int U = 4;  // searches in flight per thread
+            for (int e0 = threadIdx.x; e0 < n; e0 += U * BLOCK) {
+                int key[U], lo[U], hi[U], sb[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int e = e0 + u * BLOCK;
+                    key[u] = e < n ? src[e] : 0;
+                    sb[u] = e < n ? ((e / run) ^ 1) * run : n;  // the other run [sb, sb + run)
+                    lo[u] = min(sb[u], n);
+                    hi[u] = min(sb[u] + run, n);
+                }
+                for (int len = run; len > 0; len >>= 1) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (lo[u] < hi[u]) {
+                            const int m = (lo[u] + hi[u]) >> 1;
+                            if (src[m] < key[u])
+                                lo[u] = m + 1;
+                            else
+                                hi[u] = m;
+                        }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int e = e0 + u * BLOCK;
+                    if (e < n) {
+                        // pair start + own place in its run + smaller keys of the other run
+                        const int p = (e / (2 * run)) * (2 * run) + (e & (run - 1)) + (lo[u] - min(sb[u], n));
+                        dst[p] = key[u];
+                        dq[p] = sq[e];
+                    }
+                }
+            }
+            int *ts = src;
+            src = dst;
+            dst = ts;
+            unsigned short *tq = sq;
+            sq = dq;
+            dq = tq;
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < n; q += BLOCK) a.put(c, o + q, src[q], a.tmp_w[t + sq[q]]);
+        __syncthreads();
     }
 }
 
-// Table chunks of bitmap-ranked rows: rank = popcounts of the row's bitmap
-// before the key.
+// Rows of more than kSortMax pairs (blockIdx.y): every key sets its bit in the
+// row's bitmap of `words` words; a key's rank is the count of set bits before
+// it (pref: exclusive prefix of the words' popcounts over all rows).
 template <typename WT>
-__global__ void __launch_bounds__(256) k_big_rank(AggArgs<WT> a, BigArgs b, long long ntwork)
+__global__ void __launch_bounds__(256) k_sort_mark(SortArgs<WT> a, unsigned *bits, long long words)
 {
-    for (long long wi = blockIdx.x; wi < ntwork; wi += gridDim.x) {
-        const int i = b.twork[wi];
-        if (b.gwords[i] == 0) continue;
-        const long long j0 = (wi - b.tcoff[i]) * kChunk;
-        const long long T = b.T[i];
-        const int c = b.list[i];
-        const WT *vals = big_vals<WT>(b, i);
-        const int *keys = b.pool + b.toff[i];
-        const bool dense = b.mode[i];
-        const long long o = a.tmp_off[c];
-        const unsigned *bits = b.bits + b.gofs[i];
-        const unsigned *pref = b.pref + b.gofs[i];
-        const unsigned base = pref[0];
-        for (long long s = j0 + threadIdx.x; s < j0 + kChunk && s < T; s += blockDim.x) {
-            const WT val = vals[s];
-            const int key = dense ? (val > 0 ? (int)s : -1) : keys[s];
-            if (key < 0) continue;
-            const unsigned r = pref[key >> 5] - base + __popc(bits[key >> 5] & ((1u << (key & 31)) - 1u));
-            a.tmp_nbr[o + r] = key;
-            a.tmp_w[o + r] = val;
-        }
-    }
+    const int c = a.list[(kSortLists - 1) * a.lstride + blockIdx.y];
+    const int n = a.kc[c];
+    const int32_t *nbr = a.tmp_nbr + a.tmp_off[c];
+    unsigned *b = bits + blockIdx.y * words;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+        atomicOr(&b[nbr[q] >> 5], 1u << (nbr[q] & 31));
 }
-
-// Rows with at most kSortMax distinct neighbours: one CTA sorts the row in
-// shared memory.
 template <typename WT>
-__global__ void __launch_bounds__(1024) k_big_sort(AggArgs<WT> a, BigArgs b)
+__global__ void __launch_bounds__(256) k_sort_place(SortArgs<WT> a, const unsigned *__restrict__ bits,
+                                                    const unsigned *__restrict__ pref, long long words)
 {
-    extern __shared__ long long sm_ll[];
-    int *lk = (int *)sm_ll;
-    WT *lv = (WT *)(lk + kSortMax);
-    const int cnt = a.st->small_cnt[kLongCls];
-    for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
-        if (b.gwords[i] != 0) continue;
-        const int c = b.list[i];
-        const int k = b.kdist[i];
-        const long long o = a.tmp_off[c];
-        const int P = next_pow2_int(k);
-        for (int j = threadIdx.x; j < P; j += blockDim.x) {
-            lk[j] = j < k ? a.tmp_nbr[o + j] : 0x7fffffff;
-            lv[j] = j < k ? a.tmp_w[o + j] : 0;
-        }
-        __syncthreads();
-        bitonic_sort_smem(lk, lv, P);
-        for (int j = threadIdx.x; j < k; j += blockDim.x) {
-            a.tmp_nbr[o + j] = lk[j];
-            a.tmp_w[o + j] = lv[j];
-        }
-        __syncthreads();
+    const int c = a.list[(kSortLists - 1) * a.lstride + blockIdx.y];
+    const int n = a.kc[c];
+    const long long t = a.tmp_off[c], o = a.new_offs[c];
+    const unsigned *b = bits + blockIdx.y * words, *p = pref + blockIdx.y * words;
+    const unsigned first = p[0];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const int key = a.tmp_nbr[t + q];
+        const unsigned r = p[key >> 5] - first + __popc(b[key >> 5] & ((1u << (key & 31)) - 1u));
+        a.put(c, o + r, key, a.tmp_w[t + q]);
     }
 }
 
@@ -1766,34 +1765,9 @@ __global__ void k_contract_reset(DevStats *st)
     st->err = 0;
     st->ccount = 0;
     st->new_entries = 0;
-    st->big_slots = st->big_nwork = st->big_ntwork = st->big_lwork = 0;
+    st->big_slots = st->big_nwork = st->big_lwork = 0;
     st->rad_nb = st->rad_nitems = st->rad_nacc = st->rad_next = 0;
-}
-
-// Shared memory of the table kernels: int keys plus WT values per slot.
-template <typename WT>
-constexpr size_t mid1_smem()
-{
-    return (1024 + kMid1Max) * (sizeof(int) + sizeof(WT));
-}
-template <typename WT>
-constexpr size_t mid2_smem()
-{
-    return (8192 + kMid2Max) * (sizeof(int) + sizeof(WT));
-}
-template <typename WT>
-constexpr size_t sort_smem()
-{
-    return kSortMax * (sizeof(int) + sizeof(WT));
-}
-
-template <typename WT>
-static void configure_mid()
-{
-    cudaFuncSetAttribute(k_agg_mid<WT, 128, 1024, kMid1Max>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)mid1_smem<WT>());
-    cudaFuncSetAttribute(k_agg_mid<WT, 256, 8192, kMid2Max>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)mid2_smem<WT>());
+    for (int k = 0; k < kSortLists; ++k) st->sort_cnt[k] = 0;
 }
 
 template <typename WT>
@@ -1805,9 +1779,10 @@ constexpr size_t list_smem(int tmax)
 template <typename WT>
 static void configure_t()
 {
-    configure_mid<WT>();
-
-    cudaFuncSetAttribute(k_big_sort<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem<WT>());
+    cudaFuncSetAttribute(k_sort_cta<WT, 256, kSortCta2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sort_cta_smem(kSortCta2));
+    cudaFuncSetAttribute(k_sort_cta<WT, 1024, kSortMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sort_cta_smem(kSortMax));
     cudaFuncSetAttribute(k_big_insert_sm<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)big_sm_smem<WT>());
     cudaFuncSetAttribute(k_rad_combine<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rad_combine_smem<WT>());
     cudaFuncSetAttribute(k_rad_agg<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rad_agg_smem<WT>());
@@ -1883,10 +1858,6 @@ static long long big_pool_half(const ContractBuffers &b)
     return (b.big_pool_ints / (1 + vints)) & ~1LL;  // even: the values start 8-byte aligned
 }
 
-// Rows longer than kMid3Max entries (kMid2Max when sorted; class kLongCls),
-// at most cnt_max of them.  Counts, table sizes and the scratch check stay on
-// the device; only sorted rows read their bitmap sizes on the host.  Returns
-// false on failure.
 // Whether the key-range path fits the pool for any level of n rows and E
 // entries (C <= n, every long row longer than kMid3Max entries).
 template <typename WT>
@@ -1900,9 +1871,11 @@ static bool rad_fits(long long n, long long E, const ContractBuffers &b)
     return rad_layout(cnt, E / kChunk + cnt, nb, vints).end <= b.big_pool_ints;
 }
 
+// Rows longer than kMid3Max entries (class kLongCls), at most cnt_max of
+// them.  Counts, table sizes and the scratch check stay on the device.
 template <typename WT>
-static bool contract_long_rows(const AggArgs<WT> &a, ContractBuffers &b, const int32_t *list, int cnt_max,
-                               cudaStream_t st, gala_status *status, bool sort_rows, long long n, long long E)
+static void contract_long_rows(const AggArgs<WT> &a, ContractBuffers &b, const int32_t *list, int cnt_max,
+                               cudaStream_t st, long long n, long long E)
 {
     const int nsm = sm_count();
     const int cap = nsm * 8;
@@ -1912,22 +1885,15 @@ static bool contract_long_rows(const AggArgs<WT> &a, ContractBuffers &b, const i
     ba.list = list;
     ba.T = b.big_T;
     ba.chunks = b.big_chunks;
-    ba.tchunks = b.big_tchunks;
     ba.toff = b.big_toff;
     ba.coff = b.big_coff;
-    ba.tcoff = b.big_tcoff;
     ba.mode = b.big_mode;
     ba.work = b.big_work;
-    ba.twork = b.big_twork;
-    ba.kdist = b.big_kdist;
     ba.cursor = b.big_cursor;
-    ba.gwords = b.big_gwords;
-    ba.gofs = b.big_gofs;
     ba.pool = b.big_pool;
     ba.pool_half = big_pool_half<WT>(b);
     ba.work_cap = b.big_work_cap;
-    ba.twork_cap = b.big_twork_cap;
-    if (!sort_rows && b.long_rows_mode == 0 && rad_fits<WT>(n, E, b)) {
+    if (b.long_rows_mode == 0 && rad_fits<WT>(n, E, b)) {
         constexpr long long vints = sizeof(WT) / sizeof(int32_t);
         k_rad_plan<WT><<<grid_cap(cnt_max, 256, cap), 256, 0, st>>>(a, ba, b.big_pool, b.big_pool_ints);
         exclusive_scan_dev(b.big_chunks, b.big_coff, cnt_max, dcnt, OpIdentity(), b.scan_partial, &ds->big_nwork, st,
@@ -1941,69 +1907,32 @@ static bool contract_long_rows(const AggArgs<WT> &a, ContractBuffers &b, const i
             a, ba, b.big_pool, b.stream_key, (const WT *)b.stream_w, vints);
         k_big_len<WT><<<grid_cap(cnt_max, 256, cap), 256, 0, st>>>(a, ba);
         note_launch(6);
-        return true;
+        return;
     }
     k_big_plan<WT><<<grid_cap(cnt_max, 256, cap), 256, 0, st>>>(a, ba);
     exclusive_scan_dev(b.big_T, b.big_toff, cnt_max, dcnt, OpIdentity(), b.scan_partial, &ds->big_slots, st,
                        &ds->err);
     exclusive_scan_dev(b.big_chunks, b.big_coff, cnt_max, dcnt, OpIdentity(), b.scan_partial, &ds->big_nwork, st,
                        &ds->err);
-    exclusive_scan_dev(b.big_tchunks, b.big_tcoff, cnt_max, dcnt, OpIdentity(), b.scan_partial, &ds->big_ntwork,
-                       st, &ds->err);
     k_big_tail<<<1, 1, 0, st>>>(ba, ds);
     k_big_clear<WT><<<cap, 256, 0, st>>>(ba, ds);
     k_big_work<WT><<<grid_cap((long long)cnt_max * 32, 256, cap), 256, 0, st>>>(a, ba);
-    k_big_insert_sm<WT><<<nsm * 2, 512, big_sm_smem<WT>(), st>>>(a, ba, sort_rows ? 0 : 1);
+    k_big_insert_sm<WT><<<nsm * 2, 512, big_sm_smem<WT>(), st>>>(a, ba);
     note_launch(5);
-    if (!sort_rows) {
-        // rows in table order: collect from the slot lists, no table scans
-        long long *lch = b.big_tchunks, *lcoff = b.big_tcoff;
-        k_big_lchunks<<<grid_cap(cnt_max, 256, cap), 256, 0, st>>>(ba.cursor, ds, lch);
-        exclusive_scan_dev(lch, lcoff, cnt_max, dcnt, OpIdentity(), b.scan_partial, &ds->big_lwork, st, &ds->err);
-        k_big_collect_list<WT><<<nsm * 8, 256, 0, st>>>(a, ba, lcoff, &ds->big_lwork);
-        k_big_len<WT><<<grid_cap(cnt_max, 256, cap), 256, 0, st>>>(a, ba);
-        note_launch(3);
-        return true;
-    }
-    // sorted rows: the bitmap sizes come back to the host
-    DevStats hs;
-    if (!read_stats(&hs, ds, st, status, "contraction: long rows")) return false;
-    const int cnt3 = hs.small_cnt[kLongCls];
-    if (cnt3 == 0 || (hs.err & kErrCapacity)) return true;  // a capacity error is reported at the end
-    const long long ntwork = hs.big_ntwork;
-    k_big_mark<WT><<<grid_cap(cnt3, 256, cap), 256, 0, st>>>(a, ba, 1);
-    exclusive_scan(b.big_gwords, b.big_gofs, cnt3, OpIdentity(), b.scan_partial, &ds->total, st, &ds->err);
-    note_launch(1);
-    if (!read_stats(&hs, ds, st, status, "contraction: long-row bitmaps")) return false;
-    const long long words = hs.total;
-    if (2 * words > b.big_bitmap_words) {
-        set_error("contraction: %lld bitmap words needed, scratch holds %lld", 2 * words, b.big_bitmap_words);
-        *status = GALA_ERR_CAPACITY;
-        return false;
-    }
-    ba.bits = (unsigned *)b.big_bitmap;
-    ba.pref = (unsigned *)b.big_bitmap + words;
-    if (words > 0) cudaMemsetAsync(ba.bits, 0, (size_t)words * sizeof(unsigned), st);
-    const int tgrid = (int)(ntwork < nsm * 8 ? ntwork : nsm * 8);
-    if (tgrid > 0) {
-        k_big_collect<WT><<<tgrid, 256, 0, st>>>(a, ba, ntwork);
-        note_launch(1);
-    }
-    if (words > 0 && tgrid > 0) {
-        exclusive_scan(ba.bits, ba.pref, words, OpPopc(), b.scan_partial, &ds->total, st, &ds->err);
-        k_big_rank<WT><<<tgrid, 256, 0, st>>>(a, ba, ntwork);
-        note_launch(1);
-    }
-    k_big_sort<WT><<<cnt3 < nsm * 2 ? cnt3 : nsm * 2, 1024, sort_smem<WT>(), st>>>(a, ba);
-    note_launch(1);
-    return true;
+    // collect from the slot lists, no table scans
+    long long *lch = b.big_tchunks, *lcoff = b.big_tcoff;
+    k_big_lchunks<<<grid_cap(cnt_max, 256, cap), 256, 0, st>>>(ba.cursor, ds, lch);
+    exclusive_scan_dev(lch, lcoff, cnt_max, dcnt, OpIdentity(), b.scan_partial, &ds->big_lwork, st, &ds->err);
+    k_big_collect_list<WT><<<nsm * 8, 256, 0, st>>>(a, ba, lcoff, &ds->big_lwork);
+    k_big_len<WT><<<grid_cap(cnt_max, 256, cap), 256, 0, st>>>(a, ba);
+    note_launch(3);
 }
 
 // Returns the community count C (>= 1) or -1 on failure (*status set).
 // new_offs receives C+1 offsets (leading 0).  orig_map (length n_orig) is
 // composed with the new labels.  C, the size classes and the new entry count
-// stay on the device: the host reads them once, after the compaction (and,
-// for sorted long rows, once more for their bitmap sizes).
+// stay on the device: the host reads them once, after the compaction (sorted
+// rows of more than kSortMax pairs are ranked after that read).
 template <typename WT>
 static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers &b, int64_t *new_offs,
                       int32_t *new_nbr, WT *new_w, int32_t *orig_map, int32_t n_orig, int64_t *new_E,
@@ -2068,7 +1997,7 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
         }
         note_launch(1);
     }
-    k_classify<<<grid_cap(n, 256, cap), 256, 0, st>>>(b.ec, b.cls_list, n, b.kc, ds, sort_rows ? 1 : 0);
+    k_classify<<<grid_cap(n, 256, cap), 256, 0, st>>>(b.ec, b.cls_list, n, b.kc, ds);
     exclusive_scan_dev(b.ec, b.tmp_off, n, dC, OpCapDev{dC}, b.scan_partial, &ds->total, st, &ds->err);
     note_launch(1);
 
@@ -2089,9 +2018,8 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
         const long long c = E / min_entries;
         return (int)(c < n ? c : n);
     };
-    const int n_small = most(1), n_warp = sort_rows ? 0 : most(kSmallMax + 1);
-    const int n_mid1 = most(sort_rows ? kSmallMax + 1 : kWarpAggMax + 1), n_mid2 = most(kMid1Max + 1);
-    const int n_mid3 = sort_rows ? 0 : most(kMid2Max + 1), n_long = most((sort_rows ? kMid2Max : kMid3Max) + 1);
+    const int n_small = most(1), n_warp = most(kSmallMax + 1), n_mid1 = most(kWarpAggMax + 1);
+    const int n_mid2 = most(kMid1Max + 1), n_mid3 = most(kMid2Max + 1), n_long = most(kMid3Max + 1);
     // The classes are independent (disjoint tmp ranges and kc entries): with
     // auxiliary streams they aggregate concurrently, the long rows (the
     // longest chain of launches) first.
@@ -2102,35 +2030,27 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
         cs[i] = par ? b.aux[i] : st;
         if (par) cudaStreamWaitEvent(cs[i], b.fork_ev, 0);
     }
-    bool ok = n_long == 0 ||
-              contract_long_rows(a, b, b.cls_list + (long long)kLongCls * n, n_long, cs[3], status, sort_rows, n, E);
-    if (ok && n_mid2 > 0) {
+    if (n_long > 0) contract_long_rows(a, b, b.cls_list + (long long)kLongCls * n, n_long, cs[3], n, E);
+    if (n_mid2 > 0) {
         const int grid = n_mid2 < nsm * 2 ? n_mid2 : nsm * 2;
-        if (sort_rows)
-            k_agg_mid<WT, 256, 8192, kMid2Max><<<grid, 256, mid2_smem<WT>(), cs[2]>>>(a, b.cls_list + 2LL * n, 2);
-        else
-            k_agg_mid_list<WT, 1024, 8192><<<grid, 1024, list_smem<WT>(8192), cs[2]>>>(a, b.cls_list + 2LL * n, 2);
+        k_agg_mid_list<WT, 1024, 8192><<<grid, 1024, list_smem<WT>(8192), cs[2]>>>(a, b.cls_list + 2LL * n, 2);
         note_launch(1);
     }
-    if (ok && n_mid3 > 0) {  // 4097-8192 entries, rows in table order
+    if (n_mid3 > 0) {  // 4097-8192 entries
         const int grid = n_mid3 < nsm ? n_mid3 : nsm;
         k_agg_mid_list<WT, 1024, 16384><<<grid, 1024, list_smem<WT>(16384), cs[2]>>>(a, b.cls_list + 3LL * n, 3);
         note_launch(1);
     }
-    if (ok && n_mid1 > 0) {
+    if (n_mid1 > 0) {
         const int grid = n_mid1 < nsm * 16 ? n_mid1 : nsm * 16;
-        if (sort_rows)
-            k_agg_mid<WT, 128, 1024, kMid1Max><<<grid, 128, mid1_smem<WT>(), cs[1]>>>(a, b.cls_list + (long long)n, 1);
-        else
-            k_agg_mid_list<WT, 128, 1024><<<grid, 128, list_smem<WT>(1024), cs[1]>>>(a, b.cls_list + (long long)n,
-                                                                                      1);
+        k_agg_mid_list<WT, 128, 1024><<<grid, 128, list_smem<WT>(1024), cs[1]>>>(a, b.cls_list + (long long)n, 1);
         note_launch(1);
     }
-    if (ok && n_small > 0) {
+    if (n_small > 0) {
         k_agg_small<WT><<<grid_cap((long long)n_small * 32, 256, cap), 256, 0, cs[0]>>>(a, b.cls_list);
         note_launch(1);
     }
-    if (ok && n_warp > 0) {
+    if (n_warp > 0) {
         k_agg_warp_list<WT><<<grid_cap((long long)n_warp * 32, 256, cap), 256, 0, cs[0]>>>(
             a, b.cls_list + (long long)kWarpCls * n);
         note_launch(1);
@@ -2140,11 +2060,48 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
             cudaEventRecord(b.join_ev[i], cs[i]);
             cudaStreamWaitEvent(st, b.join_ev[i], 0);
         }
-    if (!ok) return -1;
     exclusive_scan_dev(b.kc, new_offs, n, dC, OpIdentity(), b.scan_partial, &ds->new_entries, st, &ds->err);
     k_set_last_offset<<<1, 1, 0, st>>>(new_offs, ds);
     note_launch(1);
-    if (E > 0) {  // the new level has at most E entries
+    SortArgs<WT> sa{b.tmp_off,      b.tmp_nbr,  (const WT *)b.tmp_w, b.kc, new_offs, new_nbr, new_w,
+                    (WT *)nli.self, b.cls_list, n,                   ds};
+    if (E > 0 && sort_rows) {
+        // the longest rows first; rows of a class: at most E over its shortest
+        k_sort_list<WT><<<grid_cap(n, 256, cap), 256, 0, st>>>(sa);
+        const int n_warp = most(kSortSmall + 1), n_cta1 = most(kSortWarp + 1), n_cta2 = most(kSortCta1 + 1),
+                  n_cta3 = most(kSortCta2 + 1);
+        note_launch(1);
+        if (par) {
+            cudaEventRecord(b.fork_ev, st);
+            for (int i = 0; i < ContractBuffers::kAux; ++i) cudaStreamWaitEvent(cs[i], b.fork_ev, 0);
+        }
+        if (n_cta3 > 0) {
+            k_sort_cta<WT, 1024, kSortMax><<<std::min(n_cta3, nsm), 1024, sort_cta_smem(kSortMax), cs[3]>>>(sa, 3);
+            note_launch(1);
+        }
+        if (n_cta2 > 0) {
+            const int g = resident_grid(k_sort_cta<WT, 256, kSortCta2>, 256, sort_cta_smem(kSortCta2));
+            k_sort_cta<WT, 256, kSortCta2><<<std::min(n_cta2, g), 256, sort_cta_smem(kSortCta2), cs[2]>>>(sa, 2);
+            note_launch(1);
+        }
+        if (n_cta1 > 0) {
+            const int g = resident_grid(k_sort_cta<WT, 64, kSortCta1>, 64, sort_cta_smem(kSortCta1));
+            k_sort_cta<WT, 64, kSortCta1><<<std::min(n_cta1, g), 64, sort_cta_smem(kSortCta1), cs[1]>>>(sa, 1);
+            note_launch(1);
+        }
+        if (n_warp > 0) {
+            const int g = resident_grid(k_sort_warp<WT>, 128);
+            k_sort_warp<WT><<<std::min(grid_cap((long long)n_warp * 32, 128, g), g), 128, 0, cs[0]>>>(sa);
+            note_launch(1);
+        }
+        k_sort_small<WT><<<grid_cap((long long)n * 32, 256, cap), 256, 0, cs[0]>>>(sa);
+        note_launch(1);
+        if (par)
+            for (int i = 0; i < ContractBuffers::kAux; ++i) {
+                cudaEventRecord(b.join_ev[i], cs[i]);
+                cudaStreamWaitEvent(st, b.join_ev[i], 0);
+            }
+    } else if (E > 0) {  // the new level has at most E entries
         build_walk_list(new_offs, n, 0, b, st, ShiftCompact{b.tmp_off}, dC, &ds->new_entries);
         // a second wave of blocks measured faster here than a resident grid
         k_compact<WT><<<grid_cap((E + kRangeEntries - 1) / kRangeEntries * 32, 256, cap), 256, 0, st>>>(
@@ -2154,9 +2111,8 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
     }
     if (!read_stats(&hs, ds, st, status, "contraction")) return -1;
     if (hs.err & kErrCapacity) {
-        set_error("contraction: long rows need %lld table slots / %lld + %lld chunks, scratch holds %lld / %lld / "
-                  "%lld",
-                  hs.big_slots, hs.big_nwork, hs.big_ntwork, big_pool_half<WT>(b), b.big_work_cap, b.big_twork_cap);
+        set_error("contraction: long rows need %lld table slots / %lld chunks, scratch holds %lld / %lld", hs.big_slots,
+                  hs.big_nwork, big_pool_half<WT>(b), b.big_work_cap);
         *status = GALA_ERR_CAPACITY;
         return -1;
     }
@@ -2166,6 +2122,34 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
         return -1;
     }
     *new_E = hs.new_entries;
+    if (const int rows = sort_rows ? hs.sort_cnt[kSortLists - 1] : 0) {
+        const long long words = (hs.ccount + 31) >> 5, all = rows * words;
+        if (2 * all > b.big_bitmap_words) {
+            set_error("contraction: %lld bitmap words needed, scratch holds %lld", 2 * all, b.big_bitmap_words);
+            *status = GALA_ERR_CAPACITY;
+            return -1;
+        }
+        unsigned *bits = (unsigned *)b.big_bitmap, *pref = bits + all;
+        cudaMemsetAsync(bits, 0, (size_t)all * sizeof(unsigned), st);
+        for (int y0 = 0; y0 < rows; y0 += 65535) {  // grid rows
+            SortArgs<WT> part = sa;
+            part.list += y0;
+            const dim3 g((unsigned)std::max(1, std::min(64, cap / std::min(rows, 65535))),
+                         (unsigned)std::min(rows - y0, 65535));
+            k_sort_mark<WT><<<g, 256, 0, st>>>(part, bits + y0 * words, words);
+            note_launch(1);
+        }
+        exclusive_scan(bits, pref, all, OpPopc(), b.scan_partial, &ds->total, st, &ds->err);
+        for (int y0 = 0; y0 < rows; y0 += 65535) {
+            SortArgs<WT> part = sa;
+            part.list += y0;
+            const dim3 g((unsigned)std::max(1, std::min(64, cap / std::min(rows, 65535))),
+                         (unsigned)std::min(rows - y0, 65535));
+            k_sort_place<WT><<<g, 256, 0, st>>>(part, bits + y0 * words, pref + y0 * words, words);
+            note_launch(1);
+        }
+        if (!read_stats(&hs, ds, st, status, "contraction: long sorted rows")) return -1;
+    }
     return (int)hs.ccount;
 }
 

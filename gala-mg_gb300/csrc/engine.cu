@@ -1326,8 +1326,8 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
          dalloc(ctx, &c.big_chunks, n) && dalloc(ctx, &c.big_toff, n + 1) && dalloc(ctx, &c.big_coff, n + 1) &&
          dalloc(ctx, &c.big_mode, n) && dalloc(ctx, &c.big_work, (size_t)c.big_work_cap) &&
          dalloc(ctx, &c.big_tchunks, n) && dalloc(ctx, &c.big_tcoff, n + 1) &&
-         dalloc(ctx, &c.big_twork, (size_t)c.big_twork_cap) && dalloc(ctx, &c.big_kdist, n) &&
-         dalloc(ctx, &c.big_cursor, n) && dalloc(ctx, &c.big_gwords, n) && dalloc(ctx, &c.big_gofs, n + 1);
+         dalloc(ctx, &c.big_twork, (size_t)c.big_twork_cap) &&
+         dalloc(ctx, &c.big_cursor, n);
     ok = ok && dalloc(ctx, &b.moved, n) && dalloc(ctx, &b.mv_pre, (size_t)n + 1);
     ok = ok && dalloc(ctx, &b.act_flag, n) && dalloc(ctx, &ctx->hub_px, (size_t)c.big_twork_cap) &&
          dalloc(ctx, &ctx->hub_pc, (size_t)c.big_twork_cap) && dalloc8(ctx, &ctx->hub_pw, (size_t)c.big_twork_cap) &&

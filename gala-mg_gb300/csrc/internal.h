@@ -328,11 +328,8 @@ struct ContractBuffers {
     long long *big_tcoff;     // n+1: table chunk offsets
     int32_t *big_twork;       // table chunk -> list index
     long long big_twork_cap;
-    int32_t *big_kdist;       // n: distinct neighbour communities
-    int32_t *big_cursor;      // n: unsorted emission cursor
-    long long *big_gwords;    // n: bitmap words of rows ranked by bitmap (0 = sorted in smem)
-    long long *big_gofs;      // n+1: bitmap word offsets
-    int32_t *big_bitmap;      // per-CTA bitmaps over communities (emission)
+    int32_t *big_cursor;      // n: emission cursor
+    int32_t *big_bitmap;      // bitmaps over communities of sorted long rows
     long long big_bitmap_words;
     long long *scan_partial;
     DevStats *stats;

@@ -311,8 +311,8 @@ gala_status gala_context_set_update_mode(gala_context *ctx, int32_t mode);
  * (row, bucket) is summed in one shared-memory table, whenever the level has
  * at most 2^24 rows and the scratch holds the work lists; mode 1: every chunk
  * adds its sums into a global hash table of the row.  Both give the same rows
- * up to their order, and the same results.  Sorted rows
- * (gala_contract_device) always take the global tables. */
+ * up to their order (the same rows where they are sorted,
+ * gala_contract_device), and the same results. */
 gala_status gala_context_set_long_rows(gala_context *ctx, int32_t mode);
 /* Host -> device copy of gala_louvain: with chunks = 2..16 (8 by default) a
  * page-locked (gala_graph_pin) unweighted graph of at least 2^22 entries has
