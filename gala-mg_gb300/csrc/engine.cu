@@ -315,6 +315,116 @@ long long decide_bytes_for(long long nv, long long ne, bool weighted)
 constexpr int64_t kSmallLevelEntries = 1 << 22;
 bool small_level(const LevelGraph &g) { return g.E <= kSmallLevelEntries; }
 
+// Hub tables and chunk lists: the long-row buffers of the contraction, which
+// are idle during phase 1.
+void hub_arrays(gala_context *ctx, HubPlan &hp)
+{
+    ContractBuffers &cb = ctx->cb;
+    hp.T = cb.big_T;
+    hp.chunks = cb.big_chunks;
+    hp.tchunks = cb.big_tchunks;
+    hp.toff = cb.big_toff;
+    hp.coff = cb.big_coff;
+    hp.tcoff = cb.big_tcoff;
+    hp.work = cb.big_work;
+    hp.twork = cb.big_twork;
+    hp.pool = cb.big_pool;
+    hp.px = ctx->hub_px;
+    hp.pc = ctx->hub_pc;
+    hp.pw = ctx->hub_pw;
+    hp.pt = ctx->hub_pt;
+    hp.pwc = ctx->hub_pwc;
+    hp.pdq = ctx->hub_pdq;
+    hp.pfc = ctx->hub_pfc;
+    hp.t_cap = ctx->hub_table_cap;
+}
+
+// Phase 1 of a small level: level init and all sweeps in one launch (more
+// launches when a level takes over kSmallSweeps sweeps).  The rules and the
+// results are those of phase1 below.
+gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, double min_mod, bool verbose,
+                         std::vector<double> *trace, Phase1Out *out, int fp64_only, const int32_t *init)
+{
+    cudaStream_t st = ctx->stream;
+    Phase1Buffers &b = ctx->p1;
+    ContractBuffers &cb = ctx->cb;
+    SmallOut &o = *ctx->h_small_out;
+    const bool weighted = g.w != nullptr;
+    gala_status s;
+    b.features_on = 0;
+    b.wide = g.wide;
+    ctx->sym_state = 0;  // (later levels are no larger: never updated incrementally)
+    HubPlan hp{};
+    hub_arrays(ctx, hp);
+    double prev_q = 0;
+    int iteration = 1;
+    cudaEventRecord(ctx->ev[0], st);
+    for (bool done = false; !done;) {
+        const SmallRun r{ctx->small_ctl, ctx->small_out, init, cb.big_pool_ints, cb.big_work_cap, cb.big_twork_cap, m2,
+                         min_mod, prev_q, fp64_only, iteration};
+        if ((s = check(small_level_run(g, b, hp, r, st), "small level"))) return s;
+        cudaEventRecord(ctx->ev[1], st);
+        cudaMemcpyAsync(&o, ctx->small_out, sizeof(SmallOut), cudaMemcpyDeviceToHost, st);
+        if ((s = sync_check(st, "small level"))) return s;
+        if (iteration == 1) {
+            if (m2 == 0) {  // first level: total weight m2 = sum of K (louvain.cu:165-167)
+                m2 = (long long)o.sum_k;
+                if (m2 <= 0) {
+                    set_error("graph has no edges (total weight 0)");
+                    return GALA_ERR_INVALID;
+                }
+                if (!g.wide && m2 > 0x7fffffffLL) {
+                    set_error("total weight %lld exceeds the int32 range of community totals", m2);
+                    return GALA_ERR_INVALID;
+                }
+            }
+            if (o.status == 1) {
+                set_error("level weight %llu differs from total weight %lld", o.sum_k, m2);
+                return GALA_ERR_INVALID;
+            }
+            if (o.status == 2) {
+                set_error("hub tables need %lld slots, pool holds %lld", o.hub_slots, cb.big_pool_ints / 2);
+                return GALA_ERR_CAPACITY;
+            }
+            if (!o.err) {
+                if (trace) trace->push_back(o.q0);
+                if (verbose) printf("Iteration:%d Q:%f\n", 0, o.q0);
+            }
+            out->nv = o.nv;
+        }
+        if (o.err) {
+            set_error("phase 1: device error bits %d", o.err);
+            return GALA_ERR_OVERFLOW;
+        }
+        for (int k = 0; k < o.sweeps; ++k) {
+            if (trace) trace->push_back(o.trace[k]);
+            if (verbose) printf("Iteration:%d Q:%f\n", iteration + k, o.trace[k]);
+        }
+        const long long dec_nv = o.decisions + (iteration == 1 ? out->nv : 0);
+        const long long dec_ne = (long long)o.entries + (iteration == 1 ? g.E : 0);
+        out->decisions += dec_nv;
+        out->movers += o.movers;
+        out->active_entries += dec_ne;
+        out->decide_ms += (double)o.decide_ns * 1e-6;
+        out->update_ms += (double)o.update_ns * 1e-6;
+        out->decide_bytes += decide_bytes_for(dec_nv, dec_ne, weighted);
+        out->update_bytes += o.sweeps * (out->nv * (2 * 8 + 4 * 4) + g.E * (8 + (weighted ? 4 : 0)));
+        out->sweeps += o.sweeps;
+        prev_q = o.q;
+        done = o.done != 0;
+        iteration += o.sweeps - (done ? 1 : 0);
+    }
+    out->total_ms = ev_ms(ctx->ev[0], ctx->ev[1]);
+    out->q = prev_q;
+    out->iterations = iteration;
+    if (verbose) {
+        printf("time without data init = %fms\n", out->total_ms);
+        printf("decideandmove time = %fms weight updating time = %fms remaining time = %fms\n", out->decide_ms,
+               out->update_ms, out->total_ms - out->decide_ms - out->update_ms);
+    }
+    return GALA_OK;
+}
+
 // One phase-1 run on level graph g (louvain_main_process).  The accepted
 // partition is left in ctx->p1.comm.
 //
@@ -357,14 +467,8 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     int32_t *const d_cnt = d_lo + (PendingRows::kMax + 1) * kNumBins;
     const int32_t *const h_lo = ctx->h_chunk + PendingRows::kMax + 1;
 
-    // a small level runs all its sweeps in one launch, with its own bin limits
-    const bool small = small_level(g) && !pend && !bt && pmode == GALA_PROPOSAL_OFF && !use_graphs &&
-                       ctx->update_mode != 2;
-    struct LimGuard {
-        BinLimits &l, keep;
-        ~LimGuard() { l = keep; }
-    } lim_guard{b.lim, b.lim};
-    if (small) b.lim = small_limits(b.lim, g.wide);
+    if (small_level(g) && !pend && !bt && pmode == GALA_PROPOSAL_OFF && !use_graphs && ctx->update_mode != 2)
+        return phase1_small(ctx, g, m2, min_mod, verbose, trace, out, fp64_only, init);
 
     p1_reset_level_stats(b, st);
     p1_level_init(g, b, st);
@@ -421,24 +525,8 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     hp.H = level_cnt[7];
     if (hp.H > 0) {
         ContractBuffers &cb = ctx->cb;
+        hub_arrays(ctx, hp);
         hp.hubs = b.order + bin_start[7];
-        hp.T = cb.big_T;
-        hp.chunks = cb.big_chunks;
-        hp.tchunks = cb.big_tchunks;
-        hp.toff = cb.big_toff;
-        hp.coff = cb.big_coff;
-        hp.tcoff = cb.big_tcoff;
-        hp.work = cb.big_work;
-        hp.twork = cb.big_twork;
-        hp.pool = cb.big_pool;
-        hp.px = ctx->hub_px;
-        hp.pc = ctx->hub_pc;
-        hp.pw = ctx->hub_pw;
-        hp.pt = ctx->hub_pt;
-        hp.pwc = ctx->hub_pwc;
-        hp.pdq = ctx->hub_pdq;
-        hp.pfc = ctx->hub_pfc;
-        hp.t_cap = ctx->hub_table_cap;
         p1_hub_plan_launch(g, b, hp, st);
         if ((s = check(cudaMemcpyAsync(h, b.stats, sizeof(DevStats), cudaMemcpyDeviceToHost, st), "hub plan")) ||
             (s = sync_check(st, "hub plan")))
@@ -558,35 +646,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     // enqueued only after a sweep that moved under a third of them)
     unsigned long long prev_mv_edges = ~0ull;
     cudaEventRecord(ctx->ev[0], st);
-    for (bool done = false; small && !done;) {
-        SmallRun r{ctx->small_ctl, ctx->small_out, bin_start, m2, min_tot_init, min_mod, prev_q, fp64_only, iteration};
-        if ((s = check(small_level_run(g, b, hp, r, st), "small level"))) return s;
-        SmallOut &o = *ctx->h_small_out;
-        cudaMemcpyAsync(&o, ctx->small_out, sizeof(SmallOut), cudaMemcpyDeviceToHost, st);
-        if ((s = sync_check(st, "small level"))) return s;
-        if (o.err) {
-            set_error("phase 1: device error bits %d", o.err);
-            return GALA_ERR_OVERFLOW;
-        }
-        for (int k = 0; k < o.sweeps; ++k) {
-            if (trace) trace->push_back(o.trace[k]);
-            if (verbose) printf("Iteration:%d Q:%f\n", iteration + k, o.trace[k]);
-        }
-        const long long dec_nv = o.decisions + (iteration == 1 ? act_nv : 0);
-        const long long dec_ne = (long long)o.entries + (iteration == 1 ? act_ne : 0);
-        out->decisions += dec_nv;
-        out->movers += o.movers;
-        out->active_entries += dec_ne;
-        out->decide_ms += (double)o.decide_ns * 1e-6;
-        out->update_ms += (double)o.update_ns * 1e-6;
-        out->decide_bytes += decide_bytes_for(dec_nv, dec_ne, weighted);
-        out->update_bytes += o.sweeps * (nv_all * (2 * 8 + 4 * 4) + g.E * (8 + (weighted ? 4 : 0)));
-        out->sweeps += o.sweeps;
-        prev_q = o.q;
-        done = o.done != 0;
-        iteration += o.sweeps - (done ? 1 : 0);
-    }
-    while (!small) {
+    for (;;) {
         const int nxt = cur ^ 1;
         const int32_t *lists = iteration == 1 ? b.order : b.act[cur];
         const int *counts = &b.stats->act_count[cur][0];

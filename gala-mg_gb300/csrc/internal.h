@@ -205,27 +205,31 @@ void p1_hub_decide(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, doub
 void p1_hub_update(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, int next, int bin_start, double constant,
                    long long m2, cudaStream_t st);
 
-// ---- all sweeps of a small level in one launch (small_level.cu) ----
+// ---- phase 1 of a small level in one launch (small_level.cu) ----
 constexpr int kSmallSweeps = 256;  // sweeps of one launch at most
 struct SmallOut {  // what a launch reports (copied to the host in one piece)
-    double q;      // Q of the partition kept
-    int32_t sweeps, done, err, pad;
+    double q, q0;  // Q of the partition kept, and (first launch) of the start
+    int32_t sweeps, done, err;
+    int32_t status;               // 0, 1: sum_k is not the total weight, 2: the hub tables do not fit
+    unsigned long long sum_k;     // total weight of the level
+    int32_t nv, pad;              // vertices with edges
+    long long hub_slots;
     long long movers, decisions;  // decisions, entries: without the level's first sweep
     unsigned long long entries, decide_ns, update_ns;
     double trace[kSmallSweeps];
 };
 struct SmallRun {
-    void *ctl;       // small_ctl_bytes() of device memory, kept between launches of a level
-    SmallOut *out;   // device
-    const int *bin_start;
-    long long m2, min_tot_init;
+    void *ctl;             // small_ctl_bytes() of device memory, kept between launches of a level
+    SmallOut *out;         // device
+    const int32_t *init;   // starting community of every vertex (null: its own)
+    long long pool_ints, work_cap, twork_cap;  // hub scratch
+    long long m2;          // total weight (0: the level's)
     double min_mod, prev_q;
     int fp64_only;
-    int s0;          // first sweep (1 = the level's first: every vertex is active)
+    int s0;                // first sweep (1 = the level's first, which the level init precedes)
 };
 size_t small_ctl_bytes();
-// Degree-bin limits of a level run this way (rows above go to the hub path).
-BinLimits small_limits(const BinLimits &lim, bool wide);
+// hp: the arrays of the hub plan (its counts are found on the device).
 cudaError_t small_level_run(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, const SmallRun &r,
                             cudaStream_t st);
 

@@ -1053,12 +1053,7 @@ __global__ void k_hub_plan(HubPlan p, const int64_t *__restrict__ offs)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.H; i += gridDim.x * blockDim.x) {
         const int v = p.hubs[i];
-        const long long deg = offs[v + 1] - offs[v];
-        long long T = next_pow2_ll(deg + deg / 2);  // load at most 2/3
-        if (p.t_cap > 0 && T > p.t_cap) T = p.t_cap;  // capped: inserts may run out of slots
-        p.T[i] = T;
-        p.chunks[i] = (deg + kHubChunk - 1) / kHubChunk;
-        p.tchunks[i] = (T + kHubChunk - 1) / kHubChunk;
+        hub_table(offs[v + 1] - offs[v], p.t_cap, p.T[i], p.chunks[i], p.tchunks[i]);
     }
 }
 
@@ -1071,16 +1066,7 @@ __global__ void k_hub_tail(HubPlan p, const DevStats *st)
 
 __global__ void k_hub_work(HubPlan p)
 {
-    const int lane = threadIdx.x & 31;
-    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int i = wg; i < p.H; i += nw) {
-        long long o = p.coff[i], k = p.coff[i + 1] - o;
-        for (long long j = lane; j < k; j += 32) p.work[o + j] = i;
-        o = p.tcoff[i];
-        k = p.tcoff[i + 1] - o;
-        for (long long j = lane; j < k; j += 32) p.twork[o + j] = i;
-    }
+    hub_work(p, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
 }
 
 template <typename WT, bool W>

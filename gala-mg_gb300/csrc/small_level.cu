@@ -1,6 +1,7 @@
 // small_level.cu - all sweeps of a small level's phase 1 in one cooperative
 // launch (louvain_main_process.cu:571-1034 in the reference, which returns to
-// the host between the steps of every iteration).
+// the host between the steps of every iteration), the level init included
+// (louvain_main_process.cu:268-375, init_communities kernel_functions.cu:34-73).
 //
 // A sweep of a small level is bound by its launches: some twenty kernels over
 // the degree bins, the events that fork and join their streams, and a host
@@ -23,6 +24,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "scan.cuh"
 #include "sweep.cuh"
 
 namespace gala {
@@ -41,29 +43,40 @@ struct SweepSlot {
     int act_count[kNumBins];
 };
 
+constexpr int kSmallMaxGrid = 1024;
 struct SmallCtl {
+    // reset before every launch
     unsigned arrive;  // grid barrier: arrivals since the launch
     int dead;         // a barrier wait gave up: every CTA leaves
+    // reset before a level's first launch
+    unsigned long long sum_k, sum_k2, sum_k2_hi, sum_self;
+    // kept between a level's launches
     SweepSlot slot[3];
+    int bin_start[kNumBins + 1];
+    long long half, nwork, ntwork;          // hub plan
+    int part[kSmallMaxGrid][kNumBinSlots];  // vertices per block and bin
 };
 
 template <typename WT>
 struct SmallArgs {
     DecideArgs<WT, false> d;
     UpdateArgs<WT, false> u;
-    HubPlan hp;
+    HubPlan hp;  // arrays; H, half, nwork and ntwork come from the level
+    long long pool_ints, work_cap, twork_cap;
     int n;
-    int bin_start[kNumBins + 1];
-    const int32_t *order;
+    BinLimits lim;
+    bool ks_ready;        // K and Self are given (else summed over the rows)
+    const int32_t *init;  // starting community of every vertex (null: its own)
+    int32_t *order;
     int32_t *act[2];
     int32_t *comm, *size;
-    WT *Tot, *In;
+    WT *K, *Self, *Tot, *In;
     uint8_t *act_flag;
     SmallCtl *ctl;
     SmallOut *out;
     double min_mod, prev_q;
-    long long min_tot_init;
-    int s0;  // first sweep of this launch (1 = the level's first)
+    long long m2;  // total weight (0: this level's sum of K)
+    int s0;        // first sweep of this launch (1 = the level's first)
 };
 
 // Warp-table slots per warp: the tables of all warps together are the CTA
@@ -74,6 +87,17 @@ struct SmallTable {
     static constexpr int kSlots = kWarpSlots * kSmallWarps;
     static constexpr size_t kBytes = (size_t)kSlots * (sizeof(int) + sizeof(WT)) + kSlots / 2 * sizeof(unsigned short);
 };
+
+BinLimits small_limits(const BinLimits &lim, bool wide)
+{
+    BinLimits l = lim;
+    const int row4 = (wide ? SmallTable<long long>::kWarpSlots : SmallTable<int>::kWarpSlots) / 2;
+    const int row6 = (wide ? SmallTable<long long>::kSlots : SmallTable<int>::kSlots) / 2;
+    l.m4 = std::min(l.m4, row4);
+    l.m5 = std::min(l.m5, row6);
+    l.m6 = std::min(l.m6, row6);
+    return l;
+}
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
 {
@@ -153,19 +177,227 @@ __device__ __forceinline__ void apply_moves(const SmallArgs<WT> &a, int nm, int 
     }
 }
 
+// K and Self of the rows of a list (lane groups of G; a row of a vertex that
+// lists itself in several lanes' entries sums those, as k_init_rows_group).
+template <typename WT, int G, bool W>
+__device__ __forceinline__ void init_rows(const SmallArgs<WT> &a, const int32_t *list, int count, int wg, int nw,
+                                          unsigned long long &sk, typename SqSum<WT>::T &sk2, unsigned long long &ss)
+{
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), gw = lane / G;
+    constexpr int GPW = 32 / G;
+    for (int base = wg * GPW; base < count; base += nw * GPW) {
+        const int idx = base + gw;
+        const bool has = idx < count;
+        const int v = has ? list[idx] : 0;
+        const long long s = has ? a.d.offs[v] : 0, e = has ? a.d.offs[v + 1] : 0;
+        WT k = 0, sf = 0;
+        for (long long j = s + sub; j < e; j += G) {
+            const WT wt = W ? a.d.w[j] : 1;
+            k += wt;
+            if (a.d.nbr[j] == v) sf = wt;
+        }
+#pragma unroll
+        for (int o = G / 2; o >= 1; o >>= 1) {
+            k += __shfl_xor_sync(GALA_FULL_MASK, k, o);
+            sf += __shfl_xor_sync(GALA_FULL_MASK, sf, o);
+        }
+        if (has && sub == 0) {
+            a.K[v] = k;
+            a.Tot[v] = k;
+            a.Self[v] = sf;
+            a.In[v] = sf;
+            sk += (unsigned long long)k;
+            sk2 += SqSum<WT>::sq(k);
+            ss += (unsigned long long)sf;
+        }
+    }
+}
+
+// The same for long rows, a block per row: 256 of its threads, as
+// k_init_rows_cta.
+template <typename WT, bool W>
+__device__ __forceinline__ void init_rows_cta(const SmallArgs<WT> &a, const int32_t *list, int count,
+                                              unsigned long long &sk, typename SqSum<WT>::T &sk2,
+                                              unsigned long long &ss)
+{
+    __shared__ WT rk[8], rs[8];
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
+        const int v = list[i];
+        const long long s = a.d.offs[v], e = a.d.offs[v + 1];
+        if (threadIdx.x < 256) {
+            WT k = 0, sf = 0;
+            for (long long j = s + threadIdx.x; j < e; j += 256) {
+                const WT wt = W ? a.d.w[j] : 1;
+                k += wt;
+                if (a.d.nbr[j] == v) sf = wt;
+            }
+            k = warp_sum(k);
+            sf = warp_sum(sf);
+            if ((threadIdx.x & 31) == 0) {
+                rk[threadIdx.x >> 5] = k;
+                rs[threadIdx.x >> 5] = sf;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            WT k = 0, sf = 0;
+            for (int q = 0; q < 8; ++q) {
+                k += rk[q];
+                sf += rs[q];
+            }
+            a.K[v] = k;
+            a.Tot[v] = k;
+            a.Self[v] = sf;
+            a.In[v] = sf;
+            sk += (unsigned long long)k;
+            sk2 += SqSum<WT>::sq(k);
+            ss += (unsigned long long)sf;
+        }
+        __syncthreads();
+    }
+}
+
+// Level init, one block's contiguous run of vertices.  place = false: labels,
+// sizes, totals and the block's vertices per degree bin (ctl->part); place =
+// true, after a barrier: the vertices into the bin-ordered list (offsets from
+// every block's counts), bin starts into s_bin.
+template <typename WT>
+__device__ __forceinline__ void level_vertices(const SmallArgs<WT> &a, bool place, int *s_bin)
+{
+    __shared__ int s_cnt[kNumBinSlots], s_pos[kNumBinSlots];
+    SmallCtl *ctl = a.ctl;
+    const int nb = gridDim.x, bid = blockIdx.x, lane = threadIdx.x & 31;
+    const int per = (a.n + nb - 1) / nb;
+    const int v0 = (int)min((long long)per * bid, (long long)a.n), v1 = (int)min((long long)v0 + per, (long long)a.n);
+    if (threadIdx.x < kNumBinSlots) s_cnt[threadIdx.x] = s_pos[threadIdx.x] = 0;
+    __syncthreads();
+    if (place) {
+        // s_cnt: vertices per bin; s_pos: those of the blocks before this one
+        for (int i = threadIdx.x; i < nb * kNumBinSlots; i += kSmallBlock) {
+            const int c = ctl->part[i / kNumBinSlots][i % kNumBinSlots];
+            if (c) {
+                atomicAdd(&s_cnt[i % kNumBinSlots], c);
+                if (i / kNumBinSlots < bid) atomicAdd(&s_pos[i % kNumBinSlots], c);
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int run = 0;
+            for (int k = 0; k < kNumBinSlots; ++k) {
+                if (k <= kNumBins) s_bin[k] = run;
+                s_pos[k] += run;
+                run += s_cnt[k];
+            }
+            if (bid == 0)
+                for (int k = 0; k <= kNumBins; ++k) ctl->bin_start[k] = s_bin[k];
+        }
+        __syncthreads();
+    }
+    unsigned long long sk = 0, ss = 0;
+    typename SqSum<WT>::T sk2 = 0;
+    for (int t = v0; t < v1; t += kSmallBlock) {  // block-uniform
+        const int v = t + threadIdx.x;
+        int b = -1;
+        if (v < v1) {
+            b = bin_of_degree(a.d.offs[v + 1] - a.d.offs[v], a.lim);
+            if (!place) {
+                a.comm[v] = a.init ? a.init[v] : v;
+                a.size[v] = a.init ? 0 : 1;
+                a.act_flag[v] = 1;
+                WT k = 0, sf = 0;
+                if (a.ks_ready) {
+                    k = a.K[v];
+                    sf = a.Self[v];
+                    sk += (unsigned long long)k;
+                    sk2 += SqSum<WT>::sq(k);
+                    ss += (unsigned long long)sf;
+                } else {  // the rows' sums follow; vertices without entries stay 0
+                    a.K[v] = 0;
+                    a.Self[v] = 0;
+                }
+                a.Tot[v] = a.init ? (WT)0 : k;
+                a.In[v] = a.init ? (WT)0 : sf;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kNumBinSlots; ++k) {
+            const unsigned m = __ballot_sync(GALA_FULL_MASK, b == k);
+            if (m == 0) continue;
+            int p = 0;
+            if (lane == __ffs((int)m) - 1) p = atomicAdd(place ? &s_pos[k] : &s_cnt[k], __popc(m));
+            p = __shfl_sync(GALA_FULL_MASK, p, __ffs((int)m) - 1);
+            if (place && b == k) a.order[p + __popc(m & lanemask_lt())] = v;
+        }
+        if (place && a.init) {  // Tot and size of the starting communities
+            const bool has = v < v1;
+            if (has) {
+                atomic_add_w(&a.Tot[a.init[v]], a.K[v]);
+                atomicAdd(&a.size[a.init[v]], 1);
+            }
+        }
+    }
+    if (!place) {
+        __syncthreads();
+        if (threadIdx.x < kNumBinSlots) ctl->part[bid][threadIdx.x] = s_cnt[threadIdx.x];
+        if (a.ks_ready) {
+            block_add_u64(sk, &ctl->sum_k);
+            SqSum<WT>::add(sk2, &ctl->sum_k2, &ctl->sum_k2_hi);
+            block_add_u64(ss, &ctl->sum_self);
+        }
+    }
+}
+
+// Hub plan by one block: table sizes, chunk counts and their prefixes.
+template <typename WT>
+__device__ __forceinline__ void plan_hubs(const SmallArgs<WT> &a, const HubPlan &p)
+{
+    __shared__ long long wt[32], tot;
+    long long c0 = 0, c1 = 0, c2 = 0;
+    for (int t = 0; t < p.H; t += kSmallBlock) {
+        const int i = t + threadIdx.x;
+        long long T = 0, ch = 0, tc = 0;
+        if (i < p.H) {
+            const int v = p.hubs[i];
+            hub_table(a.d.offs[v + 1] - a.d.offs[v], p.t_cap, T, ch, tc);
+            p.T[i] = T;
+        }
+        long long x = block_exclusive_scan<long long>(T, wt, &tot);
+        if (i < p.H) p.toff[i] = c0 + x;
+        c0 += tot;
+        __syncthreads();
+        x = block_exclusive_scan<long long>(ch, wt, &tot);
+        if (i < p.H) p.coff[i] = c1 + x;
+        c1 += tot;
+        __syncthreads();
+        x = block_exclusive_scan<long long>(tc, wt, &tot);
+        if (i < p.H) p.tcoff[i] = c2 + x;
+        c2 += tot;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        p.toff[p.H] = c0;
+        p.coff[p.H] = c1;
+        p.tcoff[p.H] = c2;
+        a.ctl->half = c0;
+        a.ctl->nwork = c1;
+        a.ctl->ntwork = c2;
+    }
+}
+
 template <typename WT, bool W>
 __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_constant__ SmallArgs<WT> a)
 {
     using Tab = SmallTable<WT>;
     extern __shared__ long long small_sm[];
     __shared__ int stage_buf[kSmallWarps][3 * kStageM];
-    __shared__ int s_go;
+    __shared__ int s_go, s_bin[kNumBins + 1];
     static_assert(kStageN <= 3 * kStageM, "the two stages share their buffer");
     WT *vals = (WT *)small_sm;
     int *keys = (int *)(vals + Tab::kSlots);
     unsigned short *occ = (unsigned short *)(keys + Tab::kSlots);
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int bid = blockIdx.x, nb = gridDim.x;
+    const bool boss = bid == 0 && threadIdx.x == 0;
     // warp tasks go over the CTAs first, from the last CTA down (the CTA rows
     // go to the first CTAs)
     const int wg = wib * nb + (nb - 1 - bid), nw = nb * kSmallWarps;
@@ -175,8 +407,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         vals[j] = 0;
     }
     SmallCtl *ctl = a.ctl;
-    const HubPlan &hp = a.hp;
-    const bool hubs = hp.H > 0;
+    HubPlan hp = a.hp;
     int *const err = a.d.err;
     auto clear_hubs = [&]() {
         int *hk = hp.pool;
@@ -186,33 +417,103 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             hv[j] = 0;
         }
     };
-    if (hubs) clear_hubs();
-    if (bid == 0 && threadIdx.x == 0) clear_slot(ctl->slot[a.s0 % 3], a.min_tot_init);
-    if (!grid_sync(ctl, target, err)) return;
-
+    const bool fresh = a.s0 == 1;
+    const long long min_tot_cap = WideOf<WT>::exact ? 0x7fffffffLL : 0x7fffffffffffffffLL;
+    if (fresh) {
+        // ---- level init
+        if (boss) *err = 0;
+        level_vertices(a, false, s_bin);
+        if (!grid_sync(ctl, target, err)) return;
+        level_vertices(a, true, s_bin);
+    } else {
+        if (threadIdx.x <= kNumBins) s_bin[threadIdx.x] = ctl->bin_start[threadIdx.x];
+        __syncthreads();
+    }
+    hp.H = s_bin[8] - s_bin[7];
+    hp.hubs = a.order + s_bin[7];
+    const bool hubs = hp.H > 0;
+    if (fresh) {
+        if (!a.ks_ready || hubs || a.init) {
+            if (!grid_sync(ctl, target, err)) return;
+            if (!a.ks_ready) {
+                unsigned long long sk = 0, ss = 0;
+                typename SqSum<WT>::T sk2 = 0;
+                init_rows_cta<WT, W>(a, a.order + s_bin[6], s_bin[8] - s_bin[6], sk, sk2, ss);
+                init_rows<WT, 32, W>(a, a.order + s_bin[3], s_bin[6] - s_bin[3], wg, nw, sk, sk2, ss);
+                init_rows<WT, 16, W>(a, a.order + s_bin[2], s_bin[3] - s_bin[2], wg, nw, sk, sk2, ss);
+                init_rows<WT, 8, W>(a, a.order + s_bin[1], s_bin[2] - s_bin[1], wg, nw, sk, sk2, ss);
+                init_rows<WT, 4, W>(a, a.order + s_bin[0], s_bin[1] - s_bin[0], wg, nw, sk, sk2, ss);
+                block_add_u64(sk, &ctl->sum_k);
+                SqSum<WT>::add(sk2, &ctl->sum_k2, &ctl->sum_k2_hi);
+                block_add_u64(ss, &ctl->sum_self);
+            }
+            if (hubs && bid == nb - 1) plan_hubs(a, hp);
+        }
+        if (!grid_sync(ctl, target, err)) return;
+    }
+    const long long m2 = a.m2 ? a.m2 : (long long)ctl->sum_k;
+    hp.half = ctl->half;
+    hp.nwork = ctl->nwork;
+    hp.ntwork = ctl->ntwork;
+    const long long min_tot_init = min(m2, min_tot_cap);
     double prev_q = a.prev_q;
+    if (fresh) {
+        const bool fits = !hubs || ((1 + (long long)(sizeof(WT) / sizeof(int))) * hp.half <= a.pool_ints &&
+                                    hp.nwork <= a.work_cap && hp.ntwork <= a.twork_cap);
+        const bool sum_ok = m2 > 0 && m2 <= min_tot_cap && (long long)ctl->sum_k == m2;
+        if (boss) {
+            SmallOut *o = a.out;
+            o->sum_k = ctl->sum_k;
+            o->nv = s_bin[8];
+            o->hub_slots = hubs ? hp.half : 0;
+            o->sweeps = 0;
+            o->done = 1;
+            o->err = 0;
+            o->status = !sum_ok ? 1 : (!fits ? 2 : 0);
+        }
+        if (!sum_ok || !fits) return;  // the same for every block
+        if (!a.init && threadIdx.x == 0) {
+            SweepSlot q0;
+            q0.sum_in = ctl->sum_self;
+            q0.sum_tot2 = ctl->sum_k2;
+            q0.sum_tot2_hi = ctl->sum_k2_hi;
+            prev_q = slot_q(q0, m2);
+            if (bid == 0) a.out->q0 = prev_q;
+        }
+        if (boss) {
+            clear_slot(ctl->slot[0], min_tot_init);
+            clear_slot(ctl->slot[1], min_tot_init);
+        }
+        if (hubs) {
+            hub_work(hp, wg, nw);
+            clear_hubs();
+        }
+        if (!grid_sync(ctl, target, err)) return;
+    }
+
     long long movers = 0, decisions = 0;  // block 0, thread 0
     unsigned long long entries = 0, dec_ns = 0, upd_ns = 0;
-    int done = 0, s = a.s0;
+    int done = 0, s = fresh && a.init ? 0 : a.s0;  // sweep 0: In and Q of a starting partition
     for (;; ++s) {
         SweepSlot *const cur = &ctl->slot[s % 3];
         const SweepSlot *const prev = &ctl->slot[(s + 2) % 3];
         const bool first = s == 1;
         const int32_t *const lists = first ? a.order : a.act[(s + 1) & 1];
-        auto count = [&](int bin) { return first ? a.bin_start[bin + 1] - a.bin_start[bin] : prev->act_count[bin]; };
-        const bool boss = bid == 0 && threadIdx.x == 0;
+        auto count = [&](int bin) { return first ? s_bin[bin + 1] - s_bin[bin] : prev->act_count[bin]; };
         unsigned long long t0 = 0;
         if (boss) t0 = now_ns();
 
         // ---- decide
-        {
+        if (s > 0) {
             DecideArgs<WT, false> d = a.d;
             d.n_movers = &cur->n_movers;
+            d.m2 = m2;
+            d.constant = __ddiv_rn(1.0, (double)m2);
             int c = count(6);
-            decide_cta<WT, kSmallBlock, W>(d, lists + a.bin_start[6], c, bid, nb, Tab::kSlots, 0, INT_MAX, keys, vals,
+            decide_cta<WT, kSmallBlock, W>(d, lists + s_bin[6], c, bid, nb, Tab::kSlots, 0, INT_MAX, keys, vals,
                                            occ);
             const int off5 = c % nb;
-            decide_cta<WT, kSmallBlock, W>(d, lists + a.bin_start[5], count(5), (bid + nb - off5) % nb, nb,
+            decide_cta<WT, kSmallBlock, W>(d, lists + s_bin[5], count(5), (bid + nb - off5) % nb, nb,
                                            Tab::kSlots, 0, INT_MAX, keys, vals, occ);
             if (hubs) hub_insert<WT, W>(d, hp, a.act_flag, nb - 1 - bid, nb);
             WarpStage<kStageM, 3> stage{stage_buf[wib], 0};
@@ -224,16 +525,16 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             };
             constexpr int WS = Tab::kWarpSlots;
             c = count(4);
-            decide_warp<WT, W, WS>(d, lists + a.bin_start[4], c, start(c), nw, 0, INT_MAX, keys + wib * WS,
+            decide_warp<WT, W, WS>(d, lists + s_bin[4], c, start(c), nw, 0, INT_MAX, keys + wib * WS,
                                    vals + wib * WS, occ + wib * (WS / 2));
             c = count(3);
-            decide_group<WT, 32, W>(d, lists + a.bin_start[3], c, start(c), nw, stage);
+            decide_group<WT, 32, W>(d, lists + s_bin[3], c, start(c), nw, stage);
             c = count(2);
-            decide_group<WT, 16, W>(d, lists + a.bin_start[2], c, start((c + 1) / 2), nw, stage);
+            decide_group<WT, 16, W>(d, lists + s_bin[2], c, start((c + 1) / 2), nw, stage);
             c = count(1);
-            decide_group<WT, 8, W>(d, lists + a.bin_start[1], c, start((c + 3) / 4), nw, stage);
+            decide_group<WT, 8, W>(d, lists + s_bin[1], c, start((c + 3) / 4), nw, stage);
             c = count(0);
-            decide_group<WT, 4, W>(d, lists + a.bin_start[0], c, start((c + 7) / 8), nw, stage);
+            decide_group<WT, 4, W>(d, lists + s_bin[0], c, start((c + 7) / 8), nw, stage);
             int *const mlists[3] = {a.d.mv_v, a.d.mv_old, a.d.mv_new};
             stage.flush(mlists, &cur->n_movers);
             if (!grid_sync(ctl, target, err)) return;
@@ -244,13 +545,15 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 if (!grid_sync(ctl, target, err)) return;
             }
         }
-        if (boss) dec_ns += now_ns() - t0;
+        if (boss && s > 0) dec_ns += now_ns() - t0;
 
         // ---- apply
-        apply_moves(a, cur->n_movers, +1);
-        if (hubs)
-            for (int i = bid * kSmallBlock + threadIdx.x; i < hp.H; i += nb * kSmallBlock) a.In[hp.hubs[i]] = 0;
-        if (!grid_sync(ctl, target, err)) return;
+        if (s > 0) {
+            apply_moves(a, cur->n_movers, +1);
+            if (hubs)
+                for (int i = bid * kSmallBlock + threadIdx.x; i < hp.H; i += nb * kSmallBlock) a.In[hp.hubs[i]] = 0;
+            if (!grid_sync(ctl, target, err)) return;
+        }
 
         // ---- totals; hub rows' In and their cleared tables on the side
         {
@@ -272,9 +575,9 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 clear_hubs();
             }
             if (boss) {
-                clear_slot(ctl->slot[(s + 1) % 3], a.min_tot_init);
+                clear_slot(ctl->slot[(s + 1) % 3], min_tot_init);
                 movers += cur->n_movers;
-                if (!first) {
+                if (s > 1) {
                     decisions += prev->act_vertices;
                     entries += prev->act_edges;
                 }
@@ -286,13 +589,15 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         // ---- update and prune
         {
             UpdateArgs<WT, false> u = a.u;
+            u.m2 = m2;
+            u.constant = __ddiv_rn(1.0, (double)m2);
             const long long mt = cur->min_tot;
             UpdateSums sums;
             WarpStage<kStageN, 1> stage{stage_buf[wib], 0};
             int off = 0;
             auto bin = [&](int b, int G) {  // list, count and this warp's first task of a bin
-                const int c = a.bin_start[b + 1] - a.bin_start[b], tasks = (c + 32 / G - 1) / (32 / G);
-                u.act_list = a.act[s & 1] + a.bin_start[b];
+                const int c = s_bin[b + 1] - s_bin[b], tasks = (c + 32 / G - 1) / (32 / G);
+                u.act_list = a.act[s & 1] + s_bin[b];
                 u.act_counter = &cur->act_count[b];
                 const int w0 = wg - off;
                 off = (off + tasks) % nw;
@@ -300,11 +605,11 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             };
             bin(6, 32);
             off = 0;
-            update_cta<WT, W>(u, a.order + a.bin_start[6], a.bin_start[7] - a.bin_start[6], mt, bid, nb, sums);
+            update_cta<WT, W>(u, a.order + s_bin[6], s_bin[7] - s_bin[6], mt, bid, nb, sums);
 #define GALA_SMALL_UPD(B, G)                                                                                         \
     do {                                                                                                             \
         const int w0 = bin(B, G);                                                                                    \
-        update_group<WT, G, W>(u, a.order + a.bin_start[B], a.bin_start[B + 1] - a.bin_start[B], mt, w0, nw, stage,  \
+        update_group<WT, G, W>(u, a.order + s_bin[B], s_bin[B + 1] - s_bin[B], mt, w0, nw, stage,  \
                                sums);                                                                                \
     } while (0)
             GALA_SMALL_UPD(5, 32);
@@ -315,7 +620,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             GALA_SMALL_UPD(0, 4);
 #undef GALA_SMALL_UPD
             if (hubs) {
-                u.act_list = a.act[s & 1] + a.bin_start[7];
+                u.act_list = a.act[s & 1] + s_bin[7];
                 u.act_counter = &cur->act_count[7];
                 hub_in_final(u, hp, mt, bid, nb, sums);
             }
@@ -327,8 +632,13 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
 
         // ---- convergence (louvain_main_process.cu:1004-1007)
         const int k = s - a.s0;  // sweeps of this launch before this one
+        if (s == 0) {
+            if (threadIdx.x == 0) prev_q = slot_q(*cur, m2);
+            if (boss) a.out->q0 = prev_q;
+            continue;
+        }
         if (threadIdx.x == 0) {
-            const double q = slot_q(*cur, a.d.m2);
+            const double q = slot_q(*cur, m2);
             int go = 1;
             if (*(volatile int *)err)
                 go = 0;
@@ -381,42 +691,16 @@ int small_resident()
 }
 
 template <typename WT, bool W>
-cudaError_t launch_small(const LevelGraph &g, const Phase1Buffers &b, const HubPlan &hp, const SmallRun &r,
-                         const DecideArgs<WT, false> &d, const UpdateArgs<WT, false> &u, cudaStream_t st)
+cudaError_t launch_small(const LevelGraph &g, SmallArgs<WT> &a, cudaStream_t st)
 {
-    SmallArgs<WT> a;
-    a.d = d;
-    a.u = u;
-    a.hp = hp;
-    a.n = g.n;
-    long long tasks = 0;  // warps that a sweep over every vertex keeps busy
-    const int per[kNumBins] = {8, 4, 2, 1, 1, 1, 1, 1};
-    for (int i = 0; i <= kNumBins; ++i) a.bin_start[i] = r.bin_start[i];
-    for (int i = 0; i < kNumBins; ++i) {
-        const long long c = r.bin_start[i + 1] - r.bin_start[i];
-        tasks += i < 5 ? (c + per[i] - 1) / per[i] : c * kSmallWarps;
-    }
-    if (hp.H > 0) tasks = std::max<long long>(tasks, hp.ntwork * kSmallWarps);
-    a.order = b.order;
-    a.act[0] = b.act[0];
-    a.act[1] = b.act[1];
-    a.comm = b.comm;
-    a.size = b.size;
-    a.Tot = (WT *)b.Tot;
-    a.In = (WT *)b.In;
-    a.act_flag = b.act_flag;
-    a.ctl = (SmallCtl *)r.ctl;
-    a.out = r.out;
-    a.min_mod = r.min_mod;
-    a.prev_q = r.prev_q;
-    a.min_tot_init = r.min_tot_init;
-    a.s0 = r.s0;
     const int per_sm = small_resident<WT, W>();
     if (per_sm <= 0) return cudaErrorLaunchOutOfResources;
+    // warps a sweep keeps busy: about 1.5 lanes per entry, at most 8 vertices
+    // a warp
+    const long long tasks = g.E * 3 / 64 + g.n / 32;
     long long grid = (tasks + kSmallWarps - 1) / kSmallWarps;
-    grid = std::max(1LL, std::min<long long>(grid, (long long)hub_grid_size() * per_sm));
-    // the barrier's counter (the sweep slots carry over between launches)
-    cudaMemsetAsync(r.ctl, 0, offsetof(SmallCtl, slot), st);
+    grid = std::max(1LL, std::min<long long>(grid, std::min(hub_grid_size() * per_sm, kSmallMaxGrid)));
+    cudaMemsetAsync(a.ctl, 0, a.s0 == 1 ? offsetof(SmallCtl, slot) : offsetof(SmallCtl, sum_k), st);
     void *args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_small_level<WT, W>, dim3((unsigned)grid),
                                                       dim3(kSmallBlock), args, SmallTable<WT>::kBytes, st);
@@ -427,7 +711,8 @@ cudaError_t launch_small(const LevelGraph &g, const Phase1Buffers &b, const HubP
 template <typename WT>
 cudaError_t small_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, const SmallRun &r, cudaStream_t st)
 {
-    DecideArgs<WT, false> d;
+    SmallArgs<WT> a{};
+    DecideArgs<WT, false> &d = a.d;
     d.offs = g.offs;
     d.nbr = g.nbr;
     d.w = (const WT *)g.w;
@@ -439,19 +724,10 @@ cudaError_t small_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, co
     d.mv_v = b.mv_v;
     d.mv_old = b.mv_old;
     d.mv_new = b.mv_new;
-    d.n_movers = nullptr;  // per sweep
     d.err = &b.stats->err;
     d.fp64_decisions = &b.stats->fp64_decisions;
-    d.constant = 1 / (double)r.m2;
-    d.m2 = r.m2;
     d.fp64_only = r.fp64_only;
-    d.feat_gain = nullptr;
-    d.feat_ndist = nullptr;
-    d.gid = nullptr;
-    d.m2g = nullptr;
-    d.cg = nullptr;
-    d.stop = nullptr;
-    UpdateArgs<WT, false> u;
+    UpdateArgs<WT, false> &u = a.u;
     u.offs = g.offs;
     u.nbr = g.nbr;
     u.w = (const WT *)g.w;
@@ -461,36 +737,39 @@ cudaError_t small_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, co
     u.Tot = (const WT *)b.Tot;
     u.In = (WT *)b.In;
     u.act_flag = b.act_flag;
-    u.act_list = nullptr;  // per bin
-    u.act_counter = nullptr;
     u.st = b.stats;
-    u.constant = d.constant;
-    u.m2 = r.m2;
-    u.next = 0;
-    u.gid = nullptr;
-    u.m2g = nullptr;
-    u.cg = nullptr;
-    u.stop = nullptr;
-    u.min_tot_g = nullptr;
+    a.hp = hp;
+    a.pool_ints = r.pool_ints;
+    a.work_cap = r.work_cap;
+    a.twork_cap = r.twork_cap;
+    a.n = g.n;
+    a.lim = small_limits(b.lim, g.wide);
+    a.ks_ready = g.ks_ready;
+    a.init = r.init;
+    a.order = b.order;
+    a.act[0] = b.act[0];
+    a.act[1] = b.act[1];
+    a.comm = b.comm;
+    a.size = b.size;
+    a.K = (WT *)b.K;
+    a.Self = (WT *)b.Self;
+    a.Tot = (WT *)b.Tot;
+    a.In = (WT *)b.In;
+    a.act_flag = b.act_flag;
+    a.ctl = (SmallCtl *)r.ctl;
+    a.out = r.out;
+    a.min_mod = r.min_mod;
+    a.prev_q = r.prev_q;
+    a.m2 = r.m2;
+    a.s0 = r.s0;
     if constexpr (WideOf<WT>::exact)
-        if (!g.w) return launch_small<WT, false>(g, b, hp, r, d, u, st);
-    return launch_small<WT, true>(g, b, hp, r, d, u, st);
+        if (!g.w) return launch_small<WT, false>(g, a, st);
+    return launch_small<WT, true>(g, a, st);
 }
 
 }  // namespace
 
 size_t small_ctl_bytes() { return sizeof(SmallCtl); }
-
-BinLimits small_limits(const BinLimits &lim, bool wide)
-{
-    BinLimits l = lim;
-    const int row4 = (wide ? SmallTable<long long>::kWarpSlots : SmallTable<int>::kWarpSlots) / 2;
-    const int row6 = (wide ? SmallTable<long long>::kSlots : SmallTable<int>::kSlots) / 2;
-    l.m4 = std::min(l.m4, row4);
-    l.m5 = std::min(l.m5, row6);
-    l.m6 = std::min(l.m6, row6);
-    return l;
-}
 
 cudaError_t small_level_run(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, const SmallRun &r,
                             cudaStream_t st)

@@ -66,9 +66,10 @@ struct SqSum<long long> {
 // ------------------------------------------------------------------------
 // Decide-and-move
 // ------------------------------------------------------------------------
-// Labels, totals and sizes are read-only for a kernel that runs one sweep
-// (RO), so their loads may take the non-coherent path; a kernel that runs
-// several sweeps with grid barriers between them (!RO) writes them too.
+// Labels, totals, sizes and weighted degrees are read-only for a kernel that
+// runs one sweep (RO), so their loads may take the non-coherent path; a kernel
+// that runs a whole level with grid barriers between its steps (!RO) writes
+// them too.
 template <typename T, bool RO>
 struct SweepPtr {
     using type = const T *__restrict__;
@@ -84,8 +85,8 @@ struct DecideArgs {
     const int32_t *__restrict__ nbr;
     const WT *__restrict__ w;
     typename SweepPtr<int32_t, RO>::type comm;
-    const WT *__restrict__ K;
-    const WT *__restrict__ Self;
+    typename SweepPtr<WT, RO>::type K;
+    typename SweepPtr<WT, RO>::type Self;
     typename SweepPtr<WT, RO>::type Tot;
     typename SweepPtr<int32_t, RO>::type size;
     int32_t *mv_v, *mv_old, *mv_new;
@@ -830,6 +831,30 @@ __device__ __forceinline__ void decide_cta(const DecideArgs<WT, RO> &a, const in
 // ------------------------------------------------------------------------
 constexpr int kHubChunk = 4096;
 
+// Table slots, row chunks and table chunks of a hub of degree deg (t_cap: the
+// caller's cap on the slots, 0 = none).
+__device__ __forceinline__ void hub_table(long long deg, long long t_cap, long long &T, long long &chunks,
+                                          long long &tchunks)
+{
+    T = next_pow2_ll(deg + deg / 2);  // load at most 2/3
+    if (t_cap > 0 && T > t_cap) T = t_cap;  // capped: inserts may run out of slots
+    chunks = (deg + kHubChunk - 1) / kHubChunk;
+    tchunks = (T + kHubChunk - 1) / kHubChunk;
+}
+
+// Chunk -> hub lists, one warp per hub.
+__device__ __forceinline__ void hub_work(const HubPlan &p, int wg, int nw)
+{
+    const int lane = threadIdx.x & 31;
+    for (int i = wg; i < p.H; i += nw) {
+        long long o = p.coff[i], k = p.coff[i + 1] - o;
+        for (long long j = lane; j < k; j += 32) p.work[o + j] = i;
+        o = p.tcoff[i];
+        k = p.tcoff[i + 1] - o;
+        for (long long j = lane; j < k; j += 32) p.twork[o + j] = i;
+    }
+}
+
 // Values of a hub table (WT per slot, after the keys of all tables).
 template <typename WT>
 __device__ __forceinline__ WT *hub_vals(const HubPlan &p, long long i)
@@ -1086,8 +1111,8 @@ struct UpdateArgs {
     const int32_t *__restrict__ nbr;
     const WT *__restrict__ w;
     typename SweepPtr<int32_t, RO>::type comm;
-    const WT *__restrict__ K;
-    const WT *__restrict__ Self;
+    typename SweepPtr<WT, RO>::type K;
+    typename SweepPtr<WT, RO>::type Self;
     typename SweepPtr<WT, RO>::type Tot;
     WT *In;
     uint8_t *act_flag;  // per-vertex copy of the next active set
