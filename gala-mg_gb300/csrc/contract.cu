@@ -4,7 +4,8 @@
 // kernels at kernel_functions.cu:1083-1694 of the reference).  Steps:
 //   1. community sizes (histogram) and dense renumbering in ascending label
 //      order: exclusive scan of (size > 0), no sort
-//   2. members of each community (counting-sort buckets)
+//   2. entries of each community (sum of its members' row lengths) and their
+//      prefix, where every member row claims its place
 //   3. the community-ordered edge stream: for every member edge the new id of
 //      the neighbour's community and the weight, contiguous per community
 //   4. per community, sum the weights per neighbour community, by row length:
@@ -62,13 +63,6 @@ constexpr int kChunk = 4096;
 constexpr int kSortMax = 16384;
 constexpr int kRangeEntries = 1024;  // CSR entries per warp task
 
-struct OpDegOf {
-    const int64_t *offs;
-    __device__ __forceinline__ long long operator()(int32_t v, long long) const
-    {
-        return (long long)(offs[v + 1] - offs[v]);
-    }
-};
 struct OpPopc {
     __device__ __forceinline__ long long operator()(unsigned x, long long) const { return __popc(x); }
 };
@@ -108,24 +102,30 @@ __global__ void k_nz_scatter(const int64_t *__restrict__ offs, int n, const int3
             const int p = pos[i];
             nz_rows[p] = i;
             nz_offs[p] = s;
-            nz_shift[p] = shift(i, s);
+            nz_shift[p] = shift(i, s, e);
             for (long long t = (s + kRangeEntries - 1) / kRangeEntries; t * kRangeEntries < e; ++t)
                 task_row[t] = p;
         }
     }
 }
 
-// Shifts of the two walks: the stream fill writes entry j of vertex v's row
-// to medge[mpos[v]] + (j - offs[v]); the compaction reads entry j of
-// community c's new row from tmp_off[c] + (j - new_offs[c]).
+// Shifts of the two walks: vertex v's row [s, e) claims the next e - s places
+// of its community's stream range, so the stream fill writes entry j to
+// ebase[c] + claimed + (j - s); the compaction reads entry j of community c's
+// new row from tmp_off[c] + (j - new_offs[c]).
 struct ShiftStream {
-    const int32_t *__restrict__ mpos;
-    const long long *__restrict__ medge;
-    __device__ __forceinline__ long long operator()(int v, long long s) const { return medge[mpos[v]] - s; }
+    const int32_t *__restrict__ lab;
+    const long long *__restrict__ ebase;
+    unsigned long long *taken;  // entries claimed per community
+    __device__ __forceinline__ long long operator()(int v, long long s, long long e) const
+    {
+        const int c = lab[v];
+        return ebase[c] + (long long)atomicAdd(&taken[c], (unsigned long long)(e - s)) - s;
+    }
 };
 struct ShiftCompact {
     const long long *__restrict__ tmp_off;
-    __device__ __forceinline__ long long operator()(int c, long long s) const { return tmp_off[c] - s; }
+    __device__ __forceinline__ long long operator()(int c, long long s, long long) const { return tmp_off[c] - s; }
 };
 
 // Caller-supplied labels must lie in [0, n) before they index any array.
@@ -143,24 +143,41 @@ __global__ void k_hist(const int32_t *__restrict__ comm, int n, int32_t *cnt)
         atomicAdd(&cnt[comm[v]], 1);
 }
 
-// New label of every vertex and member count of every new community (its
-// entry count ec and, with self_out, its Self start at 0); with tot/k_out,
-// K_new of community c is its total Tot[c] (the weight of the new row equals
-// the weighted degrees of its members, exactly).
+// New label of every vertex and entries of every new community (ec, zero on
+// entry: the row lengths of its members; equal labels of a warp are added
+// together first, a few large communities take most vertices of some levels).
+// With tot/k_out, K_new of community c is its total Tot[c] (the weight of the
+// new row equals the weighted degrees of its members, exactly); with self_out
+// its Self starts at 0.
 template <typename WT>
 __global__ void k_relabel(const int32_t *__restrict__ comm, const int32_t *__restrict__ newid,
-                          const int32_t *__restrict__ cnt, int n, int32_t *lab, int32_t *csz, long long *ec,
-                          const WT *__restrict__ tot, WT *k_out, WT *self_out)
+                          const int32_t *__restrict__ cnt, const int64_t *__restrict__ offs, int n, int32_t *lab,
+                          long long *ec, const WT *__restrict__ tot, WT *k_out, WT *self_out)
 {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        lab[v] = newid[comm[v]];
-        int k = cnt[v];
-        if (k > 0) {
-            const int c = newid[v];
-            csz[c] = k;
-            ec[c] = 0;
-            if (k_out) k_out[c] = tot[v];
-            if (self_out) self_out[c] = 0;
+    const int lane = threadIdx.x & 31;
+    for (int v0 = blockIdx.x * blockDim.x + threadIdx.x - lane; v0 < n; v0 += gridDim.x * blockDim.x) {
+        const int v = v0 + lane;
+        int c = -1;
+        unsigned d = 0;
+        if (v < n) {
+            c = newid[comm[v]];
+            lab[v] = c;
+            if (ec) d = (unsigned)(offs[v + 1] - offs[v]);
+            if (cnt[v] > 0) {
+                const int m = newid[v];
+                if (k_out) k_out[m] = tot[v];
+                if (self_out) self_out[m] = 0;
+            }
+        }
+        if (ec) {
+            const unsigned m = __match_any_sync(GALA_FULL_MASK, d ? c : -1);
+            // row lengths below 2^26 add up in 32 bits
+            if (__any_sync(GALA_FULL_MASK, d >> 26)) {
+                if (d) atomicAdd((unsigned long long *)&ec[c], (unsigned long long)d);
+            } else {
+                const unsigned t = __reduce_add_sync(m, d);
+                if (d && lane == __ffs((int)m) - 1) atomicAdd((unsigned long long *)&ec[c], (unsigned long long)t);
+            }
         }
     }
 }
@@ -171,27 +188,11 @@ __global__ void k_compose(int32_t *orig, int n_orig, const int32_t *__restrict__
         orig[i] = lab[orig[i]];
 }
 
-// Member buckets: csz[c] counts down to 0, so the members of c fill
-// [moff[c], moff[c] + size) from the end (no cursor copy of moff).
-__global__ void k_member_scatter(const int32_t *__restrict__ lab, const int64_t *__restrict__ offs, int n,
-                                 const int32_t *__restrict__ moff, int32_t *csz, int32_t *members, int32_t *mpos,
-                                 long long *ec)
-{
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        int c = lab[v];
-        int p = moff[c] + atomicSub(&csz[c], 1) - 1;
-        members[p] = v;
-        mpos[v] = p;
-        long long d = offs[v + 1] - offs[v];
-        if (d) atomicAdd((unsigned long long *)&ec[c], (unsigned long long)d);
-    }
-}
-
 // Community-ordered edge stream over contiguous entry ranges: entry j of row
-// v goes to medge[mpos[v]] + (j - offs[v]).  Unweighted levels (W false)
+// v goes to place j + nz_shift of its row.  Unweighted levels (W false)
 // write no weights: the aggregation counts every entry as 1.  Rows are walked through the
-// list of rows with entries (nz_rows / nz_offs); each row's destination
-// (medge[mpos[v]] - offs[v]) is loaded once per row window.
+// list of rows with entries (nz_rows / nz_offs); each row's shift is loaded
+// once per row window.
 template <typename WT, bool W>
 __global__ void __launch_bounds__(256) k_stream_fill(long long E, const int32_t *__restrict__ nbr,
                                                      const WT *__restrict__ w, const int32_t *__restrict__ lab,
@@ -333,8 +334,7 @@ __global__ void __launch_bounds__(256) k_classify(const long long *__restrict__ 
 
 template <typename WT>
 struct AggArgs {
-    const int32_t *__restrict__ moff;
-    const long long *__restrict__ medge;
+    const long long *__restrict__ ebase;  // first stream entry of a community
     const long long *__restrict__ ec;
     const int32_t *__restrict__ skey;
     const WT *__restrict__ sw;  // null: unweighted level, every entry weighs 1
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256) k_agg_small(AggArgs<WT> a, const int32_t 
     const int cnt = a.st->small_cnt[0];
     for (int i = wg; i < cnt; i += nw) {
         const int c = list[i];
-        const long long st = a.medge[a.moff[c]];
+        const long long st = a.ebase[c];
         const int E = (int)a.ec[c];
         const bool valid = lane < E;
         int key = -1;
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(256) k_agg_warp_list(AggArgs<WT> a, const int3
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int i = wg; i < cnt; i += nw) {
         const int c = list[i];
-        const long long st = a.medge[a.moff[c]];
+        const long long st = a.ebase[c];
         const int E = (int)a.ec[c];  // 33..kWarpAggMax
         int nocc = 0;
         for (int b0 = 0; b0 < E; b0 += 32) {
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(BLOCK) k_agg_mid_list(AggArgs<WT> a, const int
     const int cnt = a.st->small_cnt[cls];
     for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
         const int c = list[i];
-        const long long st = a.medge[a.moff[c]];
+        const long long st = a.ebase[c];
         const int E = (int)a.ec[c];
         agg_insert_list(a, st, E, keys, vals, TMAX, lg, occ, &s_k);
         __syncthreads();
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(512) k_big_insert_sm(AggArgs<WT> a, BigArgs b)
         const long long j = wi - b.coff[i];
         const int c = b.list[i];
         const long long E = a.ec[c];
-        const long long st = a.medge[a.moff[c]] + j * kChunk;
+        const long long st = a.ebase[c] + j * kChunk;
         const int len = (int)((E - j * kChunk) < kChunk ? (E - j * kChunk) : kChunk);
         const long long T = b.T[i];
         WT *vals = big_vals<WT>(b, i);
@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(kRadCombineThreads, 2) k_rad_combine(AggArgs<W
         const int c = b.list[i];
         const long long j = wi - b.coff[i];
         const long long E = a.ec[c];
-        const long long s0 = a.medge[a.moff[c]] + j * kChunk;
+        const long long s0 = a.ebase[c] + j * kChunk;
         const int len = (int)((E - j * kChunk) < kChunk ? (E - j * kChunk) : kChunk);
         constexpr int kPer = kChunk / kRadCombineThreads;  // entries per thread, loaded before the inserts
         int kk[kPer];
@@ -1082,7 +1082,7 @@ __global__ void k_rad_items(AggArgs<WT> a, BigArgs b, int32_t *pool, long long v
     for (int i = wg; i < cnt; i += nw) {
         const int nch = (int)b.chunks[i];
         const int c = b.list[i];
-        const long long r_sbase = a.medge[a.moff[c]], r_dst = a.tmp_off[c], r_w0 = b.coff[i], r_e = a.ec[c];
+        const long long r_sbase = a.ebase[c], r_dst = a.tmp_off[c], r_w0 = b.coff[i], r_e = a.ec[c];
         const int32_t *trow = pool + (long long)i * nb;
         long long carry = 0;  // pairs of the buckets before the tile
         int prev_big = 0;
@@ -1751,12 +1751,6 @@ __global__ void __launch_bounds__(256) k_compact(const int64_t *__restrict__ new
     }
 }
 
-__global__ void k_contract_set_tail(int32_t *moff, const DevStats *st, int n, long long *medge, long long E)
-{
-    moff[st->ccount] = n;
-    medge[n] = E;
-}
-
 __global__ void k_set_last_offset(int64_t *offs, const DevStats *st) { offs[st->ccount] = st->new_entries; }
 
 __global__ void k_contract_reset(DevStats *st)
@@ -1963,8 +1957,13 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
     cudaMemsetAsync(b.cnt, 0, ((size_t)n + 1) * sizeof(int32_t), st);
     k_hist<<<grid_cap(n, 256, cap), 256, 0, st>>>(comm, n, b.cnt);
     exclusive_scan(b.cnt, b.newid, n, OpPositive(), b.scan_partial, &ds->ccount, st, &ds->err);
-    k_relabel<WT><<<grid_cap(n, 256, cap), 256, 0, st>>>(comm, b.newid, b.cnt, n, b.lab, b.csz, b.ec,
-                                                         (const WT *)nli.tot, (WT *)nli.k, (WT *)nli.self);
+    if (!labels_only) {
+        cudaMemsetAsync(b.ec, 0, (size_t)n * sizeof(long long), st);
+        cudaMemsetAsync(b.taken, 0, (size_t)n * sizeof(long long), st);
+    }
+    k_relabel<WT><<<grid_cap(n, 256, cap), 256, 0, st>>>(comm, b.newid, b.cnt, g.offs, n, b.lab,
+                                                         labels_only ? nullptr : b.ec, (const WT *)nli.tot,
+                                                         (WT *)nli.k, (WT *)nli.self);
     note_launch(2);
     if (orig_map) {
         k_compose<<<grid_cap(n_orig, 256, cap), 256, 0, st>>>(orig_map, n_orig, b.lab);
@@ -1975,16 +1974,10 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
         *new_E = 0;
         return (int)hs.ccount;
     }
-    exclusive_scan_dev(b.csz, b.moff, n, dC, OpIdentity(), b.scan_partial, &ds->total, st, &ds->err);
-    k_member_scatter<<<grid_cap(n, 256, cap), 256, 0, st>>>(b.lab, g.offs, n, b.moff, b.csz, b.members, b.mpos,
-                                                            b.ec);
-    exclusive_scan(b.members, b.medge, n, OpDegOf{g.offs}, b.scan_partial, &ds->total, st, &ds->err);
-    // moff[C] = n and medge[n] = E close the last segments
-    k_contract_set_tail<<<1, 1, 0, st>>>(b.moff, ds, n, b.medge, E);
-    note_launch(2);
+    exclusive_scan_dev(b.ec, b.ebase, n, dC, OpIdentity(), b.scan_partial, &ds->total, st, &ds->err);
     const bool weighted = g.w != nullptr;
     if (E > 0) {
-        build_walk_list(g.offs, n, E, b, st, ShiftStream{b.mpos, b.medge});
+        build_walk_list(g.offs, n, E, b, st, ShiftStream{b.lab, b.ebase, (unsigned long long *)b.taken});
         const int tasks = grid_cap((E + kRangeEntries - 1) / kRangeEntries * 32, 256, cap);
         if (weighted) {
             const int grid = std::min(tasks, resident_grid(k_stream_fill<WT, true>, 256));
@@ -2002,8 +1995,7 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
     note_launch(1);
 
     AggArgs<WT> a;
-    a.moff = b.moff;
-    a.medge = b.medge;
+    a.ebase = b.ebase;
     a.ec = b.ec;
     a.skey = b.stream_key;
     a.sw = weighted ? (const WT *)b.stream_w : nullptr;

@@ -1371,9 +1371,7 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
          dalloc(ctx, &b.prop_list, n);
     ContractBuffers &c = ctx->cb;
     ok = ok && dalloc(ctx, &c.cnt, n + 1) && dalloc(ctx, &c.newid, n + 1) && dalloc(ctx, &c.lab, n) &&
-         dalloc(ctx, &c.csz, n + 1) && dalloc(ctx, &c.moff, n + 1) && dalloc(ctx, &c.cursor, n + 1) &&
-         dalloc(ctx, &c.members, n) && dalloc(ctx, &c.mpos, n) && dalloc(ctx, &c.ec, n + 1) &&
-         dalloc(ctx, &c.medge, n + 1) && dalloc(ctx, &c.stream_key, E) && dalloc8(ctx, &c.stream_w, E) &&
+         dalloc(ctx, &c.ec, n + 1) && dalloc(ctx, &c.ebase, n + 1) && dalloc(ctx, &c.taken, n + 1) && dalloc(ctx, &c.stream_key, E) && dalloc8(ctx, &c.stream_w, E) &&
          dalloc(ctx, &c.tmp_off, n + 1) && dalloc(ctx, &c.tmp_nbr, E) && dalloc8(ctx, &c.tmp_w, E) &&
          dalloc(ctx, &c.kc, n + 1) && dalloc(ctx, &c.cls_list, 6 * n);
     // tables of the rows longer than 4096 entries (hubs of a small level: 2048):

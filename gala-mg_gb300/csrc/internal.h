@@ -297,13 +297,9 @@ struct ContractBuffers {
     int32_t *cnt;        // n+1
     int32_t *newid;      // n
     int32_t *lab;        // n
-    int32_t *csz;        // n+1
-    int32_t *moff;       // n+1 member offsets
-    int32_t *cursor;     // n
-    int32_t *members;    // n
-    int32_t *mpos;       // n: member position of each vertex
     long long *ec;       // n+1 edges per community
-    long long *medge;    // n+1 prefix of member degrees
+    long long *ebase;    // n+1 prefix of ec: first stream entry per community
+    long long *taken;    // n: stream entries claimed by member rows
     int32_t *stream_key; // E
     int32_t *stream_w;   // E weights (int32, or int64 when wide: allocated 8 bytes per entry)
     long long *tmp_off;  // n+1
