@@ -2145,15 +2145,42 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
     return (int)hs.ccount;
 }
 
+// Levels contracted in one launch (small_contract.cu): there the general path
+// costs its fifty launches, about 200 us whatever the size.  Whole runs, general
+// path / one launch (ms): 80-vertex SBM 0.76 / 0.60, 1,024-vertex SBM 0.88 /
+// 0.74, R-MAT scale 16 2.79 / 2.52; with levels up to 2^20 entries 2.97 (few
+// large communities, few blocks at work), and levels of over 2^16 vertices
+// gain nothing (R-MAT scale 22, mostly isolated vertices, 18.63 / 18.72).
+constexpr int32_t kSmallContractVertices = 1 << 16;
+constexpr int64_t kSmallContractEntries = 1 << 18;
 int contract_run(const LevelGraph &g, const int32_t *comm, ContractBuffers &b, int64_t *new_offs,
                  int32_t *new_nbr, void *new_w, int32_t *orig_map, int32_t n_orig, int64_t *new_E,
                  cudaStream_t st, gala_status *status, bool validate_labels, bool sort_rows,
-                 const NextLevelInit &nli, bool labels_only)
+                 const NextLevelInit &nli, bool labels_only, const LevelOrder &order)
 {
     if ((nli.k != nullptr) != (nli.tot != nullptr)) {
         set_error("contraction: K_new needs the community totals");
         *status = GALA_ERR_INVALID;
         return -1;
+    }
+    if (order.order && !sort_rows && !validate_labels && b.long_rows_mode == 0 && g.n <= kSmallContractVertices &&
+        g.E <= kSmallContractEntries) {
+        *status = GALA_OK;
+        const cudaError_t ce = contract_small(g, comm, b, order.order, order.bin_start, new_offs, new_nbr, new_w,
+                                              orig_map, n_orig, nli, labels_only, st);
+        if (ce != cudaSuccess) {
+            *status = cuda_fail(ce, "contraction of a small level");
+            return -1;
+        }
+        DevStats hs;
+        if (!read_stats(&hs, b.stats, st, status, "contraction")) return -1;
+        if (hs.err) {
+            set_error("contraction: device error bits %d", hs.err);
+            *status = hs.err & kErrCapacity ? GALA_ERR_CAPACITY : GALA_ERR_OVERFLOW;
+            return -1;
+        }
+        *new_E = labels_only ? 0 : hs.new_entries;
+        return (int)hs.ccount;
     }
     if (g.wide)
         return contract_t<long long>(g, comm, b, new_offs, new_nbr, (long long *)new_w, orig_map, n_orig, new_E, st,

@@ -1,0 +1,57 @@
+// coop.cuh - pieces shared by the kernels that run a whole small level in one
+// cooperative launch (small_level.cu, small_contract.cu).
+#pragma once
+#include "common.cuh"
+
+namespace gala {
+
+constexpr int kSmallBlock = 512;
+constexpr int kSmallWarps = kSmallBlock / 32;
+constexpr int kSmallMaxGrid = 1024;
+
+// Shared-memory table: the warps' tables (one each) together are the CTA's
+// table (rows up to half of it), 53-74 KB, so that two CTAs fit an SM.
+template <typename WT>
+struct SmallTable {
+    static constexpr int kWarpSlots = WideOf<WT>::exact ? 512 : 256;
+    static constexpr int kSlots = kWarpSlots * kSmallWarps;
+    static constexpr size_t kBytes = (size_t)kSlots * (sizeof(int) + sizeof(WT)) + kSlots / 2 * sizeof(unsigned short);
+};
+
+struct GridBarrier {
+    unsigned arrive;  // arrivals since the launch
+    int dead;         // a wait gave up: every CTA leaves
+};
+
+// Grid barrier (the launch is cooperative: all CTAs are resident).  False when
+// the wait gave up after a few seconds, for every thread of the block; the
+// launch then ends with kErrBarrier.  The block's writes are released with its
+// arrival, the others' acquired by one fence after the last poll (the polls
+// are relaxed: an acquire per poll invalidates the L1 each time).
+__device__ __forceinline__ bool grid_sync(GridBarrier *c, unsigned &target, int *err)
+{
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        target += gridDim.x;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&c->arrive) : "memory");
+        int ok = 1;
+        for (unsigned spin = 0;; ++spin) {
+            unsigned v;
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&c->arrive) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if ((spin & 63) == 63 && (spin > (1u << 22) || *(volatile int *)&c->dead)) {
+                atomicExch(&c->dead, 1);
+                atomicOr(err, kErrBarrier);
+                ok = 0;
+                break;
+            }
+        }
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+}  // namespace gala

@@ -203,6 +203,7 @@ struct Phase1Out {
     long long verify_sweeps = 0;  // full plain sweeps run to judge convergence
     long long movers = 0;         // moves applied (kept or dropped)
     long long nv = 0;             // vertices with edges (the degree-bin order)
+    int bin_start[kNumBins + 1] = {};  // starts of the bins in that order
     long long active_entries = 0; // row entries decided
     long long incr_sweeps = 0;    // sweeps with the incremental weight update
 };
@@ -391,6 +392,7 @@ gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, 
                 if (verbose) printf("Iteration:%d Q:%f\n", 0, o.q0);
             }
             out->nv = o.nv;
+            for (int k = 0; k <= kNumBins; ++k) out->bin_start[k] = o.bin_start[k];
         }
         if (o.err) {
             set_error("phase 1: device error bits %d", o.err);
@@ -625,6 +627,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     note_launch(1);
     long long act_nv = nv_all, act_ne = g.E;
     out->nv = nv_all;
+    for (int k = 0; k <= kNumBins; ++k) out->bin_start[k] = bin_start[k];
     int cur = 0;
     const long long min_tot_init = (!g.wide && m2 > 0x7fffffffLL) ? 0x7fffffffLL : m2;
     unsigned long long skipped0 = h->skipped, skipped_e0 = h->skipped_edges;
@@ -1137,7 +1140,7 @@ gala_status run_levels(gala_context *ctx, int32_t n0, int64_t E0, const int64_t 
             nli.tot = ctx->ref.Kr;
         }
         C = contract_run(g, ccomm, ctx->cb, ctx->offs[buf], ctx->nbr[buf], ctx->w[buf], ctx->orig, n0, &newE, st,
-                         &cs, false, opt && opt->sorted_levels == 1, nli, last);
+                         &cs, false, opt && opt->sorted_levels == 1, nli, last, LevelOrder{ctx->p1.order, po.bin_start});
         if (C < 0) return cs;
         if (do_refine) refine_next_init(ctx->p1.comm, ctx->cb.lab, g.n, ctx->ref, st);
         have_init = do_refine;
@@ -1354,10 +1357,12 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
     ok = ok && cudaMallocHost(&ctx->h_chunk, kChunkInts * sizeof(int32_t)) == cudaSuccess;
     ok = ok && cudaMallocHost(&ctx->h_stats2, sizeof(DevStats)) == cudaSuccess;
     ok = ok && dalloc(ctx, &ctx->d_chunk, kChunkInts) && dalloc(ctx, &ctx->d_stats2, 1);
-    char *ctl = nullptr;
-    ok = ok && dalloc(ctx, &ctl, small_ctl_bytes()) && dalloc(ctx, &ctx->small_out, 1);
+    char *ctl = nullptr, *cctl = nullptr;
+    ok = ok && dalloc(ctx, &ctl, small_ctl_bytes()) && dalloc(ctx, &cctl, contract_ctl_bytes()) &&
+         dalloc(ctx, &ctx->small_out, 1);
     ok = ok && cudaMallocHost(&ctx->h_small_out, sizeof(SmallOut)) == cudaSuccess;
     ctx->small_ctl = ctl;
+    ctx->cb.small_ctl = cctl;
     for (int i = 0; i < 2 && ok; ++i)
         ok = dalloc(ctx, &ctx->offs[i], n + 1) && dalloc(ctx, &ctx->nbr[i], E) && dalloc8(ctx, &ctx->w[i], E);
     Phase1Buffers &b = ctx->p1;

@@ -212,7 +212,8 @@ struct SmallOut {  // what a launch reports (copied to the host in one piece)
     int32_t sweeps, done, err;
     int32_t status;               // 0, 1: sum_k is not the total weight, 2: the hub tables do not fit
     unsigned long long sum_k;     // total weight of the level
-    int32_t nv, pad;              // vertices with edges
+    int32_t nv;                   // vertices with edges
+    int32_t bin_start[9];         // of the degree-bin order
     long long hub_slots;
     long long movers, decisions;  // decisions, entries: without the level's first sweep
     unsigned long long entries, decide_ns, update_ns;
@@ -338,6 +339,7 @@ struct ContractBuffers {
     cudaStream_t aux[kAux] = {};
     cudaEvent_t fork_ev = nullptr;
     cudaEvent_t join_ev[kAux] = {};
+    void *small_ctl = nullptr;  // contract_ctl_bytes() for the one-launch path
 };
 // sort_rows = false (the level-to-level contraction of a Louvain run) leaves
 // every new row in hash-table order: phase 1 does not depend on the order of
@@ -388,9 +390,22 @@ struct NextLevelInit {
     void *k = nullptr;          // receives K_new (WT per new vertex)
     void *self = nullptr;       // receives Self_new (WT per new vertex)
 };
+// The level's degree-bin order (phase 1's list and its bin starts): with it, a
+// level of few entries is contracted in one launch (small_contract.cu).
+struct LevelOrder {
+    const int32_t *order = nullptr;
+    const int *bin_start = nullptr;  // host
+};
 int contract_run(const LevelGraph &g, const int32_t *comm, ContractBuffers &b, int64_t *new_offs,
                  int32_t *new_nbr, void *new_w, int32_t *orig_map, int32_t n_orig,
                  int64_t *new_E, cudaStream_t st, gala_status *status, bool validate_labels = false,
-                 bool sort_rows = true, const NextLevelInit &nli = NextLevelInit(), bool labels_only = false);
+                 bool sort_rows = true, const NextLevelInit &nli = NextLevelInit(), bool labels_only = false,
+                 const LevelOrder &order = LevelOrder());
+// One cooperative launch (small_contract.cu): rows in any order; C, the entry
+// count and the error bits are left in the stats block.
+size_t contract_ctl_bytes();
+cudaError_t contract_small(const LevelGraph &g, const int32_t *comm, ContractBuffers &b, const int32_t *order,
+                           const int *bin_start, int64_t *new_offs, int32_t *new_nbr, void *new_w, int32_t *orig_map,
+                           int32_t n_orig, const NextLevelInit &nli, bool labels_only, cudaStream_t st);
 
 }  // namespace gala

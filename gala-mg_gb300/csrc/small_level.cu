@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "coop.cuh"
 #include "internal.h"
 #include "scan.cuh"
 #include "sweep.cuh"
@@ -30,9 +31,6 @@
 namespace gala {
 
 namespace {
-
-constexpr int kSmallBlock = 512;
-constexpr int kSmallWarps = kSmallBlock / 32;
 
 // Counters of one sweep; three slots in turn, so that a slot is cleared two
 // barriers after its last reader and two before its next writer.
@@ -43,11 +41,9 @@ struct SweepSlot {
     int act_count[kNumBins];
 };
 
-constexpr int kSmallMaxGrid = 1024;
 struct SmallCtl {
     // reset before every launch
-    unsigned arrive;  // grid barrier: arrivals since the launch
-    int dead;         // a barrier wait gave up: every CTA leaves
+    GridBarrier bar;
     // reset before a level's first launch
     unsigned long long sum_k, sum_k2, sum_k2_hi, sum_self;
     // kept between a level's launches
@@ -79,15 +75,6 @@ struct SmallArgs {
     int s0;        // first sweep of this launch (1 = the level's first)
 };
 
-// Warp-table slots per warp: the tables of all warps together are the CTA
-// table (rows up to half of it), 53-74 KB, so that two CTAs fit an SM.
-template <typename WT>
-struct SmallTable {
-    static constexpr int kWarpSlots = WideOf<WT>::exact ? 512 : 256;
-    static constexpr int kSlots = kWarpSlots * kSmallWarps;
-    static constexpr size_t kBytes = (size_t)kSlots * (sizeof(int) + sizeof(WT)) + kSlots / 2 * sizeof(unsigned short);
-};
-
 BinLimits small_limits(const BinLimits &lim, bool wide)
 {
     BinLimits l = lim;
@@ -97,40 +84,6 @@ BinLimits small_limits(const BinLimits &lim, bool wide)
     l.m5 = std::min(l.m5, row6);
     l.m6 = std::min(l.m6, row6);
     return l;
-}
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Grid barrier (the launch is cooperative: all CTAs are resident).  False when
-// the wait gave up after a few seconds, for every thread of the block; the launch
-// then ends with kErrBarrier.
-__device__ __forceinline__ bool grid_sync(SmallCtl *c, unsigned &target, int *err)
-{
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        target += gridDim.x;
-        __threadfence();
-        atomicAdd(&c->arrive, 1u);
-        int ok = 1;
-        for (unsigned spin = 0; (int)(ld_acquire(&c->arrive) - target) < 0; ++spin) {
-            if (spin > (1u << 22) || *(volatile int *)&c->dead) {
-                atomicExch(&c->dead, 1);
-                atomicOr(err, kErrBarrier);
-                ok = 0;
-                break;
-            }
-        }
-        __threadfence();
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
 }
 
 __device__ __forceinline__ unsigned long long now_ns()
@@ -423,7 +376,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         // ---- level init
         if (boss) *err = 0;
         level_vertices(a, false, s_bin);
-        if (!grid_sync(ctl, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err)) return;
         level_vertices(a, true, s_bin);
     } else {
         if (threadIdx.x <= kNumBins) s_bin[threadIdx.x] = ctl->bin_start[threadIdx.x];
@@ -434,7 +387,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
     const bool hubs = hp.H > 0;
     if (fresh) {
         if (!a.ks_ready || hubs || a.init) {
-            if (!grid_sync(ctl, target, err)) return;
+            if (!grid_sync(&ctl->bar, target, err)) return;
             if (!a.ks_ready) {
                 unsigned long long sk = 0, ss = 0;
                 typename SqSum<WT>::T sk2 = 0;
@@ -449,7 +402,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             }
             if (hubs && bid == nb - 1) plan_hubs(a, hp);
         }
-        if (!grid_sync(ctl, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err)) return;
     }
     const long long m2 = a.m2 ? a.m2 : (long long)ctl->sum_k;
     hp.half = ctl->half;
@@ -465,6 +418,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             SmallOut *o = a.out;
             o->sum_k = ctl->sum_k;
             o->nv = s_bin[8];
+            for (int k = 0; k <= kNumBins; ++k) o->bin_start[k] = s_bin[k];
             o->hub_slots = hubs ? hp.half : 0;
             o->sweeps = 0;
             o->done = 1;
@@ -488,7 +442,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             hub_work(hp, wg, nw);
             clear_hubs();
         }
-        if (!grid_sync(ctl, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err)) return;
     }
 
     long long movers = 0, decisions = 0;  // block 0, thread 0
@@ -537,12 +491,12 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             decide_group<WT, 4, W>(d, lists + s_bin[0], c, start((c + 7) / 8), nw, stage);
             int *const mlists[3] = {a.d.mv_v, a.d.mv_old, a.d.mv_new};
             stage.flush(mlists, &cur->n_movers);
-            if (!grid_sync(ctl, target, err)) return;
+            if (!grid_sync(&ctl->bar, target, err)) return;
             if (hubs) {
                 hub_scan<WT, kSmallBlock>(d, hp, a.act_flag, bid, nb);
-                if (!grid_sync(ctl, target, err)) return;
+                if (!grid_sync(&ctl->bar, target, err)) return;
                 hub_final(d, hp, a.act_flag, wg, nw);
-                if (!grid_sync(ctl, target, err)) return;
+                if (!grid_sync(&ctl->bar, target, err)) return;
             }
         }
         if (boss && s > 0) dec_ns += now_ns() - t0;
@@ -552,7 +506,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             apply_moves(a, cur->n_movers, +1);
             if (hubs)
                 for (int i = bid * kSmallBlock + threadIdx.x; i < hp.H; i += nb * kSmallBlock) a.In[hp.hubs[i]] = 0;
-            if (!grid_sync(ctl, target, err)) return;
+            if (!grid_sync(&ctl->bar, target, err)) return;
         }
 
         // ---- totals; hub rows' In and their cleared tables on the side
@@ -583,7 +537,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 }
             }
         }
-        if (!grid_sync(ctl, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err)) return;
         if (boss) t0 = now_ns();
 
         // ---- update and prune
@@ -628,7 +582,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             block_add_u64(sums.edges, &cur->act_edges);
             block_add_i32(sums.act, &cur->act_vertices);
         }
-        if (!grid_sync(ctl, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err)) return;
 
         // ---- convergence (louvain_main_process.cu:1004-1007)
         const int k = s - a.s0;  // sweeps of this launch before this one
