@@ -1749,11 +1749,9 @@ gala_status batch_per_graph(gala_context *ctx, BatchRun &bt, const gala_graph *c
         };
         BatchCtaArgs &a = bt.cta;
         const size_t nv = (size_t)ctx->n_cap, nvo = nv + (size_t)G + 1, ne = (size_t)std::max<int64_t>(ctx->e_cap, 1);
-        int32_t **vert[] = {&a.K, &a.Self, &a.Tot, &a.In, &a.prev, &a.cur, &a.size, &a.cnt, &a.newid, &a.rl,
-                            &a.cursor, &a.members, &a.kc};
+        int32_t **vert[] = {&a.K, &a.Self, &a.size, &a.ec, &a.members, &a.llen[0], &a.llen[1]};
         for (auto p : vert) dal(p, nv);
         dal(&a.moff, nvo);
-        dal(&a.active, nv);
         for (int k = 0; k < 2; ++k) {
             dal(&a.loffs[k], nvo);
             dal(&a.lnbr[k], ne);
@@ -1768,7 +1766,7 @@ gala_status batch_per_graph(gala_context *ctx, BatchRun &bt, const gala_graph *c
         dal(&a.iters_out, G);
         dal(&a.queue, 2);
         // dense tables of long rows: one per warp of the largest grid
-        dal(&a.gacc, batch_cta_gacc_ints(batch_cta_grid(1 << 30), kCtaMaxN));
+        dal(&a.gacc, batch_cta_gacc_ints(batch_cta_grid(1 << 30, 1), kCtaMaxN));
         hal(&bt.h_order, G);
         hal(&bt.h_q, G);
         hal(&bt.h_c, G);
@@ -1800,7 +1798,7 @@ gala_status batch_per_graph(gala_context *ctx, BatchRun &bt, const gala_graph *c
         const int64_t ex = graphs[x]->entries(), ey = graphs[y]->entries();
         return ex != ey ? ex > ey : x < y;
     });
-    const int grid = batch_cta_grid(G);
+    const int grid = batch_cta_grid(G, nmax);
     cudaMemcpyAsync((void *)a.order, bt.h_order, (size_t)G * sizeof(int32_t), cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(a.queue, 0, 2 * sizeof(int), st);
     cudaMemsetAsync(a.gacc, 0, batch_cta_gacc_ints(grid, nmax) * sizeof(int32_t), st);

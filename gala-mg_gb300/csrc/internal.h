@@ -274,9 +274,8 @@ struct BatchCtaArgs {
     const int64_t *u_offs;  // union CSR (device layout)
     const int32_t *u_nbr;
     const int32_t *u_w;     // null: unit weights
-    int32_t *K, *Self, *Tot, *In, *prev, *cur, *size, *cnt, *newid, *rl, *cursor, *members, *kc, *moff;
-    uint8_t *active;
-    int32_t *loffs[2], *lnbr[2], *lw[2];  // contracted level graphs (ping-pong)
+    int32_t *K, *Self, *size, *ec, *members, *moff;
+    int32_t *loffs[2], *llen[2], *lnbr[2], *lw[2];  // contracted level graphs (ping-pong): row starts and lengths
     int32_t *labels;  // out: every input vertex's community, local to its graph
     double *q_out;
     int32_t *c_out, *rounds_out, *iters_out;
@@ -287,7 +286,7 @@ struct BatchCtaArgs {
     int32_t *gacc;  // per warp of the grid: nmax ints, zero (dense tables of long rows)
 };
 void batch_cta_configure();
-int batch_cta_grid(int G);
+int batch_cta_grid(int G, int nmax);
 size_t batch_cta_gacc_ints(int grid, int nmax);
 void batch_cta_launch(const BatchCtaArgs &a, int grid, cudaStream_t st);
 // labels[v] -= goff[g] for the input vertices v of every graph g.
