@@ -26,6 +26,7 @@ namespace gala {
 
 namespace {
 
+constexpr int kContractOneCta = 1024;
 struct ContractCtl {
     // reset before every launch
     GridBarrier bar;
@@ -558,7 +559,8 @@ cudaError_t launch_contract(ContractArgs<WT> &a, cudaStream_t st)
     if (per_sm < 0) return cudaErrorLaunchOutOfResources;
     // a thread per vertex and per four entries
     const long long items = std::max<long long>(a.n, std::max<long long>(a.E / 4, a.n_orig / 4));
-    const long long want = std::max(1LL, (items + kSmallBlock - 1) / kSmallBlock);
+    // (few items stay on one CTA, as in small_level.cu)
+    const long long want = items <= kContractOneCta ? 1 : (items + kSmallBlock - 1) / kSmallBlock;
     const long long grid = std::min<long long>(want, std::min(hub_grid_size() * per_sm, kSmallMaxGrid));
     cudaMemsetAsync(a.ctl, 0, offsetof(ContractCtl, part), st);
     void *args[] = {&a};

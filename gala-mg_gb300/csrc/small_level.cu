@@ -41,6 +41,7 @@ struct SweepSlot {
     int act_count[kNumBins];
 };
 
+constexpr int kSmallOneCta = 64;
 struct SmallCtl {
     // reset before every launch
     GridBarrier bar;
@@ -652,7 +653,9 @@ cudaError_t launch_small(const LevelGraph &g, SmallArgs<WT> &a, cudaStream_t st)
     // warps a sweep keeps busy: about 1.5 lanes per entry, at most 8 vertices
     // a warp
     const long long tasks = g.E * 3 / 64 + g.n / 32;
-    long long grid = (tasks + kSmallWarps - 1) / kSmallWarps;
+    // (a level of few tasks stays on one CTA, which needs no grid barriers and
+    // keeps the level in its L1)
+    long long grid = tasks <= kSmallOneCta ? 1 : (tasks + kSmallWarps - 1) / kSmallWarps;
     grid = std::max(1LL, std::min<long long>(grid, std::min(hub_grid_size() * per_sm, kSmallMaxGrid)));
     cudaMemsetAsync(a.ctl, 0, a.s0 == 1 ? offsetof(SmallCtl, slot) : offsetof(SmallCtl, sum_k), st);
     void *args[] = {&a};
