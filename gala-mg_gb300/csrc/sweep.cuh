@@ -313,10 +313,57 @@ __device__ __forceinline__ void write_features(const DecideArgs<WT, RO> &a, cons
     }
 }
 
+// FP32 as int32 of the same order.
+__device__ __forceinline__ int ordered(float f)
+{
+    const int i = __float_as_int(f);
+    return i ^ ((i >> 31) & 0x7fffffff);
+}
+
+// Merge over a whole warp whose lanes hold different communities: the result of
+// the butterfly merge below from a few warp reductions (a butterfly step moves
+// five or six values).
+__device__ __forceinline__ void warp_best(Cand<int> &b)
+{
+    const int mh = __reduce_max_sync(GALA_FULL_MASK, (int)(b.x >> 32));
+    if (mh < 0) return;  // no candidate in any lane (warp-uniform)
+    const bool top = (int)(b.x >> 32) == mh;
+    const unsigned ml = __reduce_max_sync(GALA_FULL_MASK, top ? (unsigned)b.x : 0u);
+    const bool win = top && (unsigned)b.x == ml;
+    const unsigned wins = __ballot_sync(GALA_FULL_MASK, win);
+    int src = __ffs((int)wins) - 1, t = b.t;
+    if (wins & (wins - 1)) {  // equal best X: the lowest id, a tie when the weights differ
+        const int w0 = __shfl_sync(GALA_FULL_MASK, b.w, src);
+        t = __any_sync(GALA_FULL_MASK, win && (b.t || b.w != w0));
+        const unsigned c0 = __reduce_min_sync(GALA_FULL_MASK, win ? (unsigned)b.c : 0xffffffffu);
+        src = __ffs((int)__ballot_sync(GALA_FULL_MASK, win && (unsigned)b.c == c0)) - 1;
+    }
+    b.c = __shfl_sync(GALA_FULL_MASK, b.c, src);
+    b.w = __shfl_sync(GALA_FULL_MASK, b.w, src);
+    b.t = __shfl_sync(GALA_FULL_MASK, t, src);
+    b.x = ((long long)mh << 32) | ml;
+}
+__device__ __forceinline__ void warp_best(Cand<long long> &b)
+{
+    const int ml = __reduce_max_sync(GALA_FULL_MASK, ordered(b.lo));
+    const int src = __ffs((int)__ballot_sync(GALA_FULL_MASK, ordered(b.lo) == ml)) - 1;
+    const bool win = (int)(threadIdx.x & 31) == src;
+    const int m2 = __reduce_max_sync(GALA_FULL_MASK, ordered(win ? b.hi2 : fmaxf(b.hi, b.hi2)));
+    b.lo = __shfl_sync(GALA_FULL_MASK, b.lo, src);
+    b.hi = __shfl_sync(GALA_FULL_MASK, b.hi, src);
+    b.c = __shfl_sync(GALA_FULL_MASK, b.c, src);
+    b.hi2 = __int_as_float(m2 ^ ((m2 >> 31) & 0x7fffffff));
+}
+
 // Merge over `width` lanes: the candidate and the weight to the own community.
 template <typename WT>
 __device__ __forceinline__ void warp_merge(Cand<WT> &x, WT &wc, int width)
 {
+    if (width == 32) {
+        wc = group_sum(GALA_FULL_MASK, wc);
+        warp_best(x);
+        return;
+    }
     for (int o = width / 2; o >= 1; o >>= 1) {
         wc += __shfl_xor_sync(GALA_FULL_MASK, wc, o);
         x.merge(x.shfl_xor(o));
