@@ -335,7 +335,7 @@ __device__ __forceinline__ int decide_vertex(const LevelView &g, const CtaShared
         const bool ok = lane < deg;
         mc = ok ? (int)lab[u0] : -1;
         const unsigned m = __match_any_sync(GALA_FULL_MASK, mc);
-        ms = g.w ? (int)__reduce_add_sync(m, (unsigned)w0) : __popc(m);
+        ms = g.w ? match_sum(m, ok, w0) : __popc(m);
         lead = ok && __ffs((int)m) - 1 == lane;
         const unsigned own = __ballot_sync(GALA_FULL_MASK, lead && mc == cv);
         if (own) wc = __shfl_sync(GALA_FULL_MASK, ms, __ffs((int)own) - 1);

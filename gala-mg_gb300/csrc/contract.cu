@@ -175,7 +175,7 @@ __global__ void k_relabel(const int32_t *__restrict__ comm, const int32_t *__res
             if (__any_sync(GALA_FULL_MASK, d >> 26)) {
                 if (d) atomicAdd((unsigned long long *)&ec[c], (unsigned long long)d);
             } else {
-                const unsigned t = __reduce_add_sync(m, d);
+                const unsigned t = (unsigned)match_sum(m, d != 0, (int)d);
                 if (d && lane == __ffs((int)m) - 1) atomicAdd((unsigned long long *)&ec[c], (unsigned long long)t);
             }
         }
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(256) k_agg_small(AggArgs<WT> a, const int32_t 
             wt = a.w_at(st + lane);
         }
         const unsigned m = __match_any_sync(GALA_FULL_MASK, key);
-        const WT sum = group_sum(m, wt);
+        const WT sum = match_sum(m, valid, wt);
         const bool head = valid && (__ffs(m) - 1 == lane);
         const unsigned hm = __ballot_sync(GALA_FULL_MASK, head);
         if (head) {

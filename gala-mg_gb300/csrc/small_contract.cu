@@ -126,7 +126,7 @@ template <typename T>
 __device__ __forceinline__ void add_by_label(T *a, int c, unsigned v)
 {
     const unsigned m = __match_any_sync(GALA_FULL_MASK, v ? c : -1);
-    const unsigned t = __reduce_add_sync(m, v);
+    const unsigned t = (unsigned)match_sum(m, v != 0, (int)v);
     if (v && (int)(threadIdx.x & 31) == __ffs((int)m) - 1) {
         if constexpr (sizeof(T) == 8)
             atomicAdd((unsigned long long *)&a[c], (unsigned long long)t);
@@ -246,7 +246,7 @@ __device__ __forceinline__ int row_match(const ContractArgs<WT> &a, const WT *sw
     const int key = ok ? a.skey[e0 + lane] : -1;
     const WT w = ok ? (sw ? sw[e0 + lane] : (WT)1) : (WT)0;
     const unsigned m = __match_any_sync(GALA_FULL_MASK, key);
-    const WT sum = group_sum(m, w);
+    const WT sum = match_sum(m, ok, w);
     const bool head = ok && __ffs((int)m) - 1 == lane;
     const unsigned hm = __ballot_sync(GALA_FULL_MASK, head);
     if (head) {

@@ -483,7 +483,7 @@ __device__ __forceinline__ void decide_group(const DecideArgs<WT, RO> &a, const 
         bool leader;
         if constexpr (G == 32) {
             const unsigned m = __match_any_sync(GALA_FULL_MASK, c);
-            wsum = W ? group_sum(m, wt) : (WT)__popc(m);
+            wsum = W ? match_sum(m, valid, wt) : (WT)__popc(m);
             leader = valid && (__ffs(m) - 1 == lane);
         } else {
             wsum = wt;
@@ -493,7 +493,7 @@ __device__ __forceinline__ void decide_group(const DecideArgs<WT, RO> &a, const 
                 const int osub = (sub + o) & (G - 1);
                 const int src = (lane & ~(G - 1)) | osub;
                 const int oc = __shfl_sync(GALA_FULL_MASK, c, src);
-                const WT ow = __shfl_sync(GALA_FULL_MASK, wt, src);
+                const WT ow = W ? __shfl_sync(GALA_FULL_MASK, wt, src) : (WT)1;
                 if (oc == c) {
                     wsum += ow;
                     if (osub < sub) leader = false;
@@ -1134,13 +1134,13 @@ __device__ __forceinline__ void move_totals(bool valid, int from, int to, WT k, 
 {
     const int lane = threadIdx.x & 31;
     const unsigned mt = __match_any_sync(GALA_FULL_MASK, to);
-    const WT kt = group_sum(mt, k);
+    const WT kt = match_sum(mt, valid, k);
     if (valid && lane == __ffs(mt) - 1) {
         atomic_add_w(&Tot[to], kt);
         atomicAdd(&size[to], __popc(mt));
     }
     const unsigned mf = __match_any_sync(GALA_FULL_MASK, from);
-    const WT kf = group_sum(mf, k);
+    const WT kf = match_sum(mf, valid, k);
     if (valid && lane == __ffs(mf) - 1) {
         atomic_add_w(&Tot[from], (WT)-kf);
         atomicSub(&size[from], __popc(mf));
