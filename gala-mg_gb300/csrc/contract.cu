@@ -2148,10 +2148,12 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
 // Levels contracted in one launch (small_contract.cu): there the general path
 // costs its fifty launches, about 200 us whatever the size.  Whole runs, general
 // path / one launch (ms): 80-vertex SBM 0.76 / 0.60, 1,024-vertex SBM 0.88 /
-// 0.74, R-MAT scale 16 2.79 / 2.52; with levels up to 2^20 entries 2.97 (few
-// large communities, few blocks at work), and levels of over 2^16 vertices
-// gain nothing (R-MAT scale 22, mostly isolated vertices, 18.63 / 18.72).
-constexpr int32_t kSmallContractVertices = 1 << 16;
+// 0.74, R-MAT scale 16 2.79 / 2.52, scale 20 (three levels of 0.5M vertices,
+// nearly all isolated) 7.89 / 7.69; with levels up to 2^20 entries scale 16
+// takes 2.97 (few large communities, few blocks at work).  Labels alone take
+// six launches in the general path: over 2^16 vertices those are faster (scale
+// 22, 2.2M vertices: 18.63 / 18.72).
+constexpr int32_t kSmallContractVertices = 1 << 20, kSmallLabelsVertices = 1 << 16;
 constexpr int64_t kSmallContractEntries = 1 << 18;
 int contract_run(const LevelGraph &g, const int32_t *comm, ContractBuffers &b, int64_t *new_offs,
                  int32_t *new_nbr, void *new_w, int32_t *orig_map, int32_t n_orig, int64_t *new_E,
@@ -2163,7 +2165,7 @@ int contract_run(const LevelGraph &g, const int32_t *comm, ContractBuffers &b, i
         *status = GALA_ERR_INVALID;
         return -1;
     }
-    if (order.order && !sort_rows && !validate_labels && b.long_rows_mode == 0 && g.n <= kSmallContractVertices &&
+    if (order.order && !sort_rows && !validate_labels && b.long_rows_mode == 0 && g.n <= (labels_only ? kSmallLabelsVertices : kSmallContractVertices) &&
         g.E <= kSmallContractEntries) {
         *status = GALA_OK;
         const cudaError_t ce = contract_small(g, comm, b, order.order, order.bin_start, new_offs, new_nbr, new_w,

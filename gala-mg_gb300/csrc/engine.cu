@@ -310,10 +310,11 @@ long long decide_bytes_for(long long nv, long long ne, bool weighted)
 // Levels whose sweeps run in one cooperative launch (small_level.cu).  Below
 // this many entries a sweep costs less than its launches and its host read:
 // phase 1 of planted graphs (one GB300, ms per call, separate launches / one
-// launch) 2.28 / 1.03 at 0.4M entries, 2.57 / 1.90 at 2.4M, 7.75 / 7.72 at
+// launch) 2.28 / 1.03 at 0.4M entries, 2.57 / 1.90 at 2.4M, 6.49 / 7.02 at
 // 9.6M, and 17.3 / 22.3 at 16M, where the one-bin kernels' higher occupancy
-// (48-64 warps per SM against 32) counts for more.
-constexpr int64_t kSmallLevelEntries = 1 << 22;
+// (48-64 warps per SM against 32) counts for more; refined LFR run with a level
+// of 4.7M entries 8.23 / 7.98.
+constexpr int64_t kSmallLevelEntries = 1 << 23;
 bool small_level(const LevelGraph &g) { return g.E <= kSmallLevelEntries; }
 
 // Hub tables and chunk lists: the long-row buffers of the contraction, which
