@@ -1015,17 +1015,18 @@ static void update_t(const LevelGraph &g, Phase1Buffers &b, int bin, const int32
             k_update_group<WT, GV, UV, false><<<grid_lanes(GV), 256, 0, st>>>(a, list, count);         \
     } while (0)
     // groups narrower than the rows, with one predicated batch of loads per lane
-    // up to 32 entries: a warp serves 4-8 vertices and every load of a row is in
-    // flight at once.  Phase 1 of 100k vertices 1.63 -> 1.49 ms, batch of 128
-    // graphs 33.2 -> 32.2 ms, R-MAT scale 22 18.27 -> 18.09 ms against groups of
-    // 4 / 8 / 8 / 16 lanes whose remainder entries load one after the other.
+    // up to 32 entries: a warp serves 8-16 vertices and every load of a row is in
+    // flight at once.  Batch of 128 graphs 33.2 -> 31.9 ms, R-MAT scale 22 18.27
+    // -> 17.96 ms against groups of 4 / 8 / 8 / 16 lanes whose remainder entries
+    // load one after the other (small_level.cu, with half the warps, measured
+    // best with groups of 4 / 4 / 4 / 8).
     switch (bin) {
-    case 0: GALA_UG(4, 1); break;
-    case 1: GALA_UG(4, 2); break;
+    case 0: GALA_UG(2, 2); break;
+    case 1: GALA_UG(2, 4); break;
     case 2: GALA_UG(4, 4); break;
-    case 3: GALA_UG(8, 4); break;
-    case 4: GALA_UG(8, 4); break;
-    case 5: GALA_UG(32, 4); break;
+    case 3: GALA_UG(4, 8); break;
+    case 4: GALA_UG(8, 8); break;
+    case 5: GALA_UG(32, 8); break;
     default: {
         int grid = count < cap ? count : cap;
         if (W)
