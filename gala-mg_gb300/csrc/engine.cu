@@ -548,13 +548,11 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     }
     cudaMemsetAsync(b.act_flag, 1, (size_t)g.n, st);
     // incremental weight updates: plain runs (single graphs and batches) on a
-    // symmetric graph (the symmetry hash of the run's first level, summed by
-    // its level-init row kernels, is 0)
+    // symmetric graph (its symmetry hash is 0; summed once a run, when a sweep
+    // first wants the incremental update or, while rows are being copied, with
+    // the rows' first sweep; contraction keeps the symmetry)
     const bool incr_level = pmode == GALA_PROPOSAL_OFF && ctx->update_mode != 1;
-    if (incr_level) {
-        cudaMemsetAsync(b.moved, 0, (size_t)g.n, st);
-        if (ctx->sym_state < 0 && !pend) ctx->sym_state = (!g.ks_ready && h->sym_hash == 0) ? 1 : 0;
-    }
+    if (incr_level) cudaMemsetAsync(b.moved, 0, (size_t)g.n, st);
     b.features_on = pmode != GALA_PROPOSAL_OFF;
     b.wide = g.wide;
     if (b.features_on) p1_features_init(b, g.n, st);
@@ -670,9 +668,18 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
         // of at least 2^23 entries (below, the full update takes tens of
         // microseconds), after a sweep whose movers held under a third of the
         // entries (otherwise its launches would mostly return at once)
-        const bool incr = incr_level && ctx->sym_state == 1 && iteration > 1 &&
-                          (ctx->update_mode == 2 ||
-                           (g.E >= (1LL << 23) && prev_mv_edges * 3 < (unsigned long long)g.E));
+        bool incr = incr_level && ctx->sym_state != 0 && iteration > 1 &&
+                    (ctx->update_mode == 2 || (g.E >= (1LL << 23) && prev_mv_edges * 3 < (unsigned long long)g.E));
+        if (incr && ctx->sym_state < 0) {
+            p1_sym_hash(g, b, st);
+            unsigned long long hash = 0;
+            if ((s = check(cudaMemcpyAsync(&hash, &b.stats->sym_hash, sizeof(hash), cudaMemcpyDeviceToHost, st),
+                           "symmetry")) ||
+                (s = sync_check(st, "symmetry")))
+                return s;
+            ctx->sym_state = hash == 0 ? 1 : 0;
+            incr = ctx->sym_state == 1;
+        }
         // the sweep: decide, apply, reductions, update, counters to the host
         auto enqueue = [&](bool capturing) {
             // timing events become event nodes of a captured graph
@@ -997,7 +1004,7 @@ gala_status run_levels(gala_context *ctx, int32_t n0, int64_t E0, const int64_t 
                   ctx->n_cap, (long long)ctx->e_cap);
         return GALA_ERR_CAPACITY;
     }
-    ctx->sym_state = -1;  // checked with the first level
+    ctx->sym_state = -1;  // not checked yet
     // degree-bin tuning
     {
         BinLimits lim;
@@ -2122,7 +2129,7 @@ gala_status gala_phase1_device(gala_context *ctx, int32_t n, const int64_t *d_of
     long long m2 = 0;
     std::vector<double> trace;
     Phase1Out po;
-    ctx->sym_state = -1;  // a new graph: checked with its first sweep
+    ctx->sym_state = -1;  // a new graph: not checked yet
     if ((s = phase1(ctx, g, m2, min_modularity, false, &trace, &po))) return s;
     if ((s = check(cudaMemcpyAsync(d_community_out, ctx->p1.comm, (size_t)n * sizeof(int32_t),
                                    cudaMemcpyDeviceToDevice, st),

@@ -196,6 +196,7 @@ struct PendingRows {
 void p1_configure_kernels();
 void contract_configure_kernels();
 void p1_reset_level_stats(Phase1Buffers &b, cudaStream_t st);
+void p1_sym_hash(const LevelGraph &g, Phase1Buffers &b, cudaStream_t st);
 int hub_grid_size();
 void p1_hub_plan_launch(const LevelGraph &g, Phase1Buffers &b, HubPlan &p, cudaStream_t st);
 void p1_hub_work_launch(HubPlan &p, cudaStream_t st);

@@ -150,11 +150,84 @@ __device__ __forceinline__ unsigned long long sym_term(int v, int u, unsigned lo
     return dir_hash(v, u, w) - dir_hash(u, v, w);
 }
 
+// Symmetry hash of a level, summed when a sweep first wants the incremental
+// update: summed in every level init it cost 2 % of a run on 2^22 R-MAT
+// vertices (17.98 ms against 17.65), which never asks for it.  A warp takes 1024 consecutive entries
+// whatever rows they belong to: each lane finds its first entry's row by
+// bisection and walks the offsets from there, so that a hub costs no more than
+// the same entries in short rows (eight lanes per row cost 0.3 ms on 2^20 R-MAT
+// vertices, most of it the hubs' tail).
+constexpr int kHashChunk = 1024;
+template <typename WT, bool W>
+__global__ void __launch_bounds__(256) k_sym_hash(int n, long long E, const int64_t *__restrict__ offs,
+                                                  const int32_t *__restrict__ nbr, const WT *__restrict__ w,
+                                                  DevStats *st)
+{
+    constexpr int U = 8;
+    const int lane = threadIdx.x & 31;
+    const long long c0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kHashChunk;
+    const long long c1 = c0 + kHashChunk < E ? c0 + kHashChunk : E;
+    unsigned long long hs = 0;
+    if (c0 < E) {
+        int lo = 0, hi = n;  // offs[lo] <= c0 < offs[hi]
+        while (hi - lo > 1) {
+            const int mid = lo + ((hi - lo) >> 1);
+            if (offs[mid] <= c0) lo = mid;
+            else hi = mid;
+        }
+        int r = lo;
+        long long end = offs[r + 1];
+        for (long long j = c0 + lane; j < c1; j += U * 32) {
+            int u[U];
+            WT wt[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const bool in = j + q * 32 < c1;
+                u[q] = in ? nbr[j + q * 32] : 0;
+                wt[q] = W && in ? w[j + q * 32] : (WT)1;
+            }
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                if (j + q * 32 >= c1) break;
+                while (end <= j + q * 32) end = offs[++r + 1];
+                hs += sym_term(r, u[q], (unsigned long long)wt[q]);
+            }
+        }
+    }
+    block_add_u64(hs, &st->sym_hash);
+}
+
+// Weight, self-loop weight (the last one seen) and, with H, symmetry hash of
+// the entries j, j + step, ... < e of vertex v's row.
+template <typename WT, bool W, bool H>
+__device__ __forceinline__ void row_sums(const int32_t *__restrict__ nbr, const WT *__restrict__ w, long long j,
+                                         long long e, int step, int v, WT &k, WT &sf, unsigned long long &hs)
+{
+    constexpr int U = 4;
+    for (; j < e; j += (long long)U * step) {
+        int u[U];
+        WT wt[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const long long i = j + (long long)q * step;
+            u[q] = i < e ? nbr[i] : -1;
+            wt[q] = i < e ? (W ? w[i] : (WT)1) : (WT)0;
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            if (H && u[q] < 0) break;
+            k += wt[q];
+            if (u[q] == v) sf = wt[q];
+            if (H) hs += sym_term(v, u[q], (unsigned long long)wt[q]);
+        }
+    }
+}
+
 // K = row weight sum, Self = self-loop weight (init_communities,
 // kernel_functions.cu:34-73); Tot = K, In = Self.  Accumulates sum(K),
-// sum(K^2) and sum(Self) for the modularity of the singleton partition, and
-// the symmetry hash.
-template <typename WT, int G, bool W>
+// sum(K^2) and sum(Self) for the modularity of the singleton partition and, with
+// H, the symmetry hash.  Four entries per lane in flight.
+template <typename WT, int G, bool W, bool H>
 __global__ void __launch_bounds__(256) k_init_rows_group(const int32_t *__restrict__ list, int count,
                                                          const int64_t *__restrict__ offs,
                                                          const int32_t *__restrict__ nbr,
@@ -178,13 +251,7 @@ __global__ void __launch_bounds__(256) k_init_rows_group(const int32_t *__restri
             e = offs[v + 1];
         }
         WT k = 0, sf = 0;
-        for (long long j = s + sub; j < e; j += G) {
-            WT wt = W ? w[j] : 1;
-            const int u = nbr[j];
-            k += wt;
-            if (u == v) sf = wt;
-            hs += sym_term(v, u, (unsigned long long)wt);
-        }
+        row_sums<WT, W, H>(nbr, w, s + sub, e, G, v, k, sf, hs);
 #pragma unroll
         for (int o = G / 2; o >= 1; o >>= 1) {
             k += __shfl_xor_sync(GALA_FULL_MASK, k, o);
@@ -203,10 +270,10 @@ __global__ void __launch_bounds__(256) k_init_rows_group(const int32_t *__restri
     block_add_u64(sk, &st->sum_k);
     SqSum<WT>::add(sk2, &st->sum_tot2, &st->sum_tot2_hi);
     block_add_u64(ss, &st->sum_in);
-    block_add_u64(hs, &st->sym_hash);
+    if (H) block_add_u64(hs, &st->sym_hash);
 }
 
-template <typename WT, bool W>
+template <typename WT, bool W, bool H>
 __global__ void __launch_bounds__(256) k_init_rows_cta(const int32_t *__restrict__ list, int count,
                                                        const int64_t *__restrict__ offs,
                                                        const int32_t *__restrict__ nbr,
@@ -220,13 +287,7 @@ __global__ void __launch_bounds__(256) k_init_rows_cta(const int32_t *__restrict
         int v = list[i];
         long long s = offs[v], e = offs[v + 1];
         WT k = 0, sf = 0;
-        for (long long j = s + threadIdx.x; j < e; j += blockDim.x) {
-            WT wt = W ? w[j] : 1;
-            const int u = nbr[j];
-            k += wt;
-            if (u == v) sf = wt;
-            hs += sym_term(v, u, (unsigned long long)wt);
-        }
+        row_sums<WT, W, H>(nbr, w, s + threadIdx.x, e, blockDim.x, v, k, sf, hs);
         k = warp_sum(k);
         sf = warp_sum(sf);
         if ((threadIdx.x & 31) == 0) {
@@ -254,7 +315,7 @@ __global__ void __launch_bounds__(256) k_init_rows_cta(const int32_t *__restrict
     block_add_u64(sk, &st->sum_k);
     SqSum<WT>::add(sk2, &st->sum_tot2, &st->sum_tot2_hi);
     block_add_u64(ss, &st->sum_in);
-    block_add_u64(hs, &st->sym_hash);
+    if (H) block_add_u64(hs, &st->sym_hash);
 }
 
 __global__ void k_reset_level_stats(DevStats *st)
@@ -267,7 +328,21 @@ __global__ void k_reset_level_stats(DevStats *st)
     st->max_deg = 0;
     st->err = 0;
     st->n_movers = 0;
-    st->sym_hash = 0;
+}
+
+// Symmetry hash of level g (stats->sym_hash).
+void p1_sym_hash(const LevelGraph &g, Phase1Buffers &b, cudaStream_t st)
+{
+    cudaMemsetAsync(&b.stats->sym_hash, 0, sizeof(b.stats->sym_hash), st);
+    const int grid = (int)((g.E + 8 * kHashChunk - 1) / (8 * kHashChunk));
+    if (grid == 0) return;
+    if (g.wide)
+        k_sym_hash<long long, true><<<grid, 256, 0, st>>>(g.n, g.E, g.offs, g.nbr, (const long long *)g.w, b.stats);
+    else if (g.w)
+        k_sym_hash<int, true><<<grid, 256, 0, st>>>(g.n, g.E, g.offs, g.nbr, (const int *)g.w, b.stats);
+    else
+        k_sym_hash<int, false><<<grid, 256, 0, st>>>(g.n, g.E, g.offs, g.nbr, nullptr, b.stats);
+    note_launch(1);
 }
 
 void p1_reset_level_stats(Phase1Buffers &b, cudaStream_t st)
@@ -276,7 +351,7 @@ void p1_reset_level_stats(Phase1Buffers &b, cudaStream_t st)
     note_launch(1);
 }
 
-template <typename WT>
+template <typename WT, bool H = false>
 static void launch_init_rows(const LevelGraph &g, Phase1Buffers &b, int bin, const int32_t *list, int cnt,
                              cudaStream_t st, DevStats *stats = nullptr)
 {
@@ -293,11 +368,11 @@ static void launch_init_rows(const LevelGraph &g, Phase1Buffers &b, int bin, con
 #define GALA_INIT_GROUP(GV)                                                                              \
     do {                                                                                                 \
         if (W)                                                                                           \
-            k_init_rows_group<WT, GV, true><<<grid_for(GV), 256, 0, st>>>(list, cnt, g.offs, g.nbr, w, K,  \
-                                                                          Self, Tot, In, stats);         \
+            k_init_rows_group<WT, GV, true, H><<<grid_for(GV), 256, 0, st>>>(list, cnt, g.offs, g.nbr,   \
+                                                                             w, K, Self, Tot, In, stats); \
         else                                                                                             \
-            k_init_rows_group<WT, GV, false><<<grid_for(GV), 256, 0, st>>>(list, cnt, g.offs, g.nbr, w, K, \
-                                                                           Self, Tot, In, stats);        \
+            k_init_rows_group<WT, GV, false, H><<<grid_for(GV), 256, 0, st>>>(list, cnt, g.offs, g.nbr,  \
+                                                                              w, K, Self, Tot, In, stats); \
     } while (0)
     switch (bin) {
     case 0: GALA_INIT_GROUP(4); break;
@@ -309,9 +384,9 @@ static void launch_init_rows(const LevelGraph &g, Phase1Buffers &b, int bin, con
     default: {
         int grid = cnt < cap ? cnt : cap;
         if (W)
-            k_init_rows_cta<WT, true><<<grid, 256, 0, st>>>(list, cnt, g.offs, g.nbr, w, K, Self, Tot, In, stats);
+            k_init_rows_cta<WT, true, H><<<grid, 256, 0, st>>>(list, cnt, g.offs, g.nbr, w, K, Self, Tot, In, stats);
         else
-            k_init_rows_cta<WT, false><<<grid, 256, 0, st>>>(list, cnt, g.offs, g.nbr, w, K, Self, Tot, In, stats);
+            k_init_rows_cta<WT, false, H><<<grid, 256, 0, st>>>(list, cnt, g.offs, g.nbr, w, K, Self, Tot, In, stats);
     }
     }
 #undef GALA_INIT_GROUP
@@ -398,9 +473,9 @@ void p1_init_rows_range(const LevelGraph &g, Phase1Buffers &b, int bin, const in
                         cudaStream_t st)
 {
     if (g.wide)
-        launch_init_rows<long long>(g, b, bin, list, cnt, st, stats);
+        launch_init_rows<long long, true>(g, b, bin, list, cnt, st, stats);
     else
-        launch_init_rows<int>(g, b, bin, list, cnt, st, stats);
+        launch_init_rows<int, true>(g, b, bin, list, cnt, st, stats);
 }
 
 void p1_level_init_rows(const LevelGraph &g, Phase1Buffers &b, const int *bin_start, cudaStream_t st)

@@ -11,8 +11,8 @@
 // exact, and In, the pruning bound, the next active lists and the sums equal
 // those of the full update bit for bit.  A sweep takes this path when its
 // movers' rows hold a small share of the level's entries, on a graph whose
-// entries all have mirrors (the level-init row kernels of phase1.cu sum a
-// hash of every entry minus its mirror).  A batch's union takes it too: its
+// entries all have mirrors (k_sym_hash sums a hash of every entry minus its
+// mirror when the path is first wanted in a run).  A batch's union takes it too: its
 // sweeps after the first few move little (128 graphs, 58M entries, 107 sweeps:
 // the run goes from 45.5 to 41.7 ms).
 #include "common.cuh"

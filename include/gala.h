@@ -294,7 +294,7 @@ gala_status gala_context_set_hub_table_cap(gala_context *ctx, int64_t slots);
  * third of the level's entries updates In incrementally - each mover's In is
  * summed again over its row and +-w is pushed from each mover to its
  * neighbours that did not move - on graphs whose every entry (v, u, w) has a
- * mirror (u, v, w), checked once per run; mode 1: always the full update;
+ * mirror (u, v, w), checked once per run when first needed; mode 1: always the full update;
  * mode 2: incrementally whenever allowed (symmetric graph, from a level's
  * second sweep on).  Integer sums: every mode gives the same In, active sets
  * and results bit for bit.  Plain runs, of one graph or of a batch's union;
