@@ -426,7 +426,7 @@ class Context:
         PROPOSAL_SKIP decides only the vertices it proposes; `refine` turns
         on the Leiden-style refinement."""
         n, _, _ = graph.info()
-        labels = np.zeros(n, dtype=np.int32)
+        labels = np.empty(n, dtype=np.int32)
         trace = np.zeros(iter_capacity, dtype=np.float64)
         r = Result()
         r.iter_modularity = _ptr(trace, _f64p)
@@ -464,7 +464,7 @@ class Context:
         counts plus the batch timings."""
         G = len(graphs)
         sizes = [g.info()[0] for g in graphs]
-        labels = np.zeros(sum(sizes), dtype=np.int32)
+        labels = np.empty(sum(sizes), dtype=np.int32)
         q = np.zeros(G, dtype=np.float64)
         c = np.zeros(G, dtype=np.int32)
         hs = (_vp * G)(*[g.h for g in graphs])
