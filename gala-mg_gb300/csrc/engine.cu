@@ -408,7 +408,7 @@ gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, 
     int iteration = 1;
     cudaEventRecord(ctx->ev[0], st);
     for (bool done = false; !done;) {
-        const SmallRun r{ctx->small_ctl, ctx->small_out, init, cb.big_pool_ints, cb.big_work_cap, cb.big_twork_cap, m2,
+        const SmallRun r{ctx->small_ctl, ctx->small_out, cb.ebase, init, cb.big_pool_ints, cb.big_work_cap, cb.big_twork_cap, m2,
                          min_mod, prev_q, fp64_only, iteration};
         if ((s = check(small_level_run(g, b, hp, r, st), "small level"))) return s;
         cudaEventRecord(ctx->ev[1], st);

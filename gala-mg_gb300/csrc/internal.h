@@ -223,6 +223,7 @@ struct SmallOut {  // what a launch reports (copied to the host in one piece)
 struct SmallRun {
     void *ctl;             // small_ctl_bytes() of device memory, kept between launches of a level
     SmallOut *out;         // device
+    void *tot_next;        // n totals (8 bytes each), kept between launches of a level
     const int32_t *init;   // starting community of every vertex (null: its own)
     long long pool_ints, work_cap, twork_cap;  // hub scratch
     long long m2;          // total weight (0: the level's)

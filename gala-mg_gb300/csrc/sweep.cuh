@@ -90,6 +90,7 @@ struct DecideArgs {
     typename SweepPtr<WT, RO>::type Tot;
     typename SweepPtr<int32_t, RO>::type size;
     int32_t *mv_v, *mv_old, *mv_new;
+    WT *tot_next;  // !RO: totals after the sweep, moved along with the mover lists
     int *n_movers, *err;
     unsigned long long *fp64_decisions;
     double constant;  // 1 / m2
@@ -417,6 +418,31 @@ struct CandRow<long long, N> {
     }
 };
 
+constexpr int kStageN = 256;  // staged active-list appends per warp
+constexpr int kStageM = 128;  // staged movers per warp
+
+// Totals and sizes of a warp's movers (Tot += Tot_update, size += size_update,
+// louvain_main_process.cu:949-953), or one of the two.  Movers of one warp that
+// share a source or a target community add to its Tot and size once (many
+// movers of a sweep head for the same large community).  All 32 lanes call.
+template <typename WT, bool TOT = true, bool SIZE = true>
+__device__ __forceinline__ void move_totals(bool valid, int from, int to, WT k, WT *Tot, int32_t *size)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned mt = __match_any_sync(GALA_FULL_MASK, to);
+    const WT kt = TOT ? match_sum(mt, valid, k) : (WT)0;
+    if (valid && lane == __ffs(mt) - 1) {
+        if (TOT) atomic_add_w(&Tot[to], kt);
+        if (SIZE) atomicAdd(&size[to], __popc(mt));
+    }
+    const unsigned mf = __match_any_sync(GALA_FULL_MASK, from);
+    const WT kf = TOT ? match_sum(mf, valid, k) : (WT)0;
+    if (valid && lane == __ffs(mf) - 1) {
+        if (TOT) atomic_add_w(&Tot[from], (WT)-kf);
+        if (SIZE) atomicSub(&size[from], __popc(mf));
+    }
+}
+
 template <typename WT, bool RO>
 __device__ __forceinline__ void append_mover(const DecideArgs<WT, RO> &a, bool move, int v, int cur, int best)
 {
@@ -432,15 +458,41 @@ __device__ __forceinline__ void append_mover(const DecideArgs<WT, RO> &a, bool m
         a.mv_v[p] = v;
         a.mv_old[p] = cur;
         a.mv_new[p] = best;
+        if constexpr (!RO) {
+            const WT k = a.K[v];
+            atomic_add_w(&a.tot_next[best], k);
+            atomic_add_w(&a.tot_next[cur], (WT)-k);
+        }
     }
+}
+
+// A warp's staged movers to the lists; with !RO their totals move too.
+template <typename WT, bool RO>
+__device__ __forceinline__ void flush_movers(const DecideArgs<WT, RO> &a, WarpStage<kStageM, 3> &stage)
+{
+    int *const lists[3] = {a.mv_v, a.mv_old, a.mv_new};
+    if constexpr (!RO) {
+        __syncwarp();
+        for (int i0 = 0; i0 < stage.n; i0 += 32) {
+            const int i = i0 + (threadIdx.x & 31);
+            const bool valid = i < stage.n;
+            int from = -1, to = -1;
+            WT k = 0;
+            if (valid) {
+                k = a.K[stage.buf[i]];
+                from = stage.buf[kStageM + i];
+                to = stage.buf[2 * kStageM + i];
+            }
+            move_totals<WT, true, false>(valid, from, to, k, a.tot_next, nullptr);
+        }
+    }
+    stage.flush(lists, a.n_movers);
 }
 
 // Degree <= G: one lane per neighbour.  Lanes holding the same neighbour
 // community are found with __match_any_sync (the key carries the group index
 // so groups of one warp stay apart) and their weights summed with
 // __reduce_add_sync; the lowest lane of each set evaluates the gain.
-constexpr int kStageN = 256;  // staged active-list appends per warp
-constexpr int kStageM = 128;  // staged movers per warp
 // A warp takes the tasks (32 / G vertices each) wg, wg + nw, ... of the list.
 template <typename WT, int G, bool W, bool RO>
 __device__ __forceinline__ void decide_group(const DecideArgs<WT, RO> &a, const int32_t *list, int count, int wg,
@@ -546,6 +598,7 @@ __device__ __forceinline__ void decide_group(const DecideArgs<WT, RO> &a, const 
             if (has && sub == 0) write_features(a, sc, v, best, wc, sf, ki, __popc(lb & gmask));
         }
         const int item[3] = {v, cur, bc};
+        if (!RO && stage.n + 32 > kStageM) flush_movers(a, stage);
         stage.push(move, item, mlists, a.n_movers);
     }
 }
@@ -1122,28 +1175,6 @@ __device__ __forceinline__ void hub_final(const DecideArgs<WT, RO> &a, const Hub
         }
         const bool move = lane == 0 && dec == 1 && guard_ok(a, cur, bc);
         append_mover(a, move, v, cur, bc);
-    }
-}
-
-// Totals and sizes of a warp's movers (Tot += Tot_update, size += size_update,
-// louvain_main_process.cu:949-953).  Movers of one warp that share a source or
-// a target community add to its Tot and size once (many movers of a sweep head
-// for the same large community).  All 32 lanes call.
-template <typename WT>
-__device__ __forceinline__ void move_totals(bool valid, int from, int to, WT k, WT *Tot, int32_t *size)
-{
-    const int lane = threadIdx.x & 31;
-    const unsigned mt = __match_any_sync(GALA_FULL_MASK, to);
-    const WT kt = match_sum(mt, valid, k);
-    if (valid && lane == __ffs(mt) - 1) {
-        atomic_add_w(&Tot[to], kt);
-        atomicAdd(&size[to], __popc(mt));
-    }
-    const unsigned mf = __match_any_sync(GALA_FULL_MASK, from);
-    const WT kf = match_sum(mf, valid, k);
-    if (valid && lane == __ffs(mf) - 1) {
-        atomic_add_w(&Tot[from], (WT)-kf);
-        atomicSub(&size[from], __popc(mf));
     }
 }
 
