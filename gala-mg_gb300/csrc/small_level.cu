@@ -91,6 +91,8 @@ BinLimits small_limits(const BinLimits &lim, bool wide)
     return l;
 }
 
+// (read twice a launch: the steps are timed in SM cycles, since a read of the
+// global timer takes a good part of a step of a tiny level)
 __device__ __forceinline__ unsigned long long now_ns()
 {
     unsigned long long t;
@@ -100,9 +102,8 @@ __device__ __forceinline__ unsigned long long now_ns()
 
 // Q from exact sums, the host's expression (q_from_sums in engine.cu) in the
 // same order.
-__device__ double slot_q(const SweepSlot &s, long long m2)
+__device__ double slot_q(const SweepSlot &s, double c)
 {
-    const double c = __ddiv_rn(1.0, (double)m2);
     const double t2 = __dadd_rn(__dmul_rn((double)s.sum_tot2_hi, 18446744073709551616.0), (double)s.sum_tot2);
     return __dsub_rn(__dmul_rn((double)(long long)s.sum_in, c), __dmul_rn(__dmul_rn(t2, c), c));
 }
@@ -344,6 +345,34 @@ __device__ __forceinline__ void plan_hubs(const SmallArgs<WT> &a, const HubPlan 
     }
 }
 
+// The block's share of In, active entries and active vertices to the sweep's
+// counters, in one reduction.
+__device__ __forceinline__ void block_sums(const UpdateSums &sums, SweepSlot &slot)
+{
+    __shared__ unsigned long long s_sums[3][kSmallWarps];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    unsigned long long x[3] = {sums.in, sums.edges, (unsigned long long)sums.act};
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) x[k] += __shfl_xor_sync(GALA_FULL_MASK, x[k], o);
+    if (lane < 3) s_sums[lane][wib] = lane == 0 ? x[0] : (lane == 1 ? x[1] : x[2]);
+    __syncthreads();
+    if (wib == 0) {  // (the sums' next writer comes after a grid barrier)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            x[k] = s_sums[k][lane & (kSmallWarps - 1)];
+#pragma unroll
+            for (int o = kSmallWarps / 2; o >= 1; o >>= 1) x[k] += __shfl_xor_sync(GALA_FULL_MASK, x[k], o);
+        }
+        if (lane == 0) {
+            if (x[0]) atomicAdd(&slot.sum_in, x[0]);
+            if (x[1]) atomicAdd(&slot.act_edges, x[1]);
+            if (x[2]) atomicAdd(&slot.act_vertices, (int)x[2]);
+        }
+    }
+}
+
 template <typename WT, bool W>
 __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_constant__ SmallArgs<WT> a)
 {
@@ -351,6 +380,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
     extern __shared__ long long small_sm[];
     __shared__ int stage_buf[kSmallWarps][3 * kStageM];
     __shared__ int s_go, s_bin[kNumBins + 1];
+    __shared__ long long s_min[kSmallWarps];
     static_assert(kStageN <= 3 * kStageM, "the two stages share their buffer");
     WT *vals = (WT *)small_sm;
     int *keys = (int *)(vals + Tab::kSlots);
@@ -412,6 +442,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         if (!grid_sync(&ctl->bar, target, err)) return;
     }
     const long long m2 = a.m2 ? a.m2 : (long long)ctl->sum_k;
+    const double constant = __ddiv_rn(1.0, (double)m2);
     hp.half = ctl->half;
     hp.nwork = ctl->nwork;
     hp.ntwork = ctl->ntwork;
@@ -438,7 +469,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             q0.sum_in = ctl->sum_self;
             q0.sum_tot2 = ctl->sum_k2;
             q0.sum_tot2_hi = ctl->sum_k2_hi;
-            prev_q = slot_q(q0, m2);
+            prev_q = slot_q(q0, constant);
             if (bid == 0) a.out->q0 = prev_q;
         }
         if (boss) {
@@ -454,23 +485,29 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
     }
 
     long long movers = 0, decisions = 0;  // block 0, thread 0
-    unsigned long long entries = 0, dec_ns = 0, upd_ns = 0;
+    unsigned long long entries = 0;
+    const unsigned long long ns0 = boss ? now_ns() : 0;
+    const long long cyc0 = clock64();
+    long long dec_cyc = 0, upd_cyc = 0;
     int done = 0, s = fresh && a.init ? 0 : a.s0;  // sweep 0: In and Q of a starting partition
     for (;; ++s) {
         SweepSlot *const cur = &ctl->slot[s % 3];
         const SweepSlot *const prev = &ctl->slot[(s + 2) % 3];
         const bool first = s == 1;
         const int32_t *const lists = first ? a.order : a.act[(s + 1) & 1];
-        auto count = [&](int bin) { return first ? s_bin[bin + 1] - s_bin[bin] : prev->act_count[bin]; };
-        unsigned long long t0 = 0;
-        if (boss) t0 = now_ns();
+        // rows of the bins, one bin per lane: one read after the barrier instead
+        // of one in front of every bin
+        int counts = 0;
+        if (lane < kNumBins) counts = first ? s_bin[lane + 1] - s_bin[lane] : prev->act_count[lane];
+        auto count = [&](int bin) { return __shfl_sync(GALA_FULL_MASK, counts, bin); };
+        long long t0 = clock64();
 
         // ---- decide
         if (s > 0) {
             DecideArgs<WT, false> d = a.d;
             d.n_movers = &cur->n_movers;
             d.m2 = m2;
-            d.constant = __ddiv_rn(1.0, (double)m2);
+            d.constant = constant;
             int c = count(6);
             decide_cta<WT, kSmallBlock, W>(d, lists + s_bin[6], c, bid, nb, Tab::kSlots, 0, INT_MAX, keys, vals,
                                            occ);
@@ -506,7 +543,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 if (!grid_sync(&ctl->bar, target, err)) return;
             }
         }
-        if (boss && s > 0) dec_ns += now_ns() - t0;
+        if (s > 0) dec_cyc += clock64() - t0;
 
         // ---- labels and sizes; with hub rows a step of their own, since these
         // rows' In is summed over the new labels in the next one
@@ -532,8 +569,14 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             }
 #pragma unroll
             for (int o = 16; o >= 1; o >>= 1) mn = min(mn, __shfl_xor_sync(GALA_FULL_MASK, mn, o));
-            if (lane == 0 && mn != 0x7fffffffffffffffLL) atomicMin(&cur->min_tot, mn);
-            SqSum<WT>::add(s2, &cur->sum_tot2, &cur->sum_tot2_hi);
+            if (lane == 0) s_min[wib] = mn;
+            SqSum<WT>::add(s2, &cur->sum_tot2, &cur->sum_tot2_hi);  // (block barriers inside)
+            if (wib == 0) {
+                mn = s_min[lane & (kSmallWarps - 1)];
+#pragma unroll
+                for (int o = kSmallWarps / 2; o >= 1; o >>= 1) mn = min(mn, __shfl_xor_sync(GALA_FULL_MASK, mn, o));
+                if (lane == 0 && mn != 0x7fffffffffffffffLL) atomicMin(&cur->min_tot, mn);
+            }
             if (hubs) {
                 hub_in_partial<WT, W>(a.u, hp, nb - 1 - bid, nb);
                 clear_hubs();
@@ -548,13 +591,13 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             }
         }
         if (!grid_sync(&ctl->bar, target, err)) return;
-        if (boss) t0 = now_ns();
+        t0 = clock64();
 
         // ---- update and prune
         {
             UpdateArgs<WT, false> u = a.u;
             u.m2 = m2;
-            u.constant = __ddiv_rn(1.0, (double)m2);
+            u.constant = constant;
             const long long mt = cur->min_tot;
             UpdateSums sums;
             WarpStage<kStageN, 1> stage{stage_buf[wib], 0};
@@ -588,21 +631,19 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 u.act_counter = &cur->act_count[7];
                 hub_in_final(u, hp, mt, bid, nb, sums);
             }
-            block_add_u64(sums.in, &cur->sum_in);
-            block_add_u64(sums.edges, &cur->act_edges);
-            block_add_i32(sums.act, &cur->act_vertices);
+            block_sums(sums, *cur);
         }
         if (!grid_sync(&ctl->bar, target, err)) return;
 
         // ---- convergence (louvain_main_process.cu:1004-1007)
         const int k = s - a.s0;  // sweeps of this launch before this one
         if (s == 0) {
-            if (threadIdx.x == 0) prev_q = slot_q(*cur, m2);
+            if (threadIdx.x == 0) prev_q = slot_q(*cur, constant);
             if (boss) a.out->q0 = prev_q;
             continue;
         }
         if (threadIdx.x == 0) {
-            const double q = slot_q(*cur, m2);
+            const double q = slot_q(*cur, constant);
             int go = 1;
             if (*(volatile int *)err)
                 go = 0;
@@ -612,7 +653,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 prev_q = q;
             s_go = go;
             if (bid == 0) {
-                upd_ns += now_ns() - t0;
+                upd_cyc += clock64() - t0;
                 a.out->trace[k] = q;
             }
         }
@@ -635,8 +676,9 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         o->movers = movers;
         o->decisions = decisions;
         o->entries = entries;
-        o->decide_ns = dec_ns;
-        o->update_ns = upd_ns;
+        const double ns = (double)(now_ns() - ns0) / (double)max(clock64() - cyc0, 1LL);  // per cycle
+        o->decide_ns = (unsigned long long)((double)dec_cyc * ns);
+        o->update_ns = (unsigned long long)((double)upd_cyc * ns);
     }
 }
 
