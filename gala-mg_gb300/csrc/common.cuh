@@ -341,7 +341,12 @@ struct WarpStage {
         const int lane = threadIdx.x & 31;
         int base = 0;
         if (lane == 0) base = atomicAdd(counter, n);
-        base = __shfl_sync(GALA_FULL_MASK, base, 0);
+        store(lists, __shfl_sync(GALA_FULL_MASK, base, 0));
+    }
+    // All items to the lists from position base on.
+    __device__ __forceinline__ void store(int *const *lists, int base)
+    {
+        const int lane = threadIdx.x & 31;
 #pragma unroll
         for (int k = 0; k < K; ++k)
             for (int i = lane; i < n; i += 32) lists[k][base + i] = buf[k * N + i];

@@ -345,6 +345,21 @@ __device__ __forceinline__ void plan_hubs(const SmallArgs<WT> &a, const HubPlan 
     }
 }
 
+// log2 of the rows per warp task of the update, bins 0 to 5.
+__device__ constexpr int kUpdShift[6] = {3, 3, 3, 2, 2, 0};
+
+// Warp wg's first task of every bin, one bin per lane (tasks: the bin's, 0 in
+// the other lanes), when the bins from the highest down share the nw warps round
+// robin.
+__device__ __forceinline__ int first_tasks(int tasks, int wg, int nw)
+{
+    int sum = tasks;  // of this lane's bin and those above
+#pragma unroll
+    for (int o = 1; o < 8; o *= 2) sum += __shfl_down_sync(GALA_FULL_MASK, sum, o);
+    const int w0 = wg - (sum - tasks) % nw;
+    return w0 < 0 ? w0 + nw : w0;
+}
+
 // The block's share of In, active entries and active vertices to the sweep's
 // counters, in one reduction.
 __device__ __forceinline__ void block_sums(const UpdateSums &sums, SweepSlot &slot)
@@ -381,6 +396,10 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
     __shared__ int stage_buf[kSmallWarps][3 * kStageM];
     __shared__ int s_go, s_bin[kNumBins + 1];
     __shared__ long long s_min[kSmallWarps];
+    __shared__ struct {
+        long long movers, decisions, cyc0, dec_cyc, upd_cyc;
+        unsigned long long entries, ns0;
+    } s_stat;  // block 0's
     static_assert(kStageN <= 3 * kStageM, "the two stages share their buffer");
     WT *vals = (WT *)small_sm;
     int *keys = (int *)(vals + Tab::kSlots);
@@ -484,11 +503,23 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         if (!grid_sync(&ctl->bar, target, err)) return;
     }
 
-    long long movers = 0, decisions = 0;  // block 0, thread 0
-    unsigned long long entries = 0;
-    const unsigned long long ns0 = boss ? now_ns() : 0;
-    const long long cyc0 = clock64();
-    long long dec_cyc = 0, upd_cyc = 0;
+    // counts of the run, kept by a thread that has nothing else on its path
+    const bool clerk = bid == 0 && threadIdx.x == kSmallBlock - 1;
+    if (clerk) s_stat.movers = s_stat.decisions = s_stat.entries = 0;
+    if (boss) {
+        s_stat.ns0 = now_ns();
+        s_stat.cyc0 = clock64();
+        s_stat.dec_cyc = s_stat.upd_cyc = 0;
+    }
+    int upd_w0;  // this warp's first update task per bin, one bin per lane
+    {
+        int tasks = 0;
+        if (lane < 6) {
+            const int sh = kUpdShift[lane];
+            tasks = (s_bin[lane + 1] - s_bin[lane] + (1 << sh) - 1) >> sh;
+        }
+        upd_w0 = first_tasks(tasks, wg, nw);
+    }
     int done = 0, s = fresh && a.init ? 0 : a.s0;  // sweep 0: In and Q of a starting partition
     for (;; ++s) {
         SweepSlot *const cur = &ctl->slot[s % 3];
@@ -500,7 +531,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         int counts = 0;
         if (lane < kNumBins) counts = first ? s_bin[lane + 1] - s_bin[lane] : prev->act_count[lane];
         auto count = [&](int bin) { return __shfl_sync(GALA_FULL_MASK, counts, bin); };
-        long long t0 = clock64();
+        if (boss) s_stat.dec_cyc -= s > 0 ? clock64() : 0;
 
         // ---- decide
         if (s > 0) {
@@ -511,29 +542,25 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             int c = count(6);
             decide_cta<WT, kSmallBlock, W>(d, lists + s_bin[6], c, bid, nb, Tab::kSlots, 0, INT_MAX, keys, vals,
                                            occ);
-            const int off5 = c % nb;
-            decide_cta<WT, kSmallBlock, W>(d, lists + s_bin[5], count(5), (bid + nb - off5) % nb, nb,
-                                           Tab::kSlots, 0, INT_MAX, keys, vals, occ);
+            const int b5 = bid - (c < nb ? c : c % nb);
+            decide_cta<WT, kSmallBlock, W>(d, lists + s_bin[5], count(5), b5 < 0 ? b5 + nb : b5, nb, Tab::kSlots, 0,
+                                           INT_MAX, keys, vals, occ);
             if (hubs) hub_insert<WT, W>(d, hp, a.act_flag, nb - 1 - bid, nb);
             WarpStage<kStageM, 3> stage{stage_buf[wib], 0};
-            int off = 0;
-            auto start = [&](int tasks) {  // this warp's first task of the next bin
-                const int w0 = wg - off;
-                off = (off + tasks) % nw;
-                return w0 < 0 ? w0 + nw : w0;
-            };
+            const int w0s = first_tasks(lane < 5 ? (counts + (8 >> min(lane, 3)) - 1) >> (3 - min(lane, 3)) : 0, wg, nw);
+            auto start = [&](int bin) { return __shfl_sync(GALA_FULL_MASK, w0s, bin); };
             constexpr int WS = Tab::kWarpSlots;
             c = count(4);
-            decide_warp<WT, W, WS>(d, lists + s_bin[4], c, start(c), nw, 0, INT_MAX, keys + wib * WS,
+            decide_warp<WT, W, WS>(d, lists + s_bin[4], c, start(4), nw, 0, INT_MAX, keys + wib * WS,
                                    vals + wib * WS, occ + wib * (WS / 2));
             c = count(3);
-            decide_group<WT, 32, W>(d, lists + s_bin[3], c, start(c), nw, stage);
+            decide_group<WT, 32, W>(d, lists + s_bin[3], c, start(3), nw, stage);
             c = count(2);
-            decide_group<WT, 16, W>(d, lists + s_bin[2], c, start((c + 1) / 2), nw, stage);
+            decide_group<WT, 16, W>(d, lists + s_bin[2], c, start(2), nw, stage);
             c = count(1);
-            decide_group<WT, 8, W>(d, lists + s_bin[1], c, start((c + 3) / 4), nw, stage);
+            decide_group<WT, 8, W>(d, lists + s_bin[1], c, start(1), nw, stage);
             c = count(0);
-            decide_group<WT, 4, W>(d, lists + s_bin[0], c, start((c + 7) / 8), nw, stage);
+            decide_group<WT, 4, W>(d, lists + s_bin[0], c, start(0), nw, stage);
             flush_movers(d, stage);
             if (!grid_sync(&ctl->bar, target, err)) return;
             if (hubs) {
@@ -543,10 +570,12 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 if (!grid_sync(&ctl->bar, target, err)) return;
             }
         }
-        if (s > 0) dec_cyc += clock64() - t0;
+        if (boss && s > 0) s_stat.dec_cyc += clock64();
 
         // ---- labels and sizes; with hub rows a step of their own, since these
         // rows' In is summed over the new labels in the next one
+        const int c0 = bid * kSmallBlock + threadIdx.x;  // (the first total is read ahead)
+        WT t = c0 < a.n ? a.d.tot_next[c0] : (WT)0;
         if (s > 0) {
             apply_moves<WT, false>(a, cur->n_movers);
             if (hubs) {
@@ -559,8 +588,15 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         {
             long long mn = 0x7fffffffffffffffLL;
             typename SqSum<WT>::T s2 = 0;
-            for (int c = bid * kSmallBlock + threadIdx.x; c < a.n; c += nb * kSmallBlock) {
-                const WT t = a.d.tot_next[c];
+            int nm = 0, dv = 0;
+            unsigned long long de = 0;
+            if (clerk) {
+                nm = cur->n_movers;
+                dv = prev->act_vertices;
+                de = prev->act_edges;
+            }
+            for (int c = c0; c < a.n; c += nb * kSmallBlock) {
+                if (c != c0) t = a.d.tot_next[c];
                 a.Tot[c] = t;
                 if (t != 0) {
                     mn = min(mn, (long long)t);
@@ -581,17 +617,17 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 hub_in_partial<WT, W>(a.u, hp, nb - 1 - bid, nb);
                 clear_hubs();
             }
-            if (boss) {
+            if (clerk) {
                 clear_slot(ctl->slot[(s + 1) % 3], min_tot_init);
-                movers += cur->n_movers;
+                s_stat.movers += nm;
                 if (s > 1) {
-                    decisions += prev->act_vertices;
-                    entries += prev->act_edges;
+                    s_stat.decisions += dv;
+                    s_stat.entries += de;
                 }
             }
         }
         if (!grid_sync(&ctl->bar, target, err)) return;
-        t0 = clock64();
+        if (boss) s_stat.upd_cyc -= s > 0 ? clock64() : 0;
 
         // ---- update and prune
         {
@@ -601,21 +637,17 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             const long long mt = cur->min_tot;
             UpdateSums sums;
             WarpStage<kStageN, 1> stage{stage_buf[wib], 0};
-            int off = 0;
-            auto bin = [&](int b, int G) {  // list, count and this warp's first task of a bin
-                const int c = s_bin[b + 1] - s_bin[b], tasks = (c + 32 / G - 1) / (32 / G);
+            auto bin = [&](int b) {  // active list of a bin; this warp's first task
                 u.act_list = a.act[s & 1] + s_bin[b];
                 u.act_counter = &cur->act_count[b];
-                const int w0 = wg - off;
-                off = (off + tasks) % nw;
-                return w0 < 0 ? w0 + nw : w0;
+                return __shfl_sync(GALA_FULL_MASK, upd_w0, b);
             };
-            bin(6, 32);
-            off = 0;
+            bin(6);
             update_cta<WT, W>(u, a.order + s_bin[6], s_bin[7] - s_bin[6], mt, bid, nb, sums);
 #define GALA_SMALL_UPD(B, G, U)                                                                                      \
     do {                                                                                                             \
-        const int w0 = bin(B, G);                                                                                    \
+        static_assert(32 / G == 1 << kUpdShift[B], "tasks of the bin");                                              \
+        const int w0 = bin(B);                                                                                       \
         update_group<WT, G, U, W>(u, a.order + s_bin[B], s_bin[B + 1] - s_bin[B], mt, w0, nw, stage,  \
                                sums);                                                                                \
     } while (0)
@@ -643,9 +675,10 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             continue;
         }
         if (threadIdx.x == 0) {
+            const int e = *(volatile int *)err;
             const double q = slot_q(*cur, constant);
             int go = 1;
-            if (*(volatile int *)err)
+            if (e)
                 go = 0;
             else if (__dsub_rn(q, prev_q) < a.min_mod)
                 go = -1;
@@ -653,7 +686,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 prev_q = q;
             s_go = go;
             if (bid == 0) {
-                upd_cyc += clock64() - t0;
+                s_stat.upd_cyc += clock64();
                 a.out->trace[k] = q;
             }
         }
@@ -667,18 +700,20 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         // (every thread reads s_go before the next sweep's barriers let thread
         // 0 write it again)
     }
-    if (bid == 0 && threadIdx.x == 0) {
+    if (clerk) {
+        a.out->movers = s_stat.movers;
+        a.out->decisions = s_stat.decisions;
+        a.out->entries = s_stat.entries;
+    }
+    if (boss) {
         SmallOut *o = a.out;
         o->q = prev_q;
         o->sweeps = s - a.s0 + 1;
         o->done = done;
         o->err = *(volatile int *)err;
-        o->movers = movers;
-        o->decisions = decisions;
-        o->entries = entries;
-        const double ns = (double)(now_ns() - ns0) / (double)max(clock64() - cyc0, 1LL);  // per cycle
-        o->decide_ns = (unsigned long long)((double)dec_cyc * ns);
-        o->update_ns = (unsigned long long)((double)upd_cyc * ns);
+        const double ns = (double)(now_ns() - s_stat.ns0) / (double)max(clock64() - s_stat.cyc0, 1LL);  // per cycle
+        o->decide_ns = (unsigned long long)((double)s_stat.dec_cyc * ns);
+        o->update_ns = (unsigned long long)((double)s_stat.upd_cyc * ns);
     }
 }
 

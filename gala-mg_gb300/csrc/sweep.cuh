@@ -473,6 +473,9 @@ __device__ __forceinline__ void flush_movers(const DecideArgs<WT, RO> &a, WarpSt
     int *const lists[3] = {a.mv_v, a.mv_old, a.mv_new};
     if constexpr (!RO) {
         __syncwarp();
+        if (stage.n == 0) return;
+        int base = 0;  // its place in the lists, asked for ahead of the totals
+        if ((threadIdx.x & 31) == 0) base = atomicAdd(a.n_movers, stage.n);
         for (int i0 = 0; i0 < stage.n; i0 += 32) {
             const int i = i0 + (threadIdx.x & 31);
             const bool valid = i < stage.n;
@@ -485,8 +488,10 @@ __device__ __forceinline__ void flush_movers(const DecideArgs<WT, RO> &a, WarpSt
             }
             move_totals<WT, true, false>(valid, from, to, k, a.tot_next, nullptr);
         }
+        stage.store(lists, __shfl_sync(GALA_FULL_MASK, base, 0));
+    } else {
+        stage.flush(lists, a.n_movers);
     }
-    stage.flush(lists, a.n_movers);
 }
 
 // Degree <= G: one lane per neighbour.  Lanes holding the same neighbour
