@@ -1776,8 +1776,8 @@ namespace {
 // One persistent launch over the batch's graphs (batch_cta.cu): each CTA runs
 // whole graphs.  The union CSR is in ctx->offs[1] / nbr[1] / w[1].
 gala_status batch_per_graph(gala_context *ctx, BatchRun &bt, const gala_graph *const *graphs, int G, int32_t n,
-                            long long e_tot, int nmax, bool weighted, const gala_options *opt, int32_t *community_out,
-                            PageTouch &pages, double *modularity_out, int32_t *communities_out,
+                            long long e_tot, int nmax, bool weighted, bool gather, const gala_options *opt,
+                            int32_t *community_out, PageTouch &pages, double *modularity_out, int32_t *communities_out,
                             gala_batch_result *res)
 {
     cudaStream_t st = ctx->stream;
@@ -1845,6 +1845,8 @@ gala_status batch_per_graph(gala_context *ctx, BatchRun &bt, const gala_graph *c
     a.u_offs = ctx->offs[1];
     a.u_nbr = ctx->nbr[1];
     a.u_w = weighted ? ctx->w[1] : nullptr;
+    a.gather = gather;
+    a.src = bt.src();
     a.labels = ctx->orig;
     a.min_mod = opt ? opt->min_modularity : 1e-6;
     a.max_levels = opt ? opt->max_levels : 0;
@@ -2078,6 +2080,9 @@ gala_status gala_louvain_batch(gala_context *ctx, const gala_graph *const *graph
             bt.h_tab[2LL * bt.cap + i] = (int64_t)(uintptr_t)graphs[i]->dev_w;
         }
     }
+    int nmax = 0;
+    for (int i = 0; i < G; ++i) nmax = std::max(nmax, graphs[i]->n);
+    const bool per_graph = !(opt && opt->batch_mode == 1) && nmax <= kCtaMaxN;
     long long l0 = gala_kernel_launch_count();
     cudaEventRecord(ctx->ev[6], st);
     const int32_t *dw = weighted ? ctx->w[1] : nullptr;
@@ -2087,7 +2092,8 @@ gala_status gala_louvain_batch(gala_context *ctx, const gala_graph *const *graph
     cudaMemcpyAsync(bt.estart(), bt.h_estart(), ((size_t)G + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st);
     if (mapped) {
         cudaMemcpyAsync(bt.tab, bt.h_tab, 3 * (size_t)bt.cap * sizeof(int64_t), cudaMemcpyHostToDevice, st);
-        batch_gather(G, bt.src(), ctx->offs[1], ctx->nbr[1], weighted ? ctx->w[1] : nullptr, st);
+        // (one CTA per graph: it copies its graph itself)
+        if (!per_graph) batch_gather(G, bt.src(), ctx->offs[1], ctx->nbr[1], weighted ? ctx->w[1] : nullptr, st);
     } else {
         cudaMemcpyAsync(ctx->offs[1], bt.h_offs, ((size_t)n + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st);
         cudaMemcpyAsync(ctx->nbr[1], bt.h_nbr, (size_t)e_tot * sizeof(int32_t), cudaMemcpyHostToDevice, st);
@@ -2097,13 +2103,11 @@ gala_status gala_louvain_batch(gala_context *ctx, const gala_graph *const *graph
     }
     cudaMemcpyAsync(bt.goff, bt.h_goff, ((size_t)G + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st);
     cudaEventRecord(ctx->ev[7], st);
-    batch_gid_fill(G, bt.goff, bt.gid, st);
+    if (!per_graph) batch_gid_fill(G, bt.goff, bt.gid, st);
     if ((s = sync_check(st, "batch host to device copy"))) return s;
     res->time_h2d_ms = ev_ms(ctx->ev[6], ctx->ev[7]);
-    int nmax = 0;
-    for (int i = 0; i < G; ++i) nmax = std::max(nmax, graphs[i]->n);
-    if (!(opt && opt->batch_mode == 1) && nmax <= kCtaMaxN) {
-        s = batch_per_graph(ctx, bt, graphs, G, n, e_tot, nmax, weighted, opt, community_out, pages, modularity_out,
+    if (per_graph) {
+        s = batch_per_graph(ctx, bt, graphs, G, n, e_tot, nmax, weighted, mapped, opt, community_out, pages, modularity_out,
                             communities_out, res);
         if (s) return s;
         res->h2d_bytes = ((long long)n + 1) * 8 + e_tot * 4 * (weighted ? 2 : 1) + ((long long)G + 1) * 8 +

@@ -273,9 +273,14 @@ struct BatchCtaArgs {
     int G;
     const int32_t *order;  // graphs, largest first
     const int64_t *vstart, *estart;
-    const int64_t *u_offs;  // union CSR (device layout)
-    const int32_t *u_nbr;
-    const int32_t *u_w;     // null: unit weights
+    // union CSR (u_w null: unit weights); with `gather` every CTA first copies
+    // its graph there from page-locked host memory (src; neighbours keep the
+    // graph's own ids)
+    int64_t *u_offs;
+    int32_t *u_nbr;
+    int32_t *u_w;
+    bool gather;
+    BatchSrc src;
     int32_t *K, *Self, *size, *ec, *members, *moff;
     int32_t *loffs[2], *llen[2], *lnbr[2], *lw[2];  // contracted level graphs (ping-pong): row starts and lengths
     int32_t *labels;  // out: every input vertex's community, local to its graph

@@ -362,7 +362,8 @@ typedef struct {
     int32_t reserved;
     int64_t vertices;          /* union vertices */
     int64_t entries;           /* union CSR entries */
-    double time_total_ms;      /* all rounds, device-resident union */
+    double time_total_ms;      /* all rounds, device-resident union; with one CTA
+                                * per graph and pinned graphs also their copies */
     double time_phase1_ms;
     double time_contract_ms;
     double time_h2d_ms;
