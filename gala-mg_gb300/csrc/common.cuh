@@ -106,6 +106,8 @@ struct DevStats {
     unsigned long long sym_hash;  // 0 when the graph is symmetric (hash of every entry minus its mirror)
     int push_mode;                // 1: this sweep updates In incrementally (the per-bin updates return at once)
     int push_len;                 // movers in the prefix scan (0 unless push_mode)
+    // batches: graphs whose phase 1 goes on after this sweep, graphs that drop it
+    int batch_running, batch_rejects;
 };
 
 constexpr int kErrHashOverflow = 1;

@@ -272,13 +272,15 @@ struct BatchRun {
     long long *m2g = nullptr;
     double *cg = nullptr;
     uint8_t *stop = nullptr, *reject = nullptr;
+    double *prev_qg = nullptr;  // accepted Q of the current level
     int32_t *min_tot = nullptr, *ncomm = nullptr;
     unsigned long long *sum_in = nullptr, *sum_tot2 = nullptr, *sum_k = nullptr;
     int64_t *goff = nullptr;  // G+1 vertex offsets of the current level
     // pinned host mirrors
     unsigned long long *h_sum_in = nullptr, *h_sum_tot2 = nullptr, *h_sum_k = nullptr;
     int32_t *h_ncomm = nullptr;
-    uint8_t *h_stop = nullptr, *h_reject = nullptr;
+    uint8_t *h_stop = nullptr;
+    double *h_prev_q = nullptr;
     int64_t *h_goff = nullptr;
     // source table of the input graphs, 5G+2 words: device-mapped offsets,
     // neighbour and weight addresses (G each), then the first vertex and the
@@ -633,6 +635,9 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
             if (bt->m2[i] > 0) bt->prev_q[i] = q_from_sums(bt->h_sum_in[i], bt->h_sum_tot2[i], bt->m2[i]);
         }
         cudaMemcpyAsync(bt->stop, bt->h_stop, G, cudaMemcpyHostToDevice, st);
+        memcpy(bt->h_prev_q, bt->prev_q.data(), G * sizeof(double));
+        cudaMemcpyAsync(bt->prev_qg, bt->h_prev_q, G * sizeof(double), cudaMemcpyHostToDevice, st);
+        batch_sums_reset(kSumIn | kSumTot2 | kMinTot, G, nullptr, bt->sums(), st);
     }
 
     if (init) {
@@ -792,7 +797,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
             p1_apply_movers(b, +1, g.n, st, iteration, g.offs, incr ? b.moved : nullptr);
             if (pmode == GALA_PROPOSAL_TRACE && iteration > 1) p1_trace_labels(b, ps, st);
             if (bt)
-                batch_graph_sums(kMinTot | kSumTot2, G, bt->goff, bt->stop, b, bt->sums(), st);
+                batch_graph_sums(kMinTot | kSumTot2, G, bt->goff, bt->stop, b, bt->sums(), st, false);
             else
                 p1_tot_reduce(b, g.n, st);
             rec(ctx->ev[4]);
@@ -810,14 +815,11 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
                               m2, aux_for(ctx, k));
             }
             join(ctx);
-            if (bt) {
-                batch_graph_sums(kSumIn, G, bt->goff, bt->stop, b, bt->sums(), st);
-                cudaMemcpyAsync(bt->h_sum_in, bt->sum_in, G * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                st);
-                cudaMemcpyAsync(bt->h_sum_tot2, bt->sum_tot2, G * sizeof(unsigned long long),
-                                cudaMemcpyDeviceToHost, st);
-            }
+            if (bt) batch_graph_sums(kSumIn, G, bt->goff, bt->stop, b, bt->sums(), st, false);
             rec(ctx->ev[5]);
+            if (bt)
+                batch_converge(b, G, bt->sums(), bt->cg, min_mod, bt->prev_qg, bt->stop, bt->reject, bt->gid, g.n,
+                               st);
             cudaMemcpyAsync(h, b.stats, sizeof(DevStats), cudaMemcpyDeviceToHost, st);
             if (pend && iteration == 1)
                 cudaMemcpyAsync(ctx->h_stats2, ctx->d_stats2, sizeof(DevStats), cudaMemcpyDeviceToHost, st);
@@ -887,31 +889,16 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
         act_nv = h->act_vertices[nxt];
         act_ne = (long long)h->act_edges[nxt];
         if (bt) {
-            // per-graph convergence (louvain_main_process.cu:1004-1007 for
-            // every graph): a graph whose Q did not grow by min_mod drops
-            // this iteration's moves and stops
-            bool running = false, any_reject = false;
-            for (int i = 0; i < G; ++i) {
-                bt->h_reject[i] = 0;
-                if (bt->h_stop[i]) continue;
-                const double qg = q_from_sums(bt->h_sum_in[i], bt->h_sum_tot2[i], bt->m2[i]);
-                if (qg - bt->prev_q[i] < min_mod) {
-                    bt->h_reject[i] = 1;
-                    bt->h_stop[i] = 1;
-                    any_reject = true;
-                } else {
-                    bt->prev_q[i] = qg;
-                    running = true;
-                }
+            // (per-graph convergence on the device: batch_converge)
+            if (h->batch_running == 0) {
+                if ((s = check(cudaMemcpyAsync(bt->h_prev_q, bt->prev_qg, G * sizeof(double), cudaMemcpyDeviceToHost,
+                                               st),
+                               "batch Q")) ||
+                    (s = sync_check(st, "batch Q")))
+                    return s;
+                bt->prev_q.assign(bt->h_prev_q, bt->h_prev_q + G);
+                break;
             }
-            if (any_reject) {
-                cudaMemcpyAsync(bt->reject, bt->h_reject, G, cudaMemcpyHostToDevice, st);
-                cudaMemcpyAsync(bt->stop, bt->h_stop, G, cudaMemcpyHostToDevice, st);
-                batch_revert(b, bt->gid, bt->reject, g.n, st);
-                // the host arrays must stay unchanged until the copies ran
-                if ((s = sync_check(st, "batch revert"))) return s;
-            }
-            if (!running) break;
             cur = nxt;
             iteration++;
             continue;
@@ -1990,6 +1977,7 @@ gala_status gala_louvain_batch(gala_context *ctx, const gala_graph *const *graph
         dal(&bt.cg, G);
         dal(&bt.stop, G);
         dal(&bt.reject, G);
+        dal(&bt.prev_qg, G);
         dal(&bt.min_tot, G);
         dal(&bt.ncomm, G);
         dal(&bt.sum_in, G);
@@ -2002,7 +1990,7 @@ gala_status gala_louvain_batch(gala_context *ctx, const gala_graph *const *graph
         hal(&bt.h_sum_k, G);
         hal(&bt.h_ncomm, G);
         hal(&bt.h_stop, G);
-        hal(&bt.h_reject, G);
+        hal(&bt.h_prev_q, G);
         hal(&bt.h_goff, (size_t)G + 1);
         hal(&bt.h_tab, 5 * (size_t)G + 2);
         if (!ok) {

@@ -243,8 +243,14 @@ struct GraphSums {  // per-graph outputs (device arrays of G entries)
     int32_t *min_tot, *ncomm;
 };
 void batch_graph_sums(int what, int G, const int64_t *goff, const uint8_t *stop, const Phase1Buffers &b,
-                      const GraphSums &out, cudaStream_t st);
-void batch_revert(Phase1Buffers &b, const int32_t *gid, const uint8_t *reject, int n, cudaStream_t st);
+                      const GraphSums &out, cudaStream_t st, bool reset = true);
+// `what` of the graphs that have not stopped to the sums' starting values.
+void batch_sums_reset(int what, int G, const uint8_t *stop, const GraphSums &out, cudaStream_t st);
+// Convergence of every graph after a sweep, from its sums (which are reset for
+// the next one): prev_q, stop, and stats->batch_running; the moves of graphs that
+// stop are undone.
+void batch_converge(Phase1Buffers &b, int G, const GraphSums &sums, const double *cg, double min_mod, double *prev_q,
+                    uint8_t *stop, uint8_t *reject, const int32_t *gid, int n, cudaStream_t st);
 void batch_gid_fill(int G, const int64_t *goff, int32_t *gid, cudaStream_t st);
 // Source arrays of a batch of page-locked host graphs (device-mapped
 // addresses, one per graph) and each graph's first vertex and entry in the

@@ -996,6 +996,8 @@ __global__ void k_iter_reset(DevStats *st, int next, long long min_tot_init)
     st->mv_edges = 0;
     st->push_mode = 0;
     st->push_len = 0;
+    st->batch_running = 0;
+    st->batch_rejects = 0;
     st->sum_in = 0;
     st->sum_tot2 = 0;
     st->sum_tot2_hi = 0;
