@@ -778,7 +778,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
                         cudaStreamWaitEvent(aux_for(ctx, k), pend->ev[hub_chunk], 0);
                         p1_init_rows_range(g, b, 7, b.order + bin_start[7], level_cnt[7], ctx->d_stats2,
                                            aux_for(ctx, k));
-                        p1_hub_decide(g, b, hp, constant, m2, fp64_only, aux_for(ctx, k));
+                        p1_hub_decide(g, b, hp, constant, m2, fp64_only, g.distinct, aux_for(ctx, k));
                     }
                 }
                 for (int k = 0; k < kNumBins; ++k) cudaStreamWaitEvent(aux_for(ctx, k), last, 0);
@@ -786,7 +786,8 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
                 for (int k = 0; k < kNumBins; ++k) {
                     const int bin = kBinLaunchOrder[k];
                     if (bin == 7)
-                        p1_hub_decide(g, b, hp, constant, m2, fp64_only, aux_for(ctx, k));
+                        p1_hub_decide(g, b, hp, constant, m2, fp64_only, iteration == 1 && g.distinct && !init,
+                                      aux_for(ctx, k));
                     else
                         p1_decide(g, b, bin, lists + bin_start[bin], counts + bin, level_cnt[bin], constant, m2,
                                   fp64_only, iteration == 1 && g.distinct && !init, aux_for(ctx, k));

@@ -201,7 +201,7 @@ int hub_grid_size();
 void p1_hub_plan_launch(const LevelGraph &g, Phase1Buffers &b, HubPlan &p, cudaStream_t st);
 void p1_hub_work_launch(HubPlan &p, cudaStream_t st);
 void p1_hub_decide(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, double constant, long long m2,
-                   int fp64_only, cudaStream_t st);
+                   int fp64_only, bool first, cudaStream_t st);
 // Weight update + pruning of the hub bin (bin 7), chunked over many CTAs.
 void p1_hub_update(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, int next, int bin_start, double constant,
                    long long m2, cudaStream_t st);

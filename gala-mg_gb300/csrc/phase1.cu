@@ -1167,6 +1167,86 @@ __global__ void __launch_bounds__(256) k_hub_final(DecideArgs<WT> a, HubPlan p, 
     hub_final(a, p, flag, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
 }
 
+// First sweep of a level, distinct neighbours: a hub's entries are its
+// candidates, so its row's chunks are evaluated as they are, without the table
+// (its clearing, the label gather, the atomic inserts and a scan over at least
+// 1.5 slots per entry).  Partials as hub_scan's, at the first table chunks of
+// the hub; 2^22 R-MAT vertices 17.79 ms with the tables, 16.99 without, 2^20 from
+// the host 7.54 and 7.31.
+template <typename WT, bool W>
+__global__ void __launch_bounds__(256) k_hub_first(DecideArgs<WT> a, HubPlan p, const uint8_t *__restrict__ flag)
+{
+    constexpr int NW = 256 / 32;
+    __shared__ double r_dq[NW];
+    __shared__ int r_c[NW];
+    __shared__ CandRow<WT, NW> r_best;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (long long wi = blockIdx.x; wi < p.nwork; wi += gridDim.x) {
+        const int i = p.work[wi];
+        const int v = p.hubs[i];
+        if (!flag[v] || stopped(a, v)) continue;  // block-uniform
+        const Scale sc = scale_of(a, v);
+        const int cur = a.comm[v];  // = v
+        const WT ki = a.K[v], tcur = a.Tot[cur];
+        const long long chunk = wi - p.coff[i], s = a.offs[v] + chunk * kHubChunk, left = a.offs[v + 1] - s;
+        const int len = (int)(left < kHubChunk ? left : kHubChunk);
+        const long long out = p.tcoff[i] + chunk;
+        const GainTerms<WT> gt(sc, ki, tcur);
+        Cand<WT> best(cur);
+        WT wc = 0;
+        first_scan_best<WT, W>(a, gt, s, len, v, threadIdx.x, 256, best, wc);
+        warp_merge(best, wc, 32);
+        if (lane == 0) r_best.put(wid, best, wc);
+        __syncthreads();
+        if (wid == 0) {
+            r_best.get(lane, NW, cur, best, wc);
+            warp_merge(best, wc, 32);
+            if (lane == 0) {
+                hub_put(p, out, best, wc);
+                r_best.put(0, best, wc);
+            }
+        }
+        __syncthreads();
+        if (needs_fp64(a, sc, ki)) {  // block-uniform
+            double dq = 0.0;
+            int fc = cur;
+            r_best.get(0, 1, cur, best, wc);
+            first_scan<WT, W>(a, sc, gt, best, s, len, v, threadIdx.x, 256, ki, tcur, dq, fc);
+            warp_argmax(dq, fc);
+            if (lane == 0) {
+                r_dq[wid] = dq;
+                r_c[wid] = fc;
+            }
+            __syncthreads();
+            if (wid == 0) {
+                dq = lane < NW ? r_dq[lane] : 0.0;
+                fc = lane < NW ? r_c[lane] : cur;
+                warp_argmax(dq, fc);
+                if (lane == 0) {
+                    p.pdq[out] = dq;
+                    p.pfc[out] = fc;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// One warp per hub over its chunks' partials, then over the row itself for the
+// rare rounding cases.
+template <typename WT, bool W>
+__global__ void __launch_bounds__(256) k_hub_first_final(DecideArgs<WT> a, HubPlan p, const uint8_t *__restrict__ flag)
+{
+    hub_final(
+        a, p, flag, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+        [&](int i) { return p.tcoff[i] + p.coff[i + 1] - p.coff[i]; },
+        [&](int, int v, const Scale &sc, const GainTerms<WT> &gt, const Cand<WT> &best, int, WT ki, WT tcur, double &dq,
+            int &fc) {
+            first_scan<WT, W>(a, sc, gt, best, a.offs[v], (int)(a.offs[v + 1] - a.offs[v]), v, threadIdx.x & 31, 32, ki,
+                              tcur, dq, fc);
+        });
+}
+
 // Per level: table sizes, chunk counts and their offsets (the caller reads
 // the three totals from the stats block before p1_hub_work_launch).
 void p1_hub_plan_launch(const LevelGraph &g, Phase1Buffers &b, HubPlan &p, cudaStream_t st)
@@ -1188,10 +1268,24 @@ void p1_hub_work_launch(HubPlan &p, cudaStream_t st)
 
 template <typename WT>
 static void hub_decide_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, double constant, long long m2,
-                         int fp64_only, cudaStream_t st)
+                         int fp64_only, bool first, cudaStream_t st)
 {
     const DecideArgs<WT> a = decide_args<WT>(g, b, constant, m2, fp64_only);
     const int cap = num_sms() * 8;
+    // (a capped table may hold fewer partials than the row has chunks, and its
+    // overflow is to be seen)
+    if (first && p.t_cap == 0) {
+        const int grid = (int)(p.nwork < cap ? p.nwork : cap), gf = (p.H * 32 + 255) / 256;
+        if (g.w) {
+            k_hub_first<WT, true><<<grid, 256, 0, st>>>(a, p, b.act_flag);
+            k_hub_first_final<WT, true><<<gf, 256, 0, st>>>(a, p, b.act_flag);
+        } else {
+            k_hub_first<WT, false><<<grid, 256, 0, st>>>(a, p, b.act_flag);
+            k_hub_first_final<WT, false><<<gf, 256, 0, st>>>(a, p, b.act_flag);
+        }
+        note_launch(2);
+        return;
+    }
     cudaMemsetAsync(p.pool, 0xff, (size_t)p.half * sizeof(int32_t), st);
     cudaMemsetAsync(p.pool + p.half, 0, (size_t)p.half * sizeof(WT), st);
     const int g1 = (int)(p.nwork < cap ? p.nwork : cap);
@@ -1208,13 +1302,13 @@ static void hub_decide_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p
 // tables follow all keys: p.half int32 keys, then p.half values of the
 // weight type (the caller sized the pool for it).
 void p1_hub_decide(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, double constant, long long m2,
-                   int fp64_only, cudaStream_t st)
+                   int fp64_only, bool first, cudaStream_t st)
 {
     if (p.H <= 0) return;
     if (g.wide)
-        hub_decide_t<long long>(g, b, p, constant, m2, fp64_only, st);
+        hub_decide_t<long long>(g, b, p, constant, m2, fp64_only, first, st);
     else
-        hub_decide_t<int>(g, b, p, constant, m2, fp64_only, st);
+        hub_decide_t<int>(g, b, p, constant, m2, fp64_only, first, st);
 }
 
 template <typename WT>

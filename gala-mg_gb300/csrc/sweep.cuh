@@ -1139,9 +1139,11 @@ __device__ __forceinline__ void hub_scan(const DecideArgs<WT, RO> &a, const HubP
     }
 }
 
-template <typename WT, bool RO>
+// end(i): past hub i's last partial; rescan: the hub's candidates in FP64, by
+// the warp.
+template <typename WT, bool RO, typename End, typename Rescan>
 __device__ __forceinline__ void hub_final(const DecideArgs<WT, RO> &a, const HubPlan &p, const uint8_t *flag, int wg,
-                                          int nw)
+                                          int nw, End end, Rescan rescan)
 {
     const int lane = threadIdx.x & 31;
     for (int i = wg; i < p.H; i += nw) {
@@ -1152,7 +1154,8 @@ __device__ __forceinline__ void hub_final(const DecideArgs<WT, RO> &a, const Hub
         const WT ki = a.K[v], sf = a.Self[v], tcur = a.Tot[cur];
         Cand<WT> best(cur);
         WT wc = 0;
-        for (long long q = p.tcoff[i] + lane; q < p.tcoff[i + 1]; q += 32) {
+        const long long q1 = end(i);
+        for (long long q = p.tcoff[i] + lane; q < q1; q += 32) {
             WT own;
             best.merge(hub_get(p, q, best, own));
             wc += own;
@@ -1164,14 +1167,13 @@ __device__ __forceinline__ void hub_final(const DecideArgs<WT, RO> &a, const Hub
             double dq = 0.0;
             int fc = cur;
             if (needs_fp64(a, sc, ki)) {  // chunk-wise FP64 partials from k_hub_scan
-                for (long long q = p.tcoff[i] + lane; q < p.tcoff[i + 1]; q += 32)
+                for (long long q = p.tcoff[i] + lane; q < q1; q += 32)
                     if (cand_better(p.pdq[q], p.pfc[q], dq, fc)) {
                         dq = p.pdq[q];
                         fc = p.pfc[q];
                     }
-            } else {  // rare rounding cases: rescan the table in FP64
-                scan_table(a, sc, GainTerms<WT>(sc, ki, tcur), best, p.pool + p.toff[i], hub_vals<WT>(p, i),
-                           (int)p.T[i], lane, 32, cur, ki, tcur, dq, fc);
+            } else {  // rare rounding cases
+                rescan(i, v, sc, GainTerms<WT>(sc, ki, tcur), best, cur, ki, tcur, dq, fc);
             }
             warp_argmax(dq, fc);
             bc = fc;
@@ -1181,6 +1183,20 @@ __device__ __forceinline__ void hub_final(const DecideArgs<WT, RO> &a, const Hub
         const bool move = lane == 0 && dec == 1 && guard_ok(a, cur, bc);
         append_mover(a, move, v, cur, bc);
     }
+}
+
+// The same over the hubs' tables.
+template <typename WT, bool RO>
+__device__ __forceinline__ void hub_final(const DecideArgs<WT, RO> &a, const HubPlan &p, const uint8_t *flag, int wg,
+                                          int nw)
+{
+    hub_final(
+        a, p, flag, wg, nw, [&](int i) { return p.tcoff[i + 1]; },
+        [&](int i, int, const Scale &sc, const GainTerms<WT> &gt, const Cand<WT> &best, int cur, WT ki, WT tcur,
+            double &dq, int &fc) {
+            scan_table(a, sc, gt, best, p.pool + p.toff[i], hub_vals<WT>(p, i), (int)p.T[i], threadIdx.x & 31, 32, cur,
+                       ki, tcur, dq, fc);
+        });
 }
 
 // ------------------------------------------------------------------------
