@@ -87,6 +87,7 @@ struct gala_context {
     RefineBuffers ref{};  // allocated on the first run with gala_options.refine
     DevStats *d_stats = nullptr;
     DevStats *h_stats = nullptr;
+    void *h_block = nullptr;  // page-locked: h_stats, h_stats2, h_chunk, h_small_out
     int32_t *scratch = nullptr;
     long long scratch_ints = 0;
     // per table chunk of the hub bin: best candidate of the chunk
@@ -358,10 +359,11 @@ long long decide_bytes_for(long long nv, long long ne, bool weighted)
 // Levels whose sweeps run in one cooperative launch (small_level.cu).  Below
 // this many entries a sweep costs less than its launches and its host read:
 // phase 1 of planted graphs (one GB300, ms per call, separate launches / one
-// launch) 2.28 / 1.03 at 0.4M entries, 2.57 / 1.90 at 2.4M, 6.49 / 7.02 at
-// 9.6M, and 17.3 / 22.3 at 16M, where the one-bin kernels' higher occupancy
+// launch) 2.06 / 0.69 at 0.4M entries, 2.11 / 1.33 at 2.4M, 6.27 / 5.90 at
+// 9.6M, and 15.0 / 18.1 at 16M, where the one-bin kernels' higher occupancy
 // (48-64 warps per SM against 32) counts for more; refined LFR run with a level
-// of 4.7M entries 8.23 / 7.98.
+// of 4.7M entries 8.68 / 7.65, float LFR run with a level of 13M entries and 30
+// sweeps 14.2 / 15.6.
 constexpr int64_t kSmallLevelEntries = 1 << 23;
 bool small_level(const LevelGraph &g) { return g.E <= kSmallLevelEntries; }
 
@@ -1327,7 +1329,7 @@ void gala_context_destroy(gala_context *ctx)
         delete ctx->batch;
     }
     for (void *p : ctx->allocs) cudaFree(p);
-    if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
+    if (ctx->h_block) cudaFreeHost(ctx->h_block);
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
     for (int i = 0; i < gala_context::kAux; ++i) {
@@ -1344,9 +1346,6 @@ void gala_context_destroy(gala_context *ctx)
     for (auto &e : ctx->copy_ev)
         if (e) cudaEventDestroy(e);
     if (ctx->offs_ev) cudaEventDestroy(ctx->offs_ev);
-    if (ctx->h_chunk) cudaFreeHost(ctx->h_chunk);
-    if (ctx->h_stats2) cudaFreeHost(ctx->h_stats2);
-    if (ctx->h_small_out) cudaFreeHost(ctx->h_small_out);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     cudaSetDevice(prev);
     delete ctx;
@@ -1390,25 +1389,45 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
         ok = ok && cudaStreamCreateWithFlags(&ctx->aux[i], cudaStreamNonBlocking) == cudaSuccess;
         ok = ok && cudaEventCreateWithFlags(&ctx->join_ev[i], cudaEventDisableTiming) == cudaSuccess;
     }
-    ok = ok && cudaMallocHost(&ctx->h_stats, sizeof(DevStats)) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
     for (auto &e : ctx->copy_ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->offs_ev, cudaEventDisableTiming) == cudaSuccess;
     for (auto &e : ctx->pend_store.ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     constexpr int kChunkInts = (PendingRows::kMax + 1) + (PendingRows::kMax + 1) * kNumBins + PendingRows::kMax * kNumBins;
-    ok = ok && cudaMallocHost(&ctx->h_chunk, kChunkInts * sizeof(int32_t)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&ctx->h_stats2, sizeof(DevStats)) == cudaSuccess;
-    ok = ok && dalloc(ctx, &ctx->d_chunk, kChunkInts) && dalloc(ctx, &ctx->d_stats2, 1);
-    char *ctl = nullptr, *cctl = nullptr;
-    ok = ok && dalloc(ctx, &ctl, small_ctl_bytes()) && dalloc(ctx, &cctl, contract_ctl_bytes()) &&
-         dalloc(ctx, &ctx->small_out, 1);
-    ok = ok && cudaMallocHost(&ctx->h_small_out, sizeof(SmallOut)) == cudaSuccess;
-    ctx->small_ctl = ctl;
-    ctx->cb.small_ctl = cctl;
+    // the small blocks: one page-locked and one device allocation, 256-byte slices
+    {
+        char *hp = nullptr, *dp = nullptr;
+        size_t hn = 0, dn = 0;
+        auto slice = [](size_t &at, size_t bytes) {
+            const size_t o = at;
+            at += (bytes + 255) / 256 * 256;
+            return o;
+        };
+        const size_t h0 = slice(hn, sizeof(DevStats)), h1 = slice(hn, sizeof(DevStats)),
+                     h2 = slice(hn, kChunkInts * sizeof(int32_t)), h3 = slice(hn, sizeof(SmallOut));
+        const size_t d0 = slice(dn, sizeof(DevStats)), d1 = slice(dn, sizeof(DevStats)),
+                     d2 = slice(dn, kChunkInts * sizeof(int32_t)), d3 = slice(dn, sizeof(SmallOut)),
+                     d4 = slice(dn, small_ctl_bytes()), d5 = slice(dn, contract_ctl_bytes());
+        ok = ok && cudaMallocHost(&hp, hn) == cudaSuccess;
+        ctx->h_block = hp;
+        ok = ok && dalloc(ctx, &dp, dn);
+        if (ok) {
+            ctx->h_stats = (DevStats *)(hp + h0);
+            ctx->h_stats2 = (DevStats *)(hp + h1);
+            ctx->h_chunk = (int32_t *)(hp + h2);
+            ctx->h_small_out = (SmallOut *)(hp + h3);
+            ctx->d_stats = (DevStats *)(dp + d0);
+            ctx->d_stats2 = (DevStats *)(dp + d1);
+            ctx->d_chunk = (int32_t *)(dp + d2);
+            ctx->small_out = (SmallOut *)(dp + d3);
+            ctx->small_ctl = dp + d4;
+            ctx->cb.small_ctl = dp + d5;
+        }
+    }
     for (int i = 0; i < 2 && ok; ++i)
         ok = dalloc(ctx, &ctx->offs[i], n + 1) && dalloc(ctx, &ctx->nbr[i], E) && dalloc8(ctx, &ctx->w[i], E);
     Phase1Buffers &b = ctx->p1;
-    ok = ok && dalloc(ctx, &ctx->orig, n) && dalloc(ctx, &ctx->d_stats, 1) && dalloc(ctx, &b.comm, n) &&
+    ok = ok && dalloc(ctx, &ctx->orig, n) && dalloc(ctx, &b.comm, n) &&
          dalloc8(ctx, &b.K, n) && dalloc8(ctx, &b.Self, n) && dalloc8(ctx, &b.Tot, n) && dalloc(ctx, &b.size, n) &&
          dalloc8(ctx, &b.In, n) && dalloc(ctx, &b.order, n) && dalloc(ctx, &b.act[0], n) &&
          dalloc(ctx, &b.act[1], n) && dalloc(ctx, &b.mv_v, n) && dalloc(ctx, &b.mv_old, n) &&
