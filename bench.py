@@ -556,7 +556,7 @@ def batch_arm(ffi, args, torch, device):
     return {"config": dict(b, vertices=sum(ns), edges=m, max_vertices=max(ns), min_vertices=min(ns)),
             "metric": "batched Louvain edges/s (host graphs in, labels out)", "value": m / sec, "unit": "edges/s",
             "seconds": sec, "device_ms": r["time_total_ms"], "h2d_ms": r["time_h2d_ms"], "d2h_ms": r["time_d2h_ms"],
-            "input": ("page-locked host graphs, read in place by the GPU (one gather kernel)" if pinned == len(gs)
+            "input": ("page-locked host graphs, read in place by the GPU" if pinned == len(gs)
                       else "host graphs (%d of %d page-locked): raw copies into the context's pinned staging, one "
                            "transfer, ids shifted on the device" % (pinned, len(gs))),
             "phase1_ms": r["time_phase1_ms"],

@@ -26,7 +26,7 @@
 // vertex's first entries in flight while it decides one.
 // 4,096 planted-partition graphs of 200-3500 vertices, 121M entries: 31.4 ms
 // with labels and totals in global memory and a hash table per row, 15.4 ms
-// so.
+// so (15.6 with the copies of the graphs from page-locked memory).
 #include "common.cuh"
 #include "internal.h"
 #include "scan.cuh"
@@ -681,7 +681,7 @@ __device__ __forceinline__ void cta_copy(const T *__restrict__ from, int n, Put 
 
 // The CTA's graph from host memory to its part of the union CSR.  A gather of
 // the whole batch ahead of this kernel runs at the link's rate with the SMs idle
-// (4096 graphs, 0.4 GB: 2.9 ms of 20.4); here the other CTAs work meanwhile.
+// (4096 graphs, 0.5 GB: 2.9 ms of 20.3); here the other CTAs work meanwhile.
 __device__ __forceinline__ void cta_gather(const BatchCtaArgs &a, int gi, int vb, int n0, long long eb, int E0)
 {
     int64_t *const o = a.u_offs + vb;

@@ -25,6 +25,10 @@ namespace gala {
 //                               by many CTAs (4096-entry / 4096-slot chunks)
 //   bin 8   : deg 0          -> never processed (the reference bins start at 1,
 //                               louvain_main_process.cu:278)
+// Levels of at most 2^23 entries, which run in one launch (small_level.cu), end
+// bin 4 at 256 (64-bit weights: 128) and bins 5 and 6 at 4096 (2048).  In a level's
+// first sweep over distinct neighbours no row needs a table (k_first_*,
+// k_hub_first).
 // ---------------------------------------------------------------------------
 constexpr int kNumBins = 8;
 constexpr int kNumBinSlots = 9;
@@ -123,8 +127,8 @@ constexpr int kErrCapacity = 16;  // contraction: long-row tables exceed their s
 // taken in exact integer arithmetic.  Float-weight graphs run with
 // WT = int64_t: every float weight is held as an exact 64-bit fixed-point
 // integer (weight * 2^S), so all sums (K, Tot, In, contracted weights) are
-// exact and independent of the order of the atomics, and every gain is
-// evaluated with the FP64 expressions.
+// exact and independent of the order of the atomics, and the FP64 expressions
+// decide (behind FP32 bounds, Cand<long long> in sweep.cuh).
 // ---------------------------------------------------------------------------
 template <typename WT>
 struct WideOf {

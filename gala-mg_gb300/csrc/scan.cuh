@@ -1,5 +1,5 @@
-// scan.cuh - exclusive prefix sum over device arrays in one pass (tiles chained
-// by decoupled look-back).
+// scan.cuh - exclusive prefix sum over device arrays, reduce then scan over a
+// resident grid.
 // Used for the degree-bin counting sort, the community renumbering and the
 // CSR offsets of the contraction.  Input values pass through a functor, so a
 // flag (x > 0) or a cap (min(x, C)) needs no separate pass.

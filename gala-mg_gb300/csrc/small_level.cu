@@ -15,13 +15,14 @@
 // The decide step moves the totals in a second array, so that its own reads
 // see those before the sweep, and the next step copies them over while it reads
 // them all anyway: one step and one barrier less than with the totals in one
-// array (a phase 1 at 20k vertices, 0.2M entries 0.88 -> 0.76 ms, at 100k and
-// 2.4M 1.48 -> 1.39).
-// and every CTA takes the convergence decision from the same exact sums.
-// What bounds it: at 14k entries the barriers and one dependent chain per step
-// (21 us a sweep against 110), at 2.4M entries the label and total gathers
-// (82 us against 122).  Whole runs, separate launches / one launch per level:
-// 1,024-vertex SBM 1.62 / 1.08 ms, 50k-vertex float LFR 5.2 / 3.5 ms.  The
+// array (phase 1 at 20k vertices and 0.4M entries 0.88 -> 0.76 ms, at 100k and
+// 2.4M 1.48 -> 1.39).  Every CTA takes the convergence decision from the same
+// exact sums.
+// What bounds it: at 14k entries the barriers (about 3k SM cycles each) and one
+// chain of dependent L2 reads per step (18 us a sweep against 110), at 2.4M
+// entries the label and total gathers (64 us against 100).  Whole runs,
+// separate launches / one launch per level: 1,024-vertex SBM 1.42 / 0.64 ms,
+// 50k-vertex float LFR 4.52 / 2.43 ms.  The
 // bodies per degree bin are those of the one-bin kernels (sweep.cuh), so the
 // partition and every Q are the same bit for bit.
 #include <algorithm>

@@ -218,8 +218,10 @@ gala_status gala_graph_info(const gala_graph *g, int32_t *n, int64_t *num_entrie
  * int32): weights must be positive and finite.  The engine holds them as
  * exact 64-bit fixed-point integers round(w * 2^S) (S chosen from the total
  * weight so that it stays below 2^62), accumulates K, Tot, In and contracted
- * weights exactly in those integers and evaluates every gain and the pruning
- * bound with the FP64 expressions.  Results repeat bit-exactly; modularity is
+ * weights exactly in those integers and decides every move and the pruning
+ * with the FP64 expressions (FP32 bounds discard what cannot win or clearly
+ * stays; the results are those of evaluating every gain in FP64).  Results
+ * repeat bit-exactly; modularity is
  * reported from the fixed-point sums.  gala_graph_load_bin / store_bin with
  * weighted = 2 read / write the .bin layout with a float32 weight block. */
 gala_status gala_graph_from_csr_f32(int32_t n, const int64_t *offsets_inclusive,
@@ -278,8 +280,9 @@ void gala_context_destroy(gala_context *ctx);
  * (louvain_main_process.cu:594-857); here all work of a context is ordered
  * on one stream and only that stream is synchronised. */
 gala_status gala_context_set_stream(gala_context *ctx, void *stream);
-/* Cap the global hash table of every hub (a vertex of degree > 8192 whose
- * neighbour communities are summed by many CTAs) at `slots` (a power of two
+/* Cap the global hash table of every hub (a vertex of degree > 8192, on levels
+ * of at most 2^23 entries > 4096, with float weights > 2048, whose neighbour
+ * communities are summed by many CTAs) at `slots` (a power of two
  * >= 32; 0 = sized by degree, at most 2/3 full, the default).  A cap below a
  * hub's count of distinct neighbour communities makes that table's bounded
  * probes run out: the run stops with GALA_ERR_OVERFLOW instead of dropping
