@@ -1116,7 +1116,7 @@ gala_status run_levels(gala_context *ctx, int32_t n0, int64_t E0, const int64_t 
         if (!(dalloc(ctx, &rb.R, nc) && dalloc(ctx, &rb.target, nc) && dalloc(ctx, &rb.marks, nc) &&
               dalloc(ctx, &rb.sz, nc) && dalloc(ctx, &wC, nc) && dalloc(ctx, &ext, nc) && dalloc(ctx, &Kr, nc) &&
               dalloc(ctx, &rb.pmin, nc) && dalloc(ctx, &rb.init, nc) && dalloc(ctx, &rb.list, nc) &&
-              dalloc(ctx, &rb.list2, nc) && dalloc(ctx, &rb.moved, 4))) {
+              dalloc(ctx, &rb.list2, nc) && dalloc(ctx, &rb.ctl, kRefineCtlInts))) {
             rb = RefineBuffers{};
             set_error("refinement: out of device memory");
             return GALA_ERR_CAPACITY;

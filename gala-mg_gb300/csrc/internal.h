@@ -359,6 +359,7 @@ struct ContractBuffers {
 // skipped.  gala_contract_device sorts, as the oracle does.
 // Leiden-style refinement (refine.cu).  All arrays hold one entry per level
 // vertex (int32: integer-weight graphs only).
+constexpr int kRefineCtlInts = 64;
 struct RefineBuffers {
     int32_t *R = nullptr;       // sub-community of every vertex (a vertex id)
     int32_t *target = nullptr;  // the sub-community a singleton joins this sweep, or -1
@@ -370,7 +371,7 @@ struct RefineBuffers {
     void *Kr = nullptr;         // weighted degree of a sub-community
     int32_t *pmin = nullptr;    // per community: its sub-community of lowest new id
     int32_t *init = nullptr;    // starting community of every vertex of the next level
-    int32_t *moved = nullptr;   // 3 ints: moves of the sweep, long rows listed, candidates listed
+    int32_t *ctl = nullptr;     // kRefineCtlInts ints: barrier and counters of one launch
     int32_t *list = nullptr;    // vertices with rows longer than 32 entries
     int32_t *list2 = nullptr;   // the singletons that may move
 };

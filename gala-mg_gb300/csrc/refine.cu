@@ -17,7 +17,10 @@
 // sums below 2^62, products in 128 bits.  Passes walk the level's vertices
 // with edges (the degree-bin order); candidates are decided one warp each,
 // their candidate sub-communities summed in a per-warp shared-memory table.
+#include <algorithm>
+
 #include "common.cuh"
+#include "coop.cuh"
 #include "internal.h"
 
 namespace gala {
@@ -63,7 +66,7 @@ __device__ __forceinline__ WT wt_of(const WT *w, long long j)
 
 // Per vertex with edges: wC = weight to the rest of its community.
 template <typename WT>
-__global__ void __launch_bounds__(256) k_ref_start(const int32_t *__restrict__ order, int nv,
+__device__ __forceinline__ void ref_start(const int32_t *__restrict__ order, int nv,
                                                    const int64_t *__restrict__ offs,
                                                    const int32_t *__restrict__ nbr, const WT *__restrict__ w,
                                                    const int32_t *__restrict__ P, WT *wC)
@@ -83,7 +86,7 @@ __global__ void __launch_bounds__(256) k_ref_start(const int32_t *__restrict__ o
     }
 }
 
-__global__ void k_iota(int32_t *a, int n)
+__device__ __forceinline__ void ref_iota(int32_t *a, int n)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = i;
 }
@@ -92,10 +95,10 @@ __global__ void k_iota(int32_t *a, int n)
 // One thread per vertex; rows longer than 32 entries are listed for the warp
 // kernel below, which adds their ext share.
 template <typename WT>
-__global__ void __launch_bounds__(256) k_ref_sums(const int32_t *__restrict__ order, int n,
+__device__ __forceinline__ void ref_sums(const int32_t *__restrict__ order, int n,
                                                   const int64_t *__restrict__ offs,
                                                   const int32_t *__restrict__ nbr, const WT *__restrict__ w,
-                                                  const int32_t *__restrict__ P, const int32_t *__restrict__ R,
+                                                  const int32_t *__restrict__ P, const int32_t *R,
                                                   const WT *__restrict__ K, WT *ext, WT *Kr, int32_t *sz,
                                                   int32_t *big, int32_t *nbig)
 {
@@ -123,10 +126,10 @@ __global__ void __launch_bounds__(256) k_ref_sums(const int32_t *__restrict__ or
 }
 
 template <typename WT>
-__global__ void __launch_bounds__(256) k_ref_sums_big(const int32_t *__restrict__ big, const int32_t *__restrict__ nbig,
+__device__ __forceinline__ void ref_sums_big(const int32_t *big, const int32_t *nbig,
                                                       const int64_t *__restrict__ offs,
                                                       const int32_t *__restrict__ nbr, const WT *__restrict__ w,
-                                                      const int32_t *__restrict__ P, const int32_t *__restrict__ R,
+                                                      const int32_t *__restrict__ P, const int32_t *R,
                                                       WT *ext)
 {
     const int lane = threadIdx.x & 31;
@@ -147,11 +150,11 @@ __global__ void __launch_bounds__(256) k_ref_sums_big(const int32_t *__restrict_
 
 // Per sweep: the singletons that may move (listed; every target starts -1).
 template <typename WT>
-__global__ void __launch_bounds__(256) k_ref_cand(const int32_t *__restrict__ order, int n,
+__device__ __forceinline__ void ref_cand(const int32_t *__restrict__ order, int n,
                                                   const int64_t *__restrict__ offs,
-                                                  const int32_t *__restrict__ P, const int32_t *__restrict__ R,
-                                                  const WT *__restrict__ K, const WT *__restrict__ wC,
-                                                  const WT *__restrict__ TotC, const int32_t *__restrict__ sz,
+                                                  const int32_t *__restrict__ P, const int32_t *R,
+                                                  const WT *__restrict__ K, const WT *wC,
+                                                  const WT *__restrict__ TotC, const int32_t *sz,
                                                   long long m2, int32_t *target, int32_t *cand, int32_t *ncand)
 {
     using M = RefMath<WT>;
@@ -173,11 +176,10 @@ __global__ void __launch_bounds__(256) k_ref_cand(const int32_t *__restrict__ or
 
 // Per sweep: the target of every listed candidate (or -1).
 template <typename WT>
-__global__ void __launch_bounds__(32 * ref_warps<WT>())
-    k_ref_decide(const int32_t *__restrict__ cand, const int32_t *__restrict__ ncand,
+__device__ __forceinline__ void ref_decide(const int32_t *cand, const int32_t *ncand,
                  const int64_t *__restrict__ offs, const int32_t *__restrict__ nbr, const WT *__restrict__ w,
-                 const int32_t *__restrict__ P, const int32_t *__restrict__ R, const WT *__restrict__ K,
-                 const WT *__restrict__ TotC, const WT *__restrict__ ext, const WT *__restrict__ Kr, long long m2,
+                 const int32_t *__restrict__ P, const int32_t *R, const WT *__restrict__ K,
+                 const WT *__restrict__ TotC, const WT *ext, const WT *Kr, long long m2,
                  int32_t *target, DevStats *st)
 {
     using M = RefMath<WT>;
@@ -272,8 +274,8 @@ __global__ void __launch_bounds__(32 * ref_warps<WT>())
     }
 }
 
-__global__ void k_ref_mark(const int32_t *__restrict__ cand, const int32_t *__restrict__ ncand,
-                           const int32_t *__restrict__ target, int32_t *marks)
+__device__ __forceinline__ void ref_mark(const int32_t *cand, const int32_t *ncand,
+                           const int32_t *target, int32_t *marks)
 {
     const int n = *ncand;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -282,8 +284,8 @@ __global__ void k_ref_mark(const int32_t *__restrict__ cand, const int32_t *__re
     }
 }
 
-__global__ void k_ref_move(const int32_t *__restrict__ cand, const int32_t *__restrict__ ncand,
-                           const int32_t *__restrict__ target, const int32_t *__restrict__ marks, int32_t *R,
+__device__ __forceinline__ void ref_move(const int32_t *cand, const int32_t *ncand,
+                           const int32_t *target, const int32_t *marks, int32_t *R,
                            int32_t *moved)
 {
     int cnt = 0;
@@ -300,6 +302,122 @@ __global__ void k_ref_move(const int32_t *__restrict__ cand, const int32_t *__re
     }
     cnt = warp_sum(cnt);
     if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(moved, cnt);
+}
+
+
+// Counters of one launch: moves, long rows listed and candidates listed of every
+// sweep, the last row for the totals after the sweeps.
+struct RefCtl {
+    GridBarrier bar;
+    int sweeps;
+    int cnt[kRefineSweeps + 1][3];
+};
+static_assert(sizeof(RefCtl) <= kRefineCtlInts * sizeof(int32_t), "the control block");
+
+template <typename WT>
+struct RefArgs {
+    const int32_t *order;
+    int n, nv;
+    const int64_t *offs;
+    const int32_t *nbr;
+    const WT *w;
+    const int32_t *P;
+    const WT *K, *TotC;
+    long long m2;
+    int32_t *R, *target, *marks, *sz, *list, *list2;
+    WT *wC, *ext, *Kr;
+    RefCtl *ctl;
+    DevStats *st;
+};
+
+// The whole refinement of a level in one cooperative launch, a grid barrier
+// between the steps (five a sweep).  Separate launches took six kernels, five
+// memsets and a host read a sweep, 0.1 ms whatever the level's size: a refined run
+// on 30k LFR vertices 3.03 -> 2.83 ms, on 200k 7.58 -> 7.38, on a 2^18 R-MAT
+// 33.1 -> 32.3.  On 2^22 R-MAT vertices, whose levels keep two million vertices
+// or tens of millions of entries, 292 -> 310: there the steps' own block counts
+// win (five resident blocks of this kernel against eight), so larger levels take
+// the launches below.
+constexpr int64_t kRefineOneLaunchEntries = 1 << 23;
+constexpr int32_t kRefineOneLaunchVertices = 1 << 20;
+template <typename WT>
+__global__ void __launch_bounds__(32 * ref_warps<WT>()) k_refine(const __grid_constant__ RefArgs<WT> a)
+{
+    unsigned target = 0;
+    int *const err = &a.st->err;
+    RefCtl *const ctl = a.ctl;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    auto zero = [&]() {
+        for (int i = t0; i < a.n; i += nt) {
+            a.ext[i] = 0;
+            a.Kr[i] = 0;
+            a.sz[i] = 0;
+        }
+    };
+    ref_iota(a.R, a.n);
+    ref_start<WT>(a.order, a.nv, a.offs, a.nbr, a.w, a.P, a.wC);
+    zero();
+    if (!grid_sync(&ctl->bar, target, err)) return;
+    int s = 0;
+    for (; s < kRefineSweeps; ++s) {
+        int *const moved = &ctl->cnt[s][0], *const nbig = &ctl->cnt[s][1], *const ncand = &ctl->cnt[s][2];
+        ref_sums<WT>(a.order, a.nv, a.offs, a.nbr, a.w, a.P, a.R, a.K, a.ext, a.Kr, a.sz, a.list, nbig);
+        for (int i = t0; i < a.n; i += nt) a.marks[i] = 0;
+        if (!grid_sync(&ctl->bar, target, err)) return;
+        ref_sums_big<WT>(a.list, nbig, a.offs, a.nbr, a.w, a.P, a.R, a.ext);
+        ref_cand<WT>(a.order, a.nv, a.offs, a.P, a.R, a.K, a.wC, a.TotC, a.sz, a.m2, a.target, a.list2, ncand);
+        if (!grid_sync(&ctl->bar, target, err)) return;
+        ref_decide<WT>(a.list2, ncand, a.offs, a.nbr, a.w, a.P, a.R, a.K, a.TotC, a.ext, a.Kr, a.m2, a.target, a.st);
+        if (!grid_sync(&ctl->bar, target, err)) return;
+        ref_mark(a.list2, ncand, a.target, a.marks);
+        zero();
+        if (!grid_sync(&ctl->bar, target, err)) return;
+        ref_move(a.list2, ncand, a.target, a.marks, a.R, moved);
+        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (*(volatile int *)moved == 0 || *(volatile int *)err) break;  // the same for every block
+    }
+    // totals of the final sub-communities (the next level's weighted degrees)
+    ref_sums<WT>(a.order, a.nv, a.offs, a.nbr, a.w, a.P, a.R, a.K, a.ext, a.Kr, a.sz, a.list,
+                 &ctl->cnt[kRefineSweeps][1]);
+    if (t0 == 0) ctl->sweeps = s;
+}
+
+// The same steps as launches of their own (large levels).
+template <typename WT>
+__global__ void __launch_bounds__(256) k_ref_start(RefArgs<WT> a)
+{
+    ref_iota(a.R, a.n);
+    ref_start<WT>(a.order, a.nv, a.offs, a.nbr, a.w, a.P, a.wC);
+}
+template <typename WT>
+__global__ void __launch_bounds__(256) k_ref_sums(RefArgs<WT> a, int *nbig)
+{
+    ref_sums<WT>(a.order, a.nv, a.offs, a.nbr, a.w, a.P, a.R, a.K, a.ext, a.Kr, a.sz, a.list, nbig);
+}
+template <typename WT>
+__global__ void __launch_bounds__(256) k_ref_sums_big(RefArgs<WT> a, const int *nbig)
+{
+    ref_sums_big<WT>(a.list, nbig, a.offs, a.nbr, a.w, a.P, a.R, a.ext);
+}
+template <typename WT>
+__global__ void __launch_bounds__(256) k_ref_cand(RefArgs<WT> a, int *ncand)
+{
+    ref_cand<WT>(a.order, a.nv, a.offs, a.P, a.R, a.K, a.wC, a.TotC, a.sz, a.m2, a.target, a.list2, ncand);
+}
+template <typename WT>
+__global__ void __launch_bounds__(32 * ref_warps<WT>()) k_ref_decide(RefArgs<WT> a, const int *ncand)
+{
+    ref_decide<WT>(a.list2, ncand, a.offs, a.nbr, a.w, a.P, a.R, a.K, a.TotC, a.ext, a.Kr, a.m2, a.target, a.st);
+}
+__global__ void __launch_bounds__(256) k_ref_mark(const int32_t *cand, const int *ncand, const int32_t *target,
+                                                  int32_t *marks)
+{
+    ref_mark(cand, ncand, target, marks);
+}
+__global__ void __launch_bounds__(256) k_ref_move(const int32_t *cand, const int *ncand, const int32_t *target,
+                                                  const int32_t *marks, int32_t *R, int32_t *moved)
+{
+    ref_move(cand, ncand, target, marks, R, moved);
 }
 
 __global__ void k_ref_pmin(int n, const int32_t *__restrict__ P, const int32_t *__restrict__ lab, int32_t *pmin)
@@ -340,40 +458,35 @@ int grid_for(long long items, int per_block)
 }
 
 template <typename WT>
-int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC, long long m2, const int32_t *order,
-             int nv, RefineBuffers &b, DevStats *stats, cudaStream_t st, gala_status *status)
+int refine_large(const RefArgs<WT> &a, RefineBuffers &b, cudaStream_t st, gala_status *status)
 {
-    const int n = g.n;
-    const WT *w = (const WT *)g.w;
-    WT *wC = (WT *)b.wC, *ext = (WT *)b.ext, *Kr = (WT *)b.Kr;
+    const int n = a.n, nv = a.nv;
+    RefCtl *const c = (RefCtl *)b.ctl;
+    WT *const ext = a.ext, *const Kr = a.Kr;
     constexpr int kDecideBlock = 32 * ref_warps<WT>();
     const int gw = grid_for((long long)nv * 32, 256);  // one warp per vertex
     const int gd = grid_for((long long)nv * 32, kDecideBlock);
     const int gt = grid_for(nv, 256);
-    k_iota<<<grid_for(n, 256), 256, 0, st>>>(b.R, n);
-    k_ref_start<WT><<<gw, 256, 0, st>>>(order, nv, g.offs, g.nbr, w, P, wC);
-    note_launch(2);
+    k_ref_start<WT><<<gw, 256, 0, st>>>(a);
+    note_launch(1);
     int sweeps = 0;
     for (; sweeps < kRefineSweeps; ++sweeps) {
         cudaMemsetAsync(ext, 0, (size_t)n * sizeof(WT), st);
         cudaMemsetAsync(Kr, 0, (size_t)n * sizeof(WT), st);
         cudaMemsetAsync(b.sz, 0, (size_t)n * sizeof(int32_t), st);
         cudaMemsetAsync(b.marks, 0, (size_t)n * sizeof(int32_t), st);
-        cudaMemsetAsync(b.moved, 0, 3 * sizeof(int32_t), st);
-        k_ref_sums<WT><<<gt, 256, 0, st>>>(order, nv, g.offs, g.nbr, w, P, b.R, K, ext, Kr, b.sz, b.list,
-                                           b.moved + 1);
-        k_ref_sums_big<WT><<<gw, 256, 0, st>>>(b.list, b.moved + 1, g.offs, g.nbr, w, P, b.R, ext);
-        k_ref_cand<WT><<<gt, 256, 0, st>>>(order, nv, g.offs, P, b.R, K, wC, TotC, b.sz, m2, b.target, b.list2,
-                                           b.moved + 2);
-        k_ref_decide<WT><<<gd, kDecideBlock, 0, st>>>(b.list2, b.moved + 2, g.offs, g.nbr, w, P, b.R, K, TotC, ext,
-                                                      Kr, m2, b.target, stats);
-        k_ref_mark<<<gt, 256, 0, st>>>(b.list2, b.moved + 2, b.target, b.marks);
-        k_ref_move<<<gt, 256, 0, st>>>(b.list2, b.moved + 2, b.target, b.marks, b.R, b.moved);
+        cudaMemsetAsync(c->cnt[0], 0, sizeof(c->cnt[0]), st);
+        k_ref_sums<WT><<<gt, 256, 0, st>>>(a, &c->cnt[0][1]);
+        k_ref_sums_big<WT><<<gw, 256, 0, st>>>(a, &c->cnt[0][1]);
+        k_ref_cand<WT><<<gt, 256, 0, st>>>(a, &c->cnt[0][2]);
+        k_ref_decide<WT><<<gd, kDecideBlock, 0, st>>>(a, &c->cnt[0][2]);
+        k_ref_mark<<<gt, 256, 0, st>>>(b.list2, &c->cnt[0][2], b.target, b.marks);
+        k_ref_move<<<gt, 256, 0, st>>>(b.list2, &c->cnt[0][2], b.target, b.marks, b.R, &c->cnt[0][0]);
         note_launch(6);
         int moved = 0, err = 0;
         cudaError_t ce = cudaGetLastError();
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(&moved, b.moved, sizeof(int), cudaMemcpyDeviceToHost, st);
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(&err, &stats->err, sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (ce == cudaSuccess) ce = cudaMemcpyAsync(&moved, &c->cnt[0][0], sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (ce == cudaSuccess) ce = cudaMemcpyAsync(&err, &a.st->err, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
         if (ce != cudaSuccess) {
             *status = cuda_fail(ce, "refinement");
@@ -390,9 +503,50 @@ int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC,
     cudaMemsetAsync(ext, 0, (size_t)n * sizeof(WT), st);
     cudaMemsetAsync(Kr, 0, (size_t)n * sizeof(WT), st);
     cudaMemsetAsync(b.sz, 0, (size_t)n * sizeof(int32_t), st);
-    cudaMemsetAsync(b.moved + 1, 0, sizeof(int32_t), st);
-    k_ref_sums<WT><<<gt, 256, 0, st>>>(order, nv, g.offs, g.nbr, w, P, b.R, K, ext, Kr, b.sz, b.list, b.moved + 1);
+    cudaMemsetAsync(&c->cnt[0][1], 0, sizeof(int32_t), st);
+    k_ref_sums<WT><<<gt, 256, 0, st>>>(a, &c->cnt[0][1]);
     note_launch(1);
+    return sweeps;
+}
+
+template <typename WT>
+int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC, long long m2, const int32_t *order,
+             int nv, RefineBuffers &b, DevStats *stats, cudaStream_t st, gala_status *status)
+{
+    constexpr int kBlock = 32 * ref_warps<WT>();
+    static int per_sm = 0;
+    if (per_sm == 0) {
+        int k = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_refine<WT>, kBlock, 0);
+        per_sm = k > 0 ? k : -1;
+    }
+    RefArgs<WT> a{order, g.n,      nv,      g.offs, g.nbr,  (const WT *)g.w, P,           K,           TotC,      m2,
+                  b.R,   b.target, b.marks, b.sz,   b.list, b.list2,         (WT *)b.wC, (WT *)b.ext, (WT *)b.Kr,
+                  (RefCtl *)b.ctl, stats};
+    if (g.E > kRefineOneLaunchEntries || g.n > kRefineOneLaunchVertices) return refine_large(a, b, st, status);
+    // a warp per vertex, as many blocks as are resident
+    const long long want = ((long long)nv * 32 + kBlock - 1) / kBlock;
+    const long long cap = (long long)hub_grid_size() * (per_sm > 0 ? per_sm : 1);
+    const int grid = (int)std::max(1LL, std::min(want, cap));
+    cudaMemsetAsync(b.ctl, 0, sizeof(RefCtl), st);
+    void *args[] = {&a};
+    cudaError_t ce = cudaLaunchCooperativeKernel((const void *)k_refine<WT>, dim3((unsigned)grid), dim3(kBlock), args,
+                                                 0, st);
+    note_launch(1);
+    int sweeps = 0, err = 0;
+    if (ce == cudaSuccess)
+        ce = cudaMemcpyAsync(&sweeps, &((RefCtl *)b.ctl)->sweeps, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(&err, &stats->err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+    if (ce != cudaSuccess) {
+        *status = cuda_fail(ce, "refinement");
+        return -1;
+    }
+    if (err) {
+        set_error("refinement: device error bits %d", err);
+        *status = GALA_ERR_OVERFLOW;
+        return -1;
+    }
     return sweeps;
 }
 
