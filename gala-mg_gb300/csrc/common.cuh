@@ -71,6 +71,7 @@ struct DevStats {
     int act_vertices[2];
     long long min_tot;              // min over non-empty communities of Tot
     int n_movers;                   // movers of the current iteration
+    int prev_movers;                // and of the one before (k_iter_reset), to undo
     int err;                        // error bits (kErr*)
     int max_deg;
     int num_communities;            // contraction: C

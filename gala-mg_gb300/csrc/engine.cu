@@ -127,6 +127,7 @@ struct gala_context {
     static constexpr int kAux = 4;
     cudaStream_t aux[kAux] = {};
     cudaEvent_t fork_ev = nullptr;
+    cudaEvent_t read_ev = nullptr;  // a sweep's counters are on the host
     cudaEvent_t join_ev[kAux] = {};
     std::vector<void *> allocs;
 };
@@ -700,6 +701,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     // row entries of the previous sweep's movers (the incremental update is
     // enqueued only after a sweep that moved under a third of them)
     unsigned long long prev_mv_edges = ~0ull;
+    bool reset_done = false;  // the counters are ready for the next sweep
     cudaEventRecord(ctx->ev[0], st);
     for (;;) {
         const int nxt = cur ^ 1;
@@ -742,7 +744,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
                 else
                     cudaEventRecord(e, st);
             };
-            p1_iter_reset(b, nxt, min_tot_init, st);
+            if (!reset_done) p1_iter_reset(b, nxt, min_tot_init, st);
             rec(ctx->ev[2]);
             if ((pmode == GALA_PROPOSAL_TRACE && iteration > 1) || proposal_sweep) {
                 p1_proposal_step(g, b, ps, lists, counts, bin_start, level_cnt, st);
@@ -826,6 +828,12 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
             cudaMemcpyAsync(h, b.stats, sizeof(DevStats), cudaMemcpyDeviceToHost, st);
             if (pend && iteration == 1)
                 cudaMemcpyAsync(ctx->h_stats2, ctx->d_stats2, sizeof(DevStats), cudaMemcpyDeviceToHost, st);
+            rec(ctx->read_ev);
+            // the counters for the next sweep (whose lists take this one's slot),
+            // while the host reads this one's: ahead of the next sweep's
+            // kernels it held them up by 5-7 us (phase 1 of 1M vertices 14.9 ->
+            // 14.7 ms, 128 graphs with 107 sweeps 30.2 -> 29.9)
+            p1_iter_reset(b, cur, min_tot_init, st);
         };
         if (graphs && iteration > 1) {
             // sweeps after the first repeat the same launches with the active
@@ -849,7 +857,10 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
         } else {
             enqueue(false);
         }
-        if ((s = sync_check(st, "iteration"))) return s;
+        reset_done = true;
+        if ((s = check(cudaEventSynchronize(ctx->read_ev), "iteration")) ||
+            (s = check(cudaGetLastError(), "iteration")))
+            return s;
         if (h->err) {
             set_error("phase 1: device error bits %d", h->err);
             return GALA_ERR_OVERFLOW;
@@ -943,6 +954,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
                 return s;
             act_nv = h->act_vertices[nxt];
             act_ne = (long long)h->act_edges[nxt];
+            reset_done = false;
             verify = true;
             cur = nxt;
             iteration++;
@@ -1337,6 +1349,7 @@ void gala_context_destroy(gala_context *ctx)
         if (ctx->join_ev[i]) cudaEventDestroy(ctx->join_ev[i]);
     }
     if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
+    if (ctx->read_ev) cudaEventDestroy(ctx->read_ev);
     for (auto &e : ctx->pend_store.ev)
         if (e) cudaEventDestroy(e);
     if (ctx->copy_stream) {
@@ -1385,6 +1398,7 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
     ctx->stream = ctx->own_stream;
     for (auto &e : ctx->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && cudaEventCreateWithFlags(&ctx->read_ev, cudaEventDisableTiming) == cudaSuccess;
     for (int i = 0; i < gala_context::kAux; ++i) {
         ok = ok && cudaStreamCreateWithFlags(&ctx->aux[i], cudaStreamNonBlocking) == cudaSuccess;
         ok = ok && cudaEventCreateWithFlags(&ctx->join_ev[i], cudaEventDisableTiming) == cudaSuccess;

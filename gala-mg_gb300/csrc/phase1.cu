@@ -1028,7 +1028,7 @@ __global__ void k_apply_movers(const int32_t *__restrict__ mv_v, const int32_t *
                                int32_t *size, const WT *__restrict__ K, int32_t *last_move, int iteration,
                                const int64_t *__restrict__ offs, uint8_t *moved)
 {
-    const int nm = stp->n_movers;
+    const int nm = sign > 0 ? stp->n_movers : stp->prev_movers;
     const int lane = threadIdx.x & 31;
     unsigned long long deg = 0;
     for (int i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < nm; i0 += gridDim.x * blockDim.x) {
@@ -1103,6 +1103,7 @@ void p1_tot_reduce(Phase1Buffers &b, int n, cudaStream_t st)
 
 __global__ void k_iter_reset(DevStats *st, int next, long long min_tot_init)
 {
+    st->prev_movers = st->n_movers;
     st->n_movers = 0;
     st->mv_edges = 0;
     st->push_mode = 0;
