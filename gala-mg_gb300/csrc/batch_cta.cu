@@ -298,12 +298,13 @@ __device__ __forceinline__ void warp_best_x(long long &x, int &c, int w, int &t,
     const bool win = top && (unsigned)x == ml;
     const unsigned wins = __ballot_sync(GALA_FULL_MASK, win);
     int src = __ffs((int)wins) - 1;
-    t = __shfl_sync(GALA_FULL_MASK, t, src);
-    if (wins & (wins - 1)) {  // several: the lowest id
+    if (wins & (wins - 1)) {  // several: the lowest id; a tie in any of their lanes or between them counts
         const int bc = (int)__reduce_min_sync(GALA_FULL_MASK, win ? (unsigned)c : 0xffffffffu);
         const int bw = __shfl_sync(GALA_FULL_MASK, w, src);
-        t = __any_sync(GALA_FULL_MASK, win && w != bw) ? 1 : __any_sync(GALA_FULL_MASK, win && t);
+        t = __any_sync(GALA_FULL_MASK, win && (t || w != bw));
         src = __ffs((int)__ballot_sync(GALA_FULL_MASK, win && c == bc)) - 1;
+    } else {
+        t = __shfl_sync(GALA_FULL_MASK, t, src);
     }
     c = __shfl_sync(GALA_FULL_MASK, c, src);
     x = ((long long)mh << 32) | ml;
