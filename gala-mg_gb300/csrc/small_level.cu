@@ -43,6 +43,8 @@ struct SweepSlot {
     unsigned long long sum_in, sum_tot2, sum_tot2_hi, act_edges;
     long long min_tot;
     int act_vertices, n_movers;
+    int err;  // error bits of the sweep's decisions: read behind its last barrier, while
+              // a faster block may already set bits of the next sweep (in the next slot)
     int act_count[kNumBins];
 };
 
@@ -113,7 +115,7 @@ __device__ void clear_slot(SweepSlot &s, long long min_tot_init)
 {
     s.sum_in = s.sum_tot2 = s.sum_tot2_hi = s.act_edges = 0;
     s.min_tot = min_tot_init;
-    s.act_vertices = s.n_movers = 0;
+    s.act_vertices = s.n_movers = s.err = 0;
     for (int b = 0; b < kNumBins; ++b) s.act_count[b] = 0;
 }
 
@@ -538,6 +540,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         if (s > 0) {
             DecideArgs<WT, false> d = a.d;
             d.n_movers = &cur->n_movers;
+            d.err = &cur->err;
             d.m2 = m2;
             d.constant = constant;
             int c = count(6);
@@ -676,7 +679,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             continue;
         }
         if (threadIdx.x == 0) {
-            const int e = *(volatile int *)err;
+            const int e = *(volatile int *)&cur->err;
             const double q = slot_q(*cur, constant);
             int go = 1;
             if (e)
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         o->q = prev_q;
         o->sweeps = s - a.s0 + 1;
         o->done = done;
-        o->err = *(volatile int *)err;
+        o->err = *(volatile int *)err | *(volatile int *)&ctl->slot[s % 3].err;
         const double ns = (double)(now_ns() - s_stat.ns0) / (double)max(clock64() - s_stat.cyc0, 1LL);  // per cycle
         o->decide_ns = (unsigned long long)((double)s_stat.dec_cyc * ns);
         o->update_ns = (unsigned long long)((double)s_stat.upd_cyc * ns);
