@@ -119,7 +119,7 @@ constexpr int kErrHashOverflow = 1;
 constexpr int kErrProbeLimit = 2;
 constexpr int kErrBadLabel = 4;
 constexpr int kErrBadIndex = 8;
-constexpr int kErrBarrier = 32;   // a grid barrier gave up waiting
+constexpr int kErrBarrier = 32;   // a grid barrier gave up waiting (coop.cuh)
 constexpr int kErrCapacity = 16;  // contraction: long-row tables exceed their scratch
 
 // ---------------------------------------------------------------------------

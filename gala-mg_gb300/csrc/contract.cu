@@ -2177,7 +2177,7 @@ int contract_run(const LevelGraph &g, const int32_t *comm, ContractBuffers &b, i
         DevStats hs;
         if (!read_stats(&hs, b.stats, st, status, "contraction")) return -1;
         if (hs.err) {
-            set_error("contraction: device error bits %d", hs.err);
+            set_error_bits("contraction", hs.err);
             *status = hs.err & kErrCapacity ? GALA_ERR_CAPACITY : GALA_ERR_OVERFLOW;
             return -1;
         }

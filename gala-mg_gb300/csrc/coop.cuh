@@ -24,11 +24,14 @@ struct GridBarrier {
 };
 
 // Grid barrier (the launch is cooperative: all CTAs are resident).  False when
-// the wait gave up after a few seconds, for every thread of the block; the
-// launch then ends with kErrBarrier.  The block's writes are released with its
+// the wait gave up after `polls` looks (kBarrierPolls: a few seconds), for every
+// thread of the block, which then leaves the kernel; *err gets kErrBarrier, which
+// the host reads after the launch.  A block passes only when all have arrived,
+// so what it reads behind the barrier is whole even while others give up, and
+// none passes the next one.  The block's writes are released with its
 // arrival, the others' acquired by one fence after the last poll (the polls
 // are relaxed: an acquire per poll invalidates the L1 each time).
-__device__ __forceinline__ bool grid_sync(GridBarrier *c, unsigned &target, int *err)
+__device__ __forceinline__ bool grid_sync(GridBarrier *c, unsigned &target, int *err, unsigned polls)
 {
     __shared__ int s_ok;
     __syncthreads();
@@ -37,11 +40,11 @@ __device__ __forceinline__ bool grid_sync(GridBarrier *c, unsigned &target, int 
         target += gridDim.x;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&c->arrive) : "memory");
         int ok = 1;
-        for (unsigned spin = 0;; ++spin) {
+        for (unsigned spin = 1;; ++spin) {
             unsigned v;
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&c->arrive) : "memory");
             if ((int)(v - target) >= 0) break;
-            if ((spin & 63) == 63 && (spin > (1u << 22) || *(volatile int *)&c->dead)) {
+            if (spin >= polls || ((spin & 63) == 0 && *(volatile int *)&c->dead)) {
                 atomicExch(&c->dead, 1);
                 atomicOr(err, kErrBarrier);
                 ok = 0;

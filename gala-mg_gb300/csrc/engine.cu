@@ -117,8 +117,9 @@ struct gala_context {
     int32_t *h_chunk = nullptr;      // page-locked copy of vstart and lo
     DevStats *d_stats2 = nullptr;    // level-init sums of a level whose rows were still in flight
     DevStats *h_stats2 = nullptr;
-    void *small_ctl = nullptr;       // small levels: sweep counters and result
-    SmallOut *small_out = nullptr, *h_small_out = nullptr;
+    void *small_ctl = nullptr;       // small levels: barrier, sweep counters and result
+    SmallOut *h_small_out = nullptr;
+    unsigned barrier_polls = kBarrierPolls;
     // per-graph state of gala_louvain_batch, kept between calls (reallocated
     // only for a larger batch)
     BatchRun *batch = nullptr;
@@ -131,6 +132,16 @@ struct gala_context {
     cudaEvent_t join_ev[kAux] = {};
     std::vector<void *> allocs;
 };
+
+namespace gala {
+void set_error_bits(const char *what, int bits)
+{
+    if (bits & kErrBarrier)
+        set_error("%s: a grid barrier gave up waiting (device error bits %d)", what, bits);
+    else
+        set_error("%s: device error bits %d", what, bits);
+}
+}  // namespace gala
 
 namespace {
 
@@ -413,12 +424,17 @@ gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, 
     int iteration = 1;
     cudaEventRecord(ctx->ev[0], st);
     for (bool done = false; !done;) {
-        const SmallRun r{ctx->small_ctl, ctx->small_out, cb.ebase, init, cb.big_pool_ints, cb.big_work_cap, cb.big_twork_cap, m2,
-                         min_mod, prev_q, fp64_only, iteration};
+        const SmallRun r{ctx->small_ctl,   cb.ebase,         init, cb.big_pool_ints, cb.big_work_cap,
+                         cb.big_twork_cap, m2,               min_mod, prev_q, fp64_only, iteration,
+                         ctx->barrier_polls};
         if ((s = check(small_level_run(g, b, hp, r, st), "small level"))) return s;
         cudaEventRecord(ctx->ev[1], st);
-        cudaMemcpyAsync(&o, ctx->small_out, sizeof(SmallOut), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&o, small_ctl_out(ctx->small_ctl), sizeof(SmallOut), cudaMemcpyDeviceToHost, st);
         if ((s = sync_check(st, "small level"))) return s;
+        if (o.err) {  // (nothing else of the result counts then)
+            set_error_bits("phase 1", o.err);
+            return GALA_ERR_OVERFLOW;
+        }
         if (iteration == 1) {
             if (m2 == 0) {  // first level: total weight m2 = sum of K (louvain.cu:165-167)
                 m2 = (long long)o.sum_k;
@@ -439,16 +455,10 @@ gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, 
                 set_error("hub tables need %lld slots, pool holds %lld", o.hub_slots, cb.big_pool_ints / 2);
                 return GALA_ERR_CAPACITY;
             }
-            if (!o.err) {
-                if (trace) trace->push_back(o.q0);
-                if (verbose) printf("Iteration:%d Q:%f\n", 0, o.q0);
-            }
+            if (trace) trace->push_back(o.q0);
+            if (verbose) printf("Iteration:%d Q:%f\n", 0, o.q0);
             out->nv = o.nv;
             for (int k = 0; k <= kNumBins; ++k) out->bin_start[k] = o.bin_start[k];
-        }
-        if (o.err) {
-            set_error("phase 1: device error bits %d", o.err);
-            return GALA_ERR_OVERFLOW;
         }
         for (int k = 0; k < o.sweeps; ++k) {
             if (trace) trace->push_back(o.trace[k]);
@@ -862,7 +872,7 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
             (s = check(cudaGetLastError(), "iteration")))
             return s;
         if (h->err) {
-            set_error("phase 1: device error bits %d", h->err);
+            set_error_bits("phase 1", h->err);
             return GALA_ERR_OVERFLOW;
         }
         if (pend && iteration == 1) {  // the level init's sums, from the row kernels of the first sweep
@@ -990,6 +1000,7 @@ void bind_contract_buffers(gala_context *ctx)
         cb.join_ev[i] = ctx->join_ev[i];
     }
     cb.fork_ev = ctx->fork_ev;
+    cb.polls = ctx->ref.polls = ctx->barrier_polls;
 }
 
 struct RunOut {
@@ -1420,8 +1431,8 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
         const size_t h0 = slice(hn, sizeof(DevStats)), h1 = slice(hn, sizeof(DevStats)),
                      h2 = slice(hn, kChunkInts * sizeof(int32_t)), h3 = slice(hn, sizeof(SmallOut));
         const size_t d0 = slice(dn, sizeof(DevStats)), d1 = slice(dn, sizeof(DevStats)),
-                     d2 = slice(dn, kChunkInts * sizeof(int32_t)), d3 = slice(dn, sizeof(SmallOut)),
-                     d4 = slice(dn, small_ctl_bytes()), d5 = slice(dn, contract_ctl_bytes());
+                     d2 = slice(dn, kChunkInts * sizeof(int32_t)), d3 = slice(dn, small_ctl_bytes()),
+                     d4 = slice(dn, contract_ctl_bytes());
         ok = ok && cudaMallocHost(&hp, hn) == cudaSuccess;
         ctx->h_block = hp;
         ok = ok && dalloc(ctx, &dp, dn);
@@ -1433,9 +1444,8 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
             ctx->d_stats = (DevStats *)(dp + d0);
             ctx->d_stats2 = (DevStats *)(dp + d1);
             ctx->d_chunk = (int32_t *)(dp + d2);
-            ctx->small_out = (SmallOut *)(dp + d3);
-            ctx->small_ctl = dp + d4;
-            ctx->cb.small_ctl = dp + d5;
+            ctx->small_ctl = dp + d3;
+            ctx->cb.small_ctl = dp + d4;
         }
     }
     for (int i = 0; i < 2 && ok; ++i)
@@ -1524,6 +1534,17 @@ gala_status gala_context_set_hub_table_cap(gala_context *ctx, int64_t slots)
         return GALA_ERR_INVALID;
     }
     ctx->hub_table_cap = slots;
+    return GALA_OK;
+}
+
+gala_status gala_context_set_barrier_polls(gala_context *ctx, int64_t polls)
+{
+    clear_error();
+    if (!ctx || polls < 0 || polls > 0x7fffffffLL) {
+        set_error("gala_context_set_barrier_polls: polls must be 0 .. 2^31 - 1");
+        return GALA_ERR_INVALID;
+    }
+    ctx->barrier_polls = polls ? (unsigned)polls : kBarrierPolls;
     return GALA_OK;
 }
 

@@ -56,6 +56,8 @@ ProposalView proposal_view(gala_proposal *p);
 
 // Error text of the last failure on this host thread.
 void set_error(const char *fmt, ...);
+// set_error for the error bits (kErr*) that a device step left.
+void set_error_bits(const char *what, int bits);
 void clear_error();
 gala_status cuda_fail(cudaError_t e, const char *what);
 void note_launch(int k);
@@ -206,11 +208,17 @@ void p1_hub_decide(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, doub
 void p1_hub_update(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, int next, int bin_start, double constant,
                    long long m2, cudaStream_t st);
 
+// Looks of a grid barrier (coop.cuh) before it gives up: a few seconds.
+constexpr unsigned kBarrierPolls = 1u << 22;
+
 // ---- phase 1 of a small level in one launch (small_level.cu) ----
 constexpr int kSmallSweeps = 256;  // sweeps of one launch at most
-struct SmallOut {  // what a launch reports (copied to the host in one piece)
+// What a launch reports (in the control block, zero before the launch; copied to
+// the host in one piece).
+struct SmallOut {
     double q, q0;  // Q of the partition kept, and (first launch) of the start
-    int32_t sweeps, done, err;
+    int32_t sweeps, done;
+    int32_t err;   // error bits; with any set the rest may be missing
     int32_t status;               // 0, 1: sum_k is not the total weight, 2: the hub tables do not fit
     unsigned long long sum_k;     // total weight of the level
     int32_t nv;                   // vertices with edges
@@ -222,7 +230,6 @@ struct SmallOut {  // what a launch reports (copied to the host in one piece)
 };
 struct SmallRun {
     void *ctl;             // small_ctl_bytes() of device memory, kept between launches of a level
-    SmallOut *out;         // device
     void *tot_next;        // n totals (8 bytes each), kept between launches of a level
     const int32_t *init;   // starting community of every vertex (null: its own)
     long long pool_ints, work_cap, twork_cap;  // hub scratch
@@ -230,8 +237,10 @@ struct SmallRun {
     double min_mod, prev_q;
     int fp64_only;
     int s0;                // first sweep (1 = the level's first, which the level init precedes)
+    unsigned polls;        // of a grid barrier
 };
 size_t small_ctl_bytes();
+const SmallOut *small_ctl_out(const void *ctl);  // device address of the result
 // hp: the arrays of the hub plan (its counts are found on the device).
 cudaError_t small_level_run(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, const SmallRun &r,
                             cudaStream_t st);
@@ -352,6 +361,7 @@ struct ContractBuffers {
     cudaEvent_t fork_ev = nullptr;
     cudaEvent_t join_ev[kAux] = {};
     void *small_ctl = nullptr;  // contract_ctl_bytes() for the one-launch path
+    unsigned polls = kBarrierPolls;
 };
 // sort_rows = false (the level-to-level contraction of a Louvain run) leaves
 // every new row in hash-table order: phase 1 does not depend on the order of
@@ -374,6 +384,7 @@ struct RefineBuffers {
     int32_t *ctl = nullptr;     // kRefineCtlInts ints: barrier and counters of one launch
     int32_t *list = nullptr;    // vertices with rows longer than 32 entries
     int32_t *list2 = nullptr;   // the singletons that may move
+    unsigned polls = kBarrierPolls;
 };
 // Refines the partition P of level g into R (returns the sweeps run, or -1
 // on a CUDA error with *status set); K and TotC are the level's weighted

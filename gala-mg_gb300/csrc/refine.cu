@@ -328,6 +328,7 @@ struct RefArgs {
     WT *wC, *ext, *Kr;
     RefCtl *ctl;
     DevStats *st;
+    unsigned polls;  // of a grid barrier
 };
 
 // The whole refinement of a level in one cooperative launch, a grid barrier
@@ -357,23 +358,23 @@ __global__ void __launch_bounds__(32 * ref_warps<WT>()) k_refine(const __grid_co
     ref_iota(a.R, a.n);
     ref_start<WT>(a.order, a.nv, a.offs, a.nbr, a.w, a.P, a.wC);
     zero();
-    if (!grid_sync(&ctl->bar, target, err)) return;
+    if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
     int s = 0;
     for (; s < kRefineSweeps; ++s) {
         int *const moved = &ctl->cnt[s][0], *const nbig = &ctl->cnt[s][1], *const ncand = &ctl->cnt[s][2];
         ref_sums<WT>(a.order, a.nv, a.offs, a.nbr, a.w, a.P, a.R, a.K, a.ext, a.Kr, a.sz, a.list, nbig);
         for (int i = t0; i < a.n; i += nt) a.marks[i] = 0;
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
         ref_sums_big<WT>(a.list, nbig, a.offs, a.nbr, a.w, a.P, a.R, a.ext);
         ref_cand<WT>(a.order, a.nv, a.offs, a.P, a.R, a.K, a.wC, a.TotC, a.sz, a.m2, a.target, a.list2, ncand);
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
         ref_decide<WT>(a.list2, ncand, a.offs, a.nbr, a.w, a.P, a.R, a.K, a.TotC, a.ext, a.Kr, a.m2, a.target, a.st);
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
         ref_mark(a.list2, ncand, a.target, a.marks);
         zero();
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
         ref_move(a.list2, ncand, a.target, a.marks, a.R, moved);
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
         if (*(volatile int *)moved == 0 || *(volatile int *)err) break;  // the same for every block
     }
     // totals of the final sub-communities (the next level's weighted degrees)
@@ -493,7 +494,7 @@ int refine_large(const RefArgs<WT> &a, RefineBuffers &b, cudaStream_t st, gala_s
             return -1;
         }
         if (err) {
-            set_error("refinement: device error bits %d", err);
+            set_error_bits("refinement", err);
             *status = GALA_ERR_OVERFLOW;
             return -1;
         }
@@ -522,7 +523,7 @@ int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC,
     }
     RefArgs<WT> a{order, g.n,      nv,      g.offs, g.nbr,  (const WT *)g.w, P,           K,           TotC,      m2,
                   b.R,   b.target, b.marks, b.sz,   b.list, b.list2,         (WT *)b.wC, (WT *)b.ext, (WT *)b.Kr,
-                  (RefCtl *)b.ctl, stats};
+                  (RefCtl *)b.ctl, stats, b.polls};
     if (g.E > kRefineOneLaunchEntries || g.n > kRefineOneLaunchVertices) return refine_large(a, b, st, status);
     // a warp per vertex, as many blocks as are resident
     const long long want = ((long long)nv * 32 + kBlock - 1) / kBlock;
@@ -543,7 +544,7 @@ int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC,
         return -1;
     }
     if (err) {
-        set_error("refinement: device error bits %d", err);
+        set_error_bits("refinement", err);
         *status = GALA_ERR_OVERFLOW;
         return -1;
     }

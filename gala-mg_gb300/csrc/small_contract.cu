@@ -61,6 +61,7 @@ struct ContractArgs {
     WT *new_w;
     bool labels_only;
     ContractCtl *ctl;
+    unsigned polls;  // of a grid barrier
     DevStats *st;
 };
 
@@ -277,9 +278,9 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_contract_small(const __grid_
     unsigned target = 0;
 #define GALA_SYNC()                                          \
     do {                                                     \
-        if (!grid_sync(&ctl->bar, target, err)) return;      \
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;      \
     } while (0)
-    if (bid == 0 && threadIdx.x == 0) *err = 0;
+    // (*err is 0: the level's phase 1 cleared it, and an error ends a run)
     for (int i = t0; i < a.n; i += nt) {
         a.cnt[i] = 0;
         if (!a.labels_only) a.ec[i] = a.taken[i] = 0;
@@ -612,6 +613,7 @@ cudaError_t contract_small_t(const LevelGraph &g, const int32_t *comm, ContractB
     a.new_w = (WT *)new_w;
     a.labels_only = labels_only;
     a.ctl = (ContractCtl *)b.small_ctl;
+    a.polls = b.polls;
     a.st = b.stats;
     if (g.w) return launch_contract<WT, true>(a, st);
     if constexpr (WideOf<WT>::exact) return launch_contract<WT, false>(a, st);

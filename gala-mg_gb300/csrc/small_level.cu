@@ -52,6 +52,7 @@ constexpr int kSmallOneCta = 64;
 struct SmallCtl {
     // reset before every launch
     GridBarrier bar;
+    SmallOut out;
     // reset before a level's first launch
     unsigned long long sum_k, sum_k2, sum_k2_hi, sum_self;
     // kept between a level's launches
@@ -77,7 +78,7 @@ struct SmallArgs {
     WT *K, *Self, *Tot, *In;
     uint8_t *act_flag;
     SmallCtl *ctl;
-    SmallOut *out;
+    unsigned polls;  // of a grid barrier
     double min_mod, prev_q;
     long long m2;  // total weight (0: this level's sum of K)
     int s0;        // first sweep of this launch (1 = the level's first)
@@ -419,8 +420,9 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         vals[j] = 0;
     }
     SmallCtl *ctl = a.ctl;
+    SmallOut *const out = &ctl->out;
     HubPlan hp = a.hp;
-    int *const err = a.d.err;
+    int *const err = &out->err;  // of the barriers
     auto clear_hubs = [&]() {
         int *hk = hp.pool;
         WT *hv = (WT *)(hp.pool + hp.half);
@@ -433,9 +435,9 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
     const long long min_tot_cap = WideOf<WT>::exact ? 0x7fffffffLL : 0x7fffffffffffffffLL;
     if (fresh) {
         // ---- level init
-        if (boss) *err = 0;
+        if (boss) a.u.st->err = 0;  // of the level's later kernels
         level_vertices(a, false, s_bin);
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
         level_vertices(a, true, s_bin);
     } else {
         if (threadIdx.x <= kNumBins) s_bin[threadIdx.x] = ctl->bin_start[threadIdx.x];
@@ -446,7 +448,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
     const bool hubs = hp.H > 0;
     if (fresh) {
         if (!a.ks_ready || hubs || a.init) {
-            if (!grid_sync(&ctl->bar, target, err)) return;
+            if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
             if (!a.ks_ready) {
                 unsigned long long sk = 0, ss = 0;
                 typename SqSum<WT>::T sk2 = 0;
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             }
             if (hubs && bid == nb - 1) plan_hubs(a, hp);
         }
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
     }
     const long long m2 = a.m2 ? a.m2 : (long long)ctl->sum_k;
     const double constant = __ddiv_rn(1.0, (double)m2);
@@ -475,15 +477,12 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                                     hp.nwork <= a.work_cap && hp.ntwork <= a.twork_cap);
         const bool sum_ok = m2 > 0 && m2 <= min_tot_cap && (long long)ctl->sum_k == m2;
         if (boss) {
-            SmallOut *o = a.out;
-            o->sum_k = ctl->sum_k;
-            o->nv = s_bin[8];
-            for (int k = 0; k <= kNumBins; ++k) o->bin_start[k] = s_bin[k];
-            o->hub_slots = hubs ? hp.half : 0;
-            o->sweeps = 0;
-            o->done = 1;
-            o->err = 0;
-            o->status = !sum_ok ? 1 : (!fits ? 2 : 0);
+            out->sum_k = ctl->sum_k;
+            out->nv = s_bin[8];
+            for (int k = 0; k <= kNumBins; ++k) out->bin_start[k] = s_bin[k];
+            out->hub_slots = hubs ? hp.half : 0;
+            out->done = 1;
+            out->status = !sum_ok ? 1 : (!fits ? 2 : 0);
         }
         if (!sum_ok || !fits) return;  // the same for every block
         if (!a.init && threadIdx.x == 0) {
@@ -492,7 +491,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             q0.sum_tot2 = ctl->sum_k2;
             q0.sum_tot2_hi = ctl->sum_k2_hi;
             prev_q = slot_q(q0, constant);
-            if (bid == 0) a.out->q0 = prev_q;
+            if (bid == 0) out->q0 = prev_q;
         }
         if (boss) {
             clear_slot(ctl->slot[0], min_tot_init);
@@ -503,7 +502,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             clear_hubs();
         }
         for (int c = bid * kSmallBlock + threadIdx.x; c < a.n; c += nb * kSmallBlock) a.d.tot_next[c] = a.Tot[c];
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
     }
 
     // counts of the run, kept by a thread that has nothing else on its path
@@ -566,12 +565,12 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             c = count(0);
             decide_group<WT, 4, W>(d, lists + s_bin[0], c, start(0), nw, stage);
             flush_movers(d, stage);
-            if (!grid_sync(&ctl->bar, target, err)) return;
+            if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
             if (hubs) {
                 hub_scan<WT, kSmallBlock>(d, hp, a.act_flag, bid, nb);
-                if (!grid_sync(&ctl->bar, target, err)) return;
+                if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
                 hub_final(d, hp, a.act_flag, wg, nw);
-                if (!grid_sync(&ctl->bar, target, err)) return;
+                if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
             }
         }
         if (boss && s > 0) s_stat.dec_cyc += clock64();
@@ -584,7 +583,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             apply_moves<WT, false>(a, cur->n_movers);
             if (hubs) {
                 for (int i = bid * kSmallBlock + threadIdx.x; i < hp.H; i += nb * kSmallBlock) a.In[hp.hubs[i]] = 0;
-                if (!grid_sync(&ctl->bar, target, err)) return;
+                if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
             }
         }
 
@@ -630,7 +629,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
                 }
             }
         }
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
         if (boss) s_stat.upd_cyc -= s > 0 ? clock64() : 0;
 
         // ---- update and prune
@@ -669,13 +668,13 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             }
             block_sums(sums, *cur);
         }
-        if (!grid_sync(&ctl->bar, target, err)) return;
+        if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
 
         // ---- convergence (louvain_main_process.cu:1004-1007)
         const int k = s - a.s0;  // sweeps of this launch before this one
         if (s == 0) {
             if (threadIdx.x == 0) prev_q = slot_q(*cur, constant);
-            if (boss) a.out->q0 = prev_q;
+            if (boss) out->q0 = prev_q;
             continue;
         }
         if (threadIdx.x == 0) {
@@ -691,7 +690,7 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
             s_go = go;
             if (bid == 0) {
                 s_stat.upd_cyc += clock64();
-                a.out->trace[k] = q;
+                out->trace[k] = q;
             }
         }
         __syncthreads();
@@ -705,19 +704,19 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
         // 0 write it again)
     }
     if (clerk) {
-        a.out->movers = s_stat.movers;
-        a.out->decisions = s_stat.decisions;
-        a.out->entries = s_stat.entries;
+        out->movers = s_stat.movers;
+        out->decisions = s_stat.decisions;
+        out->entries = s_stat.entries;
     }
     if (boss) {
-        SmallOut *o = a.out;
-        o->q = prev_q;
-        o->sweeps = s - a.s0 + 1;
-        o->done = done;
-        o->err = *(volatile int *)err | *(volatile int *)&ctl->slot[s % 3].err;
+        out->q = prev_q;
+        out->sweeps = s - a.s0 + 1;
+        out->done = done;
+        const int e = *(volatile int *)&ctl->slot[s % 3].err;
+        if (e) atomicOr(err, e);  // (another block may add that a barrier gave up)
         const double ns = (double)(now_ns() - s_stat.ns0) / (double)max(clock64() - s_stat.cyc0, 1LL);  // per cycle
-        o->decide_ns = (unsigned long long)((double)s_stat.dec_cyc * ns);
-        o->update_ns = (unsigned long long)((double)s_stat.upd_cyc * ns);
+        out->decide_ns = (unsigned long long)((double)s_stat.dec_cyc * ns);
+        out->update_ns = (unsigned long long)((double)s_stat.upd_cyc * ns);
     }
 }
 
@@ -772,7 +771,6 @@ cudaError_t small_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, co
     d.mv_v = b.mv_v;
     d.mv_old = b.mv_old;
     d.mv_new = b.mv_new;
-    d.err = &b.stats->err;
     d.fp64_decisions = &b.stats->fp64_decisions;
     d.fp64_only = r.fp64_only;
     UpdateArgs<WT, false> &u = a.u;
@@ -805,7 +803,7 @@ cudaError_t small_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, co
     a.In = (WT *)b.In;
     a.act_flag = b.act_flag;
     a.ctl = (SmallCtl *)r.ctl;
-    a.out = r.out;
+    a.polls = r.polls;
     a.min_mod = r.min_mod;
     a.prev_q = r.prev_q;
     a.m2 = r.m2;
@@ -818,6 +816,8 @@ cudaError_t small_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, co
 }  // namespace
 
 size_t small_ctl_bytes() { return sizeof(SmallCtl); }
+
+const SmallOut *small_ctl_out(const void *ctl) { return &((const SmallCtl *)ctl)->out; }
 
 cudaError_t small_level_run(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, const SmallRun &r,
                             cudaStream_t st)

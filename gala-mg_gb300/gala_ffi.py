@@ -29,7 +29,7 @@ EXPORTS = ["gala_last_error", "gala_status_string", "gala_kernel_launch_count", 
            "gala_proposal_logits", "gala_proposal_train", "gala_louvain_batch", "gala_generate_sbm_batch",
            "gala_graph_from_csr_f32", "gala_graph_weights_f32", "gala_generate_lfr", "gala_autotune",
            "gala_context_set_hub_table_cap", "gala_context_set_update_mode", "gala_context_set_copy_overlap",
-           "gala_context_set_long_rows"]
+           "gala_context_set_long_rows", "gala_context_set_barrier_polls"]
 
 PROPOSAL_OFF, PROPOSAL_TRACE, PROPOSAL_SKIP = 0, 1, 2
 PROPOSAL_PARAMS = 32 * 8 + 32 + 32 * 32 + 32 + 32 + 1
@@ -163,6 +163,8 @@ def load(path=LIB_PATH):
     L.gala_context_destroy.argtypes = [_vp]
     L.gala_context_destroy.restype = None
     L.gala_context_set_stream.argtypes = [_vp, _vp]
+    L.gala_context_set_barrier_polls.argtypes = [_vp, ctypes.c_int64]
+    L.gala_context_set_barrier_polls.restype = ctypes.c_int
     L.gala_context_set_hub_table_cap.argtypes = [_vp, ctypes.c_int64]
     L.gala_context_set_hub_table_cap.restype = ctypes.c_int
     L.gala_context_set_update_mode.argtypes = [_vp, ctypes.c_int32]
@@ -394,6 +396,11 @@ class Context:
         """Cap every hub's global hash table at `slots` (0 = by degree); for
         tests of the overflow status."""
         _check(load().gala_context_set_hub_table_cap(self.h, slots))
+
+    def set_barrier_polls(self, polls):
+        """Looks of a grid barrier before it gives up (0 = the default); for
+        tests of that error."""
+        _check(load().gala_context_set_barrier_polls(self.h, polls))
 
     def set_update_mode(self, mode):
         """Weight update of the sweeps: 0 = incremental when few rows moved

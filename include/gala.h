@@ -290,6 +290,12 @@ gala_status gala_context_set_stream(gala_context *ctx, void *stream);
  * src/louvain_gpu/kernel_functions.cu:217), and the context stays usable.
  * For tests of that error path; no counterpart in the reference. */
 gala_status gala_context_set_hub_table_cap(gala_context *ctx, int64_t slots);
+/* Levels of few entries run whole steps in one cooperative launch, whose thread
+ * blocks meet at grid barriers.  A barrier gives up after `polls` looks (0 =
+ * the default, a few seconds); the call then stops with GALA_ERR_OVERFLOW and
+ * the context stays usable.  For tests of that error path; no counterpart in
+ * the reference. */
+gala_status gala_context_set_barrier_polls(gala_context *ctx, int64_t polls);
 /* Weight update of the phase-1 sweeps (compute_In / compute_In_blk,
  * src/louvain_gpu/kernel_functions.cu:890-1034, sums In over every row after
  * every sweep).  mode 0 (default): on levels of at least 2^23 entries, a
