@@ -1,6 +1,8 @@
 // coop.cuh - pieces shared by the kernels that run a whole small level in one
 // cooperative launch (small_level.cu, small_contract.cu).
 #pragma once
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace gala {
@@ -17,6 +19,19 @@ struct SmallTable {
     static constexpr int kSlots = kWarpSlots * kSmallWarps;
     static constexpr size_t kBytes = (size_t)kSlots * (sizeof(int) + sizeof(WT)) + kSlots / 2 * sizeof(unsigned short);
 };
+
+// Blocks of a cooperative kernel that the current device holds at once, at most
+// `cap`; smem: its dynamic shared memory, opted in here.  0: it cannot run.
+template <typename K>
+int coop_grid(K kernel, int threads, size_t smem, int cap)
+{
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (smem > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+    return std::min(sms * per_sm, cap);
+}
 
 struct GridBarrier {
     unsigned arrive;  // arrivals since the launch

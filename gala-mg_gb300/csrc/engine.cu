@@ -120,6 +120,7 @@ struct gala_context {
     void *small_ctl = nullptr;       // small levels: barrier, sweep counters and result
     SmallOut *h_small_out = nullptr;
     unsigned barrier_polls = kBarrierPolls;
+    CoopGrids coop;
     // per-graph state of gala_louvain_batch, kept between calls (reallocated
     // only for a larger batch)
     BatchRun *batch = nullptr;
@@ -426,7 +427,7 @@ gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, 
     for (bool done = false; !done;) {
         const SmallRun r{ctx->small_ctl,   cb.ebase,         init, cb.big_pool_ints, cb.big_work_cap,
                          cb.big_twork_cap, m2,               min_mod, prev_q, fp64_only, iteration,
-                         ctx->barrier_polls};
+                         ctx->barrier_polls, ctx->coop.level[weight_kind(g)]};
         if ((s = check(small_level_run(g, b, hp, r, st), "small level"))) return s;
         cudaEventRecord(ctx->ev[1], st);
         cudaMemcpyAsync(&o, small_ctl_out(ctx->small_ctl), sizeof(SmallOut), cudaMemcpyDeviceToHost, st);
@@ -1001,6 +1002,7 @@ void bind_contract_buffers(gala_context *ctx)
     }
     cb.fork_ev = ctx->fork_ev;
     cb.polls = ctx->ref.polls = ctx->barrier_polls;
+    cb.coop = ctx->ref.coop = &ctx->coop;
 }
 
 struct RunOut {
@@ -1140,7 +1142,7 @@ gala_status run_levels(gala_context *ctx, int32_t n0, int64_t E0, const int64_t 
               dalloc(ctx, &rb.sz, nc) && dalloc(ctx, &wC, nc) && dalloc(ctx, &ext, nc) && dalloc(ctx, &Kr, nc) &&
               dalloc(ctx, &rb.pmin, nc) && dalloc(ctx, &rb.init, nc) && dalloc(ctx, &rb.list, nc) &&
               dalloc(ctx, &rb.list2, nc) && dalloc(ctx, &rb.ctl, kRefineCtlInts))) {
-            rb = RefineBuffers{};
+            rb = RefineBuffers{};  // (bound again by the next run)
             set_error("refinement: out of device memory");
             return GALA_ERR_CAPACITY;
         }
@@ -1503,6 +1505,9 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
     p1_configure_kernels();
     contract_configure_kernels();
     batch_cta_configure();
+    small_level_configure(ctx->coop);
+    contract_small_configure(ctx->coop);
+    refine_configure(ctx->coop);
     bind_contract_buffers(ctx);
     if ((ce = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) {
         gala_context_destroy(ctx);

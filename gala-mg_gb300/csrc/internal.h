@@ -211,6 +211,19 @@ void p1_hub_update(const LevelGraph &g, Phase1Buffers &b, const HubPlan &p, int 
 // Looks of a grid barrier (coop.cuh) before it gives up: a few seconds.
 constexpr unsigned kBarrierPolls = 1u << 22;
 
+// Blocks of the cooperative kernels that a device holds at once.  Residency and
+// the opt-in for large shared memory belong to a device, so every context
+// finds its own when it is created (with its device current).
+struct CoopGrids {
+    int level[3] = {};     // by weight_kind
+    int contract[3] = {};  // by weight_kind
+    int refine[2] = {};    // int32, fixed-point
+};
+inline int weight_kind(const LevelGraph &g) { return g.wide ? 2 : (g.w ? 1 : 0); }
+void small_level_configure(CoopGrids &c);
+void contract_small_configure(CoopGrids &c);
+void refine_configure(CoopGrids &c);
+
 // ---- phase 1 of a small level in one launch (small_level.cu) ----
 constexpr int kSmallSweeps = 256;  // sweeps of one launch at most
 // What a launch reports (in the control block, zero before the launch; copied to
@@ -238,6 +251,7 @@ struct SmallRun {
     int fp64_only;
     int s0;                // first sweep (1 = the level's first, which the level init precedes)
     unsigned polls;        // of a grid barrier
+    int max_grid;          // CoopGrids::level
 };
 size_t small_ctl_bytes();
 const SmallOut *small_ctl_out(const void *ctl);  // device address of the result
@@ -362,6 +376,7 @@ struct ContractBuffers {
     cudaEvent_t join_ev[kAux] = {};
     void *small_ctl = nullptr;  // contract_ctl_bytes() for the one-launch path
     unsigned polls = kBarrierPolls;
+    const CoopGrids *coop = nullptr;
 };
 // sort_rows = false (the level-to-level contraction of a Louvain run) leaves
 // every new row in hash-table order: phase 1 does not depend on the order of
@@ -385,6 +400,7 @@ struct RefineBuffers {
     int32_t *list = nullptr;    // vertices with rows longer than 32 entries
     int32_t *list2 = nullptr;   // the singletons that may move
     unsigned polls = kBarrierPolls;
+    const CoopGrids *coop = nullptr;
 };
 // Refines the partition P of level g into R (returns the sweeps run, or -1
 // on a CUDA error with *status set); K and TotC are the level's weighted

@@ -515,20 +515,13 @@ int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC,
              int nv, RefineBuffers &b, DevStats *stats, cudaStream_t st, gala_status *status)
 {
     constexpr int kBlock = 32 * ref_warps<WT>();
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int k = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_refine<WT>, kBlock, 0);
-        per_sm = k > 0 ? k : -1;
-    }
     RefArgs<WT> a{order, g.n,      nv,      g.offs, g.nbr,  (const WT *)g.w, P,           K,           TotC,      m2,
                   b.R,   b.target, b.marks, b.sz,   b.list, b.list2,         (WT *)b.wC, (WT *)b.ext, (WT *)b.Kr,
                   (RefCtl *)b.ctl, stats, b.polls};
     if (g.E > kRefineOneLaunchEntries || g.n > kRefineOneLaunchVertices) return refine_large(a, b, st, status);
     // a warp per vertex, as many blocks as are resident
     const long long want = ((long long)nv * 32 + kBlock - 1) / kBlock;
-    const long long cap = (long long)hub_grid_size() * (per_sm > 0 ? per_sm : 1);
-    const int grid = (int)std::max(1LL, std::min(want, cap));
+    const int grid = (int)std::max(1LL, std::min<long long>(want, b.coop->refine[g.wide]));
     cudaMemsetAsync(b.ctl, 0, sizeof(RefCtl), st);
     void *args[] = {&a};
     cudaError_t ce = cudaLaunchCooperativeKernel((const void *)k_refine<WT>, dim3((unsigned)grid), dim3(kBlock), args,
@@ -552,6 +545,12 @@ int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC,
 }
 
 }  // namespace
+
+void refine_configure(CoopGrids &c)
+{
+    c.refine[0] = coop_grid(k_refine<int>, 32 * ref_warps<int>(), 0, 1 << 20);
+    c.refine[1] = coop_grid(k_refine<long long>, 32 * ref_warps<long long>(), 0, 1 << 20);
+}
 
 int refine_run(const LevelGraph &g, const int32_t *P, const void *K, const void *TotC, long long m2,
                const int32_t *order, int nv, RefineBuffers &b, DevStats *stats, cudaStream_t st,

@@ -547,22 +547,14 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_contract_small(const __grid_
 }
 
 template <typename WT, bool W>
-cudaError_t launch_contract(ContractArgs<WT> &a, cudaStream_t st)
+cudaError_t launch_contract(ContractArgs<WT> &a, int max_grid, cudaStream_t st)
 {
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        int k = 0;
-        cudaFuncSetAttribute(k_contract_small<WT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)SmallTable<WT>::kBytes);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_contract_small<WT, W>, kSmallBlock, SmallTable<WT>::kBytes);
-        per_sm = k > 0 ? k : -1;
-    }
-    if (per_sm < 0) return cudaErrorLaunchOutOfResources;
+    if (max_grid <= 0) return cudaErrorLaunchOutOfResources;
     // a thread per vertex and per four entries
     const long long items = std::max<long long>(a.n, std::max<long long>(a.E / 4, a.n_orig / 4));
     // (few items stay on one CTA, as in small_level.cu)
     const long long want = items <= kContractOneCta ? 1 : (items + kSmallBlock - 1) / kSmallBlock;
-    const long long grid = std::min<long long>(want, std::min(hub_grid_size() * per_sm, kSmallMaxGrid));
+    const long long grid = std::min<long long>(want, max_grid);
     cudaMemsetAsync(a.ctl, 0, offsetof(ContractCtl, part), st);
     void *args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_contract_small<WT, W>, dim3((unsigned)grid),
@@ -615,12 +607,21 @@ cudaError_t contract_small_t(const LevelGraph &g, const int32_t *comm, ContractB
     a.ctl = (ContractCtl *)b.small_ctl;
     a.polls = b.polls;
     a.st = b.stats;
-    if (g.w) return launch_contract<WT, true>(a, st);
-    if constexpr (WideOf<WT>::exact) return launch_contract<WT, false>(a, st);
+    const int max_grid = b.coop->contract[weight_kind(g)];
+    if (g.w) return launch_contract<WT, true>(a, max_grid, st);
+    if constexpr (WideOf<WT>::exact) return launch_contract<WT, false>(a, max_grid, st);
     return cudaErrorInvalidValue;  // fixed-point levels are weighted
 }
 
 }  // namespace
+
+void contract_small_configure(CoopGrids &c)
+{
+    constexpr size_t i = SmallTable<int>::kBytes, l = SmallTable<long long>::kBytes;
+    c.contract[0] = coop_grid(k_contract_small<int, false>, kSmallBlock, i, kSmallMaxGrid);
+    c.contract[1] = coop_grid(k_contract_small<int, true>, kSmallBlock, i, kSmallMaxGrid);
+    c.contract[2] = coop_grid(k_contract_small<long long, true>, kSmallBlock, l, kSmallMaxGrid);
+}
 
 size_t contract_ctl_bytes() { return sizeof(ContractCtl); }
 

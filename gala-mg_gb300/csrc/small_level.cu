@@ -721,31 +721,16 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
 }
 
 template <typename WT, bool W>
-int small_resident()
+cudaError_t launch_small(const LevelGraph &g, SmallArgs<WT> &a, int max_grid, cudaStream_t st)
 {
-    static int r = 0;
-    if (r == 0) {
-        int k = 0;
-        cudaFuncSetAttribute(k_small_level<WT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)SmallTable<WT>::kBytes);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_small_level<WT, W>, kSmallBlock, SmallTable<WT>::kBytes);
-        r = k > 0 ? k : -1;
-    }
-    return r;
-}
-
-template <typename WT, bool W>
-cudaError_t launch_small(const LevelGraph &g, SmallArgs<WT> &a, cudaStream_t st)
-{
-    const int per_sm = small_resident<WT, W>();
-    if (per_sm <= 0) return cudaErrorLaunchOutOfResources;
+    if (max_grid <= 0) return cudaErrorLaunchOutOfResources;
     // warps a sweep keeps busy: about 1.5 lanes per entry, at most 8 vertices
     // a warp
     const long long tasks = g.E * 3 / 64 + g.n / 32;
     // (a level of few tasks stays on one CTA, which needs no grid barriers and
     // keeps the level in its L1)
     long long grid = tasks <= kSmallOneCta ? 1 : (tasks + kSmallWarps - 1) / kSmallWarps;
-    grid = std::max(1LL, std::min<long long>(grid, std::min(hub_grid_size() * per_sm, kSmallMaxGrid)));
+    grid = std::max(1LL, std::min<long long>(grid, max_grid));
     cudaMemsetAsync(a.ctl, 0, a.s0 == 1 ? offsetof(SmallCtl, slot) : offsetof(SmallCtl, sum_k), st);
     void *args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_small_level<WT, W>, dim3((unsigned)grid),
@@ -809,11 +794,19 @@ cudaError_t small_t(const LevelGraph &g, Phase1Buffers &b, const HubPlan &hp, co
     a.m2 = r.m2;
     a.s0 = r.s0;
     if constexpr (WideOf<WT>::exact)
-        if (!g.w) return launch_small<WT, false>(g, a, st);
-    return launch_small<WT, true>(g, a, st);
+        if (!g.w) return launch_small<WT, false>(g, a, r.max_grid, st);
+    return launch_small<WT, true>(g, a, r.max_grid, st);
 }
 
 }  // namespace
+
+void small_level_configure(CoopGrids &c)
+{
+    constexpr size_t i = SmallTable<int>::kBytes, l = SmallTable<long long>::kBytes;
+    c.level[0] = coop_grid(k_small_level<int, false>, kSmallBlock, i, kSmallMaxGrid);
+    c.level[1] = coop_grid(k_small_level<int, true>, kSmallBlock, i, kSmallMaxGrid);
+    c.level[2] = coop_grid(k_small_level<long long, true>, kSmallBlock, l, kSmallMaxGrid);
+}
 
 size_t small_ctl_bytes() { return sizeof(SmallCtl); }
 
