@@ -402,6 +402,7 @@ void hub_arrays(gala_context *ctx, HubPlan &hp)
     hp.pdq = ctx->hub_pdq;
     hp.pfc = ctx->hub_pfc;
     hp.t_cap = ctx->hub_table_cap;
+    hp.cap_deg = ctx->p1.lim.m6;
 }
 
 // Phase 1 of a small level: level init and all sweeps in one launch (more

@@ -1245,7 +1245,7 @@ __global__ void k_hub_plan(HubPlan p, const int64_t *__restrict__ offs)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.H; i += gridDim.x * blockDim.x) {
         const int v = p.hubs[i];
-        hub_table(offs[v + 1] - offs[v], p.t_cap, p.T[i], p.chunks[i], p.tchunks[i]);
+        hub_table(p, offs[v + 1] - offs[v], p.T[i], p.chunks[i], p.tchunks[i]);
     }
 }
 

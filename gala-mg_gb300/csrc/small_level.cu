@@ -323,7 +323,7 @@ __device__ __forceinline__ void plan_hubs(const SmallArgs<WT> &a, const HubPlan 
         long long T = 0, ch = 0, tc = 0;
         if (i < p.H) {
             const int v = p.hubs[i];
-            hub_table(a.d.offs[v + 1] - a.d.offs[v], p.t_cap, T, ch, tc);
+            hub_table(p, a.d.offs[v + 1] - a.d.offs[v], T, ch, tc);
             p.T[i] = T;
         }
         long long x = block_exclusive_scan<long long>(T, wt, &tot);

@@ -936,13 +936,14 @@ __device__ __forceinline__ void decide_cta(const DecideArgs<WT, RO> &a, const in
 // ------------------------------------------------------------------------
 constexpr int kHubChunk = 4096;
 
-// Table slots, row chunks and table chunks of a hub of degree deg (t_cap: the
-// caller's cap on the slots, 0 = none).
-__device__ __forceinline__ void hub_table(long long deg, long long t_cap, long long &T, long long &chunks,
+// Table slots, row chunks and table chunks of a hub of degree deg (p: the
+// caller's cap on the slots, which rows that only a small level makes hubs of
+// are spared).
+__device__ __forceinline__ void hub_table(const HubPlan &p, long long deg, long long &T, long long &chunks,
                                           long long &tchunks)
 {
     T = next_pow2_ll(deg + deg / 2);  // load at most 2/3
-    if (t_cap > 0 && T > t_cap) T = t_cap;  // capped: inserts may run out of slots
+    if (p.t_cap > 0 && deg > p.cap_deg && T > p.t_cap) T = p.t_cap;  // capped: inserts may run out of slots
     chunks = (deg + kHubChunk - 1) / kHubChunk;
     tchunks = (T + kHubChunk - 1) / kHubChunk;
 }

@@ -280,9 +280,8 @@ void gala_context_destroy(gala_context *ctx);
  * (louvain_main_process.cu:594-857); here all work of a context is ordered
  * on one stream and only that stream is synchronised. */
 gala_status gala_context_set_stream(gala_context *ctx, void *stream);
-/* Cap the global hash table of every hub (a vertex of degree > 8192, on levels
- * of at most 2^23 entries > 4096, with float weights > 2048, whose neighbour
- * communities are summed by many CTAs) at `slots` (a power of two
+/* Cap the global hash table of every hub (a vertex of degree > 8192 whose
+ * neighbour communities are summed by many CTAs) at `slots` (a power of two
  * >= 32; 0 = sized by degree, at most 2/3 full, the default).  A cap below a
  * hub's count of distinct neighbour communities makes that table's bounded
  * probes run out: the run stops with GALA_ERR_OVERFLOW instead of dropping
