@@ -1468,9 +1468,10 @@ gala_status gala_context_create(int32_t device, int32_t max_vertices, int64_t ma
          dalloc(ctx, &c.tmp_off, n + 1) && dalloc(ctx, &c.tmp_nbr, E) && dalloc8(ctx, &c.tmp_w, E) &&
          dalloc(ctx, &c.kc, n + 1) && dalloc(ctx, &c.cls_list, 6 * n);
     // tables of the rows longer than 4096 entries (hubs of a small level: 2048):
-    // at most 3 slots per entry of a key and up to 8 bytes of value, chunk
-    // list of at most E / 4096 + n entries
-    c.big_pool_ints = 9LL * (long long)E + 64;
+    // at most 3 slots per entry of a key and up to 8 bytes of value - 9 ints an
+    // entry where every row of a level may be a hub (small levels), else 8 - and a
+    // chunk list of at most E / 4096 + n entries
+    c.big_pool_ints = std::max(8LL * (long long)E, 9LL * std::min<long long>((long long)E, kSmallLevelEntries)) + 64;
     c.big_work_cap = (long long)E / 4096 + (long long)n + 1;
     c.big_twork_cap = (long long)E / 1024 + (long long)n + 1;  // table slots <= 4E, 4096 per chunk
     ok = ok && dalloc(ctx, &c.big_pool, (size_t)c.big_pool_ints) && dalloc(ctx, &c.big_T, n) &&
