@@ -19,6 +19,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.h"
@@ -48,14 +49,14 @@ __global__ void k_static_zero(unsigned long long *tot, int n, unsigned long long
 }
 
 // Weight (W) and own-community weight of the row entries first, first + step,
-// ... < deg.
-template <bool W>
+// ... < deg, U of them in flight.
+template <bool W, int U = 4>
 __device__ __forceinline__ void static_row(const int32_t *__restrict__ nbr, const int32_t *__restrict__ w,
                                            const int32_t *__restrict__ comm, int n, int c, long long first,
                                            long long deg, int step, unsigned long long &k, unsigned long long &in,
                                            int &bad)
 {
-    constexpr int U = 4;  // predicated batches: a short row's loads are in flight together too
+    // predicated batches: a short row's loads are in flight together too
     for (; first < deg; first += (long long)U * step) {
         int u[U], wi[U];
 #pragma unroll
@@ -84,15 +85,22 @@ __device__ __forceinline__ void static_row(const int32_t *__restrict__ nbr, cons
 
 // K (row weight) and In (weight to the own community) of every vertex;
 // community totals by atomics, sums by warp then block reduction.  A group of
-// kStaticG lanes takes a row, four loads in flight per lane and four rows per
-// warp; rows longer than kStaticLong entries go to the whole warp afterwards.
-// One wave of blocks.  300k vertices, 7.2M entries: 59 us with a warp per row,
-// 42 us so, where the label gathers (one 32-byte L2 sector each, about
-// 6 TB/s of sectors) bound it: neither more warps nor more loads in flight
-// change it.
-constexpr int kStaticG = 8;
+// G lanes takes a row, four loads in flight per lane and 32 / G rows per warp;
+// rows longer than kStaticLong entries go to the whole warp afterwards, and
+// those longer than kStaticBlock (as many as the list holds) to the whole block
+// at its end.  One wave of blocks.  300k vertices, 7.2M entries: 59 us with a
+// warp per row, 42 us with G = 8, where the label gathers (one 32-byte L2 sector
+// each, about 6 TB/s of sectors) bound it: neither more warps nor more loads in
+// flight change it.  Few vertices do not fill the chip at G = 8, and long rows
+// among them then queue in few warps: a warp per row while that is one wave,
+// half a warp up to two (calls of 300 rows of 20,000 entries 74 us with a warp
+// per row, 174 at G = 8, 59 so; 1,200 of 5,000: 48 / 76 / 46; 20,000 of 2,000:
+// 95 / 98 / 87).  A star of 2^20 vertices: 2.3 ms with its hub's row in one warp,
+// 0.29 in a block.
 constexpr int kStaticLong = 512;
-template <bool W>
+constexpr int kStaticBlock = 8192;
+constexpr int kStaticList = 16;
+template <int G, bool W>
 __global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int64_t *__restrict__ offs,
                                                         const int32_t *__restrict__ nbr,
                                                         const int32_t *__restrict__ w,
@@ -100,9 +108,12 @@ __global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int
                                                         unsigned long long *sums)
 {
     __shared__ unsigned long long s_in[8], s_k[8];
+    __shared__ int s_rows[kStaticList], s_nrows;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int sub = lane & (kStaticG - 1), gw = lane / kStaticG;
-    constexpr int GPW = 32 / kStaticG;
+    if (threadIdx.x == 0) s_nrows = 0;
+    __syncthreads();
+    const int sub = lane & (G - 1), gw = lane / G;
+    constexpr int GPW = 32 / G;
     const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     unsigned long long my_in = 0, my_k = 0;
@@ -114,15 +125,28 @@ __global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int
         const long long s = offs[v], deg = has ? offs[v + 1] - s : 0;
         const bool is_long = deg > kStaticLong;
         unsigned long long k = 0, in = 0;
-        if (!is_long) static_row<W>(nbr + s, W ? w + s : nullptr, comm, n, c, sub, deg, kStaticG, k, in, bad);
+        bool skip = false;
+        if (!is_long) static_row<W>(nbr + s, W ? w + s : nullptr, comm, n, c, sub, deg, G, k, in, bad);
         unsigned todo = __ballot_sync(GALA_FULL_MASK, is_long && sub == 0);
         while (todo) {  // warp-uniform
             const int src = __ffs((int)todo) - 1;
             todo &= todo - 1;
             const long long ls = __shfl_sync(GALA_FULL_MASK, s, src), ld = __shfl_sync(GALA_FULL_MASK, deg, src);
             const int lc = __shfl_sync(GALA_FULL_MASK, c, src);
+            if (ld > kStaticBlock) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&s_nrows, 1);
+                at = __shfl_sync(GALA_FULL_MASK, at, 0);
+                if (at < kStaticList) {
+                    if (lane == src) {
+                        s_rows[at] = v;
+                        skip = true;
+                    }
+                    continue;
+                }
+            }
             unsigned long long lk = 0, lin = 0;
-            static_row<W>(nbr + ls, W ? w + ls : nullptr, comm, n, lc, lane, ld, 32, lk, lin, bad);
+            static_row<W, W ? 4 : 8>(nbr + ls, W ? w + ls : nullptr, comm, n, lc, lane, ld, 32, lk, lin, bad);
             if (W) lk = warp_sum(lk);
             lin = warp_sum(lin);
             if (lane == src) {
@@ -131,11 +155,11 @@ __global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int
             }
         }
 #pragma unroll
-        for (int o = kStaticG / 2; o >= 1; o >>= 1) {
+        for (int o = G / 2; o >= 1; o >>= 1) {
             if (W) k += __shfl_xor_sync(GALA_FULL_MASK, k, o);
             in += __shfl_xor_sync(GALA_FULL_MASK, in, o);
         }
-        if (has && sub == 0) {
+        if (has && sub == 0 && !skip) {
             if (!W) k = (unsigned long long)deg;
             if ((unsigned)c < (unsigned)n)
                 atomicAdd(&tot[c], k);
@@ -144,6 +168,23 @@ __global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int
             my_in += in;
             my_k += k;
         }
+    }
+    __syncthreads();
+    for (int i = 0; i < min(s_nrows, kStaticList); ++i) {
+        const int v = s_rows[i], c = comm[v];
+        const long long s = offs[v], deg = offs[v + 1] - s;
+        unsigned long long k = 0, in = 0;
+        static_row<W, 8>(nbr + s, W ? w + s : nullptr, comm, n, c, threadIdx.x, deg, 256, k, in, bad);
+        if (!W) k = threadIdx.x == 0 ? (unsigned long long)deg : 0;
+        k = warp_sum(k);
+        if (lane == 0 && k) {
+            if ((unsigned)c < (unsigned)n)
+                atomicAdd(&tot[c], k);
+            else
+                bad |= 1;
+            my_k += k;
+        }
+        my_in += in;
     }
     if (bad) atomicOr(&sums[4], (unsigned long long)bad);
     my_in = warp_sum(my_in);
@@ -242,12 +283,23 @@ extern "C" gala_status gala_modularity_device_static(int32_t n, const int64_t *d
     // the scratch keeps the previous call's contents: clear it first
     const int grid = (n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024;
     k_static_zero<<<grid, 256>>>(tot, n, sums);
-    const long long rblocks = ((long long)n * kStaticG + 255) / 256, wave = (long long)hub_grid_size() * (d_weights ? 5 : 6);
-    const int rgrid = (int)(rblocks < wave ? rblocks : wave);
-    if (d_weights)
-        k_static_rows<true><<<rgrid, 256>>>(n, d_offsets, d_neighbors, d_weights, d_community, tot, sums);
+    const long long wave = (long long)hub_grid_size() * (d_weights ? 5 : 6);
+    auto rows = [&](auto lanes) {
+        constexpr int G = decltype(lanes)::value;
+        const long long blocks = ((long long)n * G + 255) / 256;
+        const int rgrid = (int)(blocks < wave ? blocks : wave);
+        if (d_weights)
+            k_static_rows<G, true><<<rgrid, 256>>>(n, d_offsets, d_neighbors, d_weights, d_community, tot, sums);
+        else
+            k_static_rows<G, false><<<rgrid, 256>>>(n, d_offsets, d_neighbors, nullptr, d_community, tot, sums);
+    };
+    // (lanes per row: see k_static_rows)
+    if ((long long)n * 32 <= wave * 256)
+        rows(std::integral_constant<int, 32>());
+    else if ((long long)n * 16 <= wave * 256 * 2)
+        rows(std::integral_constant<int, 16>());
     else
-        k_static_rows<false><<<rgrid, 256>>>(n, d_offsets, d_neighbors, nullptr, d_community, tot, sums);
+        rows(std::integral_constant<int, 8>());
     k_static_tot2<<<grid, 256>>>(n, tot, sums);
     note_launch(3);
     // a launch that failed for its configuration would leave the previous

@@ -1,0 +1,63 @@
+"""Static device modularity with rows of more than 8192 entries, which a block
+takes together (up to 16 of them, the others by warps): exact against the same
+sums on the host, bad labels and weights reported, and no slower for a star than
+a few times the same entries in short rows."""
+import time
+
+import numpy as np
+import pytest
+
+from test_batch import torch_cuda  # noqa: F401
+
+
+def _call(ffi, torch, offs, nbr, w, comm):
+    d = [torch.from_numpy(a).cuda() for a in (offs, nbr, w if w is not None else nbr, comm)]
+    torch.cuda.synchronize()
+    return lambda: ffi.modularity_device_static(len(comm), d[0].data_ptr(), d[1].data_ptr(),
+                                                d[2].data_ptr() if w is not None else None, d[3].data_ptr())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("deg", [[8191, 8192, 8193, 9000, 100003], [8193] * 70, [5, 40000, 0, 513] * 20,
+                                 [9000] + [3] * 7294, [9000] + [3] * 20000, [9000, 600] + [3] * 40000])
+def test_long_rows(ffi, torch_cuda, weighted, deg):  # noqa: F811
+    n = len(deg)
+    rng = np.random.default_rng(n)
+    offs = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    nbr = rng.integers(0, n, offs[-1]).astype(np.int32)
+    w = rng.integers(1, 1000, offs[-1]).astype(np.int32) if weighted else np.ones(offs[-1], np.int32)
+    comm = rng.integers(0, 4, n).astype(np.int32)
+    row = np.repeat(np.arange(n), deg)
+    inside, m2 = int(w[comm[row] == comm[nbr]].sum(dtype=np.int64)), int(w.sum(dtype=np.int64))
+    t2 = sum(int(w[comm[row] == c].sum(dtype=np.int64)) ** 2 for c in range(4))
+    c = 1.0 / m2
+    q = inside * c - (float(t2 >> 64) * 18446744073709551616.0 + float(t2 & (2 ** 64 - 1))) * c * c
+    assert _call(ffi, torch_cuda, offs, nbr, w if weighted else None, comm)() == q
+    v = int(np.argmax(deg))
+    bad = comm.copy()
+    bad[v] = n
+    with pytest.raises(ffi.GalaError) as e:
+        _call(ffi, torch_cuda, offs, nbr, w if weighted else None, bad)()
+    assert e.value.status == 1
+    if weighted:
+        w[offs[v + 1] - 1] = 0
+        with pytest.raises(ffi.GalaError) as e:
+            _call(ffi, torch_cuda, offs, nbr, w, comm)()
+        assert e.value.status == 1
+
+
+@pytest.mark.gpu
+def test_star_time(ffi, torch_cuda):  # noqa: F811
+    n = 1 << 20
+    comm = (np.arange(n) % 1000).astype(np.int32)
+    offs = np.concatenate([[0, n - 1], n - 1 + np.arange(1, n)]).astype(np.int64)
+    nbr = np.concatenate([np.arange(1, n, dtype=np.int32), np.zeros(n - 1, dtype=np.int32)])
+    f = _call(ffi, torch_cuda, offs, nbr, None, comm)
+    times = []
+    for _ in range(8):
+        t = time.perf_counter()
+        f()
+        times.append(time.perf_counter() - t)
+    # one warp on the hub's row: 2.3-3.1 ms; a block on it: 0.3
+    assert min(times) <= 1.5e-3, times
