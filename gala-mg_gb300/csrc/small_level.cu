@@ -84,14 +84,18 @@ struct SmallArgs {
     int s0;        // first sweep of this launch (1 = the level's first)
 };
 
+// Degree bins of a small level: the longest rows that a warp's and the CTA's table
+// take, whatever limits the caller gave bins 4 and 5 (they are tuned for the
+// one-bin launches; rows of 100 entries in 8M, bin 4 ending at 64: 4.4 ms, so
+// 1.9).  A lower limit of bin 6 still makes hubs of the rows above it.
 BinLimits small_limits(const BinLimits &lim, bool wide)
 {
-    BinLimits l = lim;
     const int row4 = (wide ? SmallTable<long long>::kWarpSlots : SmallTable<int>::kWarpSlots) / 2;
     const int row6 = (wide ? SmallTable<long long>::kSlots : SmallTable<int>::kSlots) / 2;
-    l.m4 = std::min(l.m4, row4);
-    l.m5 = std::min(l.m5, row6);
-    l.m6 = std::min(l.m6, row6);
+    BinLimits l;
+    l.m6 = std::min(lim.m6, row6);
+    l.m5 = std::min(l.m5, l.m6);
+    l.m4 = std::min(row4, l.m5);
     return l;
 }
 

@@ -82,13 +82,19 @@ typedef struct {
                                    level 0 skip aggregation; graphs built by
                                    this library are known to be distinct) */
     int32_t bin5_block;         /* threads per vertex of degree bin 5: 256
-                                   (default, 0) or 512 */
+                                   (default, 0) or 512; not for levels of at most
+                                   2^23 entries, which run in one launch (below) */
     int32_t bin_max[3];         /* upper degrees of bins 4, 5, 6 (0 = default
                                    256 / 2048 / 8192; each at most its default,
                                    non-decreasing, bin 4 at least 32); larger
                                    rows go to the next bin, above bin 6 to the
                                    multi-CTA hub path.  Any values give the same
-                                   partition; gala_autotune picks fast ones. */
+                                   partition; gala_autotune picks fast ones.
+                                   Levels of at most 2^23 entries that run in one
+                                   launch (no proposal, no use_graphs) have limits
+                                   of their own for bins 4 and 5 and send rows
+                                   above 4096 entries (float weights: 2048) to
+                                   the hub path, or above bin_max[2] if lower. */
     int32_t refine;             /* 1 = Leiden-style refinement (no counterpart in
                                    the reference): a round that gained at least
                                    min_modularity contracts the refinement of its
@@ -385,7 +391,8 @@ typedef struct {
  * candidate bin limits and bin-5 block sizes - a coordinate search over the
  * bin-4 upper degree {64, 128, 256}, bin 5 {1024, 2048}, bin 6 {4096, 8192}
  * and the bin-5 block {256, 512}, each point the minimum of `repeats` runs -
- * and returns the fastest (every candidate gives the same partition).  The
+ * and returns the fastest (every candidate gives the same partition).  Of graphs
+ * whose levels all run in one launch (see bin_max) only bin 6 matters.  The
  * other fields of opt apply to every run. */
 gala_status gala_autotune(gala_context *ctx, const gala_graph *const *graphs, int32_t count,
                           const gala_options *opt, int32_t repeats, gala_tuning *out);
