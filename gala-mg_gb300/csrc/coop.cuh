@@ -33,6 +33,21 @@ int coop_grid(K kernel, int threads, size_t smem, int cap)
     return std::min(sms * per_sm, cap);
 }
 
+// Cooperative launch of at most `grid` blocks.  A stream may hold fewer than its
+// device (a green context's stream has part of the SMs): the grid is halved
+// until it is accepted, and every grid gives the same results.
+inline cudaError_t coop_launch(const void *kernel, long long grid, int threads, void **args, size_t smem,
+                               cudaStream_t st)
+{
+    for (;;) {
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel(kernel, dim3((unsigned)grid), dim3((unsigned)threads), args, smem, st);
+        if (e != cudaErrorCooperativeLaunchTooLarge || grid <= 1) return e;
+        cudaGetLastError();
+        grid = (grid + 1) / 2;
+    }
+}
+
 struct GridBarrier {
     unsigned arrive;  // arrivals since the launch
     int dead;         // a wait gave up: every CTA leaves

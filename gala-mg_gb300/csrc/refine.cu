@@ -524,8 +524,7 @@ int refine_t(const LevelGraph &g, const int32_t *P, const WT *K, const WT *TotC,
     const int grid = (int)std::max(1LL, std::min<long long>(want, b.coop->refine[g.wide]));
     cudaMemsetAsync(b.ctl, 0, sizeof(RefCtl), st);
     void *args[] = {&a};
-    cudaError_t ce = cudaLaunchCooperativeKernel((const void *)k_refine<WT>, dim3((unsigned)grid), dim3(kBlock), args,
-                                                 0, st);
+    cudaError_t ce = coop_launch((const void *)k_refine<WT>, grid, kBlock, args, 0, st);
     note_launch(1);
     int sweeps = 0, err = 0;
     if (ce == cudaSuccess)

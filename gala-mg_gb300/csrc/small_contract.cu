@@ -557,8 +557,8 @@ cudaError_t launch_contract(ContractArgs<WT> &a, int max_grid, cudaStream_t st)
     const long long grid = std::min<long long>(want, max_grid);
     cudaMemsetAsync(a.ctl, 0, offsetof(ContractCtl, part), st);
     void *args[] = {&a};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_contract_small<WT, W>, dim3((unsigned)grid),
-                                                      dim3(kSmallBlock), args, SmallTable<WT>::kBytes, st);
+    const cudaError_t e =
+        coop_launch((const void *)k_contract_small<WT, W>, grid, kSmallBlock, args, SmallTable<WT>::kBytes, st);
     note_launch(1);
     return e;
 }

@@ -737,8 +737,8 @@ cudaError_t launch_small(const LevelGraph &g, SmallArgs<WT> &a, int max_grid, cu
     grid = std::max(1LL, std::min<long long>(grid, max_grid));
     cudaMemsetAsync(a.ctl, 0, a.s0 == 1 ? offsetof(SmallCtl, slot) : offsetof(SmallCtl, sum_k), st);
     void *args[] = {&a};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_small_level<WT, W>, dim3((unsigned)grid),
-                                                      dim3(kSmallBlock), args, SmallTable<WT>::kBytes, st);
+    const cudaError_t e =
+        coop_launch((const void *)k_small_level<WT, W>, grid, kSmallBlock, args, SmallTable<WT>::kBytes, st);
     note_launch(1);
     return e;
 }
