@@ -45,8 +45,10 @@ class PageTouch {
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
-        char *const start = (char *)((uintptr_t)p / page * page);
-        (void)madvise(start, (size_t)(p + bytes - start), MADV_POPULATE_WRITE);
+        const size_t step = std::max(page, (size_t)1 << 20);  // (short holds of the process's memory map)
+        char *const end = p + bytes;
+        for (char *q = (char *)((uintptr_t)p / page * page); q < end; q += step)
+            if (madvise(q, std::min(step, (size_t)(end - q)), MADV_POPULATE_WRITE) != 0) return;
     }
 
   public:
