@@ -143,7 +143,7 @@ def contraction_roofline(runs, peak, peak_kind):
     ach = byt / (ms / 1000.0) / 1e9
     lv = runs[-1]["levels"]
     tr = profile_traffic("contract_dram_rmat-s21.md")
-    return {"bound": "hbm", "kernel": "contraction (renumber, member buckets, row aggregation, CSR write) of "
+    return {"bound": "hbm", "kernel": "contraction (renumber, edge stream, row aggregation, CSR write) of "
                                       "every round that builds a next level",
             "achieved": ach, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": ach / peak,
             "traffic": tr * byt / len(runs) if tr else None,

@@ -26,8 +26,8 @@ namespace gala {
 //   bin 8   : deg 0          -> never processed (the reference bins start at 1,
 //                               louvain_main_process.cu:278)
 // Levels of at most 2^23 entries, which run in one launch (small_level.cu), end
-// bin 4 at 256 (64-bit weights: 128) and bins 5 and 6 at 4096 (2048).  In a level's
-// first sweep over distinct neighbours no row needs a table (k_first_*,
+// bin 4 at 256 (64-bit weights: 128), bin 5 at 2048 and bin 6 at 4096 (2048).  In
+// a larger level's first sweep over distinct neighbours no row needs a table (k_first_*,
 // k_hub_first).
 // ---------------------------------------------------------------------------
 constexpr int kNumBins = 8;

@@ -2,10 +2,13 @@
 // points of the C ABI (include/gala.h).
 //
 // A gala_context owns one CUDA stream and all device workspace for graphs up
-// to its capacity; nothing is allocated while a run is in progress.  Per
-// phase-1 iteration the host reads back one small counter block (sum of In,
-// sum of Tot^2, error bits) to decide convergence, which is the only
-// device->host traffic of the iteration.
+// to its capacity; nothing is allocated while a run is in progress.  Levels of
+// at most 2^23 entries run all sweeps of their phase 1 in one launch (up to 256
+// sweeps; small_level.cu), which decides convergence itself and returns one block
+// of results.  On larger levels the host reads back one small counter block (sum
+// of In, sum of Tot^2, error bits) per phase-1 iteration to decide convergence;
+// for a batch's union the device has judged every graph already and the block
+// says whether any goes on.
 #include <math.h>
 #include <stdio.h>
 #include <string.h>

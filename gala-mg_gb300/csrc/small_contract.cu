@@ -4,7 +4,7 @@
 // The general contraction (contract.cu) takes some fifty launches, most of
 // them prefix sums, lists and size classes; on a level of few entries each
 // finishes in two microseconds and the whole in about 200.  Here one grid runs
-// the same steps with a grid barrier between them, twelve in all (three more
+// the same steps with a grid barrier between them, eleven in all (three more
 // when a community has more than half a CTA table of entries):
 //   labels     member counts, dense renumbering in ascending label order
 //   entries    entries per community, their prefix, every row of the level

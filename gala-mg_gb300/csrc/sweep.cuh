@@ -718,9 +718,10 @@ __device__ __forceinline__ void scan_list(const DecideArgs<WT, RO> &a, const Sca
 }
 
 // Degree 33-256: one warp per vertex with a private shared-memory hash table
-// of TW slots (two launches: 256 slots for rows up to 128 entries, with eight
-// resident blocks per SM at 32 registers a thread, and 512 slots for longer
-// rows).  The table is cleared once per warp; per vertex the slots it claims
+// of TW slots (one-bin kernels, two launches: 256 slots for rows up to 128
+// entries, with eight resident blocks per SM at 32 registers a thread, and 512
+// slots for longer rows; small levels: rows up to half the table, 512 slots or 256
+// with 64-bit weights, longer ones in the CTA's table).  The table is cleared once per warp; per vertex the slots it claims
 // are listed, and only those are scanned and cleared again.
 constexpr int kWarpTable = 512;  // the full table; rows up to kWarpTable / 4 use half of it
 constexpr int kWarpWarps = 8;  // warps per block
@@ -804,8 +805,8 @@ __device__ __forceinline__ void decide_warp(const DecideArgs<WT, RO> &a, const i
     }
 }
 
-// Degree 257-8192: one CTA per vertex with a shared-memory hash table of tmax
-// slots (int keys, WT values) and the list of claimed slots, cleared once per
+// Degree 257-8192 (small levels: to 4096, 64-bit weights from 129 to 2048): one
+// CTA per vertex with a shared-memory hash table of tmax slots (int keys, WT values) and the list of claimed slots, cleared once per
 // CTA and then slot by slot after every vertex.
 template <typename WT>
 constexpr size_t cta_smem(int tmax)
@@ -929,7 +930,8 @@ __device__ __forceinline__ void decide_cta(const DecideArgs<WT, RO> &a, const in
 }
 
 // ------------------------------------------------------------------------
-// Hub vertices (degree > 8192): one global hash table per hub, filled by
+// Hub vertices (degree > 8192, on small levels > 4096 or, with 64-bit weights,
+// > 2048): one global hash table per hub, filled by
 // many CTAs in 4096-entry chunks of the hub's row, scanned by many CTAs in
 // 4096-slot chunks (each writes the best candidate of its chunk), and merged
 // by one warp per hub.  A hub's work is spread over all SMs instead of one.
