@@ -806,8 +806,9 @@ __device__ __forceinline__ void decide_warp(const DecideArgs<WT, RO> &a, const i
 }
 
 // Degree 257-8192 (small levels: to 4096, 64-bit weights from 129 to 2048): one
-// CTA per vertex with a shared-memory hash table of tmax slots (int keys, WT values) and the list of claimed slots, cleared once per
-// CTA and then slot by slot after every vertex.
+// CTA per vertex with a shared-memory hash table of tmax slots (int keys, WT
+// values) and the list of claimed slots, cleared once per CTA and then slot by
+// slot after every vertex.
 template <typename WT>
 constexpr size_t cta_smem(int tmax)
 {
@@ -931,10 +932,10 @@ __device__ __forceinline__ void decide_cta(const DecideArgs<WT, RO> &a, const in
 
 // ------------------------------------------------------------------------
 // Hub vertices (degree > 8192, on small levels > 4096 or, with 64-bit weights,
-// > 2048): one global hash table per hub, filled by
-// many CTAs in 4096-entry chunks of the hub's row, scanned by many CTAs in
-// 4096-slot chunks (each writes the best candidate of its chunk), and merged
-// by one warp per hub.  A hub's work is spread over all SMs instead of one.
+// > 2048): one global hash table per hub, filled by many CTAs in 4096-entry
+// chunks of the hub's row, scanned by many CTAs in 4096-slot chunks (each writes
+// the best candidate of its chunk), and merged by one warp per hub.  A hub's work
+// is spread over all SMs instead of one.
 // ------------------------------------------------------------------------
 constexpr int kHubChunk = 4096;
 
