@@ -416,9 +416,11 @@ void hub_arrays(gala_context *ctx, HubPlan &hp)
 
 // Phase 1 of a small level: level init and all sweeps in one launch (more
 // launches when a level takes over kSmallSweeps sweeps).  The rules and the
-// results are those of phase1 below.
+// results are those of phase1 below.  *declined: the level is left to the one-bin
+// kernels, nothing was done.
 gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, double min_mod, bool verbose,
-                         std::vector<double> *trace, Phase1Out *out, int fp64_only, const int32_t *init)
+                         std::vector<double> *trace, Phase1Out *out, int fp64_only, const int32_t *init,
+                         bool *declined)
 {
     cudaStream_t st = ctx->stream;
     Phase1Buffers &b = ctx->p1;
@@ -428,7 +430,6 @@ gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, 
     gala_status s;
     b.features_on = 0;
     b.wide = g.wide;
-    ctx->sym_state = 0;  // (later levels are no larger: never updated incrementally)
     HubPlan hp{};
     hub_arrays(ctx, hp);
     double prev_q = 0;
@@ -447,6 +448,9 @@ gala_status phase1_small(gala_context *ctx, const LevelGraph &g, long long &m2, 
             return GALA_ERR_OVERFLOW;
         }
         if (iteration == 1) {
+            *declined = o.status == 3;
+            if (*declined) return GALA_OK;
+            ctx->sym_state = 0;  // (later levels are no larger: never updated incrementally)
             if (m2 == 0) {  // first level: total weight m2 = sum of K (louvain.cu:165-167)
                 m2 = (long long)o.sum_k;
                 if (m2 <= 0) {
@@ -542,8 +546,11 @@ gala_status phase1(gala_context *ctx, const LevelGraph &g, long long &m2, double
     int32_t *const d_cnt = d_lo + (PendingRows::kMax + 1) * kNumBins;
     const int32_t *const h_lo = ctx->h_chunk + PendingRows::kMax + 1;
 
-    if (small_level(g) && !pend && !bt && pmode == GALA_PROPOSAL_OFF && !use_graphs && ctx->update_mode != 2)
-        return phase1_small(ctx, g, m2, min_mod, verbose, trace, out, fp64_only, init);
+    if (small_level(g) && !pend && !bt && pmode == GALA_PROPOSAL_OFF && !use_graphs && ctx->update_mode != 2) {
+        bool declined = false;
+        s = phase1_small(ctx, g, m2, min_mod, verbose, trace, out, fp64_only, init, &declined);
+        if (!declined) return s;
+    }
 
     p1_reset_level_stats(b, st);
     p1_level_init(g, b, st);

@@ -233,7 +233,8 @@ struct SmallOut {
     double q, q0;  // Q of the partition kept, and (first launch) of the start
     int32_t sweeps, done;
     int32_t err;   // error bits; with any set the rest may be missing
-    int32_t status;               // 0, 1: sum_k is not the total weight, 2: the hub tables do not fit
+    int32_t status;               // 0, 1: sum_k is not the total weight, 2: the hub tables do not fit,
+                                  // 3: left to the one-bin kernels (many hub rows)
     unsigned long long sum_k;     // total weight of the level
     int32_t nv;                   // vertices with edges
     int32_t bin_start[9];         // of the degree-bin order

@@ -49,6 +49,14 @@ struct SweepSlot {
 };
 
 constexpr int kSmallOneCta = 64;
+// Hub rows of an unweighted level from which the level is left to the one-bin
+// kernels: those take rows of 4097-8192 entries in shared memory, and the level's
+// first sweep without tables.  Whole runs, bipartite graphs of k rows of d entries,
+// one-bin launches (behind the launch that declines) / one launch (ms): k 200, d 4300
+// 1.15 / 1.13, d 9500 1.44 / 1.26; k 300, d 4300 1.45 / 1.49, d 6000 1.22 / 1.28, d 9500
+// 1.55 / 1.47; k 400, d 6000 1.26 / 1.46; k 800, d 4300 1.41 / 1.83.  With weights one launch is faster throughout (k 800, d 4300
+// 3.28 / 2.91), with 64-bit weights too (k 800, d 4700 3.46 / 2.86).
+constexpr int kSmallHubs = 320;
 struct SmallCtl {
     // reset before every launch
     GridBarrier bar;
@@ -450,6 +458,10 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_small_level(const __grid_con
     hp.H = s_bin[8] - s_bin[7];
     hp.hubs = a.order + s_bin[7];
     const bool hubs = hp.H > 0;
+    if (!W && fresh && hp.H > kSmallHubs) {  // the same for every block
+        if (boss) out->status = 3;
+        return;
+    }
     if (fresh) {
         if (!a.ks_ready || hubs || a.init) {
             if (!grid_sync(&ctl->bar, target, err, a.polls)) return;
