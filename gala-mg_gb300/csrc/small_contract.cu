@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_contract_small(const __grid_
     fill_rows<WT, 4, W>(a, a.bin_start[0], a.bin_start[2], wg, nw);
     GALA_SYNC();
 
-    // ---- rows
+    // ---- rows; few communities: fewer than 32 per warp, so that all warps have some
+    const int per = min(32, (C + nw - 1) / nw);
     const WT *const sw = W ? a.sw : nullptr;
     const int n_cta = ctl->n_cta, n_big = ctl->n_big;
     if (n_big > 0 && bid == nb - 1) {  // table sizes of the longest rows
@@ -403,10 +404,11 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_contract_small(const __grid_
         int *const wk = keys + wib * WS;
         WT *const wv = vals + wib * WS;
         unsigned short *const wo = occ + wib * (WS / 2);
-        for (int c0 = wg * 32; c0 < C; c0 += nw * 32) {
+        for (int c0 = wg * per; c0 < C; c0 += nw * per) {
             const int cl = c0 + lane;
-            const long long el = cl < C ? a.ec[cl] : 0;
-            if (cl < C && el == 0) a.kc[cl] = 0;
+            const bool mine = lane < per && cl < C;
+            const long long el = mine ? a.ec[cl] : 0;
+            if (mine && el == 0) a.kc[cl] = 0;
             unsigned todo = __ballot_sync(GALA_FULL_MASK, el > 0 && el <= WS / 2);
             while (todo) {  // warp-uniform
                 const int src = __ffs((int)todo) - 1;
@@ -513,9 +515,9 @@ __global__ void __launch_bounds__(kSmallBlock, 2) k_contract_small(const __grid_
     if (a.orig)
         for (int i = t0; i < a.n_orig; i += nt) a.orig[i] = a.lab[a.orig[i]];
     GALA_SYNC();
-    for (int c0 = wg * 32; c0 < C; c0 += nw * 32) {
+    for (int c0 = wg * per; c0 < C; c0 += nw * per) {
         const int cl = c0 + lane;
-        const int kl = cl < C ? a.kc[cl] : 0;
+        const int kl = lane < per && cl < C ? a.kc[cl] : 0;
         unsigned todo = __ballot_sync(GALA_FULL_MASK, kl > 0 && kl <= kHubChunk);
         while (todo) {
             const int src = __ffs((int)todo) - 1;
