@@ -96,7 +96,9 @@ __device__ __forceinline__ void static_row(const int32_t *__restrict__ nbr, cons
 // half a warp up to two (calls of 300 rows of 20,000 entries 74 us with a warp
 // per row, 174 at G = 8, 59 so; 1,200 of 5,000: 48 / 76 / 46; 20,000 of 2,000:
 // 95 / 98 / 87).  A star of 2^20 vertices: 2.3 ms with its hub's row in one warp,
-// 0.29 in a block.
+// 0.29 in a block; 160 rows of 30,000 entries on neighbouring ids among 500,000
+// vertices: 0.57 ms with a block's warps on consecutive rows, 0.13 on rows that
+// lie a grid apart.
 constexpr int kStaticLong = 512;
 constexpr int kStaticBlock = 8192;
 constexpr int kStaticList = 16;
@@ -114,7 +116,9 @@ __global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int
     __syncthreads();
     const int sub = lane & (G - 1), gw = lane / G;
     constexpr int GPW = 32 / G;
-    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // (consecutive warps' rows in different blocks: long rows often have
+    // neighbouring ids)
+    const int wg = wid * gridDim.x + blockIdx.x;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     unsigned long long my_in = 0, my_k = 0;
     int bad = 0;

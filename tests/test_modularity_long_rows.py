@@ -61,3 +61,26 @@ def test_star_time(ffi, torch_cuda):  # noqa: F811
         times.append(time.perf_counter() - t)
     # one warp on the hub's row: 2.3-3.1 ms; a block on it: 0.3
     assert min(times) <= 1.5e-3, times
+
+
+@pytest.mark.gpu
+def test_long_rows_of_neighbouring_ids(ffi, torch_cuda):  # noqa: F811
+    n, hubs, d = 500000, 160, 30000
+    rng = np.random.default_rng(3)
+    comm = rng.integers(0, 1000, n).astype(np.int32)
+    best = []
+    for ids in (np.arange(hubs), np.arange(hubs) * (n // hubs)):
+        deg = np.full(n, 8)
+        deg[ids] = d
+        offs = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+        nbr = rng.integers(0, n, offs[-1]).astype(np.int32)
+        w = rng.integers(1, 9, offs[-1]).astype(np.int32)
+        f = _call(ffi, torch_cuda, offs, nbr, w, comm)
+        times = []
+        for _ in range(8):
+            t = time.perf_counter()
+            f()
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+    print(best)
+    assert best[0] <= 1.6 * best[1], best
