@@ -1553,6 +1553,59 @@ __global__ void __launch_bounds__(256) k_sort_small(SortArgs<WT> a)
     }
 }
 
+// The same for levels of short rows (at most kSortShort entries a vertex on average):
+// rows of up to 8 pairs four per warp by rank (a key's place is the count of
+// smaller keys).  A warp takes eight consecutive rows, fewer when there are few.
+// Rows of two pairs (3.8M vertices in a path, no two merged): whole contraction
+// 2.97 ms with a warp per row, 1.57 so; R-MAT 2^20 partition, 17 entries a vertex,
+// 0.99 and 1.00.
+constexpr int kSortShort = 8;
+template <typename WT>
+__global__ void __launch_bounds__(256) k_sort_short(SortArgs<WT> a)
+{
+    constexpr int G = 8;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), gw = lane / G;
+    const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    const int C = (int)a.st->ccount;
+    const int per = min(8, (C + nw - 1) / nw);
+    for (long long c0 = (long long)wg * per; c0 < C; c0 += (long long)nw * per) {
+        const long long cl = c0 + lane;
+        const bool mine = lane < per && cl < C;
+        const int nl = mine ? a.kc[cl] : 0;
+        const long long tl = mine ? a.tmp_off[cl] : 0, ol = mine ? a.new_offs[cl] : 0;
+        unsigned todo = __ballot_sync(GALA_FULL_MASK, nl > 0 && nl <= G);
+        while (todo) {  // warp-uniform: the next four rows
+            unsigned m = todo;
+            for (int i = 0; i < gw; ++i) m &= m - 1;
+            const int src = m ? __ffs((int)m) - 1 : 0;
+            const int n = __shfl_sync(GALA_FULL_MASK, nl, src);
+            const long long t = __shfl_sync(GALA_FULL_MASK, tl, src), o = __shfl_sync(GALA_FULL_MASK, ol, src);
+            const bool ok = m && sub < n;
+            const int key = ok ? a.tmp_nbr[t + sub] : 0x7fffffff;
+            int rank = 0;
+#pragma unroll
+            for (int i = 0; i < G; ++i) rank += __shfl_sync(GALA_FULL_MASK, key, i, G) < key;
+            if (ok) a.put((int)c0 + src, o + rank, key, a.tmp_w[t + sub]);
+#pragma unroll
+            for (int i = 0; i < 32 / G; ++i) todo &= todo - 1;
+        }
+        todo = __ballot_sync(GALA_FULL_MASK, nl > G && nl <= kSortSmall);
+        while (todo) {
+            const int src = __ffs((int)todo) - 1;
+            todo &= todo - 1;
+            const int n = __shfl_sync(GALA_FULL_MASK, nl, src);
+            const int c = (int)c0 + src;
+            if (n <= 32)
+                sort_row_warp<WT, 1>(a, c, n);
+            else if (n <= 64)
+                sort_row_warp<WT, 2>(a, c, n);
+            else
+                sort_row_warp<WT, 4>(a, c, n);
+        }
+    }
+}
+
 // One warp per row of kSortSmall + 1 ... kSortWarp pairs.
 template <typename WT>
 __global__ void __launch_bounds__(128) k_sort_warp(SortArgs<WT> a)
@@ -2086,7 +2139,11 @@ static int contract_t(const LevelGraph &g, const int32_t *comm, ContractBuffers 
             k_sort_warp<WT><<<std::min(grid_cap((long long)n_warp * 32, 128, g), g), 128, 0, cs[0]>>>(sa);
             note_launch(1);
         }
-        k_sort_small<WT><<<grid_cap((long long)n * 32, 256, cap), 256, 0, cs[0]>>>(sa);
+        const int grid = grid_cap((long long)n * 32, 256, cap);
+        if (E <= (long long)kSortShort * n)
+            k_sort_short<WT><<<grid, 256, 0, cs[0]>>>(sa);
+        else
+            k_sort_small<WT><<<grid, 256, 0, cs[0]>>>(sa);
         note_launch(1);
         if (par)
             for (int i = 0; i < ContractBuffers::kAux; ++i) {
