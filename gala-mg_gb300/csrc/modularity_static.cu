@@ -94,13 +94,14 @@ __device__ __forceinline__ void static_row(const int32_t *__restrict__ nbr, cons
 // flight change it.  Few vertices do not fill the chip at G = 8, and long rows
 // among them then queue in few warps: a warp per row while that is one wave,
 // half a warp up to two (calls of 300 rows of 20,000 entries 74 us with a warp
-// per row, 174 at G = 8, 59 so; 1,200 of 5,000: 48 / 76 / 46; 20,000 of 2,000:
-// 95 / 98 / 87).  A star of 2^20 vertices: 2.3 ms with its hub's row in one warp,
-// 0.29 in a block; 160 rows of 30,000 entries on neighbouring ids among 500,000
+// per row, 174 at G = 8, 61 so; 1,200 of 5,000: 48 / 76 / 46; 20,000 of 2,000:
+// 96 / 98 / 98).  A star of 2^20 vertices: 2.3 ms with its hub's row in one warp,
+// 0.31 in a block; 160 rows of 30,000 entries on neighbouring ids among 500,000
 // vertices: 0.57 ms with a block's warps on consecutive rows, 0.13 on rows that
-// lie a grid apart.
+// lie a grid apart; 50 rows of 3,800 on neighbouring ids among 42,000: 71 us with a
+// warp per row, 95 with four to a warp, 37 by the block.
 constexpr int kStaticLong = 512;
-constexpr int kStaticBlock = 8192;
+constexpr int kStaticBlock = 1024;
 constexpr int kStaticList = 16;
 template <int G, bool W>
 __global__ void __launch_bounds__(256, W ? 5 : 6) k_static_rows(int n, const int64_t *__restrict__ offs,

@@ -1,4 +1,4 @@
-"""Static device modularity with rows of more than 8192 entries, which a block
+"""Static device modularity with rows of more than 1024 entries, which a block
 takes together (up to 16 of them, the others by warps): exact against the same
 sums on the host, bad labels and weights reported, and no slower for a star than
 a few times the same entries in short rows."""
@@ -20,7 +20,8 @@ def _call(ffi, torch, offs, nbr, w, comm):
 @pytest.mark.gpu
 @pytest.mark.parametrize("weighted", [False, True])
 @pytest.mark.parametrize("deg", [[8191, 8192, 8193, 9000, 100003], [8193] * 70, [5, 40000, 0, 513] * 20,
-                                 [9000] + [3] * 7294, [9000] + [3] * 20000, [9000, 600] + [3] * 40000])
+                                 [9000] + [3] * 7294, [9000] + [3] * 20000, [9000, 600] + [3] * 40000,
+                                 [1023, 1024, 1025, 513] * 3, [1030] * 30000])
 def test_long_rows(ffi, torch_cuda, weighted, deg):  # noqa: F811
     n = len(deg)
     rng = np.random.default_rng(n)
